@@ -18,6 +18,7 @@
 #include "mid_kernels.cuh"
 #include "generic_kernels.cuh"
 #include "tc_host.cuh"
+#include "split_stream.cuh"
 #include "ns_kernels.cuh"
 #include "ns_tc_kernels.cuh"
 #include "conv_kernels.cuh"
@@ -434,6 +435,21 @@ static int dispatch_tc(int D, int MP, F&& f) {
   if (MP == 64) return f(std::integral_constant<int, 128>{}, std::integral_constant<int, 64>{});
   return f(std::integral_constant<int, 128>{}, std::integral_constant<int, 128>{});
 }
+// The same for the split-precision kernels: head_dim 16, 32 or 64; fp32 only has the 64-landmark instances,
+// and 16-bit inputs of head_dim 64 come here with more than 64 landmarks only.
+template <class T, class F>
+static int dispatch_sx(int D, int MP, F&& f) {
+  constexpr bool k16 = !std::is_same<T, float>::value;
+  auto by_m = [&](auto dtag) -> int {
+    if constexpr (k16)
+      if (MP == 128 || decltype(dtag)::value == 64) return f(dtag, std::integral_constant<int, 128>{});
+    if constexpr (!(k16 && decltype(dtag)::value == 64)) return f(dtag, std::integral_constant<int, 64>{});
+    return fail(FNB_ERR_INVALID_ARGUMENT, "unreachable");
+  };
+  if (D == 16) return by_m(std::integral_constant<int, 16>{});
+  if (D == 32) return by_m(std::integral_constant<int, 32>{});
+  return by_m(std::integral_constant<int, 64>{});
+}
 // Co-resident tensor-core CTAs per SM: two for head_dim 64, one for head_dim 128 (shared memory).
 static int tc_ctas_per_sm(int D) { return D == 64 ? 2 : 1; }
 
@@ -452,6 +468,9 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   const int MP = p.m <= 64 ? 64 : 128;
   const bool smem_ns = p.m <= ns::kN;
   const int64_t seg_N = S.on() ? S.N_global : p.N, row_offset = S.on() ? (int64_t)S.rank * p.N : 0;
+  tc::TcSched sch_sx = tc::make_sched(p.BH, p.N, sms);   // split-precision kernels: one CTA per SM
+  const bool use_sx = !use_tc && sx::supported(a.shape.dtype, p.D, p.m, a.shape.flags) && sch_sx.nchunk <= p.nchunk;
+  if (use_sx) sch = sch_sx;
   sch.seg_N = seg_N; sch.row_offset = row_offset; sch.H = big.map_h();
   const int lmC = S.on() ? 1 : p.lm_chunks;
   float* land = S.on() ? S.xfer : w.land_partial;
@@ -463,7 +482,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   sch_fc.order = (l2 & 1) ? tc::kOrderStrided : 0;
   sch_fc.hint = hint_bits(el, 0, ef, 0);                 // Q is read again by the backward; O is not
   sch_fc.test_drop = (a.shape.flags & FNB_FLAG_TEST_DROP_LOAD) ? 1 : 0;
-  const int nchunk_b = use_tc ? sch.nchunk : p.nchunk;
+  const int nchunk_b = (use_tc || use_sx) ? sch.nchunk : p.nchunk;
   const size_t md_all = (size_t)p.BH * p.m * p.D, m_all = (size_t)p.BH * p.m;
 
   if (S.run(0)) {
@@ -573,7 +592,20 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       if (rc) return rc;
     }
   }
-  if (!use_tc) {
+  if (use_sx) {
+    int rc = dispatch_sx<T>(p.D, MP, [&](auto dtag, auto mtag) -> int {
+      constexpr int D = decltype(dtag)::value, MPc = decltype(mtag)::value;
+      L.begin();
+      auto kern = sx::sx_fwd_b_kernel<T, D, MPc>;
+      constexpr size_t smem = sx::Plan<T, D, MPc>::kFwdB;
+      if (int rc2 = set_smem(kern, smem, max_smem, "sx_fwd_b")) return rc2;
+      launch_pdl(kern, dim3((unsigned)(p.BH * sch.nchunk)), dim3(sx::kThr), smem, st, (const T*)a.k, (const T*)a.v, a.q_landmarks,
+                 w.part_acc, w.part_max, w.part_sum, sch, p.m, scale, a.device_status);
+      return L.end("sx_fwd_b");
+    });
+    if (rc) return rc;
+  }
+  if (!use_tc && !use_sx) {
     L.begin();
     size_t smem = fwd_b_smem(p.mpad, p.D);
     if (int rc = set_smem(gen_fwd_b_kernel<T>, smem, max_smem, "gen_fwd_b")) return rc;
@@ -615,8 +647,8 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       cp.acc_bh_stride = (int64_t)nchunk_b * p.m * p.D; cp.acc_chunk_stride = (int64_t)p.m * p.D;
       cp.vec_bh_stride = (int64_t)nchunk_b * p.m; cp.vec_chunk_stride = p.m;
     }
-    if (use_tc && p.D % 16 == 0) {
-      // the tensor-core output pass packs its own operand copies: merge + step2 only, spread over
+    if ((use_tc || use_sx) && p.D % 16 == 0) {
+      // the tensor-core output passes pack their own operand copies: merge + step2 only, spread over
       // D / 16 CTAs per slice
       CombineSlabParams sp2;
       sp2.part_acc = cp.part_acc; sp2.part_max = cp.part_max; sp2.part_sum = cp.part_sum; sp2.nchunk = cp.nchunk;
@@ -656,6 +688,18 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       });
     }
   }
+  if (use_sx) {
+    return dispatch_sx<T>(p.D, MP, [&](auto dtag, auto mtag) -> int {
+      constexpr int D = decltype(dtag)::value, MPc = decltype(mtag)::value;
+      L.begin();
+      auto kern = sx::sx_fwd_c_kernel<T, D, MPc>;
+      constexpr size_t smem = sx::Plan<T, D, MPc>::kFwdC;
+      if (int rc2 = set_smem(kern, smem, max_smem, "sx_fwd_c")) return rc2;
+      launch_pdl(kern, dim3((unsigned)(p.BH * sch.nchunk)), dim3(sx::kThr), smem, st, (const T*)a.q, (T*)a.out, a.lse1,
+                 a.k_landmarks, a.step2, sch, p.m, scale, a.device_status);
+      return L.end("sx_fwd_c");
+    });
+  }
   L.begin();
   {
     size_t smem = fwd_c_smem(p.mpad, p.D);
@@ -685,6 +729,12 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
                 "num_landmarks <= 64 or head_dim 128 with num_landmarks <= 128)");
   const int MP = p.m <= 64 ? 64 : 128;
   const bool smem_ns = p.m <= ns::kN;
+  tc::TcSched sch_sx = tc::make_sched(p.BH, p.N, sms);   // split-precision kernels: one CTA per SM
+  const bool use_sx = !use_tc && sx::supported(a.shape.dtype, p.D, p.m, a.shape.flags) && sch_sx.nchunk <= p.nchunk;
+  if (use_sx) {
+    sch = sch_sx;
+    sch.seg_N = seg_N; sch.row_offset = row_offset; sch.H = big.map_h();
+  }
   // With head_dim 64 on the tensor-core path the reduction of the pass-A partials and the two
   // products that follow run inside the Newton-Schulz backward kernel.
   const bool fused_mid = smem_ns && use_tc && p.D == 64 && p.J >= 1 && ns_on_tensor_cores(a.shape.flags);
@@ -724,8 +774,8 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
   const unsigned sgrid = (unsigned)(p.BH * p.nchunk);
   const unsigned tgrid = (unsigned)(p.BH * sch.nchunk);
   const size_t gsmem = bwd_ac_smem(p.mpad, p.D);
-  const int nchunk_used = use_tc ? sch.nchunk : p.nchunk;        // pass A partials
-  const int nchunk_colpass = use_tc ? sch_b.nchunk : p.nchunk;   // column pass partials
+  const int nchunk_used = (use_tc || use_sx) ? sch.nchunk : p.nchunk;                        // pass A partials
+  const int nchunk_colpass = use_tc ? sch_b.nchunk : use_sx ? sch.nchunk : p.nchunk;         // column pass partials
 
   void* qt16 = w.op16[3]; void* do3n = w.op16[5];
   CUtensorMap tm_q, tm_g, tm_dq, tm_dk;
@@ -758,7 +808,20 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       if (rc) return rc;
     }
   }
-  if (!use_tc) {
+  if (use_sx) {
+    int rc = dispatch_sx<T>(p.D, MP, [&](auto dtag, auto mtag) -> int {
+      constexpr int D = decltype(dtag)::value, MPc = decltype(mtag)::value;
+      L.begin();
+      auto kern = sx::sx_bwd_a_kernel<T, D, MPc>;
+      constexpr size_t sm = sx::Plan<T, D, MPc>::kBwdA;
+      if (int rc2 = set_smem(kern, sm, max_smem, "sx_bwd_a")) return rc2;
+      launch_pdl(kern, dim3(tgrid), dim3(sx::kThr), sm, st, (const T*)a.q, (const T*)a.d_out, a.lse1, a.k_landmarks, a.step2, w.partA,
+                 sch, p.m, scale, a.device_status);
+      return L.end("sx_bwd_a");
+    });
+    if (rc) return rc;
+  }
+  if (!use_tc && !use_sx) {
     L.begin();
     if (int rc = set_smem(gen_bwd_a_kernel<T>, gsmem, max_smem, "gen_bwd_a")) return rc;
     gen_bwd_a_kernel<T><<<sgrid, kThreads, gsmem, st>>>(sp);
@@ -908,7 +971,20 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       if (rc) return rc;
     }
   }
-  if (!use_tc) {
+  if (use_sx) {
+    int rc = dispatch_sx<T>(p.D, MP, [&](auto dtag, auto mtag) -> int {
+      constexpr int D = decltype(dtag)::value, MPc = decltype(mtag)::value;
+      L.begin();
+      auto kern = sx::sx_bwd_b_kernel<T, D, MPc>;
+      constexpr size_t sm = sx::Plan<T, D, MPc>::kBwdB;
+      if (int rc2 = set_smem(kern, sm, max_smem, "sx_bwd_b")) return rc2;
+      launch_pdl(kern, dim3(tgrid), dim3(sx::kThr), sm, st, (const T*)a.k, (const T*)a.v, (T*)a.dk, (T*)a.dv, a.lse3, w.D3,
+                 a.q_landmarks, w.dO3, w.dkt_tot, w.partB, sch, p.m, scale, a.device_status);
+      return L.end("sx_bwd_b");
+    });
+    if (rc) return rc;
+  }
+  if (!use_tc && !use_sx) {
     L.begin();
     if (int rc = set_smem(gen_bwd_b_kernel<T>, gsmem, max_smem, "gen_bwd_b")) return rc;
     gen_bwd_b_kernel<T><<<sgrid, kThreads, gsmem, st>>>(sp);
@@ -967,6 +1043,18 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
                                                  seg_N, scale);
   }
   if (L.end("dqt_reduce")) return L.status;
+  if (use_sx) {
+    return dispatch_sx<T>(p.D, MP, [&](auto dtag, auto mtag) -> int {
+      constexpr int D = decltype(dtag)::value, MPc = decltype(mtag)::value;
+      L.begin();
+      auto kern = sx::sx_bwd_c_kernel<T, D, MPc>;
+      constexpr size_t sm = sx::Plan<T, D, MPc>::kBwdC;
+      if (int rc2 = set_smem(kern, sm, max_smem, "sx_bwd_c")) return rc2;
+      launch_pdl(kern, dim3(tgrid), dim3(sx::kThr), sm, st, (const T*)a.q, (const T*)a.d_out, (T*)a.dq, a.lse1, a.k_landmarks, a.step2,
+                 w.dqt_tot, sch, p.m, scale, a.device_status);
+      return L.end("sx_bwd_c");
+    });
+  }
   L.begin();
   if (int rc = set_smem(gen_bwd_c_kernel<T>, gsmem, max_smem, "gen_bwd_c")) return rc;
   gen_bwd_c_kernel<T><<<sgrid, kThreads, gsmem, st>>>(sp);

@@ -1,0 +1,959 @@
+// Streaming passes at FP32-equivalent precision on the sm_100a tensor cores: full-precision inputs, and
+// the 16-bit shapes whose probabilities stay in more than 16 bits (head_dim 64 with more than 64
+// landmarks, head_dim 16 and 32).
+//
+// Every FP32 operand is a short sum of bf16 terms (x = x0 + x1 + ..., each term the bf16 rounding of
+// what the previous ones left over), and a product is the sum of the partial products whose weight
+// matters.  bf16 has the FP32 exponent range, so no operand needs scaling.
+//   inputs           bf16: 1 term, fp16: 2, fp32: 3 (exact in all three cases)
+//   landmark matrices, probabilities, softmax Jacobians: 3 terms (24 bits) for fp32 inputs; 2 terms
+//                    (16 bits, a sixteenth of the last place of an fp16 result) for 16-bit inputs
+// so a product takes six MMAs per K step for fp32, two or three for bf16 and fp16.
+//
+// One CTA of 16 warps per SM walks 128-row tiles of one (b,h) slice.  All warps stage the tile (global ->
+// registers -> terms -> swizzled shared memory), warp 0 issues the MMAs, all warps take the scores out
+// of tensor memory (thread = one row x a quarter of the landmark columns) and write the probabilities
+// back as operand tiles: K-major when they are contracted over landmarks, MN-major when over rows.
+// The next tile's rows are in flight in registers meanwhile, and its scores are issued together with
+// the products of the current tile wherever the buffers allow.
+//
+// What bounds it: the MMAs of the fp32 passes (24 per 128 x 64 x 64 product at 48 cycles each, the time
+// their operands take through shared memory; a tile of the column pass of the backward needs 128 of
+// them) and, for 16-bit inputs, the exp / split / store work on the probabilities, each in turn with the
+// other for want of room for a second set of buffers.  Measured on a B200, us per launch, against the
+// CUDA-core kernels of generic_kernels.cuh (fwd_b, fwd_c, bwd_a, bwd_b, bwd_c):
+//   fp32, B=1, H=16, N=16384, D=64, m=64    1135, 574, 1996, 1948, 863  ->  78, 64, 117, 130, 95
+//   bf16, B=2, H=8,  N=8192,  D=64, m=128    727, 431, 1319, 1379, 713  ->  41, 37,  50,  60, 46
+#pragma once
+#include <type_traits>
+#include "common.cuh"
+#include "tc_common.cuh"
+#include "tc_stream.cuh"
+
+namespace fnb {
+namespace sx {
+
+using namespace tc;
+typedef __nv_bfloat16 bf16;
+
+constexpr int kThr = 512;
+constexpr int kBlk = kTile * 128;   // bytes of a [128 rows x 64] bf16 block, rows 128 bytes apart
+
+template <class T> struct InTerms { static constexpr int n = 3; };
+template <> struct InTerms<__half> { static constexpr int n = 2; };
+template <> struct InTerms<bf16> { static constexpr int n = 1; };
+template <class T> struct OpTerms { static constexpr int n = std::is_same<T, float>::value ? 3 : 2; };
+
+// Shared-memory plan of one instantiation (bytes).  X: an input tile, P: a probability tile, L: a
+// landmark operand.  head_dim below 64 leaves the tail of the 128-byte rows unused.
+template <class T, int D, int MP>
+struct Plan {
+  static constexpr int NX = InTerms<T>::n, NP = OpTerms<T>::n;
+  static constexpr int kX = NX * kBlk, kP = NP * (MP / 64) * kBlk, kL = NP * MP * 128;
+  static constexpr int kPitch = D * (int)sizeof(T) + 16;      // staged output row
+  static constexpr int kStage = kTile * kPitch;
+  static constexpr int kSmall = 4 * kTile * 4 + 4 * MP * 4 + 256;   // exchange words, per-landmark vectors, barriers
+  static constexpr int kVP = kX > kP ? kX : kP;                // V tile, then P tile
+  static_assert(kStage <= kP, "outputs are staged in a probability buffer");
+  static constexpr int kFwdB = kL + 3 * kX + kP + kSmall;
+  static constexpr int kFwdC = 2 * kL + kX + kP + kSmall;
+  static constexpr int kBwdA = 2 * kL + 2 * kX + kP + kSmall;
+  static constexpr int kBwdB = 2 * kL + kX + kVP + kP + kSmall - 4 * kTile * 4;
+  static constexpr int kBwdC = 2 * kL + 2 * kX + kP + kSmall;
+  static_assert(kFwdB <= 232448 && kFwdC <= 232448 && kBwdA <= 232448 && kBwdB <= 232448 && kBwdC <= 232448, "shared memory");
+};
+
+// ---- terms ---------------------------------------------------------------------------------
+template <int NT>
+__device__ __forceinline__ void split8(const float* v, uint4* w) {
+  uint32_t* o = reinterpret_cast<uint32_t*>(w);
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float a = v[2 * p], b = v[2 * p + 1];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const uint32_t x = pack2<bf16>(a, b);
+      o[4 * t + p] = x;
+      if (t + 1 < NT) {
+        a -= __uint_as_float(x << 16);
+        b -= __uint_as_float(x & 0xffff0000u);
+      }
+    }
+  }
+}
+// Order of the three terms of a probability tile: (x1, x0, x2), so that both (x1, x0) and (x0, x2) are
+// neighbours and can be stacked along M (see contract()).
+template <int NP> __device__ __forceinline__ constexpr int slot_of(int term) { return NP == 3 ? (term == 0 ? 1 : term == 1 ? 0 : 2) : term; }
+
+// ---- input tiles: global -> registers -> terms in shared memory -----------------------------------
+template <class T, int D>
+struct InTile {
+  static constexpr int kVec = (int)sizeof(T) / 2;            // 16-byte words per eight elements
+  static constexpr int kChunks = kTile * D / 8;
+  static constexpr int kPer = (kChunks + kThr - 1) / kThr;
+  uint4 raw[kPer][kVec];
+  __device__ __forceinline__ void fetch(const T* slice, int64_t r0, int64_t N) {
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      const int idx = threadIdx.x + c * kThr, row = idx / (D / 8), ch = idx % (D / 8);
+      const bool ok = (kChunks % kThr == 0 || idx < kChunks) && r0 + row < N;
+      const uint4* src = reinterpret_cast<const uint4*>(slice + (r0 + row) * D + ch * 8);
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) raw[c][v] = ok ? __ldg(src + v) : make_uint4(0, 0, 0, 0);
+    }
+  }
+  __device__ __forceinline__ void put(uint8_t* tile) const {
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      const int idx = threadIdx.x + c * kThr;
+      if (kChunks % kThr != 0 && idx >= kChunks) return;
+      const uint32_t off = sw128_offset(idx / (D / 8), idx % (D / 8));
+      if constexpr (std::is_same<T, bf16>::value) {
+        *reinterpret_cast<uint4*>(tile + off) = raw[c][0];
+      } else {
+        constexpr int NX = InTerms<T>::n;
+        const T* e = reinterpret_cast<const T*>(raw[c]);
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = to_f<T>(e[i]);
+        uint4 w[NX];
+        split8<NX>(x, w);
+#pragma unroll
+        for (int t = 0; t < NX; ++t) *reinterpret_cast<uint4*>(tile + t * kBlk + off) = w[t];
+      }
+    }
+  }
+};
+
+// (m x D) FP32 landmark matrix times mul -> NP term tiles of [MP rows x 128 B], rows >= m zero
+template <int D, int MP, int NP>
+__device__ __forceinline__ void put_landmarks(uint8_t* op, const float* src, int m, float mul) {
+  for (int idx = threadIdx.x; idx < MP * D / 8; idx += kThr) {
+    const int r = idx / (D / 8), ch = idx % (D / 8);
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = 0.f;
+    if (r < m) {
+      const float4 a = *reinterpret_cast<const float4*>(src + r * D + ch * 8), b = *reinterpret_cast<const float4*>(src + r * D + ch * 8 + 4);
+      x[0] = a.x * mul; x[1] = a.y * mul; x[2] = a.z * mul; x[3] = a.w * mul;
+      x[4] = b.x * mul; x[5] = b.y * mul; x[6] = b.z * mul; x[7] = b.w * mul;
+    }
+    uint4 w[NP];
+    split8<NP>(x, w);
+#pragma unroll
+    for (int t = 0; t < NP; ++t) *reinterpret_cast<uint4*>(op + t * (MP * 128) + sw128_offset(r, ch)) = w[t];
+  }
+}
+
+// NC consecutive columns col0.. of row r of a probability tile
+template <int NC, int MP, int NP>
+__device__ __forceinline__ void put_probs(uint8_t* tile, int r, int col0, const float* v) {
+#pragma unroll
+  for (int c = 0; c < NC / 8; ++c) {
+    uint4 w[NP];
+    split8<NP>(v + 8 * c, w);
+    const int cc = (col0 >> 3) + c;
+    const uint32_t off = (uint32_t)(cc >> 3) * kBlk + sw128_offset(r, cc & 7);
+#pragma unroll
+    for (int t = 0; t < NP; ++t) *reinterpret_cast<uint4*>(tile + slot_of<NP>(t) * ((MP / 64) * kBlk) + off) = w[t];
+  }
+}
+
+// ---- products (warp-uniform; one elected lane issues) ------------------------------------------------
+// scores (128 x MP) = X (128 x D) L^T
+template <int D, int MP, int NX, int NP>
+__device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l) {
+  constexpr uint32_t idesc = make_idesc<bf16>(kTile, MP, false, false);
+  bool acc = false;
+#pragma unroll
+  for (int s = NP - 1; s >= 0; --s)            // small terms first
+#pragma unroll
+    for (int i = 0; i < NX; ++i) {
+      const int j = s - i;
+      if (j < 0 || j >= NP) continue;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+        umma_elect(d, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc, acc);
+        acc = true;
+      }
+    }
+}
+// rows (128 x D) = P (128 x MP) L (MP x D).  This product and the next always run with N = 64, the width
+// of a swizzled block: for a smaller head_dim the columns past D hold nothing and are never read.
+template <int MP, int NP>
+__device__ __forceinline__ void issue_rows(uint32_t d, uint32_t p, uint32_t l) {
+  constexpr uint32_t idesc = make_idesc<bf16>(kTile, 64, false, true);
+  bool acc = false;
+#pragma unroll
+  for (int s = NP - 1; s >= 0; --s)
+#pragma unroll
+    for (int i = 0; i <= s; ++i) {
+      const uint32_t pt = p + slot_of<NP>(i) * ((MP / 64) * kBlk), lt = l + (s - i) * (MP * 128);
+#pragma unroll
+      for (int k = 0; k < MP / 16; ++k) {
+        umma_elect(d, smem_desc_sw128(pt + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), smem_desc_sw128(lt + k * 2048, MP * 128, 1024), idesc, acc);
+        acc = true;
+      }
+    }
+}
+// tile sum (landmarks x D) = P^T (MP x 128) X (128 x D).  With 64 landmarks two terms of P are stacked along M
+// (lanes 0..63 and 64..127, added when the sum is read); the one partial product of three-term operands
+// that this cannot place, x2 * X0, goes to 64 columns of its own, lanes 64..127.
+// The tensor core truncates when it adds to an accumulator, and a run of such additions at full magnitude
+// drifts by about 2^-25 each (bmat was off by 5e-5 after 128 tiles).  So the small terms go first, and the
+// tile sums are added up over tiles with ordinary FP32 additions (add_tile_sum).
+template <int MP, int NX, int NP>
+__device__ __forceinline__ void issue_contract(uint32_t d, uint32_t p, uint32_t x) {
+  constexpr uint32_t idesc = make_idesc<bf16>(128, 64, true, true);
+  if (MP == 64) {
+#pragma unroll
+    for (int j = NX - 1; j >= 0; --j)
+#pragma unroll
+      for (int k = 0; k < kTile / 16; ++k)
+        umma_elect(d, smem_desc_sw128(p + k * 2048, kBlk, 1024), smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc, j < NX - 1 || k > 0);
+    if (NP == 3) {
+#pragma unroll
+      for (int k = 0; k < kTile / 16; ++k)
+        umma_elect(d + 64, smem_desc_sw128(p + kBlk + k * 2048, kBlk, 1024), smem_desc_sw128(x + k * 2048, kBlk, 1024), idesc, k > 0);
+    }
+  } else {
+    bool a = false;
+#pragma unroll
+    for (int s = NP - 1; s >= 0; --s)
+#pragma unroll
+      for (int j = 0; j < NX; ++j) {
+        const int i = s - j;
+        if (i < 0 || i >= NP) continue;
+#pragma unroll
+        for (int k = 0; k < kTile / 16; ++k) {
+          umma_elect(d, smem_desc_sw128(p + slot_of<NP>(i) * (2 * kBlk) + k * 2048, kBlk, 1024),
+                     smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc, a);
+          a = true;
+        }
+      }
+  }
+}
+template <int MP, int NP> __host__ __device__ constexpr int acc_cols() { return (MP == 64 && NP == 3) ? 128 : 64; }
+__host__ __device__ constexpr uint32_t pow2_cols(int c) { return c <= 64 ? 64u : c <= 128 ? 128u : c <= 256 ? 256u : 512u; }
+
+// ---- tensor memory -> registers, NC columns of this warp's 32 lanes ------------------------------------
+template <int NC>
+__device__ __forceinline__ void ld(uint32_t a, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  if constexpr (NC == 32) {
+    tmem_ld32(a, v);
+  } else if constexpr (NC == 16) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(a)
+        : "memory");
+  } else if constexpr (NC == 8) {
+    tmem_ld8(a, v);
+  } else {
+    static_assert(NC == 4, "columns");
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  }
+}
+
+template <int NC>
+__device__ __forceinline__ void st(uint32_t a, const float* v) {
+  const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
+  if constexpr (NC == 8) {
+    tmem_st8(a, v);
+  } else {
+    static_assert(NC == 4, "columns");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
+  }
+}
+
+// ---- common frame of the kernels --------------------------------------------------------------------
+struct Frame {
+  uint64_t* bars;          // [3] completion barriers
+  uint32_t tmem;
+  Abort ab;
+  uint32_t phase[3];
+  int warp, row, group;    // row = tile row = tensor-memory lane of this thread; group = its quarter of the columns
+  uint32_t lane_base;
+  int64_t bh;
+  int chunk, first, count;
+  __device__ __forceinline__ void wait(int b, int where) {
+    mbar_wait(bars + b, phase[b], ab, where);
+    phase[b] ^= 1u;
+    __syncwarp();
+    tc_fence_after();
+  }
+  // this thread's shared-memory stores and tensor-memory accesses are done; then every thread's are
+  __device__ __forceinline__ void publish() const {
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+  }
+};
+__device__ __forceinline__ bool open_frame(Frame& f, uint8_t* smem, uint8_t* tail, const TcSched& sch, uint32_t cols, int* status, int where) {
+  f.bars = reinterpret_cast<uint64_t*>(tail);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f.bars + 3);
+  int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
+  if (smem_u32(smem) & 1023u) {
+    if (threadIdx.x == 0 && status) atomicCAS(status, 0, (kStatusSmemAlign << 24) | where);
+    return false;
+  }
+  f.warp = threadIdx.x >> 5;
+  f.row = (f.warp & 3) * 32 + (threadIdx.x & 31);
+  f.group = f.warp >> 2;
+  f.lane_base = (uint32_t)((f.warp & 3) * 32) << 16;
+  f.phase[0] = f.phase[1] = f.phase[2] = 0;
+  f.bh = blockIdx.x / sch.nchunk;
+  f.chunk = (int)(blockIdx.x - f.bh * sch.nchunk);
+  const int tiles = (int)((sch.N + kTile - 1) / kTile);
+  f.first = f.chunk * sch.tiles_per_chunk;
+  f.count = max(0, min(sch.tiles_per_chunk, tiles - f.first));
+  if (threadIdx.x == 0) {
+    for (int b = 0; b < 3; ++b) mbar_init(f.bars + b, 1);
+    *abort_word = 0;
+    fence_mbar_init();
+  }
+  if (f.warp == 0) {
+    tmem_alloc(tmem_slot, cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_wait();
+  f.tmem = *tmem_slot;
+  f.ab = Abort{abort_word, status};
+  return true;
+}
+__device__ __forceinline__ void close_frame(const Frame& f, uint32_t cols) {
+  tc_fence_before();
+  __syncthreads();
+  if (f.warp == 0) tmem_dealloc(f.tmem, cols);
+}
+
+// D / 4 result columns of this thread's row -> staged row of the output type; then the staged tile -> global rows
+template <class T, int D>
+__device__ __forceinline__ void stage_row(uint8_t* stage, int pitch, int row, int col0, const float* o) {
+  T* dst = reinterpret_cast<T*>(stage + row * pitch) + col0;
+  constexpr int NC = D / 4;
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < NC; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < NC; j += 4) *reinterpret_cast<uint2*>(dst + j) = make_uint2(pack2<T>(o[j], o[j + 1]), pack2<T>(o[j + 2], o[j + 3]));
+  }
+}
+template <class T, int D>
+__device__ __forceinline__ void copy_out(T* slice, const uint8_t* stage, int pitch, int64_t r0, int64_t N) {
+  constexpr int VPR = D * (int)sizeof(T) / 16;
+  for (int idx = threadIdx.x; idx < kTile * VPR; idx += kThr) {
+    const int row = idx / VPR, v = idx % VPR;
+    if (r0 + row < N)
+      *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(slice + (r0 + row) * D) + v * 16) = *reinterpret_cast<const uint4*>(stage + row * pitch + v * 16);
+  }
+}
+// running sum (64 columns at `sum`) = factor * running sum + tile sum (at `tile`), FP32; with `first` the running sum
+// starts at zero.  Each thread handles its lane and a quarter of the columns.
+template <int D, int MP, int NP>
+__device__ __forceinline__ void add_tile_sum(const Frame& f, uint32_t tile, uint32_t sum, bool first) {
+  constexpr int NC = D / 4, ST = NC < 8 ? NC : 8;
+  const uint32_t off = f.tmem + f.lane_base + f.group * NC;
+#pragma unroll
+  for (int c = 0; c < NC; c += ST) {
+    float v[ST], x[ST], r[ST];
+    ld<ST>(off + tile + c, v);
+    if (MP == 64 && NP == 3) ld<ST>(off + tile + 64 + c, x);
+    if (!first) ld<ST>(off + sum + c, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ST; ++j) {
+      if (MP == 64 && NP == 3) v[j] += f.row >= 64 ? x[j] : 0.f;
+      if (!first) v[j] += r[j];
+    }
+    st<ST>(off + sum + c, v);
+  }
+  tmem_st_wait();
+}
+template <int D>
+__device__ __forceinline__ void scale_sum(const Frame& f, uint32_t sum, float factor) {
+  constexpr int NC = D / 4, ST = NC < 8 ? NC : 8;
+  const uint32_t off = f.tmem + f.lane_base + f.group * NC + sum;
+#pragma unroll
+  for (int c = 0; c < NC; c += ST) {
+    float v[ST];
+    ld<ST>(off + c, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ST; ++j) v[j] *= factor;
+    st<ST>(off + c, v);
+  }
+  tmem_st_wait();
+}
+// running sum -> global (m x D) times mul; scratch: [64][D + 4] floats of shared memory
+template <int D, int MP>
+__device__ __forceinline__ void store_sum(const Frame& f, uint32_t sum, float* scratch, float* dst, int m, float mul) {
+  constexpr int NC = D / 4, LD = D + 4;
+  const int c0 = f.group * NC;
+  float v[NC];
+  ld<NC>(f.tmem + sum + f.lane_base + c0, v);
+  tmem_ld_wait();
+  if constexpr (MP == 64) {
+    __syncthreads();
+    if (f.row >= 64) {
+#pragma unroll
+      for (int j = 0; j < NC; ++j) scratch[(f.row - 64) * LD + c0 + j] = v[j];
+    }
+    __syncthreads();
+    if (f.row < 64) {
+#pragma unroll
+      for (int j = 0; j < NC; ++j) v[j] += scratch[f.row * LD + c0 + j];
+    }
+  }
+  if (f.row < m && f.row < MP) {
+#pragma unroll
+    for (int j = 0; j < NC; j += 4)
+      *reinterpret_cast<float4*>(dst + f.row * D + c0 + j) = make_float4(v[j] * mul, v[j + 1] * mul, v[j + 2] * mul, v[j + 3] * mul);
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// Forward column pass: partial Bmat = softmax(Qt (sK)^T) V over this CTA's rows with per-landmark
+// maximum and sum.  The exponent's reference moves only when a score exceeds it by 2^8 (one compare
+// per element and one OR-barrier per tile decide it), so the accumulator is rarely rescaled.
+template <class T, int D, int MP>
+__global__ void __launch_bounds__(kThr, 1)
+sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ q_landmarks,
+                float* __restrict__ part_acc, float* __restrict__ part_max, float* __restrict__ part_sum, TcSched sch,
+                int m, float scale, int* status) {
+  using L = Plan<T, D, MP>;
+  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4;
+  constexpr uint32_t kS = 0, kTileSum = MP, kSum = MP + acc_cols<MP, NP>(), kCols = pow2_cols(kSum + 64);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_qt = smem;
+  uint8_t* s_k = s_qt + L::kL;
+  uint8_t* s_v = s_k + L::kX;               // two buffers
+  uint8_t* s_p = s_v + 2 * L::kX;
+  float* s_red = reinterpret_cast<float*>(s_p + L::kP);      // [4][128]
+  float* s_ref = s_red + 4 * kTile;                          // [MP] reference, log2 domain
+  float* s_alpha = s_ref + MP;
+  pdl_trigger();
+  Frame f;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x4000)) return;
+  const T* kk = k + f.bh * sch.N * D;
+  const T* vv = v + f.bh * sch.N * D;
+  const uint32_t a_qt = smem_u32(s_qt), a_k = smem_u32(s_k), a_p = smem_u32(s_p);
+  InTile<T, D> rk, rv;
+  auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  rk.fetch(kk, row0(0), sch.N);
+  rv.fetch(vv, row0(0), sch.N);
+  put_landmarks<D, MP, NP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  if (threadIdx.x < MP) s_ref[threadIdx.x] = -INFINITY;
+  rk.put(s_k);
+  rv.put(s_v);
+  rk.fetch(kk, row0(1), sch.N);
+  rv.fetch(vv, row0(1), sch.N);
+  f.publish();
+  if (f.warp == 0) {
+    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+    umma_commit_elect(f.bars + 0);
+  }
+  const int c0 = f.group * NC;
+  float sum[NC];
+#pragma unroll
+  for (int j = 0; j < NC; ++j) sum[j] = 0.f;
+  for (int i = 0; i < f.count; ++i) {
+    const bool valid = row0(i) + f.row < sch.N;
+    f.wait(0, 0x4100);
+    float s[NC];
+    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
+    tmem_ld_wait();
+    bool over = false;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) over = over || (s[j] - s_ref[c0 + j] > 8.f);   // (a NaN score never raises it)
+    over = over && valid;
+    if (i > 0) {
+      f.wait(1, 0x4200);                     // the product of the previous tile is done: P and its V are free
+      add_tile_sum<D, MP, NP>(f, kTileSum, kSum, i == 1);
+    }
+    if (__syncthreads_or(over)) {
+      // tile maximum of every landmark, the new reference and the factor for what has been summed so far
+#pragma unroll
+      for (int j = 0; j < NC; ++j) {
+        float x = valid ? s[j] : -INFINITY;
+        for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+        if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + c0 + j] = x;
+      }
+      __syncthreads();
+      if (threadIdx.x < MP) {
+        const int l = threadIdx.x;
+        const float old = s_ref[l];
+        const float mx = fmaxf(fmaxf(fmaxf(s_red[l], s_red[kTile + l]), fmaxf(s_red[2 * kTile + l], s_red[3 * kTile + l])), old);
+        s_alpha[l] = old == mx ? 1.f : fast_exp2(old - mx);
+        s_ref[l] = mx;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < NC; ++j) sum[j] *= s_alpha[c0 + j];
+      if (i > 0) scale_sum<D>(f, kSum, s_alpha[MP == 64 ? (f.row & 63) : f.row]);
+    }
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      s[j] = valid ? fast_exp2(s[j] - s_ref[c0 + j]) : 0.f;
+      sum[j] += s[j];
+    }
+    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+    rk.put(s_k);
+    rv.put(s_v + ((i + 1) & 1) * L::kX);
+    f.publish();
+    if (f.warp == 0) {
+      issue_contract<MP, NX, NP>(f.tmem + kTileSum, a_p, smem_u32(s_v) + (i & 1) * L::kX);
+      umma_commit_elect(f.bars + 1);
+      if (i + 1 < f.count) {
+        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+        umma_commit_elect(f.bars + 0);
+      }
+    }
+    if (i + 2 < f.count) {
+      rk.fetch(kk, row0(i + 2), sch.N);
+      rv.fetch(vv, row0(i + 2), sch.N);
+    }
+  }
+  const int64_t slot = blockIdx.x;
+  if (f.count > 0) {
+    f.wait(1, 0x4300);
+    add_tile_sum<D, MP, NP>(f, kTileSum, kSum, f.count == 1);
+    store_sum<D, MP>(f, kSum, reinterpret_cast<float*>(s_k), part_acc + slot * m * D, m, 1.f);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    float x = sum[j];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + c0 + j] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < m) {
+    const int l = threadIdx.x;
+    part_max[slot * m + l] = s_ref[l] * kLn2;
+    part_sum[slot * m + l] = (s_red[l] + s_red[kTile + l]) + (s_red[2 * kTile + l] + s_red[3 * kTile + l]);
+  }
+  close_frame(f, kCols);
+}
+
+// ------------------------------------------------------------------------------------------
+// Forward output pass: O = softmax(sQ Kt^T) step2 and lse1.
+template <class T, int D, int MP>
+__global__ void __launch_bounds__(kThr, 1)
+sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict__ lse1, const float* __restrict__ k_landmarks,
+                const float* __restrict__ step2, TcSched sch, int m, float scale, int* status) {
+  using L = Plan<T, D, MP>;
+  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4;
+  constexpr uint32_t kS = 0, kO = MP, kCols = pow2_cols(MP + 64);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_kt = smem;
+  uint8_t* s_st = s_kt + L::kL;
+  uint8_t* s_q = s_st + L::kL;
+  uint8_t* s_p = s_q + L::kX;               // probabilities, then the staged output tile
+  float* s_max = reinterpret_cast<float*>(s_p + L::kP);      // [4][128]: row maxima, then row sums
+  pdl_trigger();
+  Frame f;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_max + 4 * kTile + 4 * MP), sch, kCols, status, 0x4400)) return;
+  const T* qq = q + f.bh * sch.N * D;
+  T* oo = out + f.bh * sch.N * D;
+  const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_p = smem_u32(s_p);
+  InTile<T, D> rq;
+  auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  rq.fetch(qq, row0(0), sch.N);
+  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  rq.put(s_q);
+  rq.fetch(qq, row0(1), sch.N);
+  f.publish();
+  if (f.warp == 0) {
+    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+    umma_commit_elect(f.bars + 0);
+  }
+  const int c0 = f.group * NC;
+  for (int i = 0; i < f.count; ++i) {
+    const int64_t row = row0(i) + f.row;
+    f.wait(0, 0x4500);
+    float s[NC];
+    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
+    tmem_ld_wait();
+    float mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      if (c0 + j >= m) s[j] = -INFINITY;
+      mx = fmaxf(mx, s[j]);
+    }
+    s_max[f.group * kTile + f.row] = mx;
+    __syncthreads();                         // (also: the previous output tile has left the staging buffer)
+    mx = fmaxf(fmaxf(s_max[f.row], s_max[kTile + f.row]), fmaxf(s_max[2 * kTile + f.row], s_max[3 * kTile + f.row]));
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      s[j] = fast_exp2(s[j] - mx);
+      sum += s[j];
+    }
+    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+    rq.put(s_q);
+    __syncthreads();                         // every thread has read the maxima
+    s_max[f.group * kTile + f.row] = sum;
+    f.publish();
+    if (f.warp == 0) {
+      issue_rows<MP, NP>(f.tmem + kO, a_p, a_st);
+      umma_commit_elect(f.bars + 1);
+      if (i + 1 < f.count) {
+        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+        umma_commit_elect(f.bars + 0);
+      }
+    }
+    if (i + 2 < f.count) rq.fetch(qq, row0(i + 2), sch.N);
+    sum = (s_max[f.row] + s_max[kTile + f.row]) + (s_max[2 * kTile + f.row] + s_max[3 * kTile + f.row]);
+    if (f.group == 0 && row < sch.N) lse1[f.bh * sch.N + row] = (mx + log2f(sum)) * kLn2;
+    const float inv = 1.f / sum;
+    f.wait(1, 0x4600);
+    float o[ND];
+    ld<ND>(f.tmem + kO + f.lane_base + f.group * ND, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ND; ++j) o[j] *= inv;
+    stage_row<T, D>(s_p, L::kPitch, f.row, f.group * ND, o);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    copy_out<T, D>(oo, s_p, L::kPitch, row0(i), sch.N);
+  }
+  close_frame(f, kCols);
+}
+
+// The softmax-1 Jacobian of a tile from its scores s and dP1 = dO step2^T (both in registers; s becomes
+// P1 and g becomes dS1): P1 = exp2(S - lse1 log2e), D1 = rowsum(P1 o dP1), dS1 = P1 o (dP1 - D1).
+template <int NC>
+__device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse2, bool valid, int c0, int m) {
+  float d1 = 0.f;
+#pragma unroll
+  for (int j = 0; j < NC; ++j) {
+    s[j] = (valid && c0 + j < m) ? fast_exp2(s[j] - lse2) : 0.f;
+    d1 = fmaf(s[j], g[j], d1);
+  }
+  s_red[f.group * kTile + f.row] = d1;
+  __syncthreads();
+  d1 = (s_red[f.row] + s_red[kTile + f.row]) + (s_red[2 * kTile + f.row] + s_red[3 * kTile + f.row]);
+#pragma unroll
+  for (int j = 0; j < NC; ++j) g[j] = s[j] * (g[j] - d1);
+}
+
+// ------------------------------------------------------------------------------------------
+// First backward row pass: per-CTA partials of dstep2 = P1^T dO and dKt = dS1^T (sQ).  P1 and dS1 take
+// turns in one buffer: Q, dO, both landmark operands and one probability tile fill the SM.
+template <class T, int D, int MP>
+__global__ void __launch_bounds__(kThr, 1)
+sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const float* __restrict__ lse1,
+                const float* __restrict__ k_landmarks, const float* __restrict__ step2, float* __restrict__ partA, TcSched sch,
+                int m, float scale, int* status) {
+  using L = Plan<T, D, MP>;
+  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, AC = acc_cols<MP, NP>();
+  constexpr uint32_t kS = 0, kG = MP, kTile1 = 2 * MP, kTile2 = kTile1 + AC, kSum1 = kTile2 + AC, kSum2 = kSum1 + 64, kCols = 512;
+  static_assert(kSum2 + 64 <= 512, "tensor memory");
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_kt = smem;
+  uint8_t* s_st = s_kt + L::kL;
+  uint8_t* s_q = s_st + L::kL;
+  uint8_t* s_g = s_q + L::kX;
+  uint8_t* s_p = s_g + L::kX;
+  float* s_red = reinterpret_cast<float*>(s_p + L::kP);
+  pdl_trigger();
+  Frame f;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x4800)) return;
+  const T* qq = q + f.bh * sch.N * D;
+  const T* gg = d_out + f.bh * sch.N * D;
+  const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_g = smem_u32(s_g), a_p = smem_u32(s_p);
+  InTile<T, D> rq, rg;
+  auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  rq.fetch(qq, row0(0), sch.N);
+  rg.fetch(gg, row0(0), sch.N);
+  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  rq.put(s_q);
+  rg.put(s_g);
+  rq.fetch(qq, row0(1), sch.N);
+  rg.fetch(gg, row0(1), sch.N);
+  f.publish();
+  if (f.warp == 0) {
+    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+    umma_commit_elect(f.bars + 0);
+  }
+  const int c0 = f.group * NC;
+  for (int i = 0; i < f.count; ++i) {
+    const int64_t row = row0(i) + f.row;
+    const bool valid = row < sch.N, more = i + 1 < f.count;
+    const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
+    f.wait(0, 0x4900);
+    float s[NC], g[NC];
+    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
+    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
+    tmem_ld_wait();
+    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, c0, m);
+    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+    f.publish();
+    if (f.warp == 0) {
+      issue_contract<MP, NX, NP>(f.tmem + kTile1, a_p, a_g);
+      umma_commit_elect(f.bars + 1);
+    }
+    f.wait(1, 0x4a00);                       // P1 and dO have been used
+    put_probs<NC, MP, NP>(s_p, f.row, c0, g);
+    if (more) rg.put(s_g);
+    f.publish();
+    if (f.warp == 0) {
+      issue_contract<MP, NX, NP>(f.tmem + kTile2, a_p, a_q);
+      umma_commit_elect(f.bars + 2);
+      if (more) issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+    }
+    if (i + 2 < f.count) rg.fetch(gg, row0(i + 2), sch.N);
+    add_tile_sum<D, MP, NP>(f, kTile1, kSum1, i == 0);
+    f.wait(2, 0x4b00);                       // dS1 and Q have been used
+    if (more) {
+      rq.put(s_q);
+      if (i + 2 < f.count) rq.fetch(qq, row0(i + 2), sch.N);
+      f.publish();
+      if (f.warp == 0) {
+        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+        umma_commit_elect(f.bars + 0);
+      }
+    }
+    add_tile_sum<D, MP, NP>(f, kTile2, kSum2, i == 0);
+  }
+  float* pa = partA + (int64_t)blockIdx.x * 2 * m * D;
+  store_sum<D, MP>(f, kSum1, reinterpret_cast<float*>(s_q), pa, m, 1.f);
+  store_sum<D, MP>(f, kSum2, reinterpret_cast<float*>(s_q), pa + m * D, m, scale);
+  close_frame(f, kCols);
+}
+
+// ------------------------------------------------------------------------------------------
+// Backward column pass: dV = P3^T dO3, dK = s (dS3^T Qt + dKt_tot[l(n)] / len_l), per-CTA partials of
+// dQt = dS3 (sK).  P3 takes V's place once the scores are formed; dV and dK leave through the
+// probability buffers.
+template <class T, int D, int MP>
+__global__ void __launch_bounds__(kThr, 1)
+sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ dk, T* __restrict__ dv,
+                const float* __restrict__ lse3, const float* __restrict__ D3, const float* __restrict__ q_landmarks,
+                const float* __restrict__ dO3, const float* __restrict__ dkt_tot, float* __restrict__ partB, TcSched sch, int m,
+                float scale, int* status) {
+  using L = Plan<T, D, MP>;
+  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4, AC = acc_cols<MP, NP>();
+  constexpr uint32_t kS = 0, kG = MP, kDv = 2 * MP, kDk = kDv + 64, kTileSum = kDk + 64, kSum = kTileSum + AC, kCols = 512;
+  static_assert(kSum + 64 <= 512, "tensor memory");
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_qt = smem;
+  uint8_t* s_g3 = s_qt + L::kL;
+  uint8_t* s_k = s_g3 + L::kL;
+  uint8_t* s_p = s_k + L::kX;               // V, then P3, then the staged dV tile
+  uint8_t* s_ds = s_p + L::kVP;             // dS3, then the staged dK tile
+  float* s_l3 = reinterpret_cast<float*>(s_ds + L::kP);
+  float* s_d3 = s_l3 + MP;
+  pdl_trigger();
+  Frame f;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_l3 + 4 * MP), sch, kCols, status, 0x5000)) return;
+  const T* kk = k + f.bh * sch.N * D;
+  const T* vv = v + f.bh * sch.N * D;
+  const uint32_t a_qt = smem_u32(s_qt), a_g3 = smem_u32(s_g3), a_k = smem_u32(s_k), a_p = smem_u32(s_p), a_ds = smem_u32(s_ds);
+  InTile<T, D> rk, rv;
+  auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  rk.fetch(kk, row0(0), sch.N);
+  rv.fetch(vv, row0(0), sch.N);
+  put_landmarks<D, MP, NP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP, NP>(s_g3, dO3 + f.bh * m * D, m, 1.f);
+  if (threadIdx.x < MP) {
+    s_l3[threadIdx.x] = threadIdx.x < m ? lse3[f.bh * m + threadIdx.x] * kLog2e : INFINITY;   // exp2(S - inf) = 0
+    s_d3[threadIdx.x] = threadIdx.x < m ? D3[f.bh * m + threadIdx.x] : 0.f;
+  }
+  Segments sg(sch.seg_N, m);
+  const float* rows = dkt_tot + f.bh * m * D;
+  const int c0 = f.group * NC, d0 = f.group * ND;
+  rk.put(s_k);
+  rv.put(s_p);
+  f.publish();
+  if (f.warp == 0) {
+    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_p, a_g3);
+    umma_commit_elect(f.bars + 0);
+  }
+  for (int i = 0; i < f.count; ++i) {
+    const int64_t row = row0(i) + f.row;
+    const bool valid = row < sch.N, more = i + 1 < f.count;
+    if (more) {
+      rk.fetch(kk, row0(i + 1), sch.N);
+      rv.fetch(vv, row0(i + 1), sch.N);
+    }
+    f.wait(0, 0x5100);
+    float s[NC], g[NC];
+    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
+    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      s[j] = valid ? fast_exp2(s[j] - s_l3[c0 + j]) : 0.f;
+      g[j] = s[j] * (g[j] - s_d3[c0 + j]);
+    }
+    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+    put_probs<NC, MP, NP>(s_ds, f.row, c0, g);
+    f.publish();
+    if (f.warp == 0) {
+      issue_rows<MP, NP>(f.tmem + kDv, a_p, a_g3);
+      issue_rows<MP, NP>(f.tmem + kDk, a_ds, a_qt);
+      issue_contract<MP, NX, NP>(f.tmem + kTileSum, a_ds, a_k);
+      umma_commit_elect(f.bars + 1);
+    }
+    const int l = valid ? sg.landmark_of(sch.row_offset + row) : 0;
+    const float inv = scale / (float)sg.len(l);
+    float add[ND];
+#pragma unroll
+    for (int j = 0; j < ND; j += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(rows + l * D + d0 + j);
+      add[j] = x.x * inv; add[j + 1] = x.y * inv; add[j + 2] = x.z * inv; add[j + 3] = x.w * inv;
+    }
+    f.wait(1, 0x5200);
+    float o[ND];
+    ld<ND>(f.tmem + kDv + f.lane_base + d0, o);
+    tmem_ld_wait();
+    stage_row<T, D>(s_p, L::kPitch, f.row, d0, o);
+    ld<ND>(f.tmem + kDk + f.lane_base + d0, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);    // the operand carries s log2e
+    stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
+    if (more) rk.put(s_k);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    copy_out<T, D>(dv + f.bh * sch.N * D, s_p, L::kPitch, row0(i), sch.N);
+    copy_out<T, D>(dk + f.bh * sch.N * D, s_ds, L::kPitch, row0(i), sch.N);
+    add_tile_sum<D, MP, NP>(f, kTileSum, kSum, i == 0);
+    if (more) {
+      __syncthreads();                       // the staged tiles have been read
+      rv.put(s_p);
+      f.publish();
+      if (f.warp == 0) {
+        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX, NP>(f.tmem + kG, a_p, a_g3);
+        umma_commit_elect(f.bars + 0);
+      }
+    }
+  }
+  store_sum<D, MP>(f, kSum, reinterpret_cast<float*>(s_k), partB + (int64_t)blockIdx.x * m * D, m, scale);
+  close_frame(f, kCols);
+}
+
+// ------------------------------------------------------------------------------------------
+// Second backward row pass: dQ = s (dS1 Kt + dQt_tot[l(n)] / len_l), dS1 formed again from Q and dO.
+template <class T, int D, int MP>
+__global__ void __launch_bounds__(kThr, 1)
+sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restrict__ dq, const float* __restrict__ lse1,
+                const float* __restrict__ k_landmarks, const float* __restrict__ step2, const float* __restrict__ dqt_tot,
+                TcSched sch, int m, float scale, int* status) {
+  using L = Plan<T, D, MP>;
+  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4;
+  constexpr uint32_t kS = 0, kG = MP, kO = 2 * MP, kCols = pow2_cols(2 * MP + 64);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_kt = smem;
+  uint8_t* s_st = s_kt + L::kL;
+  uint8_t* s_q = s_st + L::kL;
+  uint8_t* s_g = s_q + L::kX;
+  uint8_t* s_ds = s_g + L::kX;              // dS1, then the staged dQ tile
+  float* s_red = reinterpret_cast<float*>(s_ds + L::kP);
+  pdl_trigger();
+  Frame f;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x5400)) return;
+  const T* qq = q + f.bh * sch.N * D;
+  const T* gg = d_out + f.bh * sch.N * D;
+  const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_g = smem_u32(s_g), a_ds = smem_u32(s_ds);
+  InTile<T, D> rq, rg;
+  auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  rq.fetch(qq, row0(0), sch.N);
+  rg.fetch(gg, row0(0), sch.N);
+  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  rq.put(s_q);
+  rg.put(s_g);
+  rq.fetch(qq, row0(1), sch.N);
+  rg.fetch(gg, row0(1), sch.N);
+  f.publish();
+  if (f.warp == 0) {
+    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+    umma_commit_elect(f.bars + 0);
+  }
+  Segments sg(sch.seg_N, m);
+  const float* rows = dqt_tot + f.bh * m * D;
+  const int c0 = f.group * NC, d0 = f.group * ND;
+  for (int i = 0; i < f.count; ++i) {
+    const int64_t row = row0(i) + f.row;
+    const bool valid = row < sch.N, more = i + 1 < f.count;
+    const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
+    f.wait(0, 0x5500);
+    float s[NC], g[NC];
+    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
+    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
+    tmem_ld_wait();
+    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, c0, m);   // (its barrier: the previous output tile has left s_ds)
+    put_probs<NC, MP, NP>(s_ds, f.row, c0, g);
+    if (more) {
+      rq.put(s_q);
+      rg.put(s_g);
+    }
+    f.publish();
+    if (f.warp == 0) {
+      issue_rows<MP, NP>(f.tmem + kO, a_ds, a_kt);
+      umma_commit_elect(f.bars + 1);
+      if (more) {
+        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+        issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+        umma_commit_elect(f.bars + 0);
+      }
+    }
+    if (i + 2 < f.count) {
+      rq.fetch(qq, row0(i + 2), sch.N);
+      rg.fetch(gg, row0(i + 2), sch.N);
+    }
+    const int l = valid ? sg.landmark_of(sch.row_offset + row) : 0;
+    const float inv = scale / (float)sg.len(l);
+    float add[ND];
+#pragma unroll
+    for (int j = 0; j < ND; j += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(rows + l * D + d0 + j);
+      add[j] = x.x * inv; add[j + 1] = x.y * inv; add[j + 2] = x.z * inv; add[j + 3] = x.w * inv;
+    }
+    f.wait(1, 0x5600);
+    float o[ND];
+    ld<ND>(f.tmem + kO + f.lane_base + d0, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);
+    stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    copy_out<T, D>(dq + f.bh * sch.N * D, s_ds, L::kPitch, row0(i), sch.N);
+  }
+  close_frame(f, kCols);
+}
+
+// The shapes these kernels take: fp32 with up to 64 landmarks and head_dim 16 .. 64; 16-bit inputs with head_dim
+// 16 .. 64 and up to 128 landmarks (head_dim 64 with up to 64 landmarks has 16-bit kernels of its own, which are
+// asked first).  The line lies where the term tiles of one 128-row tile and both landmark operands stop fitting into
+// shared memory: three terms of a 128-landmark or head_dim-128 operand pair take 96 .. 192 KB alone.  They are
+// faster than the CUDA-core kernels from one tile on (B=1, H=4, N=1024, m=32, fp32: 143 -> 76 us for the five).
+inline bool supported(int dtype, int D, int m, uint32_t flags) {
+  if ((flags & FNB_FLAG_FORCE_GENERIC) || D > 64) return false;
+  return dtype == FNB_F32 ? m <= 64 : m <= 128;
+}
+
+}  // namespace sx
+}  // namespace fnb

@@ -1,0 +1,66 @@
+"""The split-precision tensor-core passes (fp32 with up to 64 landmarks; 16-bit inputs of head_dim 16 / 32, and of
+head_dim 64 with more than 64 landmarks) against the float64 oracle, with the FP32 CUDA-core kernels
+as the yardstick: the same calls are made through both, and the split kernels may not be further
+from the oracle than the CUDA-core ones by more than what their operands drop.  fp32 operands keep 24
+bits in three bf16 terms; per product the dropped terms and the truncating accumulator stay below
+2^-22 = 2.4e-7, and the pseudoinverse (condition number up to a few tens here) amplifies it like it does the
+yardstick's own rounding: bound 1.5 x yardstick + 1e-6.  16-bit inputs: the results' own rounding (2^-12, 2^-9
+relative at most) dominates both; two-term operands add at most 2^-16 per element, amplified the same way:
+bound 1.05 x yardstick + 5e-5."""
+import pytest
+import torch
+
+from oracle import nystrom_oracle as O
+from tests._util import run_cuda, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
+
+CASES = [
+    # tile edges, one tile and a remainder, smallest landmark counts
+    (1, 2, 127, 64, 1, 6, 0.0, F32), (1, 2, 128, 64, 64, 6, 0.0, F32), (1, 2, 129, 32, 63, 6, 5.0, F32), (1, 2, 257, 16, 5, 6, 0.0, F32),
+    (1, 2, 128, 64, 65, 6, 0.0, F16), (1, 2, 129, 64, 128, 6, 5.0, BF16), (1, 2, 255, 32, 64, 6, 0.0, BF16), (1, 2, 300, 32, 65, 4, 0.0, F16),
+    (1, 1, 128, 16, 128, 6, 0.0, F16), (1, 1, 16, 16, 16, 6, 0.0, BF16),
+    # more slices than SMs, so that one CTA walks every tile of its slice: the running sums over many tiles
+    (1, 150, 2500, 64, 64, 6, 0.0, F32), (3, 50, 1300, 64, 100, 6, 0.0, BF16), (3, 50, 1300, 32, 40, 6, 0.0, F16),
+]
+
+
+def _rel(a, b):
+    a, b = a.detach().double().cpu(), b.double()
+    return float((a - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(str(x) for x in c[:7]) + str(c[7])[6:])
+def test_split_precision_against_fp32_kernels(cuda_device, case):
+    from flashnystrom_b200 import _C
+    B, H, N, D, m, J, kappa, dtype = case
+    q, k, v, dO = O.make_inputs(B, H, N, D, seed=9, dtype=dtype)
+    got = run_cuda(q, k, v, dO, m, J, kappa)
+    _C.set_force_generic(True)
+    try:
+        ref = run_cuda(q, k, v, dO, m, J, kappa)
+    finally:
+        _C.set_force_generic(False)
+    slices = [0, B * H // 2, B * H - 1]
+    pick = lambda t: t.reshape(1, B * H, *t.shape[2:])[:, slices]
+    want = run_oracle(pick(q), pick(k), pick(v), pick(dO), m, J, kappa)
+    factor, extra = (1.5, 1e-6) if dtype == F32 else (1.05, 5e-5)
+    for key in ("out", "dq", "dk", "dv", "bmat", "step2", "lse1", "lse3"):
+        a, b = _rel(pick(got[key]), want[key]), _rel(pick(ref[key]), want[key])
+        print(key, f"{a:.2e} {b:.2e}")
+        assert a <= factor * b + extra, (key, a, b)
+
+
+def test_moving_reference(cuda_device):
+    """Scores that grow along the sequence: the reference of the forward column pass moves in most tiles, and what has
+    been summed is rescaled each time."""
+    B, H, N, D, m = 1, 2, 2048, 64, 16
+    q, k, v, dO = O.make_inputs(B, H, N, D, seed=2, dtype=torch.float32)
+    k = k * torch.linspace(0.1, 12.0, N)[None, None, :, None]
+    got = run_cuda(q, k, v, dO, m, 6, 0.0)
+    want = run_oracle(q, k, v, dO, m, 6, 0.0)
+    for key in ("out", "dq", "dk", "dv", "bmat", "lse3"):
+        # scores of about 100: 2^-24 of them is an error of 6e-6 in a probability, several of which meet in a gradient
+        assert _rel(got[key], want[key]) <= 1e-4, (key, _rel(got[key], want[key]))
