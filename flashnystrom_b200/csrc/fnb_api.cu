@@ -488,11 +488,19 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   if (S.run(0)) {
     {
       L.begin();
-      int64_t grid = std::min<int64_t>(2 * p.BH * p.m * lmC, (int64_t)sms * 4);
-      auto pool = (a.shape.layout == FNB_LAYOUT_BNHD) ? landmark_partial_kernel<T, false> : landmark_partial_kernel<T, true>;
-      launch_pdl(pool, dim3((unsigned)grid), dim3(kThreads), 0, st,
-          (const T*)a.q, (const T*)a.k, land, p.BH, p.N, p.D, p.m, lmC, seg_N, row_offset, big.map_h(), big.row_stride(),
-          big.head_stride(), big.batch_stride());
+      // One warp per item where an item is at most 32 KB, the whole CTA above.  Measured (us, CTA / warp): B=32, H=16,
+      // N=2000, D=64 (4 KB items) 404 / 66, B=1, H=7, N=50001, m=33 (24 KB) 32 / 25, B=2, H=8, N=16384, D=128, m=128 (32 KB)
+      // 37 / 32, B=4, H=16, N=16384, D=128 (64 KB, and fewer than two items per warp) 93 / 103.
+      const int64_t items = 2 * p.BH * p.m * lmC, seg = seg_N / p.m;
+      if (items > 0x7fffffff) return fail(FNB_ERR_INVALID_ARGUMENT, "too many pooling items (%lld)", (long long)items);
+      const bool by_warp = (seg + lmC - 1) / lmC * p.D * (int64_t)sizeof(T) <= 32 * 1024;
+      const int64_t ctas = by_warp ? (items + kThreads / 32 - 1) / (kThreads / 32) : items;
+      auto pool = (a.shape.layout == FNB_LAYOUT_BNHD)
+                      ? (by_warp ? landmark_partial_kernel<T, false, 1> : landmark_partial_kernel<T, false, 8>)
+                      : (by_warp ? landmark_partial_kernel<T, true, 1> : landmark_partial_kernel<T, true, 8>);
+      launch_pdl(pool, dim3((unsigned)std::min<int64_t>(ctas, (int64_t)sms * 4)), dim3(kThreads), 0, st,
+          (const T*)a.q, (const T*)a.k, land, (uint32_t)p.BH, p.N, p.D, p.m, lmC, seg_N, seg, row_offset, big.map_h(),
+          big.row_stride(), big.head_stride(), big.batch_stride());
       if (L.end("landmark_partial")) return L.status;
     }
   }
@@ -1435,7 +1443,7 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
   if (!g.ok) return 0;
   using H = __half;
   const KernelEntry ks[] = {
-      {"landmark_partial<half>", (const void*)landmark_partial_kernel<H, true>, kThreads, 0},
+      {"landmark_partial<half>", (const void*)landmark_partial_kernel<H, true, 8>, kThreads, 0},
       {"ns_fwd_tc", (const void*)nstc::ns_fwd_tc_kernel, nstc::kNsTcThreads, nstc::kFwdSmem},
       {"conv_residual<half>", (const void*)conv_residual_kernel<H>, kThreads, conv_smem_bytes(64, 3)},
       {"conv_dw_partial<half,2>", (const void*)conv_dw_partial_kernel<H, 2>, kThreads, conv_smem_bytes(64, 3)},

@@ -74,97 +74,79 @@ __device__ __forceinline__ void load_small(float* dst, int ld, const float* src,
 // ------------------------------------------------------------------------------------------
 // Pass 1: raw segment sums of Q and K (landmark pooling).
 // Work items (which, bh, landmark, chunk) are walked by a grid-stride loop, so the grid can be
-// sized to the machine.  out[which][bh][l][c][D].  kContig: the slices are contiguous (row stride D,
-// slice bh at bh * N * D); the addressing of the streaming loop is then 32-bit and free of the
-// run-time strides, which this kernel is sensitive to (59 against 92 us with them at B=1, H=16,
-// N=65536, D=64).
-template <class T, bool kContig>
+// sized to the machine.  out[which][bh][l][c][D].  G warps share an item: one where the items are
+// short, so that an SM has 32 independent ones in flight and none waits at a barrier, the
+// whole CTA (G = 8) where they are long.  Either way a lane has eight predicated 16-byte loads
+// in flight, also for the last rows of an item.
+// kContig: the slices are contiguous (row stride D, slice bh at bh * N * D); the addressing of the
+// streaming loop is then 32-bit and free of the run-time strides.
+// The items are counted in 32 bits (the host refuses more), and the segment length comes from the host: the
+// four 64-bit divisions that numbering an item takes otherwise are as long as the loads of a short one.
+template <class T, bool kContig, int G>
 __global__ void __launch_bounds__(kThreads, 4)
 landmark_partial_kernel(const T* __restrict__ q, const T* __restrict__ k, float* __restrict__ out,
-                        int64_t BH, int64_t N, int D, int m, int C, int64_t seg_N, int64_t row_offset,
+                        uint32_t BH, int64_t N, int D, int m, int C, int64_t seg_N, int64_t seg, int64_t row_offset,
                         int H, int64_t row_stride, int64_t head_stride, int64_t batch_stride) {
-  constexpr int V = Vec16<T>::n;
-  __shared__ float red[kThreads * 8];
+  constexpr int V = Vec16<T>::n, U = 8;
+  __shared__ float red[G > 1 ? kThreads / 32 * kMaxD : 1];
   pdl_trigger();
+  const uint32_t per_slice = (uint32_t)(m * C), per_which = BH * per_slice, items = 2 * per_which;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int vpr = D / V, rpw = 32 / vpr;                      // lanes per row, rows per load of a warp
+  const int cv = lane % vpr, ro = lane / vpr;
+  const int w = G > 1 ? warp : 0;
+  const int rows_it = G * rpw;                                // rows per load of the warps that share the item
+  const uint32_t first = G > 1 ? blockIdx.x : blockIdx.x * (kThreads / 32) + warp;
+  const uint32_t step = G > 1 ? gridDim.x : gridDim.x * (kThreads / 32);
   pdl_wait();
-  const int64_t per_which = BH * m * C, items = 2 * per_which;
-  const int vpr = D / V, rows_per_iter = kThreads / vpr;
-  const int cv = threadIdx.x % vpr, ro = threadIdx.x / vpr;
-  // lanes that hold the same columns are vpr apart: fold them with shuffles when that tiles a warp
-  const bool warp_fold = vpr <= 32 && (vpr & (vpr - 1)) == 0;
-  Segments sg(seg_N, m);
-  for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
-    const int which = (int)(item / per_which);
-    const int64_t rest = item - which * per_which;
-    const int64_t bh = rest / (m * C);
-    const int lc = (int)(rest - bh * (m * C));
-    const int l = lc / C, c = lc - l * C;
+  for (uint32_t item = first; item < items; item += step) {
+    const int which = item >= per_which;
+    const uint32_t rest = item - (which ? per_which : 0u);
+    const uint32_t bh = rest / per_slice, lc = rest - bh * per_slice;
+    const int l = (int)lc / C, c = (int)lc - l * C;
     // slice (bh % H, bh / H); its rows are row_stride elements apart (D for the contiguous layout)
-    const T* slice = (which ? k : q) + (kContig ? bh * N * D : (bh / H) * batch_stride + (bh % H) * head_stride);
+    const T* slice = (which ? k : q) + (kContig ? (int64_t)bh * N * D : (int64_t)(bh / (uint32_t)H) * batch_stride + (int64_t)(bh % (uint32_t)H) * head_stride);
     // segment l in global rows, clipped to the rows this rank holds, in local row numbers
-    int64_t start = sg.start(l) - row_offset, end = sg.end(l) - row_offset;
+    int64_t start = seg * l - row_offset, end = (l == m - 1 ? seg_N : seg * (l + 1)) - row_offset;
     if (start < 0) start = 0;
     if (end > N) end = N;
-    const int64_t len = end > start ? end - start : 0;
-    const int64_t per = (len + C - 1) / C;
-    const int64_t r0 = start + c * per;
+    const int len = end > start ? (int)(end - start) : 0;
+    const int per = C == 1 ? len : (len + C - 1) / C;
+    const int64_t r0 = start + (int64_t)c * per;
     int64_t r1 = r0 + per;
     if (r1 > start + len) r1 = start + len;
+    const int64_t stride = kContig ? (int64_t)D : row_stride;
+    const T* ptr = slice + (r0 + w * rpw + ro) * stride + cv * V;
+    const int64_t adv = (int64_t)rows_it * stride;
+    int left = (int)(r1 - r0) - (w * rpw + ro);               // rows from this lane's first one to the end of the item
     float acc[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) acc[e] = 0.f;
-    // eight independent 16-byte loads in flight per thread
-    int64_t r = r0 + ro;
-    if constexpr (kContig) {
-      for (; r + 7 * rows_per_iter < r1; r += 8 * rows_per_iter) {
-        uint4 raw[8];
+    for (; left > 0; left -= U * rows_it) {
+      uint4 raw[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          raw[u] = __ldcs(reinterpret_cast<const uint4*>(slice + (r + u * rows_per_iter) * D + cv * V));
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const T* e16 = reinterpret_cast<const T*>(&raw[u]);
-#pragma unroll
-          for (int e = 0; e < V; ++e) acc[e] += to_f<T>(e16[e]);
-        }
+      for (int u = 0; u < U; ++u) {
+        raw[u] = make_uint4(0, 0, 0, 0);                      // (zero bits are a zero in all three types)
+        if (left > u * rows_it) raw[u] = __ldcs(reinterpret_cast<const uint4*>(ptr));
+        ptr += adv;
       }
-      for (; r < r1; r += rows_per_iter) {
-        float x[V];
-        load16<T>(slice + r * D + cv * V, x);
 #pragma unroll
-        for (int e = 0; e < V; ++e) acc[e] += x[e];
-      }
-    } else {
-      // strided rows: one running pointer, advanced by additions only
-      const T* ptr = slice + r * row_stride + cv * V;
-      const int64_t step = (int64_t)rows_per_iter * row_stride;
-      for (; r + 7 * rows_per_iter < r1; r += 8 * rows_per_iter) {
-        uint4 raw[8];
+      for (int u = 0; u < U; ++u) {
+        const T* e16 = reinterpret_cast<const T*>(&raw[u]);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          raw[u] = __ldcs(reinterpret_cast<const uint4*>(ptr));
-          ptr += step;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const T* e16 = reinterpret_cast<const T*>(&raw[u]);
-#pragma unroll
-          for (int e = 0; e < V; ++e) acc[e] += to_f<T>(e16[e]);
-        }
-      }
-      for (; r < r1; r += rows_per_iter, ptr += step) {
-        float x[V];
-        load16<T>(ptr, x);
-#pragma unroll
-        for (int e = 0; e < V; ++e) acc[e] += x[e];
+        for (int e = 0; e < V; ++e) acc[e] += to_f<T>(e16[e]);
       }
     }
-    float* dst = out + ((((size_t)which * BH + bh) * m + l) * C + c) * D;
-    if (warp_fold) {
-      for (int o = vpr; o < 32; o <<= 1)
+    // lanes that hold the same columns are vpr apart
+    for (int o = vpr; o < 32; o <<= 1)
 #pragma unroll
-        for (int e = 0; e < V; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-      const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+      for (int e = 0; e < V; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    float* dst = out + ((((size_t)which * BH + bh) * m + l) * C + c) * D;
+    if (G == 1) {
+      if (lane < vpr)
+#pragma unroll
+        for (int e = 0; e < V; e += 4) *reinterpret_cast<float4*>(dst + lane * V + e) = make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]);
+    } else {
       if (lane < vpr)
 #pragma unroll
         for (int e = 0; e < V; ++e) red[w * D + lane * V + e] = acc[e];
@@ -175,17 +157,8 @@ landmark_partial_kernel(const T* __restrict__ q, const T* __restrict__ k, float*
         for (int ww = 0; ww < kThreads / 32; ++ww) s += red[ww * D + threadIdx.x];
         dst[threadIdx.x] = s;
       }
-    } else {
-#pragma unroll
-      for (int e = 0; e < V; ++e) red[ro * D + cv * V + e] = acc[e];
-      __syncthreads();
-      if (threadIdx.x < D) {
-        float s = 0.f;
-        for (int rr = 0; rr < rows_per_iter; ++rr) s += red[rr * D + threadIdx.x];
-        dst[threadIdx.x] = s;
-      }
+      __syncthreads();   // red is reused by the next item
     }
-    __syncthreads();   // red is reused by the next item
   }
 }
 
