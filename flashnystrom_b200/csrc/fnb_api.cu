@@ -19,6 +19,7 @@
 #include "generic_kernels.cuh"
 #include "tc_host.cuh"
 #include "split_stream.cuh"
+#include "mid_tc.cuh"
 #include "ns_kernels.cuh"
 #include "ns_tc_kernels.cuh"
 #include "conv_kernels.cuh"
@@ -263,7 +264,8 @@ static FwdWs carve_fwd(const Plan& p, void* base) {
   w.part_acc = take((size_t)p.BH * p.nchunk * p.m * p.D);
   w.part_max = take((size_t)p.BH * p.nchunk * p.m);
   w.part_sum = take((size_t)p.BH * p.nchunk * p.m);
-  w.pinv = take((size_t)p.BH * kPinvFwdBufs * p.m * p.m);
+  // the images of mid_tc.cuh are the larger need (the CUDA-core kernel takes kPinvFwdBufs m x m matrices)
+  w.pinv = take(p.m > ns::kN ? (size_t)p.BH * (mx::kFwdScratchBytes / sizeof(float)) : 0);
   const int MP = p.m <= 64 ? 64 : 128;
   const size_t op16 = ((size_t)p.BH * MP * p.D + 1) / 2;   // 16-bit elements, counted in floats
   w.qt16 = take(op16); w.kt16 = take(op16); w.st16 = take(op16);
@@ -292,7 +294,7 @@ static BwdWs carve_bwd(const Plan& p, void* base) {
   w.dqt_ns = take(md); w.dkt_tot = take(md); w.dqt_tot = take(md);
   w.D3 = take((size_t)p.BH * p.m);
   w.G = take(mm); w.dK2 = take(mm);
-  w.pinv = take((size_t)kPinvBwdBufs * mm);
+  w.pinv = take(p.m > ns::kN ? (size_t)p.BH * (mx::kBwdScratchBytes / sizeof(float)) : 0);
   const int MP = p.m <= 64 ? 64 : 128;
   const size_t op16 = ((size_t)p.BH * MP * p.D + 1) / 2;
   for (int i = 0; i < 8; ++i) w.op16[i] = take(op16);
@@ -344,52 +346,7 @@ static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// Launch as thread-block clusters of `cs` CTAs along x (grid.x = number of clusters * cs).
-template <class... KArgs, class... Args>
-static cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cs,
-                                  Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = cs > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
-// CTAs per slice of the landmark-sized kernels for more than 64 landmarks when their products run on
-// the tensor cores (a thread-block cluster shares every product by output columns): eight if the
-// device can hold a cluster of eight for every slice at once (each CTA takes an SM to itself, and
-// a cluster must fit into one GPC), else four.  FNB_MID_CLUSTER in the environment at load fixes the
-// size (1, 2, 4 or 8; kept for A/B measurements).
-template <class... KArgs>
-static int mid_cluster_size(void (*kern)(KArgs...), int64_t slices, int device) {
-  static const int forced = [] {
-    const char* e = getenv("FNB_MID_CLUSTER");
-    const int v = e ? atoi(e) : 0;
-    return (v == 1 || v == 2 || v == 4 || v == 8) ? v : 0;
-  }();
-  if (forced) return forced;
-  static std::mutex mu;
-  static std::map<std::pair<const void*, int>, int> fit8;   // (kernel, device) -> clusters of eight that fit at once
-  std::lock_guard<std::mutex> lock(mu);
-  auto key = std::make_pair((const void*)kern, device);
-  auto it = fit8.find(key);
-  if (it == fit8.end()) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(8 * 64); cfg.blockDim = dim3(kMidTcThreads); cfg.dynamicSmemBytes = kTcGemmSmem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 8; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-    it = fit8.emplace(key, n).first;
-  }
-  return slices <= it->second ? 8 : 4;
-}
-
-// The Newton-Schulz kernels for num_landmarks <= 64 run on the tensor cores (three-term bf16
+// The Newton-Schulz kernels run on the tensor cores (three-term bf16
 // split, FP32-equivalent) unless the caller forces the CUDA-core path or FNB_NS_CUDA_CORES=1 is
 // set in the environment (kept for A/B measurements).
 static bool ns_on_tensor_cores(uint32_t flags) {
@@ -476,13 +433,22 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   float* land = S.on() ? S.xfer : w.land_partial;
   const int l2 = l2_mode();
   const int ef = (l2 & 2) ? 1 : 0, el = (l2 & 16) ? 2 : 0;
+  // More than 64 landmarks: the pseudoinverse takes a cluster of two SMs per slice for longer than the column
+  // pass lasts, so up to a quarter of the SMs' worth of slices the two run side by side, the column pass on the
+  // SMs that are left.  Four more stay free: a cluster needs both its SMs in one GPC.
+  const bool mid_tc = !smem_ns && ns_on_tensor_cores(a.shape.flags);
+  const bool side_mid = mid_tc && (use_tc || use_sx) && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
   tc::TcSched sch_fb = sch, sch_fc = sch;
+  if (side_mid) {
+    sch_fb = tc::make_sched(p.BH, p.N, (use_tc ? tc_ctas_per_sm(p.D) : 1) * (sms - 2 * (int)p.BH - 4));
+    sch_fb.seg_N = seg_N; sch_fb.row_offset = row_offset; sch_fb.H = big.map_h();
+  }
   sch_fb.order = (l2 & 32) ? tc::kOrderStrided : 0;
   sch_fb.hint = hint_bits(ef, ef, 0, 0);                 // K (left in L2 by the pooling pass) and V die here
   sch_fc.order = (l2 & 1) ? tc::kOrderStrided : 0;
   sch_fc.hint = hint_bits(el, 0, ef, 0);                 // Q is read again by the backward; O is not
   sch_fc.test_drop = (a.shape.flags & FNB_FLAG_TEST_DROP_LOAD) ? 1 : 0;
-  const int nchunk_b = (use_tc || use_sx) ? sch.nchunk : p.nchunk;
+  const int nchunk_b = (use_tc || use_sx) ? sch_fb.nchunk : p.nchunk;
   const size_t md_all = (size_t)p.BH * p.m * p.D, m_all = (size_t)p.BH * p.m;
 
   if (S.run(0)) {
@@ -518,12 +484,12 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
                                                                                                 : combine2_kernel<8>;
 
   if (S.run(1)) {
-  Fork fork(st, a.device, smem_ns && !L.prof && allow_inner_fork);   // side stream for the pseudoinverse (off while profiling)
+  Fork fork(st, a.device, side_mid || (smem_ns && !L.prof && allow_inner_fork));   // side stream for the pseudoinverse (off while profiling)
   // With the tensor-core kernels the landmarks are formed from the raw segment sums inside their
   // two consumers (the Newton-Schulz forward writes the FP32 copies, the column pass packs its own
   // 16-bit operand), so the finalize kernel is skipped.
   const bool fused_landmarks = smem_ns && use_tc && p.D == 64 && ns_on_tensor_cores(a.shape.flags);
-  if (smem_ns) {
+  if (smem_ns || mid_tc) {
     if (!fused_landmarks) {
     L.begin();
     {
@@ -538,6 +504,15 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
     // The pseudoinverse only feeds the combine step, so it runs beside the column pass.
     cudaStream_t ns_stream = fork.begin();
     L.begin();
+    if (mid_tc) {
+      mx::FwdParams mp;
+      mp.qt = a.q_landmarks; mp.kt = a.k_landmarks; mp.k2 = a.k2; mp.lse2 = a.lse2; mp.iterates = a.ns_iterates;
+      mp.k2inv = a.k2_inv; mp.scratch = reinterpret_cast<uint8_t*>(w.pinv); mp.m = p.m; mp.D = p.D; mp.J = p.J;
+      mp.kappa = a.shape.kappa_star; mp.status = a.device_status;
+      if (int rc = set_smem(mx::mx_fwd_kernel, mx::kSmem, max_smem, "mid_fwd")) return rc;
+      mx::mx_fwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, ns_stream>>>(mp);
+      if (L.end("mid_fwd")) return L.status;
+    } else {
     ns::NsFwdParams np;
     np.qt = a.q_landmarks; np.kt = a.k_landmarks; np.k2 = a.k2; np.lse2 = a.lse2;
     np.iterates = a.ns_iterates; np.k2inv = a.k2_inv; np.m = p.m; np.D = p.D; np.J = p.J;
@@ -552,6 +527,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       ns::ns_fwd_kernel<<<(unsigned)p.BH, kThreads, ns::kFwdSmem, ns_stream>>>(np);
     }
     if (L.end("ns_fwd")) return L.status;
+    }
     fork.end();
   } else {
     L.begin();
@@ -561,21 +537,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
     mp.iterates = a.ns_iterates; mp.k2inv = a.k2_inv; mp.scratch = w.pinv;
     mp.BH = p.BH; mp.N = seg_N; mp.m = p.m; mp.D = p.D; mp.J = p.J;
     mp.kappa = a.shape.kappa_star; mp.scale = scale;
-    mp.landmarks_only = 0;
-    mp.qt16 = use_tc ? w.qt16 : nullptr; mp.dtype = a.shape.dtype; mp.MP = MP;
-    mp.qt16_mul = scale * tc::kLog2e;
-    // products on the tensor cores unless the caller forces the CUDA-core path
-    mp.use_tc = (a.shape.flags & FNB_FLAG_FORCE_GENERIC) ? 0 : 1;
-    mp.status = a.device_status;
-    const size_t mid_smem = mp.use_tc ? kTcGemmSmem : 0;
-    if (mp.use_tc)
-      if (int rc = set_smem(mid_fwd_kernel, mid_smem, max_smem, "mid_fwd")) return rc;
-    if (mp.use_tc) {
-      const int cs = mid_cluster_size(mid_fwd_kernel, p.BH, a.device);
-      FNB_CUDA(launch_cluster(mid_fwd_kernel, dim3((unsigned)(p.BH * cs)), dim3(kMidTcThreads), mid_smem, st, cs, mp));
-    } else {
-      mid_fwd_kernel<<<(unsigned)p.BH, kThreads, mid_smem, st>>>(mp);
-    }
+    mid_fwd_kernel<<<(unsigned)p.BH, kThreads, 0, st>>>(mp);
     if (L.end("mid_fwd")) return L.status;
   }
 
@@ -592,7 +554,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
         auto kern = tc::tc_fwd_b_kernel<T, D, MPc>;
         size_t smem = tc::FwdBSmem<D, MPc>::kBytes;
         if (int rc2 = set_smem(kern, smem, max_smem, "tc_fwd_b")) return rc2;
-        launch_pdl(kern, dim3((unsigned)(p.BH * sch.nchunk)), dim3(tc::kTcThreads), smem, st,
+        launch_pdl(kern, dim3((unsigned)(p.BH * sch_fb.nchunk)), dim3(tc::kTcThreads), smem, st,
             tm_k, tm_v, tm_qt, fused_landmarks ? land : (const float*)nullptr, lmC, p.BH, scale, w.part_acc, w.part_max,
             w.part_sum, sch_fb, p.m, a.device_status);
         return L.end("tc_fwd_b");
@@ -607,8 +569,8 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       auto kern = sx::sx_fwd_b_kernel<T, D, MPc>;
       constexpr size_t smem = sx::Plan<T, D, MPc>::kFwdB;
       if (int rc2 = set_smem(kern, smem, max_smem, "sx_fwd_b")) return rc2;
-      launch_pdl(kern, dim3((unsigned)(p.BH * sch.nchunk)), dim3(sx::kThr), smem, st, (const T*)a.k, (const T*)a.v, a.q_landmarks,
-                 w.part_acc, w.part_max, w.part_sum, sch, p.m, scale, a.device_status);
+      launch_pdl(kern, dim3((unsigned)(p.BH * sch_fb.nchunk)), dim3(sx::kThr), smem, st, (const T*)a.k, (const T*)a.v, a.q_landmarks,
+                 w.part_acc, w.part_max, w.part_sum, sch_fb, p.m, scale, a.device_status);
       return L.end("sx_fwd_b");
     });
     if (rc) return rc;
@@ -751,9 +713,13 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
   // the Newton-Schulz kernel on a side stream with one SM per slice, the column pass on the rest.
   // Off while profiling (kernels are timed one by one).
   const bool side_ns = fused_mid && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
+  // With more than 64 landmarks the same holds where the column pass parks its tiles (the other passes need dKt
+  // inside the column pass): two SMs per slice for the pseudoinverse backward, four more kept free for its clusters.
+  const bool mid_tc = !smem_ns && ns_on_tensor_cores(a.shape.flags);
+  const bool side_mid = mid_tc && use_tc && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
   tc::TcSched sch_b = sch;
-  if (side_ns) {
-    sch_b = tc::make_sched(p.BH, p.N, 2 * (sms - (int)p.BH));
+  if (side_ns || side_mid) {
+    sch_b = tc::make_sched(p.BH, p.N, side_ns ? 2 * (sms - (int)p.BH) : tc_ctas_per_sm(p.D) * (sms - 2 * (int)p.BH - 4));
     sch_b.seg_N = seg_N; sch_b.row_offset = row_offset; sch_b.H = big.map_h();
   }
   int kshift = 0;
@@ -847,7 +813,7 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
 
   // ---- landmark-sized middle ------------------------------------------------------------------
   if (S.run(1)) {
-  Fork fork(st, a.device, side_ns);
+  Fork fork(st, a.device, side_ns || side_mid);
   if (smem_ns) {
     if (!fused_mid) {
     L.begin();
@@ -916,6 +882,38 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       if (int rc = set_smem(colpass_operands_kernel, (size_t)kColpassOperandSmem, max_smem, "colpass_operands")) return rc;
       launch_pdl(colpass_operands_kernel, dim3((unsigned)p.BH), dim3(kThreads), (size_t)kColpassOperandSmem, st, cp);
     }
+  } else if (mid_tc) {
+    const float* sums = partA_src;
+    if (partA_chunks > 1) {
+      L.begin();
+      reduce_chunks(partA_src, partA_chunks, 2 * p.m * p.D, w.partA_red);
+      if (L.end("reduce_partA")) return L.status;
+      sums = w.partA_red;
+    }
+    mx::BwdParams mp;
+    memset(&mp, 0, sizeof(mp));
+    mp.sums = sums; mp.qt = a.q_landmarks; mp.kt = a.k_landmarks; mp.k2 = a.k2; mp.iterates = a.ns_iterates;
+    mp.k2inv = a.k2_inv; mp.bmat = a.bmat; mp.dO3 = w.dO3; mp.D3 = w.D3; mp.dqt_ns = w.dqt_ns; mp.dkt_tot = w.dkt_tot;
+    mp.rows_k = use_tc ? w.rows_k : nullptr; mp.scratch = reinterpret_cast<uint8_t*>(w.pinv); mp.m = p.m; mp.D = p.D; mp.J = p.J;
+    mp.kappa = a.shape.kappa_star; mp.scale = scale; mp.N = seg_N; mp.status = a.device_status;
+    if (int rc = set_smem(mx::mx_bwd_kernel, mx::kSmem, max_smem, "mid_bwd")) return rc;
+    mp.head = 1; mp.tail = side_mid ? 0 : 1;
+    L.begin();
+    mx::mx_bwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, st>>>(mp);
+    if (L.end("mid_bwd")) return L.status;
+    if (side_mid) {
+      mp.head = 0; mp.tail = 1;
+      mx::mx_bwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, fork.begin()>>>(mp);
+      fork.end();
+    }
+    if (use_tc) {
+      L.begin();
+      MidPackParams pp;
+      pp.dO3 = w.dO3; pp.q_landmarks = a.q_landmarks; pp.do3n = do3n; pp.do3_scale = w.do3_scale; pp.qt16 = qt16;
+      pp.m = p.m; pp.D = p.D; pp.MP = MP; pp.dtype = a.shape.dtype; pp.qt_mul = scale * tc::kLog2e;
+      mid_pack_kernel<<<dim3((unsigned)p.BH, kMidPackSplit), kThreads, 0, st>>>(pp);
+      if (L.end("mid_pack")) return L.status;
+    }
   } else {
     L.begin();
     {
@@ -925,30 +923,10 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       mp.k2inv = a.k2_inv; mp.bmat = a.bmat;
       mp.dstep2 = w.dstep2; mp.dkt_a = w.dkt_a; mp.dO3 = w.dO3; mp.D3 = w.D3;
       mp.dqt_ns = w.dqt_ns; mp.dkt_tot = w.dkt_tot; mp.G = w.G; mp.dK2 = w.dK2; mp.scratch = w.pinv;
-      mp.m = p.m; mp.D = p.D; mp.J = p.J; mp.kappa = a.shape.kappa_star; mp.first_half_only = 0;
-      mp.use_tc = (a.shape.flags & FNB_FLAG_FORCE_GENERIC) ? 0 : 1;
-      mp.status = a.device_status;
-      const size_t mid_smem = mp.use_tc ? kTcGemmSmem : 0;
-      if (mp.use_tc)
-        if (int rc = set_smem(mid_bwd_kernel, mid_smem, max_smem, "mid_bwd")) return rc;
-      if (mp.use_tc && !mp.first_half_only) {
-        const int cs = mid_cluster_size(mid_bwd_kernel, p.BH, a.device);
-        FNB_CUDA(launch_cluster(mid_bwd_kernel, dim3((unsigned)(p.BH * cs)), dim3(kMidTcThreads), mid_smem, st, cs, mp));
-      } else {
-        mid_bwd_kernel<<<(unsigned)p.BH, kThreads, mid_smem, st>>>(mp);
-      }
+      mp.m = p.m; mp.D = p.D; mp.J = p.J; mp.kappa = a.shape.kappa_star;
+      mid_bwd_kernel<<<(unsigned)p.BH, kThreads, 0, st>>>(mp);
     }
     if (L.end("mid_bwd")) return L.status;
-    if (use_tc) {
-      // what the tensor-core column pass and the in-place pass need from the middle stage
-      L.begin();
-      MidPackParams pp;
-      pp.dO3 = w.dO3; pp.q_landmarks = a.q_landmarks; pp.dkt_tot = w.dkt_tot; pp.do3n = do3n; pp.do3_scale = w.do3_scale;
-      pp.qt16 = qt16; pp.rows_k = w.rows_k; pp.m = p.m; pp.D = p.D; pp.MP = MP; pp.dtype = a.shape.dtype;
-      pp.qt_mul = scale * tc::kLog2e; pp.scale = scale; pp.N = seg_N;
-      mid_pack_kernel<<<dim3((unsigned)p.BH, kMidPackSplit), kThreads, 0, st>>>(pp);
-      if (L.end("mid_pack")) return L.status;
-    }
   }
 
   // ---- pass B ---------------------------------------------------------------------------------
@@ -968,7 +946,7 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
         size_t sm = tc::BwdBSmem<D, MPc>::kBytes;
         if (int rc2 = set_smem(kern, sm, max_smem, "tc_bwd_b")) return rc2;
         const dim3 bgrid((unsigned)(p.BH * sch_b.nchunk));
-        if (side_ns)   // an ordinary launch: it must not claim SMs before the Newton-Schulz kernel has its own
+        if (side_ns || side_mid)   // an ordinary launch: it must not claim SMs before the Newton-Schulz kernel has its own
           kern<<<bgrid, tc::kTcThreads, sm, st>>>(tm_k, tm_v, tm_qt, tm_do3, tm_dk, tm_dv, a.lse3, w.D3, w.do3_scale, w.partB,
                                                   w.tile_scale, sch_b, p.m, scale, kshift, a.device_status);
         else
@@ -1260,7 +1238,11 @@ int fnb_sp_backward(const fnb_bwd_args* a, const fnb_sp_info* sp) {
 
 size_t fnb_debug_pinv_workspace_bytes(int64_t bh, int32_t m) {
   if (bh <= 0 || m < 1 || m > kMaxM) return 0;
-  return align256((size_t)bh * kPinvBwdBufs * m * m * sizeof(float));
+  return align256(m > ns::kN ? (size_t)bh * mx::kBwdScratchBytes + 256 : (size_t)bh * kPinvBwdBufs * m * m * sizeof(float));
+}
+// the images are copied in bulk: 16-byte aligned wherever the caller's workspace starts
+static uint8_t* pinv_scratch(void* ws) {
+  return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~(uintptr_t)255);
 }
 
 static int check_pinv_args(int64_t bh, int32_t m, int32_t J, float kappa, const void* ws,
@@ -1286,19 +1268,20 @@ int fnb_debug_pinv_forward(int64_t bh, int32_t m, int32_t J, float kappa, const 
                                   (int)nstc::kFwdSmem));
     nstc::ns_pinv_fwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kFwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, k2_inv, m, J, kappa, nullptr);
+  } else if (m > ns::kN && ns_on_tensor_cores(0)) {
+    mx::FwdParams mp;
+    memset(&mp, 0, sizeof(mp));
+    mp.k2 = const_cast<float*>(k2);      // (given softmaxed: only read)
+    mp.iterates = ns_iterates; mp.k2inv = k2_inv; mp.scratch = pinv_scratch(workspace); mp.m = m; mp.J = J; mp.kappa = kappa;
+    FNB_CUDA(cudaFuncSetAttribute(mx::mx_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
+    mx::mx_fwd_kernel<<<(unsigned)(2 * bh), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
   } else if (m <= ns::kN) {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_fwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kFwdSmem));
     ns::ns_pinv_fwd_debug_kernel<<<(unsigned)bh, kThreads, ns::kFwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, k2_inv, m, J, kappa);
   } else {
-    const int use_tc = ns_on_tensor_cores(0) ? 1 : 0;
-    if (use_tc)
-      FNB_CUDA(cudaFuncSetAttribute(pinv_fwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcGemmSmem));
-    const int cs = use_tc ? mid_cluster_size(pinv_fwd_debug_kernel, bh, device) : 1;
-    FNB_CUDA(launch_cluster(pinv_fwd_debug_kernel, dim3((unsigned)(bh * cs)), dim3(use_tc ? kMidTcThreads : kThreads),
-                            use_tc ? kTcGemmSmem : 0, (cudaStream_t)stream, cs, k2, ns_iterates, k2_inv, (float*)workspace, m,
-                            J, kappa, use_tc));
+    pinv_fwd_debug_kernel<<<(unsigned)bh, kThreads, 0, (cudaStream_t)stream>>>(k2, ns_iterates, k2_inv, (float*)workspace, m, J, kappa);
   }
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
@@ -1316,19 +1299,20 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
                                   (int)nstc::kBwdSmem));
     nstc::ns_pinv_bwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa, nullptr, nullptr, nullptr);
+  } else if (m > ns::kN && ns_on_tensor_cores(0)) {
+    mx::BwdParams mp;
+    memset(&mp, 0, sizeof(mp));
+    mp.k2 = k2; mp.iterates = ns_iterates; mp.G = d_k2_inv; mp.dK2 = d_k2; mp.scratch = pinv_scratch(workspace); mp.m = m; mp.J = J;
+    mp.kappa = kappa; mp.tail = 1;
+    FNB_CUDA(cudaFuncSetAttribute(mx::mx_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
+    mx::mx_bwd_kernel<<<(unsigned)(2 * bh), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
   } else if (m <= ns::kN) {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_bwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kBwdSmem));
     ns::ns_pinv_bwd_debug_kernel<<<(unsigned)bh, kThreads, ns::kBwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa);
   } else {
-    const int use_tc = ns_on_tensor_cores(0) ? 1 : 0;
-    if (use_tc)
-      FNB_CUDA(cudaFuncSetAttribute(pinv_bwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcGemmSmem));
-    const int cs = use_tc ? mid_cluster_size(pinv_bwd_debug_kernel, bh, device) : 1;
-    FNB_CUDA(launch_cluster(pinv_bwd_debug_kernel, dim3((unsigned)(bh * cs)), dim3(use_tc ? kMidTcThreads : kThreads),
-                            use_tc ? kTcGemmSmem : 0, (cudaStream_t)stream, cs, k2, ns_iterates, d_k2_inv, d_k2,
-                            (float*)workspace, m, J, kappa, use_tc));
+    pinv_bwd_debug_kernel<<<(unsigned)bh, kThreads, 0, (cudaStream_t)stream>>>(k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa);
   }
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
@@ -1386,10 +1370,6 @@ int fnb_pinv_backward_noalloc(int64_t bh, int32_t m, int32_t J, float kappa, con
 __attribute__((visibility("default"))) int fnb_debug_tc_trace(long long* out, int cta) {
   if (cta >= 0) { cudaMemcpyToSymbol(tc::g_tc_trace_cta, &cta, sizeof(int)); return 0; }
   return cudaMemcpyFromSymbol(out, tc::g_tc_trace, sizeof(long long) * 8 * 256) == cudaSuccess ? 0 : -1;
-}
-__attribute__((visibility("default"))) int fnb_debug_gemm_cycles(unsigned long long* out, int reset) {
-  if (reset) { unsigned long long z[8] = {}; return cudaMemcpyToSymbol(g_gemm_cycles, z, sizeof(z)) == cudaSuccess ? 0 : -1; }
-  return cudaMemcpyFromSymbol(out, g_gemm_cycles, sizeof(unsigned long long) * 8) == cudaSuccess ? 0 : -1;
 }
 __attribute__((visibility("default"))) int fnb_debug_tc_span(unsigned long long* out) {
   return cudaMemcpyFromSymbol(out, tc::g_tc_span, sizeof(unsigned long long) * 6 * 1024) == cudaSuccess ? 0 : -1;

@@ -1,0 +1,904 @@
+// Landmark-sized stages for 64 < num_landmarks <= 128 on the sm_100a tensor cores, FP32-equivalent: a
+// thread-block cluster of two CTAs per (b,h) slice works through the softmax-2, ridge and Newton-Schulz
+// products (forward and exact backward) of mid_kernels.cuh.
+//
+// Every matrix that is an operand exists once as an "image" in global memory (it stays in L2): three bf16
+// terms x = x0 + x1 + x2 (24 significant bits), padded with zeros to 128 x 128, already in the 128-byte
+// swizzle the tensor core reads, [64-column block][term][128 rows x 128 B].  The epilogue that forms a result
+// splits it once and writes its image; a consumer's operands are plain bulk copies into a ring of shared-
+// memory stages, K in chunks of 64, in whichever orientation the product needs (an image serves as left or
+// right operand, plain or transposed, by the pieces that are copied and the descriptor they are read
+// with).  CTA `rank` of the pair forms the 64 output columns [64 rank, 64 rank + 64) of every product; the
+// terms of the right operand are stacked along N, so a K step of 16 is three MMAs,
+//     x0 [y0 | y1 | y2],  x1 [y0 | y1],  x2 [y0],
+// into three column groups by weight that the epilogue adds (small ones first).
+// 16 compute warps (epilogues and element-wise phases), one warp that copies, one that issues MMAs; all run
+// through the same program.  A phase ends with an arrival of all warps of both CTAs on both CTAs'
+// `ready` barriers; operands that are older than the last phase are copied ahead of it.  All waits are
+// bounded; control flow never depends on them.
+//
+// What bounds it: the latency of a phase, about 9000 cycles with one product (result block out to L2 2000-2400,
+// meeting the peer 800, first chunk in 1550, MMAs 2400, accumulator out and split 2300), not the 144 KB a CTA copies
+// per product.  Clusters of four or eight that copied FP32 operands and split them in every CTA took, on a B200 at
+// B=2, H=8 (us, before / now): forward D=128, J=8 with ridge 326 / 203, D=64, J=6 without 234 / 147; backward
+// 651 / 406 and 478 / 290; per iteration 37 / 19 and 70 / 36.
+#pragma once
+#include "common.cuh"
+#include "small_kernels.cuh"
+#include "split_stream.cuh"
+#include "tc_common.cuh"
+
+namespace fnb {
+namespace mx {
+
+using namespace tc;
+
+constexpr int kTermBytes = 128 * 128;          // 128 rows x 64 columns of one term
+constexpr int kBlockBytes = 3 * kTermBytes;    // a 64-column block of an image
+constexpr int kImg = 2 * kBlockBytes;
+constexpr int kStages = 2;
+constexpr int kStageBytes = kBlockBytes + kBlockBytes / 2;   // left chunk (128 x 64) and right chunk (64 x 64), all terms
+constexpr int kComputeWarps = 16;
+constexpr int kThr = 32 * (kComputeWarps + 2);
+constexpr int kRedFloats = 17 * kMaxM;
+constexpr size_t kSmem = (size_t)kStages * kStageBytes + kBlockBytes + kRedFloats * sizeof(float) + 128 + 1024;
+constexpr int kAccCols = 192;                  // tensor-memory columns of one accumulator
+constexpr int kF32 = kMaxM * kMaxM;            // floats of one FP32 scratch matrix
+
+// per-slice scratch: images, then FP32 matrices
+enum FwdImg { kFK2, kFA, kFZ0, kFZ1, kFM, kFV, kFT, kFwdImgs };
+constexpr size_t kFwdScratchBytes = (size_t)kFwdImgs * kImg + kF32 * sizeof(float);
+enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBdZ0, kBdZ1, kBM, kBV, kBT, kBdT, kBdV, kBdM, kBwdImgs };
+enum BwdF32 { kGA, kGdZ, kGdK, kGg, kBwdF32s };
+constexpr size_t kBwdScratchBytes = (size_t)kBwdImgs * kImg + (size_t)kBwdF32s * kF32 * sizeof(float);
+
+enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
+
+struct Shared {
+  uint64_t full[kStages], empty[kStages], done[2], ready;
+  uint32_t tmem_slot;
+  int abort_word;
+};
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// One arrival on this CTA's barrier and one on the peer's.  The remote one is relaxed: whoever has written
+// something the peer reads has fenced it before.
+__device__ __forceinline__ void arrive_both(uint64_t* bar, int rank) {
+  uint32_t ra;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(bar)), "r"(rank ^ 1));
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(ra) : "memory");
+  mbar_arrive(bar);
+}
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, const Abort& ab, int where) {
+  uint64_t t0 = 0;
+  for (uint32_t spin = 0;; ++spin) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    if (ok) return true;
+    if ((spin & 63u) == 63u) {
+      if (ab.raised()) return false;
+      const uint64_t now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > g_wait_limit_ns) break;
+    }
+  }
+  ab.raise(where);
+  return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const uint8_t* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(uint8_t* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void compute_sync() { named_barrier(1, 32 * kComputeWarps); }
+
+// 16 values, columns 16 seg .. 16 seg + 15 of row r (seg counts over both column blocks) -> image
+__device__ __forceinline__ void put16(uint8_t* img, int r, int seg, const float* v) {
+  uint4 a[3], b[3];
+  sx::split8<3>(v, a);
+  sx::split8<3>(v + 8, b);
+  const int cg = seg & 3, odd = r & 1;
+  uint8_t* p = img + (seg >> 2) * kBlockBytes + r * 128 + (((2 * cg) ^ (r & 6)) << 4);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const uint4 lo = odd ? b[t] : a[t], hi = odd ? a[t] : b[t];
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + t * kTermBytes), "r"(lo.x), "r"(lo.y),
+                 "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
+                 : "memory");
+  }
+}
+// 4 values, columns 4 lane .. 4 lane + 3 of row r -> image (a warp writes a whole row)
+__device__ __forceinline__ void put_row(uint8_t* img, int r, int lane, const float* v) {
+  uint8_t* p = img + (lane >> 4) * kBlockBytes + sw128_offset(r, (lane >> 1) & 7) + (lane & 1) * 8;
+  float a[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const uint32_t w0 = pack2<__nv_bfloat16>(a[0], a[1]), w1 = pack2<__nv_bfloat16>(a[2], a[3]);
+    *reinterpret_cast<uint2*>(p + t * kTermBytes) = make_uint2(w0, w1);
+    a[0] -= __uint_as_float(w0 << 16); a[1] -= __uint_as_float(w0 & 0xffff0000u);
+    a[2] -= __uint_as_float(w1 << 16); a[3] -= __uint_as_float(w1 & 0xffff0000u);
+  }
+}
+// n consecutive values of an FP32 row (zero past `cols`); n a multiple of 4
+template <int n>
+__device__ __forceinline__ void get_row(const float* g, int c0, int cols, bool row_ok, float* v) {
+  const float* src = g + c0;
+  if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0 && (cols & 3) == 0) {
+#pragma unroll
+    for (int q = 0; q < n; q += 4) {
+      const float4 x = (row_ok && c0 + q < cols) ? __ldcg(reinterpret_cast<const float4*>(src + q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[q] = x.x; v[q + 1] = x.y; v[q + 2] = x.z; v[q + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < n; ++i) v[i] = (row_ok && c0 + i < cols) ? __ldcg(src + i) : 0.f;
+  }
+}
+template <int n>
+__device__ __forceinline__ void set_row(float* g, int c0, int cols, bool row_ok, const float* v) {
+  if (!row_ok) return;
+  float* dst = g + c0;
+  if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0 && (cols & 3) == 0) {
+#pragma unroll
+    for (int q = 0; q < n; q += 4)
+      if (c0 + q < cols) *reinterpret_cast<float4*>(dst + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+      if (c0 + i < cols) dst[i] = v[i];
+  }
+}
+
+// One role's walk through the program.
+template <int R>
+struct Role {
+  Shared* sh;
+  uint8_t* ring;
+  uint8_t* out;       // compute: staging of one result block, [term][128 rows x 128 B]
+  float* red;
+  uint32_t tmem;
+  Abort ab;
+  int rank, lane;
+  bool failed, pend;
+  uint32_t rphase;
+  // copy / issue: position in the ring
+  int stage;
+  uint32_t sphase, fills;   // fills: eight bits per stage (newton_iter <= 20: at most 160 fills of a stage)
+  // compute: accumulator row, column segment of 16 (over both blocks), completion parities
+  int row, seg;
+  uint32_t dphase[2];
+
+  __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status) {
+    sh = s; ring = r; out = r + (size_t)kStages * kStageBytes; red = rd; rank = rk; lane = threadIdx.x & 31;
+    tmem = s->tmem_slot;
+    ab = Abort{&s->abort_word, status};
+    failed = pend = false;
+    rphase = sphase = fills = 0; stage = 0;
+    dphase[0] = dphase[1] = 0;
+    const int w = threadIdx.x >> 5;
+    row = (w & 3) * 32 + lane;
+    seg = rank * 4 + (w >> 2);
+  }
+  // the phase published last is complete in both CTAs (and, for a compute warp that asks, what the peer's
+  // compute warps wrote with ordinary stores can be read)
+  __device__ __forceinline__ void ensure(bool read_peer = true) {
+    if (R == kCompute && read_peer && !pend) __threadfence();
+    if (!pend) return;
+    pend = false;
+    if (R == kCompute || lane == 0) {
+      if (!wait_cluster(&sh->ready, rphase, ab, 0x6000 + R)) failed = true;
+      if (R == kProducer) fence_proxy_async_all();
+      if (R == kCompute && read_peer) __threadfence();
+    }
+    if (R == kIssuer) tc_fence_after();
+    rphase ^= 1u;
+  }
+  // This warp's part of the phase is done.  Images written through put() are complete; with `plain` so are the
+  // ordinary global stores of the phase, for readers of either kind.
+  __device__ __forceinline__ void publish(bool plain) {
+    ensure(false);
+    if (R == kCompute) {
+      if (threadIdx.x < 128 && lane == 0) tma_store_wait_all();
+      if (plain || (threadIdx.x < 128 && lane == 0)) {
+        fence_proxy_async_all();
+        __threadfence();
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+    if (lane == 0) arrive_both(&sh->ready, rank);
+    pend = true;
+  }
+  // The result block of this CTA (this thread: row, 16 columns) -> image.  The four warps that hold the same 32
+  // rows stage their 4 KB per term, which one thread stores in bulk: stored straight from the accumulator layout
+  // (32 rows x 32 B per instruction) the block took 3300 cycles and its fence 2000.
+  __device__ __forceinline__ void put(uint8_t* img, const float* v) {
+    const int q = (threadIdx.x >> 5) & 3;
+    const bool storing = threadIdx.x < 128 && lane == 0;
+    if (storing) tma_store_wait_read();
+    named_barrier(2 + q, 128);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint4 a[3];
+      sx::split8<3>(v + 8 * c, a);
+      uint8_t* p = out + sw128_offset(row, (seg & 3) * 2 + c);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) *reinterpret_cast<uint4*>(p + t * kTermBytes) = a[t];
+    }
+    fence_proxy_async();
+    named_barrier(2 + q, 128);
+    if (storing) {
+      uint8_t* dst = img + rank * kBlockBytes + q * 4096;
+#pragma unroll
+      for (int t = 0; t < 3; ++t) bulk_store(dst + t * kTermBytes, smem_u32(out) + t * kTermBytes + q * 4096, 4096);
+      tma_store_commit();
+    }
+  }
+  // accumulator `acc` (+)= op(X) op(Y)[:, own columns].  fx, fy: the operand was written in the last phase.
+  template <bool LT, bool RT>
+  __device__ __forceinline__ void product(const uint8_t* X, bool fx, const uint8_t* Y, bool fy, int kchunks, int acc, bool accumulate) {
+    if (R == kProducer) {
+      if (lane == 0) {
+        for (int kc = 0; kc < kchunks; ++kc) {
+          if (!mbar_wait(&sh->empty[stage], sphase ^ 1u, ab, 0x6010)) failed = true;
+          if (!failed) mbar_expect_tx(&sh->full[stage], kStageBytes);
+          const uint32_t l = smem_u32(ring) + stage * kStageBytes, r = l + kBlockBytes;
+          if (!fx && !failed) load_left<LT>(l, X, kc);
+          if (!fy && !failed) load_right<RT>(r, Y, kc);
+          if (pend && (fx || fy)) {
+            if (!wait_cluster(&sh->ready, rphase, ab, 0x6011)) failed = true;
+            fence_proxy_async_all();
+            rphase ^= 1u;
+            pend = false;
+          }
+          if (fx && !failed) load_left<LT>(l, X, kc);
+          if (fy && !failed) load_right<RT>(r, Y, kc);
+          if (!failed) fills += 1u << (8 * stage);       // (counts modulo 256: only the parity is used)
+          advance();
+        }
+      }
+    } else if (R == kIssuer) {
+      if (lane == 0) {
+        ensure();
+        const uint32_t d = tmem + acc * kAccCols;
+        for (int kc = 0; kc < kchunks; ++kc) {
+          if (!failed && !mbar_wait(&sh->full[stage], sphase, ab, 0x6020)) failed = true;
+          if (!failed) {
+            tc_fence_after();
+            const uint32_t l = smem_u32(ring) + stage * kStageBytes, r = l + kBlockBytes;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const uint64_t b = RT ? smem_desc_sw128(r + k * 32, 16, 1024) : smem_desc_sw128(r + k * 2048, kTermBytes / 2, 1024);
+#pragma unroll
+              for (int t = 0; t < 3; ++t) {
+                const uint32_t lt = l + t * kTermBytes;
+                const uint64_t a = LT ? smem_desc_sw128(lt + k * 2048, kTermBytes / 2, 1024) : smem_desc_sw128(lt + k * 32, 16, 1024);
+                umma(d + 64 * t, a, b, make_idesc<__nv_bfloat16>(128, 64 * (3 - t), LT, !RT),
+                     (accumulate || kc > 0 || k > 0 || t > 0) ? 1u : 0u);
+              }
+            }
+            umma_commit(&sh->empty[stage]);
+          }
+          advance();
+        }
+      } else {
+        if (pend) { pend = false; rphase ^= 1u; }
+      }
+    }
+  }
+  __device__ __forceinline__ void advance() {
+    if (++stage == kStages) { stage = 0; sphase ^= 1u; }
+  }
+  template <bool LT>
+  __device__ __forceinline__ void load_left(uint32_t dst, const uint8_t* X, int kc) {
+    if (!LT) {
+      bulk_load(dst, X + (size_t)kc * kBlockBytes, kBlockBytes, &sh->full[stage]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int cb = 0; cb < 2; ++cb)
+          bulk_load(dst + t * kTermBytes + cb * (kTermBytes / 2), X + (size_t)cb * kBlockBytes + t * kTermBytes + kc * (kTermBytes / 2),
+                    kTermBytes / 2, &sh->full[stage]);
+    }
+  }
+  template <bool RT>
+  __device__ __forceinline__ void load_right(uint32_t dst, const uint8_t* Y, int kc) {
+    const uint8_t* src = RT ? Y + (size_t)kc * kBlockBytes + rank * (kTermBytes / 2) : Y + (size_t)rank * kBlockBytes + kc * (kTermBytes / 2);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) bulk_load(dst + t * (kTermBytes / 2), src + t * kTermBytes, kTermBytes / 2, &sh->full[stage]);
+  }
+  __device__ __forceinline__ void commit(int g) {
+    if (R == kIssuer && lane == 0 && !failed) umma_commit(&sh->done[g]);
+  }
+  // compute: the 16 values of this thread (row, columns 16 seg ..) of accumulator acc once group g is complete
+  __device__ __forceinline__ void result(int g, int acc, float* v) {
+    if (!mbar_wait(&sh->done[g], dphase[g], ab, 0x6030 + g)) failed = true;
+    dphase[g] ^= 1u;
+    __syncwarp();
+    tc_fence_after();
+    const uint32_t a = tmem + (uint32_t)acc * kAccCols + ((uint32_t)(row & ~31) << 16) + (uint32_t)((seg & 3) * 16);
+    float x[16], y[16];
+    sx::ld<16>(a + 128, x);
+    sx::ld<16>(a + 64, y);
+    sx::ld<16>(a, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += x[i] + y[i];
+  }
+  __device__ __forceinline__ int col0() const { return 16 * seg; }
+  __device__ __forceinline__ void add_diag(float* v, float d, int m) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += (col0() + i == row && row < m) ? d : 0.f;
+  }
+  // (rows x cols) FP32 matrix -> this CTA's half of the rows of its image
+  __device__ __forceinline__ void convert(const float* g, int rows, int cols, uint8_t* img) {
+    const int r = rank * 64 + (threadIdx.x >> 3), s = threadIdx.x & 7;
+    if (16 * s >= 64 && cols <= 64) return;      // the second block of such an operand is never copied
+    float v[16];
+    get_row<16>(g + (size_t)r * cols, 16 * s, cols, r < rows, v);
+    put16(img, r, s, v);
+  }
+  __device__ void close() {
+    ensure();
+    if (R == kProducer && lane == 0) {      // (only after a wait gave up can a copy still be in flight here)
+#pragma unroll
+      for (int s = 0; s < kStages; ++s) {
+        const uint32_t n = (fills >> (8 * s)) & 0xffu;
+        if (failed && n) mbar_drain(&sh->full[s], (n - 1) & 1u);
+      }
+    }
+  }
+};
+
+// ||A||_1, ||A||_inf and their first-occurrence argmax positions (compute warps; A: m x m in global memory)
+struct Norms { float n1, ninf; int jc, ir; };
+__device__ inline Norms norms(const float* A, int m, float* red) {
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  float* rowsum = red;
+  float* colpart = red + kMaxM;
+  float cs[4] = {0.f, 0.f, 0.f, 0.f};
+  float x[kMaxM / kComputeWarps][4];      // every load in flight at once
+#pragma unroll
+  for (int i = 0; i < kMaxM / kComputeWarps; ++i) {
+    const int r = w + i * kComputeWarps;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[i][q] = (r < m && lane + 32 * q < m) ? fabsf(__ldcg(A + (size_t)r * m + lane + 32 * q)) : 0.f;
+  }
+#pragma unroll
+  for (int i = 0; i < kMaxM / kComputeWarps; ++i) {
+    float rs = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { cs[q] += x[i][q]; rs += x[i][q]; }
+    for (int o = 16; o > 0; o >>= 1) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+    if (lane == 0) rowsum[w + i * kComputeWarps] = rs;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) colpart[w * kMaxM + lane + 32 * q] = cs[q];
+  compute_sync();
+  if (t < m) {
+    float s = 0.f;
+#pragma unroll
+    for (int ww = 0; ww < kComputeWarps; ++ww) s += colpart[ww * kMaxM + t];
+    colpart[t] = s;           // (column t of the first partial row is read by this thread alone)
+  }
+  compute_sync();
+  // every warp finds both maxima for itself
+  float b[2];
+  int bi[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float* src = k ? rowsum : colpart;
+    float best = -1.f;
+    int at = 0;
+    for (int c = lane; c < m; c += 32)
+      if (src[c] > best) { best = src[c]; at = c; }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ob > best || (ob == best && oi < at)) { best = ob; at = oi; }
+    }
+    b[k] = best; bi[k] = at;
+  }
+  compute_sync();
+  return Norms{b[0], b[1], bi[0], bi[1]};
+}
+
+// ---- forward ------------------------------------------------------------------------------------------
+struct FwdParams {
+  const float* qt; const float* kt;       // [BH][m][D]; null: k2 is given (softmaxed)
+  float* k2; float* lse2; float* iterates; float* k2inv;
+  uint8_t* scratch;                       // [BH][kFwdScratchBytes]
+  int m, D, J;
+  float kappa;
+  int* status;
+};
+
+template <int R>
+__device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int64_t bh) {
+  constexpr bool C = R == kCompute;
+  const int m = p.m, D = p.D, mm = m * m;
+  uint8_t* base = p.scratch + bh * (int64_t)kFwdScratchBytes;
+  auto img = [&](int i) { return base + (size_t)i * kImg; };
+  float* a32 = reinterpret_cast<float*>(base + (size_t)kFwdImgs * kImg);
+  float* k2 = p.k2 + bh * mm;
+  float* iterates = p.iterates + bh * (int64_t)(p.J + 1) * mm;
+  float* k2inv = p.k2inv + bh * mm;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float v[16];
+  if (p.qt) {
+    if (C) {
+      r.convert(p.qt + bh * m * D, m, D, img(kFM));
+      r.convert(p.kt + bh * m * D, m, D, img(kFV));
+    }
+    r.publish(true);
+    r.template product<false, true>(img(kFM), true, img(kFV), true, (D + 63) / 64, 0, false);
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);
+      set_row<16>(k2 + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
+    }
+    r.publish(true);
+  }
+  if (C) {
+    r.ensure();
+    // row softmax (this CTA's half of the rows, one warp per row, four columns per lane)
+    for (int i = 0; i < 4; ++i) {
+      const int row = r.rank * 64 + 4 * w + i;
+      float x[4];
+      get_row<4>(k2 + (size_t)row * m, 4 * lane, m, row < m, x);
+      if (p.qt && row < m) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) if (4 * lane + q < m) mx = fmaxf(mx, x[q]);
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float sum = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { x[q] = 4 * lane + q < m ? expf(x[q] - mx) : 0.f; sum += x[q]; }
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) x[q] /= sum;
+        if (!r.failed) set_row<4>(k2 + (size_t)row * m, 4 * lane, m, true, x);
+        if (lane == 0) p.lse2[bh * m + row] = mx + logf(sum);
+      }
+      put_row(img(kFK2), row, lane, x);
+    }
+  }
+  r.publish(true);
+  const uint8_t* A = img(kFK2);
+  const float* A32 = k2;
+  if (p.kappa > 0.f) {
+    r.template product<true, false>(img(kFK2), true, img(kFK2), true, 2, 0, false);
+    r.commit(0);
+    if (C) {
+      r.ensure();
+      const Norms nk = norms(k2, m, r.red);
+      r.result(0, 0, v);
+      r.add_diag(v, nk.n1 * nk.ninf / p.kappa, m);
+      r.put(img(kFA), v);
+      set_row<16>(a32 + (size_t)r.row * m, r.col0(), m, r.row < m, v);
+    }
+    r.publish(true);
+    A = img(kFA);
+    A32 = a32;
+  }
+  if (C) {
+    r.ensure();
+    const Norms na = norms(A32, m, r.red);
+    const float c = fmaxf(na.n1 * na.ninf, 1e-12f);
+    // Z0 = A^T / c; lanes run along the rows of Z0 (the columns of A)
+    const int row = r.rank * 64 + (threadIdx.x & 63), s = threadIdx.x >> 6;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = (row < m && 16 * s + i < m) ? __ldcg(A32 + (size_t)(16 * s + i) * m + row) / c : 0.f;
+    put16(img(kFZ0), row, s, v);
+    set_row<16>(iterates + (size_t)row * m, 16 * s, m, row < m, v);
+  }
+  r.publish(true);
+  for (int j = 0; j < p.J; ++j) {
+    uint8_t* Z = img(kFZ0 + (j & 1));
+    uint8_t* Zn = img(kFZ0 + ((j + 1) & 1));
+    float mv[16];
+    r.template product<false, false>(A, false, Z, true, 2, 0, false);           // M = A Z
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, mv);
+      r.put(img(kFM), mv);
+    }
+    r.publish(false);
+    r.template product<false, false>(img(kFM), true, img(kFM), true, 2, 0, false);
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);                                                        // V = 15 I - M (7 I - M)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, mv[i], v[i]);
+      r.add_diag(v, 15.f, m);
+      r.put(img(kFV), v);
+    }
+    r.publish(false);
+    r.template product<false, false>(img(kFM), false, img(kFV), true, 2, 0, false);
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);                                                        // T / 4 = (13 I - M V) / 4
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
+      r.add_diag(v, 3.25f, m);
+      r.put(img(kFT), v);
+    }
+    r.publish(false);
+    r.template product<false, false>(Z, false, img(kFT), true, 2, 0, false);    // Z' = Z T / 4
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);
+      r.put(Zn, v);
+      const bool ok = r.row < m && !r.failed;
+      set_row<16>(iterates + (size_t)(j + 1) * mm + (size_t)r.row * m, r.col0(), m, ok, v);
+      if (j == p.J - 1 && !(p.kappa > 0.f)) set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, ok, v);
+    }
+    r.publish(false);
+  }
+  if (p.kappa > 0.f) {
+    r.template product<false, true>(img(kFZ0 + (p.J & 1)), true, img(kFK2), false, 2, 0, false);   // Z_J K2^T
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);
+      set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
+    }
+  }
+  r.close();
+}
+
+// ---- backward -----------------------------------------------------------------------------------------
+struct BwdParams {
+  const float* sums;          // [BH][2][m][D]: dstep2, dKt sums of the row pass
+  const float* qt; const float* kt; const float* k2; const float* iterates; const float* k2inv; const float* bmat;
+  float* dO3; float* D3;      // [BH][m][D], [BH][m]
+  float* dqt_ns; float* dkt_tot; float* rows_k;   // [BH][m][D]; rows_k (scale * dkt_tot / segment length) may be null
+  const float* G;             // debug entry: dL/dk2inv given, dK2 wanted
+  float* dK2;
+  uint8_t* scratch;           // [BH][kBwdScratchBytes]
+  int m, D, J;
+  float kappa, scale;
+  int64_t N;
+  int head, tail;             // run dO3 / D3 / dK2inv; run the pseudoinverse backward and what follows
+  int* status;
+};
+
+template <int R>
+__device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int64_t bh) {
+  constexpr bool C = R == kCompute;
+  const int m = p.m, D = p.D, mm = m * m, md = m * D, J = p.J;
+  const bool ridge = p.kappa > 0.f;
+  uint8_t* base = p.scratch + bh * (int64_t)kBwdScratchBytes;
+  auto img = [&](int i) { return base + (size_t)i * kImg; };
+  auto f32 = [&](int i) { return reinterpret_cast<float*>(base + (size_t)kBwdImgs * kImg) + (size_t)i * kF32; };
+  const float* k2 = p.k2 + bh * mm;
+  const float* iterates = p.iterates + bh * (int64_t)(J + 1) * mm;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool own_d = r.rank * 64 < D;          // this CTA has columns of an (m x D) result
+  uint8_t* Gi = ridge ? img(kBdM) : img(kBdZ0 + (J & 1));   // dL/dk2inv; without the ridge it is dL/dZ_J
+  float v[16];
+  if (p.head) {
+    const float* dstep2 = p.sums + bh * 2 * md;
+    float* dO3 = p.dO3 + bh * md;
+    if (C) {
+      r.convert(p.k2inv + bh * mm, m, m, img(kBM));
+      r.convert(dstep2, m, D, img(kBT));
+      r.convert(p.bmat + bh * md, m, D, img(kBV));
+    }
+    r.publish(true);
+    if (own_d) {
+      r.template product<true, false>(img(kBM), true, img(kBT), true, 2, 0, false);       // dO3 = K2inv^T dstep2
+      r.commit(0);
+    }
+    r.template product<false, true>(img(kBT), true, img(kBV), true, (D + 63) / 64, 1, false);   // dK2inv = dstep2 Bmat^T
+    r.commit(1);
+    if (C) {
+      if (own_d) {
+        r.result(0, 0, v);
+        set_row<16>(dO3 + (size_t)r.row * D, r.col0(), D, r.row < m && !r.failed, v);
+      }
+      r.result(1, 1, v);
+      r.put(Gi, v);
+    }
+    r.publish(true);
+    if (C) {
+      r.ensure();
+      for (int i = 0; i < 4; ++i) {
+        const int row = r.rank * 64 + 4 * w + i;
+        if (row >= m) continue;
+        float s = 0.f;
+        for (int d = lane; d < D; d += 32) s = fmaf(p.bmat[bh * md + row * D + d], __ldcg(dO3 + row * D + d), s);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) p.D3[bh * m + row] = s;
+      }
+    }
+  }
+  if (!p.tail) { r.close(); return; }
+  float* out32 = p.G ? p.dK2 + bh * mm : f32(kGg);
+  if (C) {
+    if (p.G) r.convert(p.G + bh * mm, m, m, Gi);
+    r.convert(k2, m, m, img(kBK2));
+    r.convert(iterates + (size_t)(J - 1) * mm, m, m, img(kBZ0 + ((J - 1) & 1)));
+    if (ridge) r.convert(iterates + (size_t)J * mm, m, m, img(kBT));
+  }
+  r.publish(true);
+  const uint8_t* A = img(kBK2);
+  const float* A32 = k2;
+  if (ridge) {
+    r.template product<true, false>(img(kBK2), true, img(kBK2), true, 2, 0, false);
+    r.commit(0);
+    r.template product<true, false>(Gi, true, img(kBT), true, 2, 1, false);          // G^T Z_J
+    r.commit(1);
+    if (C) {
+      const Norms nk = norms(k2, m, r.red);
+      r.result(0, 0, v);
+      r.add_diag(v, nk.n1 * nk.ninf / p.kappa, m);
+      r.put(img(kBA), v);
+      set_row<16>(f32(kGA) + (size_t)r.row * m, r.col0(), m, r.row < m, v);
+      r.result(1, 1, v);
+      set_row<16>(f32(kGdK) + (size_t)r.row * m, r.col0(), m, r.row < m, v);
+    }
+    r.publish(true);
+    r.template product<false, false>(Gi, false, img(kBK2), false, 2, 0, false);      // dL/dZ_J = G K2
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);
+      r.put(img(kBdZ0 + (J & 1)), v);
+    }
+    r.publish(false);
+    A = img(kBA);
+    A32 = f32(kGA);
+  }
+  // Per iteration, with dT = Z^T dZ / 4, dV = -M^T dT, dU = -M^T dV and U = 7 I - M:
+  //   1:  M = A Z                                       | ndT = -Z^T dZ / 4
+  //   2:  V = 15 I - 7 M + M M                          | dV = M^T ndT
+  //   3:  dM = ndT V^T + dV M^T + M^T dV - 7 dV         | qT = (13 I - M V) / 4
+  //   4:  dZ' = dZ qT^T + A^T dM                        | dA += dM Z^T  (registers)
+  float dA[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) dA[i] = 0.f;
+  for (int j = J - 1; j >= 0; --j) {
+    uint8_t* Z = img(kBZ0 + (j & 1));
+    uint8_t* dZ = img(kBdZ0 + ((j + 1) & 1));
+    float mv[16], dv[16];
+    r.template product<false, false>(A, j == J - 1, Z, j == J - 1, 2, 0, false);
+    r.commit(0);
+    r.template product<true, false>(Z, false, dZ, true, 2, 1, false);
+    r.commit(1);
+    if (C) {
+      r.ensure();
+      if (j > 0) r.convert(iterates + (size_t)(j - 1) * mm, m, m, img(kBZ0 + ((j + 1) & 1)));
+      r.result(0, 0, mv);
+      r.put(img(kBM), mv);
+      r.result(1, 1, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
+      r.put(img(kBdT), v);
+    }
+    r.publish(j > 0);
+    r.template product<false, false>(img(kBM), true, img(kBM), true, 2, 0, false);
+    r.commit(0);
+    r.template product<true, false>(img(kBM), true, img(kBdT), true, 2, 1, false);
+    r.commit(1);
+    if (C) {
+      r.result(0, 0, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, mv[i], v[i]);
+      r.add_diag(v, 15.f, m);
+      r.put(img(kBV), v);
+      r.result(1, 1, dv);
+      r.put(img(kBdV), dv);
+    }
+    r.publish(false);
+    r.template product<false, false>(img(kBM), false, img(kBV), true, 2, 0, false);
+    r.commit(0);
+    r.template product<false, true>(img(kBdT), false, img(kBV), true, 2, 1, false);
+    r.template product<false, true>(img(kBdV), true, img(kBM), false, 2, 1, true);
+    r.template product<true, false>(img(kBM), false, img(kBdV), true, 2, 1, true);
+    r.commit(1);
+    if (C) {
+      r.result(0, 0, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
+      r.add_diag(v, 3.25f, m);
+      r.put(img(kBT), v);
+      r.result(1, 1, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, dv[i], v[i]);
+      r.put(img(kBdM), v);
+    }
+    r.publish(false);
+    r.template product<false, true>(dZ, false, img(kBT), true, 2, 0, false);
+    r.template product<true, false>(A, false, img(kBdM), true, 2, 0, true);
+    r.commit(0);
+    r.template product<false, true>(img(kBdM), true, Z, false, 2, 1, false);
+    r.commit(1);
+    if (C) {
+      r.result(0, 0, v);
+      if (j > 0) r.put(img(kBdZ0 + (j & 1)), v);
+      else set_row<16>(f32(kGdZ) + (size_t)r.row * m, r.col0(), m, r.row < m, v);
+      r.result(1, 1, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) dA[i] += v[i];
+    }
+    r.publish(j == 0);
+  }
+  // Z0 = A^T / c with c = ||A||_1 ||A||_inf; S = sum_{a,b} dZ0[a,b] A[b,a]
+  if (C) {
+    r.ensure();
+    const float* dZ0 = f32(kGdZ);
+    const Norms na = norms(A32, m, r.red);
+    const float craw = na.n1 * na.ninf, c = fmaxf(craw, 1e-12f);
+    // this thread's row of A against the same column of dZ0, in both blocks (each CTA forms the whole sum)
+    float part = 0.f, z[16];
+#pragma unroll
+    for (int b = 1; b >= 0; --b) {
+      const int c0 = (b ? (r.rank ^ 1) : r.rank) * 64 + (r.seg & 3) * 16;      // the own block last: v and z stay
+      get_row<16>(A32 + (size_t)r.row * m, c0, m, r.row < m, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) z[i] = (r.row < m && c0 + i < m) ? __ldcg(dZ0 + (size_t)(c0 + i) * m + r.row) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) part = fmaf(z[i], v[i], part);
+    }
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) r.red[w] = part;
+    compute_sync();
+    float S = 0.f;
+    for (int i = 0; i < kComputeWarps; ++i) S += r.red[i];
+    const bool clamped = !(craw > 1e-12f);
+    const float col_term = clamped ? 0.f : -S * na.ninf / (c * c);
+    const float row_term = clamped ? 0.f : -S * na.n1 / (c * c);
+    if (r.row < m) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int cc = r.col0() + i;
+        if (cc < m) {
+          const float sg = v[i] > 0.f ? 1.f : (v[i] < 0.f ? -1.f : 0.f);
+          float g = dA[i] + z[i] / c;
+          if (cc == na.jc) g += sg * col_term;
+          if (r.row == na.ir) g += sg * row_term;
+          dA[i] = g;
+        }
+      }
+      set_row<16>(out32 + (size_t)r.row * m, r.col0(), m, !r.failed, dA);
+    }
+  }
+  r.publish(true);
+  if (ridge) {
+    // dK2 = G^T Z_J + K2 (dA + dA^T)
+    if (C) {
+      r.ensure();
+      const int row = r.rank * 64 + (threadIdx.x & 63), s = threadIdx.x >> 6;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int cc = 16 * s + i;
+        v[i] = (row < m && cc < m) ? __ldcg(out32 + (size_t)row * m + cc) + __ldcg(out32 + (size_t)cc * m + row) : 0.f;
+      }
+      put16(img(kBT), row, s, v);
+    }
+    r.publish(true);
+    r.template product<false, false>(img(kBK2), false, img(kBT), true, 2, 0, false);
+    r.commit(0);
+    if (C) {
+      r.result(0, 0, v);
+      float x[16];
+      get_row<16>(f32(kGdK) + (size_t)r.row * m, r.col0(), m, r.row < m, x);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] += x[i];
+      set_row<16>(out32 + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
+    }
+    r.publish(true);
+  }
+  if (p.G) { r.close(); return; }
+  // softmax-2 Jacobian dS2 = K2 o (dK2 - rowsum(dK2 o K2)), then dqt_ns = dS2 Kt, dkt_tot = dkt_a + dS2^T Qt
+  if (C) {
+    r.ensure();
+    for (int i = 0; i < 4; ++i) {
+      const int row = r.rank * 64 + 4 * w + i;
+      float x[4], k[4], s = 0.f;
+      get_row<4>(out32 + (size_t)row * m, 4 * lane, m, row < m, x);
+      get_row<4>(k2 + (size_t)row * m, 4 * lane, m, row < m, k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s = fmaf(x[q], k[q], s);
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = k[q] * (x[q] - s);
+      put_row(img(kBM), row, lane, x);
+    }
+    r.convert(p.kt + bh * md, m, D, img(kBV));
+    r.convert(p.qt + bh * md, m, D, img(kBdV));
+  }
+  r.publish(true);
+  if (own_d) {
+    r.template product<false, false>(img(kBM), true, img(kBV), true, 2, 0, false);
+    r.commit(0);
+    r.template product<true, false>(img(kBM), true, img(kBdV), true, 2, 1, false);
+    r.commit(1);
+    if (C) {
+      const size_t off = (size_t)bh * md + (size_t)r.row * D;
+      const bool row_ok = r.row < m;
+      float da[16];
+      get_row<16>(p.sums + bh * 2 * md + md + (size_t)r.row * D, r.col0(), D, row_ok, da);
+      r.result(0, 0, v);
+      set_row<16>(p.dqt_ns + off, r.col0(), D, row_ok && !r.failed, v);
+      r.result(1, 1, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] += da[i];
+      set_row<16>(p.dkt_tot + off, r.col0(), D, row_ok && !r.failed, v);
+      if (p.rows_k && row_ok) {
+        Segments sg(p.N, m);
+        const float f = p.scale / (float)sg.len(r.row);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] *= f;
+        set_row<16>(p.rows_k + off, r.col0(), D, !r.failed, v);
+      }
+    }
+  }
+  r.close();
+}
+
+// ---- kernels --------------------------------------------------------------------------------------------
+template <int R, class P, class Prog>
+__device__ __forceinline__ void run_role(Shared* sh, uint8_t* ring, float* red, const P& p, Prog prog) {
+  Role<R> r;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  r.open(sh, ring, red, (int)rank, p.status);
+  prog(r, p, (int64_t)(blockIdx.x >> 1));
+}
+template <class P, class Prog>
+__device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) {
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
+  float* red = reinterpret_cast<float*>(ring + (size_t)kStages * kStageBytes + kBlockBytes);
+  Shared* sh = reinterpret_cast<Shared*>(red + kRedFloats);
+  static_assert(sizeof(Shared) <= 128, "barriers");
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
+    mbar_init(&sh->done[0], 1);
+    mbar_init(&sh->done[1], 1);
+    mbar_init(&sh->ready, 2 * (kComputeWarps + 2));
+    sh->abort_word = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(&sh->tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();          // the peer's barriers exist
+  tc_fence_after();
+  pdl_wait();
+  if (warp < kComputeWarps) run_role<kCompute>(sh, ring, red, p, prog);
+  else if (warp == kComputeWarps) run_role<kProducer>(sh, ring, red, p, prog);
+  else run_role<kIssuer>(sh, ring, red, p, prog);
+  __syncwarp();
+  const uint32_t tmem = sh->tmem_slot;
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();          // nobody arrives on this CTA's barriers any more
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+__global__ void __launch_bounds__(kThr, 1) __cluster_dims__(2, 1, 1) mx_fwd_kernel(FwdParams p) {
+  extern __shared__ uint8_t mx_dyn[];
+  run_kernel(mx_dyn, p, [](auto& r, const FwdParams& q, int64_t bh) { fwd_program(r, q, bh); });
+}
+__global__ void __launch_bounds__(kThr, 1) __cluster_dims__(2, 1, 1) mx_bwd_kernel(BwdParams p) {
+  extern __shared__ uint8_t mx_dyn[];
+  run_kernel(mx_dyn, p, [](auto& r, const BwdParams& q, int64_t bh) { bwd_program(r, q, bh); });
+}
+
+}  // namespace mx
+}  // namespace fnb

@@ -501,15 +501,13 @@ __global__ void __launch_bounds__(kThreads) combine_slab_kernel(CombineSlabParam
 }
 
 // ------------------------------------------------------------------------------------------
-// After the global-memory middle stage of the backward (num_landmarks > 64), what the tensor-core
-// column pass and the in-place pass read: the 16-bit operand copies dO3 / 2^e (with 2^e >= max |dO3|)
-// and qt_mul * Qt, padded to MP rows, and the per-landmark rows scale * dKt_tot / len.
+// With more than 64 landmarks, what the tensor-core column pass of the backward reads: the 16-bit
+// operand copies dO3 / 2^e (with 2^e >= max |dO3|) and qt_mul * Qt, padded to MP rows.
 struct MidPackParams {
-  const float* dO3; const float* q_landmarks; const float* dkt_tot;   // [BH][m][D]
-  void* do3n; float* do3_scale; void* qt16; float* rows_k;
+  const float* dO3; const float* q_landmarks;   // [BH][m][D]
+  void* do3n; float* do3_scale; void* qt16;
   int m, D, MP, dtype;
-  float qt_mul, scale;
-  int64_t N;
+  float qt_mul;
 };
 // gridDim.y CTAs share a slice: each finds the scale for itself (the slice's dO3 comes from L2) and
 // packs its share of the rows, four values per thread and step.
@@ -528,8 +526,6 @@ __global__ void __launch_bounds__(kThreads) mid_pack_kernel(MidPackParams p) {
   if (t == 0 && blockIdx.y == 0) p.do3_scale[bh] = sc;
   const size_t ob = (size_t)bh * p.MP * p.D * 2;
   const float* qt = p.q_landmarks + bh * (int64_t)md;
-  const float* dkt = p.dkt_tot + bh * (int64_t)md;
-  Segments sg(p.N, p.m);
   const int groups = p.MP * p.D / 4;       // groups of four consecutive columns of the padded operands
   for (int g = blockIdx.y * kThreads + t; g < groups; g += gridDim.y * kThreads) {
     const int l = (g * 4) / p.D;
@@ -537,9 +533,6 @@ __global__ void __launch_bounds__(kThreads) mid_pack_kernel(MidPackParams p) {
     if (l < p.m) {
       a = reinterpret_cast<const float4*>(dO3)[g];
       q = reinterpret_cast<const float4*>(qt)[g];
-      const float4 k = reinterpret_cast<const float4*>(dkt)[g];
-      const float f = p.scale / (float)sg.len(l);
-      reinterpret_cast<float4*>(p.rows_k + bh * (int64_t)md)[g] = make_float4(k.x * f, k.y * f, k.z * f, k.w * f);
     }
     reinterpret_cast<uint2*>(reinterpret_cast<char*>(p.do3n) + ob)[g] =
         make_uint2(pack2x16(p.dtype, a.x * inv_sc, a.y * inv_sc), pack2x16(p.dtype, a.z * inv_sc, a.w * inv_sc));
