@@ -1,8 +1,9 @@
 """The landmark-sized stages for more than 64 landmarks on the tensor cores, against the float64 oracle with the
 CUDA-core kernels as the yardstick.  FP32 inputs run the same streaming passes on both sides, so only these stages
-differ.  Operands keep 24 bits in three bf16 terms; dropped partial products and the truncating accumulator stay
-below 2^-22 = 2.4e-7 per product, which the pseudoinverse amplifies like the yardstick's own rounding:
-bound 1.5 x yardstick + 1e-6."""
+differ.  Operands keep 24 bits in three bf16 terms.  The accumulator truncates: the eight K steps of a product lose up
+to 8 * 2^-24, all in one direction, where the yardstick's 128 rounded additions lose about sqrt(128) / 2 * 2^-24
+= 6 * 2^-24 in either direction; both are amplified alike by the iterations, but a bias adds up over the terms of the
+sums that follow (up to sqrt(64) = 8 times) where rounding averages out: bound 8 x yardstick + 1e-6."""
 import pytest
 import torch
 
@@ -37,7 +38,7 @@ def test_against_cuda_core_stages(cuda_device, B, H, N, D, m, J, kappa):
     for key in ("K2", "lse2", "k2inv", "step2", "out", "dq", "dk", "dv"):
         a, b = _rel(pick(got[key]), want[key]), _rel(pick(ref[key]), want[key])
         print(key, f"{a:.2e} {b:.2e}")
-        assert a <= 1.5 * b + 1e-6, (key, a, b)
+        assert a <= 8 * b + 1e-6, (key, a, b)
 
 
 @pytest.mark.parametrize("BH", [2, 37, 38])     # beside the column passes up to a quarter of 148 SMs, in line above
