@@ -162,6 +162,10 @@ def check_device_status(device=None):
                                f"(status 0x{val & 0xffffffff:08x}); results of that call are invalid")
 
 
+# (the handle itself, without the Stream object torch.cuda.current_stream builds around it)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _workspace(nbytes, device):
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
@@ -248,11 +252,126 @@ def backward(dO, q_s, k_s, q_tilde, k_tilde, kernel2_inv, step2, lse1, lse2, lse
                             _ptr(dk), _ptr(dv), _ptr(ws), ws.numel(), dev.index,
                             C.c_void_p(torch.cuda.current_stream(dev).cuda_stream), _ptr(_status(dev)))
         _lib.check(lib.fnb_backward(C.byref(args)))
-    if _os.environ.get("FNB_BWD_DEBUG"):   # per-stage statistics, as FN_BWD_DEBUG does in the reference
-        for name, st in tensor_stats(dO=dO, dQ=dq, dK=dk, dV=dv, step2=step2, k2inv=kernel2_inv).items():
-            print(f"[FNB_BWD_DEBUG] {name}: absmax={st['absmax']:.4e} absmean={st['absmean']:.4e} "
-                  f"nonfinite={st['nonfinite']}")
-        check_device_status(dev)
+    if _os.environ.get("FNB_BWD_DEBUG"):
+        _print_bwd_debug(dev, dO=dO, dQ=dq, dK=dk, dV=dv, step2=step2, k2inv=kernel2_inv)
+    return [dq, dk, dv]
+
+
+def _print_bwd_debug(dev, **tensors):
+    """Per-stage statistics, as FN_BWD_DEBUG does in the reference."""
+    for name, st in tensor_stats(**tensors).items():
+        print(f"[FNB_BWD_DEBUG] {name}: absmax={st['absmax']:.4e} absmean={st['absmean']:.4e} "
+              f"nonfinite={st['nonfinite']}")
+    check_device_status(dev)
+
+
+# ---- the autograd function's path -----------------------------------------------------------------------
+# One call of forward() makes fourteen tensors and one of backward() checks as many, about half of the host time of
+# a call.  The function below it keeps all FP32 tensors the backward needs in one buffer; what depends on the
+# sizes and options alone (the shape struct, workspace sizes, offsets) is worked out once per combination.
+class _Plan:
+    __slots__ = ("shape", "fwd_ws", "bwd_ws", "floats", "offsets", "layout")
+
+    def __init__(self, lib, B, H, N, D, m, J, dtype, kappa_star, layout):
+        self.shape = _shape_struct(B, H, N, D, m, J, dtype, kappa_star, layout)
+        _lib.check(lib.fnb_check_shape(C.byref(self.shape)))
+        self.layout = layout
+        self.fwd_ws = max(lib.fnb_fwd_workspace_bytes(C.byref(self.shape)), 256)
+        self.bwd_ws = max(lib.fnb_bwd_workspace_bytes(C.byref(self.shape)), 256)
+        # lse1, q~, k~, K2, lse2, iterates, K2inv, Bmat, lse3, step2: the order of FwdArgs; 256-byte aligned, in bytes
+        BH, off, offsets = B * H, 0, []
+        for n in (N, m * D, m * D, m * m, m, (J + 1) * m * m, m * m, m * D, m, m * D):
+            offsets.append(4 * off)
+            off += (BH * n + 63) // 64 * 64
+        self.offsets, self.floats = tuple(offsets), off
+
+
+_plans = {}
+_MAX_PLANS = 256
+
+
+def _plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout):
+    if type(kappa_star) is not float and type(kappa_star) is not int:
+        return _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
+    key = (B, H, N, D, m, J, dtype, kappa_star, layout, _flags)
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
+        if len(_plans) >= _MAX_PLANS:
+            _plans.clear()
+        _plans[key] = plan
+    return plan
+
+
+def _is(t, shape, dtype, dev, layout):
+    """t is a CUDA tensor on `dev` of that shape, dtype and layout (the quick form of _check_big)."""
+    return t.shape == shape and t.dtype == dtype and t.device == dev and layout_of(t) == layout
+
+
+def forward_packed(q, k, v, num_landmarks, newton_iter, kappa_star):
+    """forward() for the autograd function: (output, buffer); the buffer holds everything backward_packed() needs
+    besides q, k and v."""
+    lib = _lib.load()
+    if not all(isinstance(t, torch.Tensor) for t in (q, k, v)) or q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
+        raise RuntimeError("q, k, v must be 4D (B, H, N, D)")
+    dtype, shape, dev = q.dtype, q.shape, q.device
+    if not (dtype == k.dtype == v.dtype):
+        raise RuntimeError("q, k, v dtypes must match")
+    B, H, N, D = shape
+    m, J = int(num_landmarks), int(newton_iter)
+    lay = layout_of(q)
+    if lay != _lib.FNB_LAYOUT_BHND and (lay is None or not tc_eligible(dtype, D, m) or layout_of(k) != lay or layout_of(v) != lay):
+        lay = _lib.FNB_LAYOUT_BHND
+    if not (q.is_cuda and _is(q, shape, dtype, dev, lay) and _is(k, shape, dtype, dev, lay) and _is(v, shape, dtype, dev, lay)):
+        for t, name in ((q, "q"), (k, "k"), (v, "v")):
+            _check_big(t, name, shape, layout=lay)
+    plan = _plan(lib, B, H, N, D, m, J, dtype, kappa_star, lay)
+    with _on_device(dev):
+        out = _empty_like_layout(q, lay)
+        saved = torch.empty(plan.floats, dtype=torch.float32, device=dev)
+        ws = torch.empty(plan.fwd_ws, dtype=torch.uint8, device=dev)
+        base = saved.data_ptr()
+        args = _lib.FwdArgs(plan.shape, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
+                            *[base + o for o in plan.offsets], ws.data_ptr(), plan.fwd_ws, dev.index,
+                            _raw_stream(dev.index), _status(dev).data_ptr())
+        _lib.check(lib.fnb_forward(C.byref(args)))
+    return out, saved
+
+
+def backward_packed(dO, q, k, v, saved, num_landmarks, newton_iter, kappa_star):
+    """[dQ, dK, dV] from what forward_packed() was given and returned."""
+    lib = _lib.load()
+    if not isinstance(dO, torch.Tensor) or dO.dim() != 4:
+        raise RuntimeError(f"dO must be 4D (B, H, N, D), got {getattr(dO, 'dim', lambda: '?')()}D")
+    dtype, shape, dev = dO.dtype, dO.shape, dO.device
+    B, H, N, D = shape
+    m, J = int(num_landmarks), int(newton_iter)
+    lay = layout_of(q)
+    if lay != _lib.FNB_LAYOUT_BNHD or not tc_eligible(dtype, D, m):
+        lay = _lib.FNB_LAYOUT_BHND
+    if dO.is_cuda:
+        dO = _to_layout(dO, lay)
+    plan = _plan(lib, B, H, N, D, m, J, dtype, kappa_star, lay)
+    if not (dO.is_cuda and _is(q, shape, dtype, dev, lay) and _is(k, shape, dtype, dev, lay) and _is(v, shape, dtype, dev, lay)):
+        _check_big(dO, "dO", layout=lay)
+        for t, name in ((q, "q_s"), (k, "k_s"), (v, "v")):
+            _check_big(t, name, shape, dtype, layout=lay)
+    if saved.device != dev or saved.shape != (plan.floats,) or saved.dtype != torch.float32 or not saved.is_contiguous():
+        _check_big(saved, "saved tensors", (plan.floats,), torch.float32)
+        raise RuntimeError("saved tensors are on another device than dO")
+    with _on_device(dev):
+        dq, dk, dv = (_empty_like_layout(dO, lay) for _ in range(3))
+        ws = torch.empty(plan.bwd_ws, dtype=torch.uint8, device=dev)
+        base = saved.data_ptr()
+        lse1, qt, kt, k2, _, iterates, k2inv, bmat, lse3, step2 = [base + o for o in plan.offsets]
+        args = _lib.BwdArgs(plan.shape, q.data_ptr(), k.data_ptr(), v.data_ptr(), dO.data_ptr(), lse1, qt, kt, k2, iterates,
+                            k2inv, bmat, lse3, step2, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), plan.bwd_ws,
+                            dev.index, _raw_stream(dev.index), _status(dev).data_ptr())
+        _lib.check(lib.fnb_backward(C.byref(args)))
+    if _os.environ.get("FNB_BWD_DEBUG"):
+        at = lambda o, n, s: saved[o // 4:o // 4 + n].view(s)
+        _print_bwd_debug(dev, dO=dO, dQ=dq, dK=dk, dV=dv, step2=at(plan.offsets[9], B * H * m * D, (B, H, m, D)),
+                         k2inv=at(plan.offsets[6], B * H * m * m, (B, H, m, m)))
     return [dq, dk, dv]
 
 
@@ -414,7 +533,9 @@ def conv_residual(v, weight, base=None, transposed=False):
     lib = _lib.load()
     v, layout = _conv_geometry(v)
     B, H, N, D = v.shape
-    w = weight.detach().to(device=v.device, dtype=torch.float32).contiguous()
+    w = weight.detach()
+    if not (w.dtype == torch.float32 and w.device == v.device and w.is_contiguous()):
+        w = w.to(device=v.device, dtype=torch.float32).contiguous()
     if w.dim() != 2 or w.shape[0] != H:
         raise RuntimeError(f"conv weight must be (heads, kernel_size) = ({H}, ks), got {tuple(w.shape)}")
     if base is not None:
@@ -424,7 +545,7 @@ def conv_residual(v, weight, base=None, transposed=False):
     result = _empty_like_layout(v, layout)
     args = _lib.ConvArgs(B, H, N, D, int(w.shape[1]), _DTYPES[v.dtype], int(layout), v.data_ptr(),
                          base.data_ptr() if base is not None else None, result.data_ptr(), w.data_ptr(),
-                         1 if transposed else 0, v.device.index, torch.cuda.current_stream(v.device).cuda_stream)
+                         1 if transposed else 0, v.device.index, _raw_stream(v.device.index))
     with _on_device(v.device):
         _lib.check(lib.fnb_conv_residual(C.byref(args)))
     return result
@@ -443,7 +564,7 @@ def conv_residual_dweight(v, d_out, kernel_size):
     ws = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=v.device)
     args = _lib.ConvDwArgs(B, H, N, D, int(kernel_size), _DTYPES[v.dtype], int(layout), v.data_ptr(), d_out.data_ptr(),
                            dw.data_ptr(), ws.data_ptr(), ws.numel(), v.device.index,
-                           torch.cuda.current_stream(v.device).cuda_stream)
+                           _raw_stream(v.device.index))
     with _on_device(v.device):
         _lib.check(lib.fnb_conv_residual_dweight(C.byref(args)))
     return dw

@@ -125,6 +125,8 @@ _lib = None
 def load(build_if_missing=True):
     """Return the loaded library, building it with nvcc first if it is absent."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

@@ -57,11 +57,8 @@ class FlashNystromFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, num_landmarks, newton_iter, fast_dk2inv, kappa_star, use_tc_pinv):
-        need_bwd = bool(q.requires_grad or k.requires_grad or v.requires_grad)
-        results = _C.forward(q, k, v, num_landmarks, newton_iter, kappa_star, use_tc_pinv, need_bwd)
-        output = results[0]
-        saved = list(results[1:]) + [v, output]
-        ctx.save_for_backward(*saved)
+        output, saved = _C.forward_packed(q, k, v, num_landmarks, newton_iter, kappa_star)
+        ctx.save_for_backward(q, k, v, output, saved)
         ctx.num_landmarks = num_landmarks
         ctx.newton_iter = newton_iter
         ctx.fast_dk2inv = fast_dk2inv
@@ -70,12 +67,10 @@ class FlashNystromFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_output):
-        s = ctx.saved_tensors
+        q, k, v, _, saved = ctx.saved_tensors
         # (the shim brings grad_output to the layout of q: no copy when both are contiguous or both
         # are head-split views of (B, N, H*D) tensors, which is what the module below produces)
-        dQ, dK, dV = _C.backward(grad_output, *s[0:12], s[12], s[13],
-                                 ctx.num_landmarks, ctx.newton_iter, ctx.fast_dk2inv,
-                                 ctx.kappa_star)
+        dQ, dK, dV = _C.backward_packed(grad_output, q, k, v, saved, ctx.num_landmarks, ctx.newton_iter, ctx.kappa_star)
         return dQ, dK, dV, None, None, None, None, None
 
 
