@@ -40,10 +40,10 @@ using ns::Norms;
 constexpr int kTileBytes = kN * 128;        // one bf16 term of a matrix
 constexpr int kSet = 3 * kTileBytes;        // the three terms of a matrix, order (x1, x0, x2)
 constexpr int kTerm0 = kTileBytes, kTerm1 = 0, kTerm2 = 2 * kTileBytes;
-constexpr int kXchBytes = kN * kLd * 4;     // FP32 exchange buffer between the lane halves
+constexpr int kXchBytes = kN * kN * 4;      // FP32 exchange buffer between the lane halves, one per accumulator
 constexpr int kFwdSlots = 7, kBwdSlots = 8;
 constexpr size_t kFwdSmem = (size_t)kFwdSlots * kSet + kXchBytes + 1024;
-constexpr size_t kBwdSmem = (size_t)kBwdSlots * kSet + kXchBytes + 1024;
+constexpr size_t kBwdSmem = (size_t)kBwdSlots * kSet + 2 * kXchBytes + 1024;
 constexpr uint32_t kFwdTmemCols = 256, kBwdTmemCols = 512;
 constexpr uint32_t kAcc0 = 0, kAcc1 = 256;  // TMEM column of the two accumulators
 
@@ -68,7 +68,7 @@ __device__ int g_ns_trace_n;
 
 struct Ctx {
   uint8_t* base;        // 1024-byte aligned start of the tile slots
-  float* xch;           // exchange buffer (row stride kLd)
+  float4* xch;          // exchange buffers: [accumulator][4][256 threads]
   uint64_t* bar;        // two completion barriers (MMA groups -> compute warps)
   uint64_t* ready;      // operand tiles written (one arrival per compute warp -> issuing thread)
   uint32_t phase[2];    // parity the next wait on each completion barrier uses
@@ -222,46 +222,41 @@ __device__ __forceinline__ void mma_single(Ctx& c, int where, Issue issue) {
 // Result of the accumulator at TMEM column `col`: after the call v[0..15] holds columns
 // c.col0 .. c.col0+15 of row c.row.  Every thread must call (warp-wide TMEM loads, pair barriers).
 __device__ __forceinline__ void acc_result(const Ctx& c, uint32_t col, float* v) {
-  float s[32], t[32];
+  float s[32], t[32], u[32];
   const uint32_t a = c.tmem + col + c.lane_off;
-  tmem_ld32(a, s);                          // lanes 0..63: x1y1 ; lanes 64..127: x0y1
-  tmem_ld32(a + 64, t);                     //              x1y0 ;                x0y0
+  tmem_ld32(a, s);                                // lanes 0..63: x1y1 ; lanes 64..127: x0y1
+  tmem_ld32(a + 64, t);                           //              x1y0 ;                x0y0
+  tmem_ld32(a + (c.part ? 128 : 192), u);         //              x0y2 ;                x2y0
   tmem_ld_wait();
 #pragma unroll
-  for (int i = 0; i < 32; ++i) s[i] += t[i];
+  for (int i = 0; i < 32; ++i) s[i] = (s[i] + t[i]) + u[i];
   NS_TRACE2();
-  tmem_ld32(a + (c.part ? 128 : 192), t);   //              x0y2 ;                x2y0
-  tmem_ld_wait();
-#pragma unroll
-  for (int i = 0; i < 32; ++i) s[i] += t[i];
-  NS_TRACE2();
-  // hand the 16 columns the partner finalises over, take the partner's share of mine
-  // (part is warp-uniform; the two branches keep every register index a constant)
-  float* rowp = c.xch + c.row * kLd + c.c32;
+  // Hand the 16 columns the partner finalises over, take the partner's share of mine (part is
+  // warp-uniform; the two branches keep every register index a constant).  A buffer is written again only
+  // after another batch of products has completed, which every warp's arrival precedes: one barrier is enough.
+  float4* x = c.xch + (col == kAcc0 ? 0 : kXchBytes / 16) + threadIdx.x;
+  const float4* y = c.xch + (col == kAcc0 ? 0 : kXchBytes / 16) + (threadIdx.x ^ 64);
   if (c.part == 0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      *reinterpret_cast<float4*>(rowp + 16 + 4 * q) = make_float4(s[16 + 4 * q], s[17 + 4 * q], s[18 + 4 * q], s[19 + 4 * q]);
+    for (int q = 0; q < 4; ++q) x[q * 256] = make_float4(s[16 + 4 * q], s[17 + 4 * q], s[18 + 4 * q], s[19 + 4 * q]);
     named_barrier(c.pair_bar, 64);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float4 x = *reinterpret_cast<const float4*>(rowp + 4 * q);
-      v[4 * q] = s[4 * q] + x.x; v[4 * q + 1] = s[4 * q + 1] + x.y;
-      v[4 * q + 2] = s[4 * q + 2] + x.z; v[4 * q + 3] = s[4 * q + 3] + x.w;
+      const float4 w = y[q * 256];
+      v[4 * q] = s[4 * q] + w.x; v[4 * q + 1] = s[4 * q + 1] + w.y;
+      v[4 * q + 2] = s[4 * q + 2] + w.z; v[4 * q + 3] = s[4 * q + 3] + w.w;
     }
   } else {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      *reinterpret_cast<float4*>(rowp + 4 * q) = make_float4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
+    for (int q = 0; q < 4; ++q) x[q * 256] = make_float4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
     named_barrier(c.pair_bar, 64);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float4 x = *reinterpret_cast<const float4*>(rowp + 16 + 4 * q);
-      v[4 * q] = s[16 + 4 * q] + x.x; v[4 * q + 1] = s[17 + 4 * q] + x.y;
-      v[4 * q + 2] = s[18 + 4 * q] + x.z; v[4 * q + 3] = s[19 + 4 * q] + x.w;
+      const float4 w = y[q * 256];
+      v[4 * q] = s[16 + 4 * q] + w.x; v[4 * q + 1] = s[17 + 4 * q] + w.y;
+      v[4 * q + 2] = s[18 + 4 * q] + w.z; v[4 * q + 3] = s[19 + 4 * q] + w.w;
     }
   }
-  named_barrier(c.pair_bar, 64);   // the partner has read: the exchange buffer may be reused
   NS_TRACE2();
 }
 
@@ -299,7 +294,7 @@ struct Shared {
 };
 __device__ __forceinline__ void ctx_open(Ctx& c, Shared& sh, uint8_t* dyn, int slots, int* status, uint32_t cols) {
   c.base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
-  c.xch = reinterpret_cast<float*>(c.base + (size_t)slots * kSet);
+  c.xch = reinterpret_cast<float4*>(c.base + (size_t)slots * kSet);
   c.bar = sh.bar;
   c.ready = &sh.ready;
   c.phase[0] = c.phase[1] = c.rphase = 0;
@@ -371,29 +366,19 @@ __device__ inline void pinv_forward_tc(Ctx& c, float* red, float* iterates, floa
   }
   Norms na = ns::norms(A, m, red);
   const float cden = fmaxf(na.n1 * na.ninf, 1e-12f);
-  {
-    // Z0 = A^T / cden -> slot 1 and iterates[0] (and the result itself when there is no iteration)
-    const int r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
-    float z[16];
+  // v: the iterate of the last step, in the layout of the epilogue.  It goes to global memory while the next
+  // product runs (in front of that product the store took 1300 of the 9300 cycles of an iteration).
+  float v[16];
+  // Z0 = A^T / cden
 #pragma unroll
-    for (int i = 0; i < 16; ++i) z[i] = A[(c0 + i) * kLd + r] / cden;
-    split_store16(c.slot(1), r, c0, z);
-    if (r < m) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (c0 + i < m) {
-          iterates[r * m + c0 + i] = z[i];
-          if (J == 0 && !(kappa > 0.f)) k2inv[r * m + c0 + i] = z[i];
-        }
-    }
-  }
+  for (int i = 0; i < 16; ++i) v[i] = A[(c.col0 + i) * kLd + c.row] / cden;
+  split_store16(c.slot(1), c.row, c.col0, v);
   convert_buf(c.slot(0), A);
   NS_TRACE();
-  float v[16];
   for (int j = 0; j < J; ++j) {
-    float* Zn = iterates + (size_t)(j + 1) * mm_;
     NS_TRACE();
     tiles_ready(c);
+    if (!c.failed) store_global16(c, iterates + (size_t)j * mm_, v, m, m, m);
     wait_group(c, 0, 0x2110);
     acc_result(c, kAcc0, v);
     split_store16(c.slot(2), c.row, c.col0, v);
@@ -413,19 +398,60 @@ __device__ inline void pinv_forward_tc(Ctx& c, float* red, float* iterates, floa
     wait_group(c, 0, 0x2113);
     acc_result(c, kAcc0, v);
     split_store16(c.slot(1), c.row, c.col0, v);
-    if (!c.failed) {
-      store_global16(c, Zn, v, m, m, m);
-      if (j == J - 1 && !(kappa > 0.f)) store_global16(c, k2inv, v, m, m, m);
-    }
   }
   NS_TRACE();
+  if (kappa > 0.f) tiles_ready(c);
+  if (!c.failed) {
+    store_global16(c, iterates + (size_t)J * mm_, v, m, m, m);
+    if (!(kappa > 0.f)) store_global16(c, k2inv, v, m, m, m);
+  }
   if (kappa > 0.f) {
     // k2inv = Z_J K2^T
-    tiles_ready(c);
     wait_group(c, 0, 0x2114);
     acc_result(c, kAcc0, v);
     if (!c.failed) store_global16(c, k2inv, v, m, m, m);
   }
+}
+
+// Row softmax of the scores in the padded buffer X, in place (rows and columns past m become zero), K2 and lse2 to
+// global memory.  Four adjacent lanes share a row, 16 columns each: two shuffles per reduction.
+__device__ inline void softmax16(float* X, const ns::NsFwdParams& p, int64_t bh) {
+  const int m = p.m, r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
+  float* row = X + r * kLd + c0;
+  float v[16], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 x = *reinterpret_cast<const float4*>(row + 4 * q);
+    v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) if (c0 + i < m) mx = fmaxf(mx, v[i]);
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    v[i] = (r < m && c0 + i < m) ? expf(v[i] - mx) : 0.f;
+    sum += v[i];
+  }
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = r < m ? v[i] / sum : 0.f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) *reinterpret_cast<float4*>(row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  if (r < m) {
+    float* g = p.k2 + bh * m * m + (size_t)r * m + c0;
+    if ((m & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (c0 + 4 * q < m) *reinterpret_cast<float4*>(g + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) if (c0 + i < m) g[i] = v[i];
+    }
+    if (c0 == 0) p.lse2[bh * m + r] = mx + logf(sum);
+  }
+  ns::ns_sync();
 }
 
 // Scores S2 = Qt Kt^T for head_dim 64 as one split product (Qt in slot 0, Kt in slot 1, both
@@ -457,7 +483,7 @@ __device__ inline void s2_softmax_tc(Ctx& c, const ns::NsFwdParams& p, int64_t b
   acc_result(c, kAcc0, v);
   store_row16(c, fwd_staging(c), v);
   ns::ns_sync();
-  ns::softmax_rows(fwd_staging(c), p, bh);
+  softmax16(fwd_staging(c), p, bh);
 }
 
 __global__ void __launch_bounds__(kNsTcThreads, 1) ns_fwd_tc_kernel(ns::NsFwdParams p, int* status) {
@@ -566,12 +592,11 @@ __device__ inline void pinv_backward_issue(Ctx& c, int J, int finish, bool head)
 template <class BeforeTail>
 __device__ __forceinline__ float* pinv_backward_tc(Ctx& c, float* red, const float* k2g, const float* iterates,
                                                    const float* G, float* spill, int m, int J, float kappa,
-                                                   BeforeTail before_tail, float* step_dz = nullptr,
-                                                   float* step_da = nullptr) {
+                                                   BeforeTail before_tail, float* znext, const float* a,
+                                                   float* step_dz = nullptr, float* step_da = nullptr) {
   // G == nullptr: dL/dk2inv is already in place (slot 2 without the ridge, staging buffer 3 with it)
+  // znext, a: Z_{J-1} and K2 as load_global16 gives them (fetched by the caller ahead of its own products)
   const int mm_ = m * m;
-  float znext[16];
-  load_global16(iterates + (size_t)(J - 1) * mm_, m, m, m, znext);
   if (kappa > 0.f) {
     float* bK2 = bwd_stage(c, 0);
     float* bA = bwd_stage(c, 1);
@@ -592,8 +617,6 @@ __device__ __forceinline__ float* pinv_backward_tc(Ctx& c, float* red, const flo
     convert_buf(c.slot(2), bdZ);
   } else {
     // A = K2 and dZ_J = G go straight from global memory into their tiles
-    float a[16];
-    load_global16(k2g, m, m, m, a);
     if (G) {
       float g[16];
       load_global16(G, m, m, m, g);
@@ -691,7 +714,10 @@ ns_pinv_bwd_tc_debug_kernel(const float* k2, const float* iterates, const float*
   if (is_compute()) {
     // step hook: one iteration (J = 1) whose "iterates" is the single matrix Z_j per slice
     const float* its = step_dz ? iterates + bh * (size_t)m * m : iterates + bh * (size_t)(J + 1) * m * m;
-    float* out = pinv_backward_tc(c, red, k2 + bh * m * m, its, G + bh * m * m, spill + bh * m * m, m, J, kappa, [] {},
+    float z[16], a[16];
+    load_global16(its + (size_t)(J - 1) * m * m, m, m, m, z);
+    load_global16(k2 + bh * m * m, m, m, m, a);
+    float* out = pinv_backward_tc(c, red, k2 + bh * m * m, its, G + bh * m * m, spill + bh * m * m, m, J, kappa, [] {}, z, a,
                                   step_dz ? step_dz + bh * m * m : nullptr, step_da ? step_da + bh * m * m : nullptr);
     if (out && !c.failed) ns::store_mat(dK2 + bh * m * m, out, m);
   } else if (is_issuer()) {
@@ -911,11 +937,14 @@ ns_bwd_tc_kernel(ns::NsBwdParams p, BwdHeadParams h, int* status) {
   const int finish_tc = p.D == NH * kN ? NH : 0;   // batches of the finishing step
   const bool head = h.partA != nullptr;      // fused middle stage (head_dim 64 only)
   if (is_compute()) {
+    float z[16], a[16];
+    load_global16(p.iterates + (bh * (size_t)(p.J + 1) + p.J - 1) * mm_, m, m, m, z);
+    load_global16(p.k2 + bh * mm_, m, m, m, a);
     if (head) bwd_head_tc(c, red, p, h, bh);
     FinishOperands fo;
     float* dK2 = pinv_backward_tc(c, red, p.k2 + bh * mm_, p.iterates + bh * (size_t)(p.J + 1) * mm_,
                                   head ? nullptr : p.G + bh * mm_,
-                                  p.spill + bh * mm_, m, p.J, p.kappa, [&] { if (finish_tc) finish_load(c, p, bh, 0, fo); });
+                                  p.spill + bh * mm_, m, p.J, p.kappa, [&] { if (finish_tc) finish_load(c, p, bh, 0, fo); }, z, a);
     NS_TRACE();
     if (finish_tc) ns_bwd_finish_tc<NH>(c, p, bh, bwd_tail(c, 0), dK2, fo);
     else if (!c.failed) ns::ns_bwd_finish(p, bh, bwd_tail(c, 0), dK2);
