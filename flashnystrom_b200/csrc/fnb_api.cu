@@ -346,7 +346,7 @@ static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// The Newton-Schulz kernels run on the tensor cores (three-term bf16
+// The Newton-Schulz kernels for num_landmarks <= 64 run on the tensor cores (three-term bf16
 // split, FP32-equivalent) unless the caller forces the CUDA-core path or FNB_NS_CUDA_CORES=1 is
 // set in the environment (kept for A/B measurements).
 static bool ns_on_tensor_cores(uint32_t flags) {
@@ -626,8 +626,10 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       sp2.vec_bh_stride = cp.vec_bh_stride; sp2.vec_chunk_stride = cp.vec_chunk_stride;
       sp2.k2inv = a.k2_inv; sp2.bmat = a.bmat; sp2.lse3 = a.lse3; sp2.step2 = a.step2; sp2.m = p.m; sp2.D = p.D;
       const size_t csm = combine_slab_smem(p.m);
-      if (int rc = set_smem(combine_slab_kernel, csm, max_smem, "combine")) return rc;
-      launch_pdl(combine_slab_kernel, dim3((unsigned)p.BH, (unsigned)(p.D / 16)), dim3(kThreads), csm, st, sp2);
+      auto slab_kern = sp2.nchunk <= 2 ? combine_slab_kernel<2> : sp2.nchunk <= 10 ? combine_slab_kernel<10>
+                                                                                    : combine_slab_kernel<kSlabMaxChunks>;
+      if (int rc = set_smem(slab_kern, csm, max_smem, "combine")) return rc;
+      launch_pdl(slab_kern, dim3((unsigned)p.BH, (unsigned)(p.D / 16)), dim3(kThreads), csm, st, sp2);
     } else {
       cp.k2inv = a.k2_inv; cp.k_landmarks = a.k_landmarks; cp.bmat = a.bmat; cp.lse3 = a.lse3;
       cp.step2 = a.step2; cp.m = p.m; cp.D = p.D;
@@ -1428,7 +1430,7 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
       {"conv_residual<half>", (const void*)conv_residual_kernel<H>, kThreads, conv_smem_bytes(64, 3)},
       {"conv_dw_partial<half,2>", (const void*)conv_dw_partial_kernel<H, 2>, kThreads, conv_smem_bytes(64, 3)},
       {"tc_fwd_b<half,64,64>", (const void*)tc::tc_fwd_b_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdBSmem<64, 64>::kBytes},
-      {"combine_slab", (const void*)combine_slab_kernel, kThreads, combine_slab_smem(64)},
+      {"combine_slab", (const void*)combine_slab_kernel<kSlabMaxChunks>, kThreads, combine_slab_smem(64)},
       {"tc_fwd_c<half,64,64>", (const void*)tc::tc_fwd_c_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdCSmem<64, 64>::kBytes},
       {"tc_bwd_a<half,64,64>", (const void*)tc::tc_bwd_a_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdASmem<64, 64>::kBytes},
       {"reduce_chunks", (const void*)reduce_chunks_kernel, kThreads, 0},

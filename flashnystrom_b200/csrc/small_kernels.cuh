@@ -429,11 +429,15 @@ struct CombineSlabParams {
   int m, D;
 };
 
-constexpr int kSlabMaxChunks = 20;   // chunks merged with every load in flight; more run in rounds
+// Chunks merged with every load in flight; more run in rounds.  Every round costs its full width in loads and
+// exponentials, so there are three widths and a launch takes the smallest that holds its chunks: with one chunk (more
+// slices than CTAs) the widest took 72 us for 512 slices, most of it for entries that do not exist.
+constexpr int kSlabMaxChunks = 20;
 
 // Dynamic shared memory: K2inv with padded rows, m (m + 1) floats (combine_slab_smem).
 __host__ __device__ inline size_t combine_slab_smem(int m) { return sizeof(float) * (size_t)m * (m + 1); }
 
+template <int CH>
 __global__ void __launch_bounds__(kThreads) combine_slab_kernel(CombineSlabParams p) {
   extern __shared__ float sK[];                        // [m][m + 1]
   __shared__ __align__(16) float sB[kMaxM * 16];
@@ -443,7 +447,9 @@ __global__ void __launch_bounds__(kThreads) combine_slab_kernel(CombineSlabParam
   const int slab = blockIdx.y, t = threadIdx.x, q = t & 3;
   const int m = p.m, D = p.D, nc = p.nchunk, d0 = 16 * slab + 4 * q, ms = m + 1;
   const float* k2inv = p.k2inv + bh * m * m;
-  for (int idx = t; idx < m * m; idx += kThreads) sK[(idx / m) * ms + idx % m] = k2inv[idx];
+#pragma unroll 4
+  for (int r = t >> 5; r < m; r += kThreads / 32)
+    for (int c = t & 31; c < m; c += 32) sK[r * ms + c] = k2inv[r * m + c];
   // thread t merges landmark rows t >> 2 and, with more than 64 landmarks, (t >> 2) + 64
   for (int l = t >> 2; l < kMaxM; l += 64) {
     float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -451,29 +457,29 @@ __global__ void __launch_bounds__(kThreads) combine_slab_kernel(CombineSlabParam
       const float* pacc = p.part_acc + bh * p.acc_bh_stride + (size_t)l * D + d0;
       const float* pmax = p.part_max + bh * p.vec_bh_stride + l;
       const float* psum = p.part_sum + bh * p.vec_bh_stride + l;
-      // with at most kSlabMaxChunks chunks (the usual case) the maxima come out of the one batch of
+      // with at most CH chunks (the usual case) the maxima come out of the one batch of
       // loads below; otherwise a first sweep finds them
       float M = -INFINITY;
-      if (nc > kSlabMaxChunks)
+      if (nc > CH)
         for (int c = 0; c < nc; ++c) M = fmaxf(M, pmax[c * p.vec_chunk_stride]);
       float Lsum = 0.f;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int c0 = 0; c0 < nc; c0 += kSlabMaxChunks) {
-        float4 x[kSlabMaxChunks];
-        float wgt[kSlabMaxChunks], ps[kSlabMaxChunks];
+      for (int c0 = 0; c0 < nc; c0 += CH) {
+        float4 x[CH];
+        float wgt[CH], ps[CH];
 #pragma unroll
-        for (int i = 0; i < kSlabMaxChunks; ++i) {
+        for (int i = 0; i < CH; ++i) {
           const int c = min(c0 + i, nc - 1);
           x[i] = *reinterpret_cast<const float4*>(pacc + (size_t)c * p.acc_chunk_stride);
           wgt[i] = pmax[c * p.vec_chunk_stride];
           ps[i] = psum[c * p.vec_chunk_stride];
         }
-        if (nc <= kSlabMaxChunks) {
+        if (nc <= CH) {
 #pragma unroll
-          for (int i = 0; i < kSlabMaxChunks; ++i) M = fmaxf(M, wgt[i]);   // entries past nc repeat the last chunk
+          for (int i = 0; i < CH; ++i) M = fmaxf(M, wgt[i]);   // entries past nc repeat the last chunk
         }
 #pragma unroll
-        for (int i = 0; i < kSlabMaxChunks; ++i) {
+        for (int i = 0; i < CH; ++i) {
           const float w = (c0 + i < nc) ? expf(wgt[i] - M) : 0.f;
           Lsum = fmaf(w, ps[i], Lsum);
           acc.x = fmaf(w, x[i].x, acc.x); acc.y = fmaf(w, x[i].y, acc.y);
