@@ -436,7 +436,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   // More than 64 landmarks: the pseudoinverse takes a cluster of two SMs per slice for longer than the column
   // pass lasts, so up to a quarter of the SMs' worth of slices the two run side by side, the column pass on the
   // SMs that are left.  Four more stay free: a cluster needs both its SMs in one GPC.
-  const bool mid_tc = !smem_ns && ns_on_tensor_cores(a.shape.flags);
+  const bool mid_tc = !smem_ns && !(a.shape.flags & FNB_FLAG_FORCE_GENERIC);
   const bool side_mid = mid_tc && (use_tc || use_sx) && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
   tc::TcSched sch_fb = sch, sch_fc = sch;
   if (side_mid) {
@@ -717,7 +717,7 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
   const bool side_ns = fused_mid && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
   // With more than 64 landmarks the same holds where the column pass parks its tiles (the other passes need dKt
   // inside the column pass): two SMs per slice for the pseudoinverse backward, four more kept free for its clusters.
-  const bool mid_tc = !smem_ns && ns_on_tensor_cores(a.shape.flags);
+  const bool mid_tc = !smem_ns && !(a.shape.flags & FNB_FLAG_FORCE_GENERIC);
   const bool side_mid = mid_tc && use_tc && !L.prof && allow_inner_fork && p.BH * 4 <= sms;
   tc::TcSched sch_b = sch;
   if (side_ns || side_mid) {
