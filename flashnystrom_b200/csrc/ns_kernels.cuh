@@ -2,7 +2,7 @@
 // cores, no cuBLAS) for num_landmarks <= 64.  One CTA of 256 threads per (b,h) slice; every
 // (m x m) matrix lives in a zero-padded 64 x 64 shared buffer with row stride 68, so all loops
 // have compile-time bounds and every operand access is a conflict-free 16-byte load.
-// Larger landmark counts use the global-memory version in mid_kernels.cuh.
+// Larger landmark counts use mid_tc.cuh (mid_kernels.cuh on the CUDA cores).
 #pragma once
 #include "common.cuh"
 #include "mid_kernels.cuh"

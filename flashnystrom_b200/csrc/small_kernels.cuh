@@ -431,7 +431,7 @@ struct CombineSlabParams {
 
 // Chunks merged with every load in flight; more run in rounds.  Every round costs its full width in loads and
 // exponentials, so there are three widths and a launch takes the smallest that holds its chunks: with one chunk (more
-// slices than CTAs) the widest took 72 us for 512 slices, most of it for entries that do not exist.
+// slices than CTAs) the widest took 72 us for 512 slices, most of it for entries that do not exist; the smallest 39.
 constexpr int kSlabMaxChunks = 20;
 
 // Dynamic shared memory: K2inv with padded rows, m (m + 1) floats (combine_slab_smem).
