@@ -74,30 +74,35 @@ __device__ __forceinline__ void load_small(float* dst, int ld, const float* src,
 // ------------------------------------------------------------------------------------------
 // Pass 1: raw segment sums of Q and K (landmark pooling).
 // Work items (which, bh, landmark, chunk) are walked by a grid-stride loop, so the grid can be
-// sized to the machine.  out[which][bh][l][c][D].  G warps share an item: one where the items are
-// short, so that an SM has 32 independent ones in flight and none waits at a barrier, the
-// whole CTA (G = 8) where they are long.  Either way a lane has eight predicated 16-byte loads
-// in flight, also for the last rows of an item.
+// sized to the machine.  out[which][bh][l][c][D].  A whole CTA shares an item where the items are
+// long (G = 8 warps); where they are short one warp does what the eight would have done, so that
+// an SM has 16 independent items in flight and none waits at a barrier.
+// The order of the additions is the same in both: of the rows that eight warps load at once, warp w holds the w-th
+// group; every lane adds up its rows in order, lanes that hold the same columns are added by doubling distance,
+// and the eight groups in order.  The single warp keeps one accumulator per group (u), its eight loads in
+// flight being one of each group.  (With one accumulator for all of them a lane added up to 64 rows one after another
+// in place of 8, and the landmarks came out in another rounding.)
 // kContig: the slices are contiguous (row stride D, slice bh at bh * N * D); the addressing of the
 // streaming loop is then 32-bit and free of the run-time strides.
 // The items are counted in 32 bits (the host refuses more), and the segment length comes from the host: the
 // four 64-bit divisions that numbering an item takes otherwise are as long as the loads of a short one.
 template <class T, bool kContig, int G>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, G == 1 ? 2 : 4)
 landmark_partial_kernel(const T* __restrict__ q, const T* __restrict__ k, float* __restrict__ out,
                         uint32_t BH, int64_t N, int D, int m, int C, int64_t seg_N, int64_t seg, int64_t row_offset,
                         int H, int64_t row_stride, int64_t head_stride, int64_t batch_stride) {
-  constexpr int V = Vec16<T>::n, U = 8;
-  __shared__ float red[G > 1 ? kThreads / 32 * kMaxD : 1];
+  static_assert(G == 1 || G == kThreads / 32, "one warp or the whole CTA per item");
+  constexpr int V = Vec16<T>::n, W = kThreads / 32, A = G == 1 ? W : 1;   // A: accumulators of a lane per column
+  __shared__ __align__(16) float red_all[W * (G == 1 ? W : 1) * kMaxD];
   pdl_trigger();
   const uint32_t per_slice = (uint32_t)(m * C), per_which = BH * per_slice, items = 2 * per_which;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int vpr = D / V, rpw = 32 / vpr;                      // lanes per row, rows per load of a warp
   const int cv = lane % vpr, ro = lane / vpr;
   const int w = G > 1 ? warp : 0;
-  const int rows_it = G * rpw;                                // rows per load of the warps that share the item
-  const uint32_t first = G > 1 ? blockIdx.x : blockIdx.x * (kThreads / 32) + warp;
-  const uint32_t step = G > 1 ? gridDim.x : gridDim.x * (kThreads / 32);
+  const uint32_t first = G > 1 ? blockIdx.x : blockIdx.x * W + warp;
+  const uint32_t step = G > 1 ? gridDim.x : gridDim.x * W;
+  float* red = red_all + (G == 1 ? warp * W * D : 0);         // [W][D]: the sums of the eight groups
   pdl_wait();
   for (uint32_t item = first; item < items; item += step) {
     const int which = item >= per_which;
@@ -116,45 +121,84 @@ landmark_partial_kernel(const T* __restrict__ q, const T* __restrict__ k, float*
     int64_t r1 = r0 + per;
     if (r1 > start + len) r1 = start + len;
     const int64_t stride = kContig ? (int64_t)D : row_stride;
+    // load u of a step: the next group of rpw rows (one warp), or this warp's group of the u-th step (CTA)
     const T* ptr = slice + (r0 + w * rpw + ro) * stride + cv * V;
-    const int64_t adv = (int64_t)rows_it * stride;
+    const int between = G * rpw;
+    const int64_t adv = (int64_t)between * stride;
     int left = (int)(r1 - r0) - (w * rpw + ro);               // rows from this lane's first one to the end of the item
-    float acc[V];
+    float acc[A][V];
 #pragma unroll
-    for (int e = 0; e < V; ++e) acc[e] = 0.f;
-    for (; left > 0; left -= U * rows_it) {
-      uint4 raw[U];
+    for (int a = 0; a < A; ++a)
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int e = 0; e < V; ++e) acc[a][e] = 0.f;
+    for (; left > 0; left -= 8 * between) {
+      uint4 raw[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
         raw[u] = make_uint4(0, 0, 0, 0);                      // (zero bits are a zero in all three types)
-        if (left > u * rows_it) raw[u] = __ldcs(reinterpret_cast<const uint4*>(ptr));
+        if (left > u * between) raw[u] = __ldcs(reinterpret_cast<const uint4*>(ptr));
         ptr += adv;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
+      for (int u = 0; u < 8; ++u) {
         const T* e16 = reinterpret_cast<const T*>(&raw[u]);
 #pragma unroll
-        for (int e = 0; e < V; ++e) acc[e] += to_f<T>(e16[e]);
+        for (int e = 0; e < V; ++e) acc[A == 1 ? 0 : u][e] += to_f<T>(e16[e]);
       }
     }
     // lanes that hold the same columns are vpr apart
-    for (int o = vpr; o < 32; o <<= 1)
+    if constexpr (G == 1) {
+      // Eight groups are folded by halves: at each of the first three distances a lane keeps half of its groups and
+      // hands over the other half (8 V shuffles at most in place of 8 V per distance).
+      static_assert(W == 8, "eight groups");
+      int u0 = 0, n = 8;                                      // this lane's groups: u0 .. u0 + n - 1, in acc[0 .. n - 1]
 #pragma unroll
-      for (int e = 0; e < V; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-    float* dst = out + ((((size_t)which * BH + bh) * m + l) * C + c) * D;
-    if (G == 1) {
-      if (lane < vpr)
+      for (int s = 0; s < 3; ++s) {
+        const int o = vpr << s, half = 4 >> s;
+        if (o >= 32) continue;
+        const bool hi = (lane & o) != 0;
 #pragma unroll
-        for (int e = 0; e < V; e += 4) *reinterpret_cast<float4*>(dst + lane * V + e) = make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]);
+        for (int i = 0; i < half; ++i)
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            const float give = hi ? acc[i][e] : acc[i + half][e], keep = hi ? acc[i + half][e] : acc[i][e];
+            acc[i][e] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        n = half;
+        u0 += hi ? half : 0;
+      }
+      if (vpr == 2) {                                         // (head_dim 16, 16-bit: a fourth distance)
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[0][e] += __shfl_xor_sync(0xffffffffu, acc[0][e], 16);
+      }
+      __syncwarp();                                           // the previous item's sums have been read
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i < n && (vpr > 2 || lane < 16))
+#pragma unroll
+          for (int e = 0; e < V; e += 4)
+            *reinterpret_cast<float4*>(red + (u0 + i) * D + cv * V + e) = make_float4(acc[i][e], acc[i][e + 1], acc[i][e + 2], acc[i][e + 3]);
+      __syncwarp();
+      float* dst = out + ((((size_t)which * BH + bh) * m + l) * C + c) * D;
+      for (int d = lane; d < D; d += 32) {
+        float s = 0.f;
+#pragma unroll
+        for (int ww = 0; ww < W; ++ww) s += red[ww * D + d];
+        dst[d] = s;
+      }
     } else {
+      for (int o = vpr; o < 32; o <<= 1)
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[0][e] += __shfl_xor_sync(0xffffffffu, acc[0][e], o);
+      float* dst = out + ((((size_t)which * BH + bh) * m + l) * C + c) * D;
       if (lane < vpr)
 #pragma unroll
-        for (int e = 0; e < V; ++e) red[w * D + lane * V + e] = acc[e];
+        for (int e = 0; e < V; ++e) red[w * D + lane * V + e] = acc[0][e];
       __syncthreads();
       if (threadIdx.x < D) {
         float s = 0.f;
 #pragma unroll
-        for (int ww = 0; ww < kThreads / 32; ++ww) s += red[ww * D + threadIdx.x];
+        for (int ww = 0; ww < W; ++ww) s += red[ww * D + threadIdx.x];
         dst[threadIdx.x] = s;
       }
       __syncthreads();   // red is reused by the next item
