@@ -414,25 +414,23 @@ __device__ inline void pinv_forward_tc(Ctx& c, float* red, float* iterates, floa
 }
 
 // Row softmax of the scores in the padded buffer X, in place (rows and columns past m become zero), K2 and lse2 to
-// global memory.  Four adjacent lanes share a row, 16 columns each: two shuffles per reduction.
+// global memory.  Four adjacent lanes share a row, lane k the columns 4 i + k: the row sum is then the tree
+// of ns::softmax_rows (columns 32 apart, 16, 8 and 4 in the lane, 2 and 1 by shuffles), bit for bit, with two
+// shuffles per reduction in place of five.
 __device__ inline void softmax16(float* X, const ns::NsFwdParams& p, int64_t bh) {
-  const int m = p.m, r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
-  float* row = X + r * kLd + c0;
+  const int m = p.m, r = threadIdx.x >> 2, k = threadIdx.x & 3;
+  float* row = X + r * kLd;
   float v[16], mx = -INFINITY, sum;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float4 x = *reinterpret_cast<const float4*>(row + 4 * q);
-    v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
-  }
+  for (int i = 0; i < 16; ++i) v[i] = row[4 * i + k];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) if (c0 + i < m) mx = fmaxf(mx, v[i]);
+  for (int i = 0; i < 16; ++i) if (4 * i + k < m) mx = fmaxf(mx, v[i]);
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    v[i] = (r < m && c0 + i < m) ? expf(v[i] - mx) : 0.f;
+    v[i] = (r < m && 4 * i + k < m) ? expf(v[i] - mx) : 0.f;
   }
-  // (a tree: added up one by one the row sums were up to 20 % less precise)
   float part[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) part[i] = v[i] + v[i + 8];
@@ -441,23 +439,23 @@ __device__ inline void softmax16(float* X, const ns::NsFwdParams& p, int64_t bh)
 #pragma unroll
     for (int i = 0; i < o; ++i) part[i] += part[i + o];
   sum = part[0];
-  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
   sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = r < m ? v[i] / sum : 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) *reinterpret_cast<float4*>(row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  for (int i = 0; i < 16; ++i) row[4 * i + k] = r < m ? v[i] / sum : 0.f;
+  __syncwarp();                              // a row's four lanes are in one warp
   if (r < m) {
+    const int c0 = 16 * k;
     float* g = p.k2 + bh * m * m + (size_t)r * m + c0;
     if ((m & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (c0 + 4 * q < m) *reinterpret_cast<float4*>(g + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        if (c0 + 4 * q < m) *reinterpret_cast<float4*>(g + 4 * q) = *reinterpret_cast<const float4*>(row + c0 + 4 * q);
     } else {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) if (c0 + i < m) g[i] = v[i];
+      for (int i = 0; i < 16; ++i) if (c0 + i < m) g[i] = row[c0 + i];
     }
-    if (c0 == 0) p.lse2[bh * m + r] = mx + logf(sum);
+    if (k == 0) p.lse2[bh * m + r] = mx + logf(sum);
   }
   ns::ns_sync();
 }

@@ -62,3 +62,35 @@ def test_segment_sums(cuda_device, BH, N, D, m, dtype, split_heads):
     for got, x in ((res[3], q), (res[4], k)):
         want = _segment_sums(x[0].float().numpy(), m, elems) * f
         assert np.array_equal(got[0].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("m", [1, 3, 31, 33, 62, 64])
+def test_softmax2_rows(cuda_device, m):
+    """Scores that every product forms exactly (one dimension, few bits), so that K2 and lse2 follow from expf, logf
+    and the order of the row sum: columns 32, 16, 8, 4, 2 and 1 apart."""
+    from flashnystrom_b200 import _C
+    D, scale = 64, np.float32(64 ** -0.25)
+
+    def preimage(t):                         # the float x with fl(x * scale) == t
+        x = np.float32(t / float(scale))
+        for y in (x, np.nextafter(x, np.float32(np.inf)), np.nextafter(x, np.float32(-np.inf))):
+            if np.float32(y * scale) == t:
+                return y
+        return None
+    rng = np.random.RandomState(m)
+    exact = [t for t in (np.arange(-96, 97) / 32).astype(np.float32) if preimage(t) is not None]
+    a, b = rng.choice(exact, m), rng.choice(exact, m)
+    q, k = torch.zeros(1, 1, m, D), torch.zeros(1, 1, m, D)
+    q[0, 0, :, 0] = torch.tensor([preimage(t) for t in a])
+    k[0, 0, :, 0] = torch.tensor([preimage(t) for t in b])
+    res = _C.forward(q.cuda(), k.cuda(), k.cuda(), m, 1)
+    s = torch.zeros(m, 64, device="cuda")
+    s[:, :m] = torch.tensor(np.outer(a, b), device="cuda")
+    live = torch.arange(64, device="cuda") < m
+    mx = torch.where(live, s, s.new_tensor(float("-inf"))).max(1, keepdim=True).values
+    e = torch.where(live, torch.exp(s - mx), s.new_zeros(()))
+    t = e
+    for o in (32, 16, 8, 4, 2, 1):
+        t = t[:, :o] + t[:, o:2 * o]
+    assert torch.equal(res[11][0, 0], (e / t)[:, :m])
+    assert torch.equal(res[8][0, 0], (mx + torch.log(t))[:, 0])
