@@ -1,21 +1,22 @@
 // Streaming passes at FP32-equivalent precision on the sm_100a tensor cores: full-precision inputs, and
-// the 16-bit shapes whose probabilities stay in more than 16 bits (head_dim 64 with more than 64
-// landmarks, head_dim 16 and 32).
+// the 16-bit shapes whose landmark matrices, probabilities and softmax Jacobians stay in FP32 (head_dim 64
+// with more than 64 landmarks, head_dim 16 and 32).
 //
 // Every FP32 operand is a short sum of bf16 terms (x = x0 + x1 + ..., each term the bf16 rounding of
 // what the previous ones left over), and a product is the sum of the partial products whose weight
 // matters.  bf16 has the FP32 exponent range, so no operand needs scaling.
 //   inputs           bf16: 1 term, fp16: 2, fp32: 3 (exact in all three cases)
-//   landmark matrices, probabilities, softmax Jacobians: 3 terms (24 bits) for fp32 inputs; 2 terms
-//                    (16 bits, a sixteenth of the last place of an fp16 result) for 16-bit inputs
-// so a product takes six MMAs per K step for fp32, two or three for bf16 and fp16.
+//   landmark matrices, probabilities, softmax Jacobians: 3 terms (24 bits)
+// Of a product, the partial products of weight 2^-16 and up are formed: six MMAs per K step for fp32 operands,
+// five and three for fp16 and bf16 inputs; what is dropped is below 2^-25 of the sum of the products' magnitudes.
 //
 // One CTA of 16 warps per SM walks 128-row tiles of one (b,h) slice.  All warps stage the tile (global ->
 // registers -> terms -> swizzled shared memory), warp 0 issues the MMAs, all warps take the scores out
-// of tensor memory (thread = one row x a quarter of the landmark columns) and write the probabilities
+// of tensor memory (thread = one row x 16 columns of each block of 64 landmarks) and write the probabilities
 // back as operand tiles: K-major when they are contracted over landmarks, MN-major when over rows.
 // The next tile's rows are in flight in registers meanwhile, and its scores are issued together with
-// the products of the current tile wherever the buffers allow.
+// the products of the current tile wherever the buffers allow.  With more than 64 landmarks a probability tile
+// is 96 KB; where that leaves no room for the rest, its two blocks take turns in one of 48 KB.
 //
 // What bounds it: the MMAs of the fp32 passes (24 per 128 x 64 x 64 product at 48 cycles each, the time
 // their operands take through shared memory; a tile of the column pass of the backward needs 128 of
@@ -42,25 +43,28 @@ constexpr int kBlk = kTile * 128;   // bytes of a [128 rows x 64] bf16 block, ro
 template <class T> struct InTerms { static constexpr int n = 3; };
 template <> struct InTerms<__half> { static constexpr int n = 2; };
 template <> struct InTerms<bf16> { static constexpr int n = 1; };
-template <class T> struct OpTerms { static constexpr int n = std::is_same<T, float>::value ? 3 : 2; };
+constexpr int kTerms = 3;           // of landmark matrices, probabilities and softmax Jacobians
+constexpr int kSmemMax = 232448;
 
-// Shared-memory plan of one instantiation (bytes).  X: an input tile, P: a probability tile, L: a
-// landmark operand.  head_dim below 64 leaves the tail of the 128-byte rows unused.
+// Shared-memory plan of one instantiation (bytes).  X: an input tile, P: a probability tile of one block of 64
+// landmarks, L: a landmark operand.  head_dim below 64 leaves the tail of the 128-byte rows unused.
+// H*: blocks of a probability tile that are held at once.
 template <class T, int D, int MP>
 struct Plan {
-  static constexpr int NX = InTerms<T>::n, NP = OpTerms<T>::n;
-  static constexpr int kX = NX * kBlk, kP = NP * (MP / 64) * kBlk, kL = NP * MP * 128;
+  static constexpr int NX = InTerms<T>::n, NB = MP / 64;
+  static constexpr int kX = NX * kBlk, kP = kTerms * kBlk, kL = kTerms * MP * 128;
   static constexpr int kPitch = D * (int)sizeof(T) + 16;      // staged output row
-  static constexpr int kStage = kTile * kPitch;
-  static constexpr int kSmall = 4 * kTile * 4 + 4 * MP * 4 + 256;   // exchange words, per-landmark vectors, barriers
-  static constexpr int kVP = kX > kP ? kX : kP;                // V tile, then P tile
-  static_assert(kStage <= kP, "outputs are staged in a probability buffer");
-  static constexpr int kFwdB = kL + 3 * kX + kP + kSmall;
-  static constexpr int kFwdC = 2 * kL + kX + kP + kSmall;
-  static constexpr int kBwdA = 2 * kL + 2 * kX + kP + kSmall;
-  static constexpr int kBwdB = 2 * kL + kX + kVP + kP + kSmall - 4 * kTile * 4;
-  static constexpr int kBwdC = 2 * kL + 2 * kX + kP + kSmall;
-  static_assert(kFwdB <= 232448 && kFwdC <= 232448 && kBwdA <= 232448 && kBwdB <= 232448 && kBwdC <= 232448, "shared memory");
+  static_assert(kTile * kPitch <= kP, "outputs are staged in a probability buffer");
+  static constexpr int kRed = 4 * kTile * 4, kVec = 2 * MP * 4, kBars = 256;   // exchange words, per-landmark vectors, barriers
+  static constexpr int fit(int rest) { return rest + NB * kP <= kSmemMax ? NB : 1; }
+  static constexpr int kFwdB0 = kL + 2 * kX + kRed + kVec + kBars, kHFwdB = fit(kFwdB0), kFwdB = kFwdB0 + kHFwdB * kP;
+  static constexpr int kRow0 = 2 * kL + kX + kRed + kBars;
+  static constexpr int kHFwdC = fit(kRow0), kFwdC = kRow0 + kHFwdC * kP;
+  static constexpr int kHBwdA = fit(kRow0 + kX), kBwdA = kRow0 + kX + kHBwdA * kP, kHBwdC = kHBwdA, kBwdC = kBwdA;
+  static constexpr int kHBwdB = 1, kBwdB = 2 * kL + kX + 2 * kP + kVec + kBars;    // V tile, then P tile; dS tile
+  static_assert(kX <= kP, "V takes the place of a probability tile");
+  static_assert(kHFwdB == NB && kHFwdC == NB, "the forward passes hold whole probability tiles");
+  static_assert(kFwdB <= kSmemMax && kFwdC <= kSmemMax && kBwdA <= kSmemMax && kBwdB <= kSmemMax, "shared memory");
 };
 
 // ---- terms ---------------------------------------------------------------------------------
@@ -82,8 +86,8 @@ __device__ __forceinline__ void split8(const float* v, uint4* w) {
   }
 }
 // Order of the three terms of a probability tile: (x1, x0, x2), so that both (x1, x0) and (x0, x2) are
-// neighbours and can be stacked along M (see contract()).
-template <int NP> __device__ __forceinline__ constexpr int slot_of(int term) { return NP == 3 ? (term == 0 ? 1 : term == 1 ? 0 : 2) : term; }
+// neighbours and can be stacked along M (see issue_contract()).
+__device__ __forceinline__ constexpr int slot_of(int term) { return term == 0 ? 1 : term == 1 ? 0 : 2; }
 
 // ---- input tiles: global -> registers -> terms in shared memory -----------------------------------
 template <class T, int D>
@@ -125,8 +129,8 @@ struct InTile {
   }
 };
 
-// (m x D) FP32 landmark matrix times mul -> NP term tiles of [MP rows x 128 B], rows >= m zero
-template <int D, int MP, int NP>
+// (m x D) FP32 landmark matrix times mul -> three term tiles of [MP rows x 128 B], rows >= m zero
+template <int D, int MP>
 __device__ __forceinline__ void put_landmarks(uint8_t* op, const float* src, int m, float mul) {
   for (int idx = threadIdx.x; idx < MP * D / 8; idx += kThr) {
     const int r = idx / (D / 8), ch = idx % (D / 8);
@@ -138,102 +142,122 @@ __device__ __forceinline__ void put_landmarks(uint8_t* op, const float* src, int
       x[0] = a.x * mul; x[1] = a.y * mul; x[2] = a.z * mul; x[3] = a.w * mul;
       x[4] = b.x * mul; x[5] = b.y * mul; x[6] = b.z * mul; x[7] = b.w * mul;
     }
-    uint4 w[NP];
-    split8<NP>(x, w);
+    uint4 w[kTerms];
+    split8<kTerms>(x, w);
 #pragma unroll
-    for (int t = 0; t < NP; ++t) *reinterpret_cast<uint4*>(op + t * (MP * 128) + sw128_offset(r, ch)) = w[t];
+    for (int t = 0; t < kTerms; ++t) *reinterpret_cast<uint4*>(op + t * (MP * 128) + sw128_offset(r, ch)) = w[t];
   }
 }
 
-// NC consecutive columns col0.. of row r of a probability tile
-template <int NC, int MP, int NP>
-__device__ __forceinline__ void put_probs(uint8_t* tile, int r, int col0, const float* v) {
+// 16 values, columns 16 group .. of block b of row r, -> a probability tile of HB blocks ([term][block][128 rows x 128 B])
+template <int HB>
+__device__ __forceinline__ void put_probs(uint8_t* tile, int r, int b, int group, const float* v) {
 #pragma unroll
-  for (int c = 0; c < NC / 8; ++c) {
-    uint4 w[NP];
-    split8<NP>(v + 8 * c, w);
-    const int cc = (col0 >> 3) + c;
-    const uint32_t off = (uint32_t)(cc >> 3) * kBlk + sw128_offset(r, cc & 7);
+  for (int c = 0; c < 2; ++c) {
+    uint4 w[kTerms];
+    split8<kTerms>(v + 8 * c, w);
+    const uint32_t off = (uint32_t)b * kBlk + sw128_offset(r, group * 2 + c);
 #pragma unroll
-    for (int t = 0; t < NP; ++t) *reinterpret_cast<uint4*>(tile + slot_of<NP>(t) * ((MP / 64) * kBlk) + off) = w[t];
+    for (int t = 0; t < kTerms; ++t) *reinterpret_cast<uint4*>(tile + slot_of(t) * (HB * kBlk) + off) = w[t];
   }
 }
 
 // ---- products (warp-uniform; one elected lane issues) ------------------------------------------------
-// scores (128 x MP) = X (128 x D) L^T
-template <int D, int MP, int NX, int NP>
+// The tensor core truncates when it adds to an accumulator.  So the small partial products go first, and the K steps
+// of the leading one may be spread over G accumulators of their own (column groups of the result's width), which the
+// epilogue adds in FP32.
+// scores (128 x MP) = X (128 x D) L^T, groups MP columns apart
+template <int D, int G> __host__ __device__ constexpr int score_groups() { return G < D / 16 ? G : D / 16; }
+template <int D, int MP, int NX, int G>
 __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l) {
   constexpr uint32_t idesc = make_idesc<bf16>(kTile, MP, false, false);
+  constexpr int K = D / 16, GE = score_groups<D, G>();
   bool acc = false;
 #pragma unroll
-  for (int s = NP - 1; s >= 0; --s)            // small terms first
+  for (int s = kTerms - 1; s >= 0; --s)
 #pragma unroll
     for (int i = 0; i < NX; ++i) {
       const int j = s - i;
-      if (j < 0 || j >= NP) continue;
+      if (j < 0 || j >= kTerms) continue;
 #pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        umma_elect(d, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc, acc);
+      for (int k = 0; k < K; ++k) {
+        const int g = s == 0 ? k * GE / K : 0;
+        const bool first = g > 0 && (k - 1) * GE / K != g;
+        umma_elect(d + g * MP, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc,
+                   g > 0 ? !first : acc);
         acc = true;
       }
     }
 }
-// rows (128 x D) = P (128 x MP) L (MP x D).  This product and the next always run with N = 64, the width
-// of a swizzled block: for a smaller head_dim the columns past D hold nothing and are never read.
-template <int MP, int NP>
-__device__ __forceinline__ void issue_rows(uint32_t d, uint32_t p, uint32_t l) {
+// rows (128 x D) = P L over the HB blocks of landmarks from blk on, which the tile p holds; groups 64 columns apart.
+// This product and the next always run with N = 64, the width of a swizzled block: for a smaller head_dim the columns
+// past D hold nothing and are never read.
+template <int MP, int HB, int G>
+__device__ __forceinline__ void issue_rows(uint32_t d, uint32_t p, uint32_t l, int blk) {
   constexpr uint32_t idesc = make_idesc<bf16>(kTile, 64, false, true);
+  constexpr int K = HB * 4;
   bool acc = false;
 #pragma unroll
-  for (int s = NP - 1; s >= 0; --s)
+  for (int s = kTerms - 1; s >= 0; --s)
 #pragma unroll
     for (int i = 0; i <= s; ++i) {
-      const uint32_t pt = p + slot_of<NP>(i) * ((MP / 64) * kBlk), lt = l + (s - i) * (MP * 128);
+      const uint32_t pt = p + slot_of(i) * (HB * kBlk), lt = l + (s - i) * (MP * 128) + blk * (64 * 128);
 #pragma unroll
-      for (int k = 0; k < MP / 16; ++k) {
-        umma_elect(d, smem_desc_sw128(pt + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), smem_desc_sw128(lt + k * 2048, MP * 128, 1024), idesc, acc);
+      for (int k = 0; k < K; ++k) {
+        const int g = s == 0 ? k * G / K : 0;
+        const bool first = g > 0 && (k - 1) * G / K != g;
+        umma_elect(d + g * 64, smem_desc_sw128(pt + (k >> 2) * kBlk + (k & 3) * 32, 16, 1024), smem_desc_sw128(lt + k * 2048, MP * 128, 1024), idesc,
+                   g > 0 ? !first : acc);
         acc = true;
       }
     }
 }
-// tile sum (landmarks x D) = P^T (MP x 128) X (128 x D).  With 64 landmarks two terms of P are stacked along M
-// (lanes 0..63 and 64..127, added when the sum is read); the one partial product of three-term operands
-// that this cannot place, x2 * X0, goes to 64 columns of its own, lanes 64..127.
-// The tensor core truncates when it adds to an accumulator, and a run of such additions at full magnitude
-// drifts by about 2^-25 each (bmat was off by 5e-5 after 128 tiles).  So the small terms go first, and the
-// tile sums are added up over tiles with ordinary FP32 additions (add_tile_sum).
-template <int MP, int NX, int NP>
+// tile sum (landmarks x D) = P^T X (128 x D), groups 64 columns apart.
+// A tile of one block: two terms of P are stacked along M (lanes 0..63 and 64..127, added when the sum is read); the
+// one partial product that this cannot place, x2 * X0, goes to the 64 columns behind the groups, lanes 64..127.
+// A tile of two blocks: the lanes are the landmarks.
+// A run of additions at full magnitude drifts by about 2^-25 each (bmat was off by 5e-5 after 128 tiles in one accumulator),
+// so the tile sums are added up over tiles with ordinary FP32 additions (add_tile_sum).
+template <int HB, int NX, int G>
 __device__ __forceinline__ void issue_contract(uint32_t d, uint32_t p, uint32_t x) {
   constexpr uint32_t idesc = make_idesc<bf16>(128, 64, true, true);
-  if (MP == 64) {
+  constexpr int K = kTile / 16;
+  bool acc = false;
+  if (HB == 1) {
 #pragma unroll
     for (int j = NX - 1; j >= 0; --j)
 #pragma unroll
-      for (int k = 0; k < kTile / 16; ++k)
-        umma_elect(d, smem_desc_sw128(p + k * 2048, kBlk, 1024), smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc, j < NX - 1 || k > 0);
-    if (NP == 3) {
+      for (int k = 0; k < K; ++k) {
+        const int g = j == 0 ? k * G / K : 0;
+        const bool first = g > 0 && (k - 1) * G / K != g;
+        umma_elect(d + g * 64, smem_desc_sw128(p + k * 2048, kBlk, 1024), smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc,
+                   g > 0 ? !first : acc);
+        acc = true;
+      }
 #pragma unroll
-      for (int k = 0; k < kTile / 16; ++k)
-        umma_elect(d + 64, smem_desc_sw128(p + kBlk + k * 2048, kBlk, 1024), smem_desc_sw128(x + k * 2048, kBlk, 1024), idesc, k > 0);
-    }
+    for (int k = 0; k < K; ++k)
+      umma_elect(d + G * 64, smem_desc_sw128(p + kBlk + k * 2048, kBlk, 1024), smem_desc_sw128(x + k * 2048, kBlk, 1024), idesc, k > 0);
   } else {
-    bool a = false;
 #pragma unroll
-    for (int s = NP - 1; s >= 0; --s)
+    for (int s = kTerms - 1; s >= 0; --s)
 #pragma unroll
       for (int j = 0; j < NX; ++j) {
         const int i = s - j;
-        if (i < 0 || i >= NP) continue;
+        if (i < 0 || i >= kTerms) continue;
 #pragma unroll
-        for (int k = 0; k < kTile / 16; ++k) {
-          umma_elect(d, smem_desc_sw128(p + slot_of<NP>(i) * (2 * kBlk) + k * 2048, kBlk, 1024),
-                     smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc, a);
-          a = true;
+        for (int k = 0; k < K; ++k) {
+          const int g = s == 0 ? k * G / K : 0;
+          const bool first = g > 0 && (k - 1) * G / K != g;
+          umma_elect(d + g * 64, smem_desc_sw128(p + slot_of(i) * (HB * kBlk) + k * 2048, kBlk, 1024),
+                     smem_desc_sw128(x + j * kBlk + k * 2048, kBlk, 1024), idesc, g > 0 ? !first : acc);
+          acc = true;
         }
       }
   }
 }
-template <int MP, int NP> __host__ __device__ constexpr int acc_cols() { return (MP == 64 && NP == 3) ? 128 : 64; }
+// tensor-memory columns of a tile sum, and of the running sums of MP landmarks
+template <int HB, int G> __host__ __device__ constexpr int tile_cols() { return 64 * (HB == 1 ? G + 1 : G); }
+template <int MP, int HB> __host__ __device__ constexpr int sum_cols() { return HB == 1 ? MP : 64; }
 __host__ __device__ constexpr uint32_t pow2_cols(int c) { return c <= 64 ? 64u : c <= 128 ? 128u : c <= 256 ? 256u : 512u; }
 
 // ---- tensor memory -> registers, NC columns of this warp's 32 lanes ------------------------------------
@@ -272,7 +296,7 @@ __device__ __forceinline__ void st(uint32_t a, const float* v) {
 
 // ---- common frame of the kernels --------------------------------------------------------------------
 struct Frame {
-  uint64_t* bars;          // [3] completion barriers
+  uint64_t* bars;          // [3] completion barriers, [1] used on the way out after a wait gave up
   uint32_t tmem;
   Abort ab;
   uint32_t phase[3];
@@ -296,7 +320,7 @@ struct Frame {
 };
 __device__ __forceinline__ bool open_frame(Frame& f, uint8_t* smem, uint8_t* tail, const TcSched& sch, uint32_t cols, int* status, int where) {
   f.bars = reinterpret_cast<uint64_t*>(tail);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f.bars + 3);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f.bars + 4);
   int* abort_word = reinterpret_cast<int*>(tmem_slot + 1);
   if (smem_u32(smem) & 1023u) {
     if (threadIdx.x == 0 && status) atomicCAS(status, 0, (kStatusSmemAlign << 24) | where);
@@ -313,7 +337,7 @@ __device__ __forceinline__ bool open_frame(Frame& f, uint8_t* smem, uint8_t* tai
   f.first = f.chunk * sch.tiles_per_chunk;
   f.count = max(0, min(sch.tiles_per_chunk, tiles - f.first));
   if (threadIdx.x == 0) {
-    for (int b = 0; b < 3; ++b) mbar_init(f.bars + b, 1);
+    for (int b = 0; b < 4; ++b) mbar_init(f.bars + b, 1);
     *abort_word = 0;
     fence_mbar_init();
   }
@@ -332,6 +356,11 @@ __device__ __forceinline__ bool open_frame(Frame& f, uint8_t* smem, uint8_t* tai
 __device__ __forceinline__ void close_frame(const Frame& f, uint32_t cols) {
   tc_fence_before();
   __syncthreads();
+  if (f.warp == 0 && f.ab.raised()) {      // products may still be running: they end before their memory is given back
+    umma_commit_elect(f.bars + 3);
+    mbar_drain(f.bars + 3, 0);
+    __syncwarp();
+  }
   if (f.warp == 0) tmem_dealloc(f.tmem, cols);
 }
 
@@ -357,22 +386,60 @@ __device__ __forceinline__ void copy_out(T* slice, const uint8_t* stage, int pit
       *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(slice + (r0 + row) * D) + v * 16) = *reinterpret_cast<const uint4*>(stage + row * pitch + v * 16);
   }
 }
-// running sum (64 columns at `sum`) = factor * running sum + tile sum (at `tile`), FP32; with `first` the running sum
+// the sum of G column groups (`stride` apart) of this thread's row, 16 columns of each of NB blocks of 64
+template <int NB, int G>
+__device__ __forceinline__ void ld_scores(const Frame& f, uint32_t at, int stride, float* v) {
+  const uint32_t a = f.tmem + at + f.lane_base + f.group * 16;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) ld<16>(a + b * 64, v + 16 * b);
+#pragma unroll
+  for (int g = 1; g < G; ++g)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      float x[16];
+      ld<16>(a + g * stride + b * 64, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[16 * b + j] += x[j];
+    }
+  tmem_ld_wait();
+}
+// the sum of G column groups (64 apart) of this thread's row, its quarter of the D result columns
+template <int D, int G>
+__device__ __forceinline__ void ld_rows(const Frame& f, uint32_t at, float* o) {
+  constexpr int ND = D / 4;
+  const uint32_t a = f.tmem + at + f.lane_base + f.group * ND;
+  ld<ND>(a, o);
+#pragma unroll
+  for (int g = 1; g < G; ++g) {
+    float x[ND];
+    ld<ND>(a + g * 64, x);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < ND; ++j) o[j] += x[j];
+  }
+  tmem_ld_wait();
+}
+// running sum (64 columns at `sum`) += tile sum (at `tile`, see issue_contract), FP32; with `first` the running sum
 // starts at zero.  Each thread handles its lane and a quarter of the columns.
-template <int D, int MP, int NP>
+template <int D, int HB, int G>
 __device__ __forceinline__ void add_tile_sum(const Frame& f, uint32_t tile, uint32_t sum, bool first) {
   constexpr int NC = D / 4, ST = NC < 8 ? NC : 8;
   const uint32_t off = f.tmem + f.lane_base + f.group * NC;
 #pragma unroll
   for (int c = 0; c < NC; c += ST) {
-    float v[ST], x[ST], r[ST];
+    float v[ST], x[G][ST], r[ST];
     ld<ST>(off + tile + c, v);
-    if (MP == 64 && NP == 3) ld<ST>(off + tile + 64 + c, x);
+#pragma unroll
+    for (int g = 1; g < G; ++g) ld<ST>(off + tile + g * 64 + c, x[g]);
+    if (HB == 1) ld<ST>(off + tile + G * 64 + c, x[0]);
     if (!first) ld<ST>(off + sum + c, r);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < ST; ++j) {
-      if (MP == 64 && NP == 3) v[j] += f.row >= 64 ? x[j] : 0.f;
+      if (HB == 1) v[j] += f.row >= 64 ? x[0][j] : 0.f;
+#pragma unroll
+      for (int g = 1; g < G; ++g) v[j] += x[g][j];
       if (!first) v[j] += r[j];
     }
     st<ST>(off + sum + c, v);
@@ -394,36 +461,40 @@ __device__ __forceinline__ void scale_sum(const Frame& f, uint32_t sum, float fa
   }
   tmem_st_wait();
 }
-// running sum -> global (m x D) times mul; scratch: [64][D + 4] floats of shared memory
-template <int D, int MP>
+// running sums of MP landmarks -> global (m x D) times mul; scratch: [64][D + 4] floats of shared memory
+template <int D, int MP, int HB>
 __device__ __forceinline__ void store_sum(const Frame& f, uint32_t sum, float* scratch, float* dst, int m, float mul) {
   constexpr int NC = D / 4, LD = D + 4;
   const int c0 = f.group * NC;
-  float v[NC];
-  ld<NC>(f.tmem + sum + f.lane_base + c0, v);
-  tmem_ld_wait();
-  if constexpr (MP == 64) {
-    __syncthreads();
-    if (f.row >= 64) {
 #pragma unroll
-      for (int j = 0; j < NC; ++j) scratch[(f.row - 64) * LD + c0 + j] = v[j];
+  for (int b = 0; b < (HB == 1 ? MP / 64 : 1); ++b) {
+    float v[NC];
+    ld<NC>(f.tmem + sum + 64 * b + f.lane_base + c0, v);
+    tmem_ld_wait();
+    if constexpr (HB == 1) {
+      __syncthreads();
+      if (f.row >= 64) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) scratch[(f.row - 64) * LD + c0 + j] = v[j];
+      }
+      __syncthreads();
+      if (f.row < 64) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) v[j] += scratch[f.row * LD + c0 + j];
+      }
     }
-    __syncthreads();
-    if (f.row < 64) {
+    const int l = 64 * b + f.row;
+    if (l < m && f.row < HB * 64) {
 #pragma unroll
-      for (int j = 0; j < NC; ++j) v[j] += scratch[f.row * LD + c0 + j];
+      for (int j = 0; j < NC; j += 4)
+        *reinterpret_cast<float4*>(dst + l * D + c0 + j) = make_float4(v[j] * mul, v[j + 1] * mul, v[j + 2] * mul, v[j + 3] * mul);
     }
-  }
-  if (f.row < m && f.row < MP) {
-#pragma unroll
-    for (int j = 0; j < NC; j += 4)
-      *reinterpret_cast<float4*>(dst + f.row * D + c0 + j) = make_float4(v[j] * mul, v[j + 1] * mul, v[j + 2] * mul, v[j + 3] * mul);
   }
 }
 
 // ------------------------------------------------------------------------------------------
 // Forward column pass: partial Bmat = softmax(Qt (sK)^T) V over this CTA's rows with per-landmark
-// maximum and sum.  The exponent's reference moves only when a score exceeds it by 2^8 (one compare
+// maximum and sum.  The exponent's reference moves only when a score exceeds it by kMove (one compare
 // per element and one OR-barrier per tile decide it), so the accumulator is rarely rescaled.
 template <class T, int D, int MP>
 __global__ void __launch_bounds__(kThr, 1)
@@ -431,38 +502,38 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
                 float* __restrict__ part_acc, float* __restrict__ part_max, float* __restrict__ part_sum, TcSched sch,
                 int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4;
-  constexpr uint32_t kS = 0, kTileSum = MP, kSum = MP + acc_cols<MP, NP>(), kCols = pow2_cols(kSum + 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GS = score_groups<D, 1>(), GT = 1;
+  constexpr uint32_t kS = 0, kTileSum = GS * MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
+  static_assert(kSum + 64 <= 512, "tensor memory");
+  constexpr float kMove = 8.f;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_qt = smem;
   uint8_t* s_k = s_qt + L::kL;
-  uint8_t* s_v = s_k + L::kX;               // two buffers
-  uint8_t* s_p = s_v + 2 * L::kX;
-  float* s_red = reinterpret_cast<float*>(s_p + L::kP);      // [4][128]
+  uint8_t* s_v = s_k + L::kX;
+  uint8_t* s_p = s_v + L::kX;
+  float* s_red = reinterpret_cast<float*>(s_p + HB * L::kP);      // [4][128]
   float* s_ref = s_red + 4 * kTile;                          // [MP] reference, log2 domain
   float* s_alpha = s_ref + MP;
   pdl_trigger();
   Frame f;
-  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x4000)) return;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_alpha + MP), sch, kCols, status, 0x4000)) return;
   const T* kk = k + f.bh * sch.N * D;
   const T* vv = v + f.bh * sch.N * D;
-  const uint32_t a_qt = smem_u32(s_qt), a_k = smem_u32(s_k), a_p = smem_u32(s_p);
+  const uint32_t a_qt = smem_u32(s_qt), a_k = smem_u32(s_k), a_v = smem_u32(s_v), a_p = smem_u32(s_p);
   InTile<T, D> rk, rv;
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };   // landmark of this thread's value j
   rk.fetch(kk, row0(0), sch.N);
   rv.fetch(vv, row0(0), sch.N);
-  put_landmarks<D, MP, NP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
   if (threadIdx.x < MP) s_ref[threadIdx.x] = -INFINITY;
   rk.put(s_k);
-  rv.put(s_v);
   rk.fetch(kk, row0(1), sch.N);
-  rv.fetch(vv, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
     umma_commit_elect(f.bars + 0);
   }
-  const int c0 = f.group * NC;
   float sum[NC];
 #pragma unroll
   for (int j = 0; j < NC; ++j) sum[j] = 0.f;
@@ -470,15 +541,14 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
     const bool valid = row0(i) + f.row < sch.N;
     f.wait(0, 0x4100);
     float s[NC];
-    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
-    tmem_ld_wait();
+    ld_scores<NB, GS>(f, kS, MP, s);
     bool over = false;
 #pragma unroll
-    for (int j = 0; j < NC; ++j) over = over || (s[j] - s_ref[c0 + j] > 8.f);   // (a NaN score never raises it)
+    for (int j = 0; j < NC; ++j) over = over || (s[j] - s_ref[col(j)] > kMove);   // (a NaN score never raises it)
     over = over && valid;
     if (i > 0) {
-      f.wait(1, 0x4200);                     // the product of the previous tile is done: P and its V are free
-      add_tile_sum<D, MP, NP>(f, kTileSum, kSum, i == 1);
+      f.wait(1, 0x4200);                     // the product of the previous tile is done: P and V are free
+      add_tile_sum<D, HB, GT>(f, kTileSum, kSum, i == 1);
     }
     if (__syncthreads_or(over)) {
       // tile maximum of every landmark, the new reference and the factor for what has been summed so far
@@ -486,7 +556,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
       for (int j = 0; j < NC; ++j) {
         float x = valid ? s[j] : -INFINITY;
         for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-        if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + c0 + j] = x;
+        if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + col(j)] = x;
       }
       __syncthreads();
       if (threadIdx.x < MP) {
@@ -498,43 +568,44 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
       }
       __syncthreads();
 #pragma unroll
-      for (int j = 0; j < NC; ++j) sum[j] *= s_alpha[c0 + j];
-      if (i > 0) scale_sum<D>(f, kSum, s_alpha[MP == 64 ? (f.row & 63) : f.row]);
+      for (int j = 0; j < NC; ++j) sum[j] *= s_alpha[col(j)];
+      if (i > 0) scale_sum<D>(f, kSum, s_alpha[HB == 1 ? (f.row & 63) : f.row]);
     }
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      s[j] = valid ? fast_exp2(s[j] - s_ref[c0 + j]) : 0.f;
+      s[j] = valid ? fast_exp2(s[j] - s_ref[col(j)]) : 0.f;
       sum[j] += s[j];
     }
-    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) put_probs<HB>(s_p, f.row, b, f.group, s + 16 * b);
     rk.put(s_k);
-    rv.put(s_v + ((i + 1) & 1) * L::kX);
+    rv.put(s_v);
     f.publish();
     if (f.warp == 0) {
-      issue_contract<MP, NX, NP>(f.tmem + kTileSum, a_p, smem_u32(s_v) + (i & 1) * L::kX);
+      issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_v);
       umma_commit_elect(f.bars + 1);
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
         umma_commit_elect(f.bars + 0);
       }
     }
-    if (i + 2 < f.count) {
-      rk.fetch(kk, row0(i + 2), sch.N);
-      rv.fetch(vv, row0(i + 2), sch.N);
+    if (i + 1 < f.count) {
+      rv.fetch(vv, row0(i + 1), sch.N);
+      if (i + 2 < f.count) rk.fetch(kk, row0(i + 2), sch.N);
     }
   }
   const int64_t slot = blockIdx.x;
   if (f.count > 0) {
     f.wait(1, 0x4300);
-    add_tile_sum<D, MP, NP>(f, kTileSum, kSum, f.count == 1);
-    store_sum<D, MP>(f, kSum, reinterpret_cast<float*>(s_k), part_acc + slot * m * D, m, 1.f);
+    add_tile_sum<D, HB, GT>(f, kTileSum, kSum, f.count == 1);
+    store_sum<D, MP, HB>(f, kSum, reinterpret_cast<float*>(s_k), part_acc + slot * m * D, m, 1.f);
   }
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     float x = sum[j];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + c0 + j] = x;
+    if ((threadIdx.x & 31) == 0) s_red[(f.warp & 3) * kTile + col(j)] = x;
   }
   __syncthreads();
   if (threadIdx.x < m) {
@@ -552,43 +623,43 @@ __global__ void __launch_bounds__(kThr, 1)
 sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict__ lse1, const float* __restrict__ k_landmarks,
                 const float* __restrict__ step2, TcSched sch, int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4;
-  constexpr uint32_t kS = 0, kO = MP, kCols = pow2_cols(MP + 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdC, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1;
+  constexpr uint32_t kS = 0, kO = GS * MP, kCols = pow2_cols(kO + GO * 64);
+  static_assert(kO + GO * 64 <= 512, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
   uint8_t* s_st = s_kt + L::kL;
   uint8_t* s_q = s_st + L::kL;
   uint8_t* s_p = s_q + L::kX;               // probabilities, then the staged output tile
-  float* s_max = reinterpret_cast<float*>(s_p + L::kP);      // [4][128]: row maxima, then row sums
+  float* s_max = reinterpret_cast<float*>(s_p + HB * L::kP);      // [4][128]: row maxima, then row sums
   pdl_trigger();
   Frame f;
-  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_max + 4 * kTile + 4 * MP), sch, kCols, status, 0x4400)) return;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_max + 4 * kTile), sch, kCols, status, 0x4400)) return;
   const T* qq = q + f.bh * sch.N * D;
   T* oo = out + f.bh * sch.N * D;
   const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_p = smem_u32(s_p);
   InTile<T, D> rq;
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };
   rq.fetch(qq, row0(0), sch.N);
-  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
-  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rq.fetch(qq, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
     umma_commit_elect(f.bars + 0);
   }
-  const int c0 = f.group * NC;
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     f.wait(0, 0x4500);
     float s[NC];
-    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
-    tmem_ld_wait();
+    ld_scores<NB, GS>(f, kS, MP, s);
     float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      if (c0 + j >= m) s[j] = -INFINITY;
+      if (col(j) >= m) s[j] = -INFINITY;
       mx = fmaxf(mx, s[j]);
     }
     s_max[f.group * kTile + f.row] = mx;
@@ -600,16 +671,17 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
       s[j] = fast_exp2(s[j] - mx);
       sum += s[j];
     }
-    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) put_probs<HB>(s_p, f.row, b, f.group, s + 16 * b);
     rq.put(s_q);
     __syncthreads();                         // every thread has read the maxima
     s_max[f.group * kTile + f.row] = sum;
     f.publish();
     if (f.warp == 0) {
-      issue_rows<MP, NP>(f.tmem + kO, a_p, a_st);
+      issue_rows<MP, HB, GO>(f.tmem + kO, a_p, a_st, 0);
       umma_commit_elect(f.bars + 1);
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -619,8 +691,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
     const float inv = 1.f / sum;
     f.wait(1, 0x4600);
     float o[ND];
-    ld<ND>(f.tmem + kO + f.lane_base + f.group * ND, o);
-    tmem_ld_wait();
+    ld_rows<D, GO>(f, kO, o);
 #pragma unroll
     for (int j = 0; j < ND; ++j) o[j] *= inv;
     stage_row<T, D>(s_p, L::kPitch, f.row, f.group * ND, o);
@@ -635,11 +706,11 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
 // The softmax-1 Jacobian of a tile from its scores s and dP1 = dO step2^T (both in registers; s becomes
 // P1 and g becomes dS1): P1 = exp2(S - lse1 log2e), D1 = rowsum(P1 o dP1), dS1 = P1 o (dP1 - D1).
 template <int NC>
-__device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse2, bool valid, int c0, int m) {
+__device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse2, bool valid, int m) {
   float d1 = 0.f;
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
-    s[j] = (valid && c0 + j < m) ? fast_exp2(s[j] - lse2) : 0.f;
+    s[j] = (valid && (j >> 4) * 64 + f.group * 16 + (j & 15) < m) ? fast_exp2(s[j] - lse2) : 0.f;
     d1 = fmaf(s[j], g[j], d1);
   }
   s_red[f.group * kTile + f.row] = d1;
@@ -652,25 +723,29 @@ __device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, 
 // ------------------------------------------------------------------------------------------
 // First backward row pass: per-CTA partials of dstep2 = P1^T dO and dKt = dS1^T (sQ).  P1 and dS1 take
 // turns in one buffer: Q, dO, both landmark operands and one probability tile fill the SM.
+// kAlias: where only one of two blocks fits, their sums fill tensor memory, the tile sums lie where the scores were,
+// and the next scores wait for the last of them.
 template <class T, int D, int MP>
 __global__ void __launch_bounds__(kThr, 1)
 sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const float* __restrict__ lse1,
                 const float* __restrict__ k_landmarks, const float* __restrict__ step2, float* __restrict__ partA, TcSched sch,
                 int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, AC = acc_cols<MP, NP>();
-  constexpr uint32_t kS = 0, kG = MP, kTile1 = 2 * MP, kTile2 = kTile1 + AC, kSum1 = kTile2 + AC, kSum2 = kSum1 + 64, kCols = 512;
-  static_assert(kSum2 + 64 <= 512, "tensor memory");
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdA, NC = 16 * NB, GS = score_groups<D, 1>(), GT = 1;
+  constexpr bool kAlias = HB < NB;
+  constexpr uint32_t kS = 0, kG = GS * MP, kTileSum = kAlias ? 0 : 2 * GS * MP, kTileCols = tile_cols<HB, GT>();
+  constexpr uint32_t kSum1 = 512 - 2 * sum_cols<MP, HB>(), kSum2 = kSum1 + sum_cols<MP, HB>(), kCols = 512;
+  static_assert(kTileSum + kTileCols <= kSum1 && 2 * GS * MP <= kSum1, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
   uint8_t* s_st = s_kt + L::kL;
   uint8_t* s_q = s_st + L::kL;
   uint8_t* s_g = s_q + L::kX;
   uint8_t* s_p = s_g + L::kX;
-  float* s_red = reinterpret_cast<float*>(s_p + L::kP);
+  float* s_red = reinterpret_cast<float*>(s_p + HB * L::kP);
   pdl_trigger();
   Frame f;
-  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x4800)) return;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile), sch, kCols, status, 0x4800)) return;
   const T* qq = q + f.bh * sch.N * D;
   const T* gg = d_out + f.bh * sch.N * D;
   const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_g = smem_u32(s_g), a_p = smem_u32(s_p);
@@ -678,68 +753,77 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
   rq.fetch(qq, row0(0), sch.N);
   rg.fetch(gg, row0(0), sch.N);
-  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
-  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rg.put(s_g);
   rq.fetch(qq, row0(1), sch.N);
   rg.fetch(gg, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
-    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
     umma_commit_elect(f.bars + 0);
   }
-  const int c0 = f.group * NC;
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     const bool valid = row < sch.N, more = i + 1 < f.count;
     const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
     f.wait(0, 0x4900);
     float s[NC], g[NC];
-    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
-    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
-    tmem_ld_wait();
-    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, c0, m);
-    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
-    f.publish();
-    if (f.warp == 0) {
-      issue_contract<MP, NX, NP>(f.tmem + kTile1, a_p, a_g);
-      umma_commit_elect(f.bars + 1);
+    ld_scores<NB, GS>(f, kS, MP, s);
+    ld_scores<NB, GS>(f, kG, MP, g);
+    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, m);
+#pragma unroll
+    for (int b0 = 0; b0 < NB; b0 += HB) {
+#pragma unroll
+      for (int b = 0; b < HB; ++b) put_probs<HB>(s_p, f.row, b, f.group, s + 16 * (b0 + b));
+      f.publish();
+      if (f.warp == 0) {
+        issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_g);
+        umma_commit_elect(f.bars + 1);
+      }
+      f.wait(1, 0x4a00);                     // P1 (and, after the last block, dO) have been used
+      add_tile_sum<D, HB, GT>(f, kTileSum, kSum1 + 64 * b0, i == 0);
     }
-    f.wait(1, 0x4a00);                       // P1 and dO have been used
-    put_probs<NC, MP, NP>(s_p, f.row, c0, g);
     if (more) rg.put(s_g);
-    f.publish();
-    if (f.warp == 0) {
-      issue_contract<MP, NX, NP>(f.tmem + kTile2, a_p, a_q);
-      umma_commit_elect(f.bars + 2);
-      if (more) issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+#pragma unroll
+    for (int b0 = 0; b0 < NB; b0 += HB) {
+#pragma unroll
+      for (int b = 0; b < HB; ++b) put_probs<HB>(s_p, f.row, b, f.group, g + 16 * (b0 + b));
+      f.publish();
+      if (f.warp == 0) {
+        issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_q);
+        umma_commit_elect(f.bars + 2);
+        if (more && !kAlias) issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+      }
+      if (b0 == 0 && i + 2 < f.count) rg.fetch(gg, row0(i + 2), sch.N);
+      f.wait(2, 0x4b00);                     // dS1 (and, after the last block, Q) have been used
+      if (kAlias || b0 + HB < NB) add_tile_sum<D, HB, GT>(f, kTileSum, kSum2 + 64 * b0, i == 0);
     }
-    if (i + 2 < f.count) rg.fetch(gg, row0(i + 2), sch.N);
-    add_tile_sum<D, MP, NP>(f, kTile1, kSum1, i == 0);
-    f.wait(2, 0x4b00);                       // dS1 and Q have been used
     if (more) {
       rq.put(s_q);
       if (i + 2 < f.count) rq.fetch(qq, row0(i + 2), sch.N);
       f.publish();
       if (f.warp == 0) {
-        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+        if (kAlias) issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
         umma_commit_elect(f.bars + 0);
       }
     }
-    add_tile_sum<D, MP, NP>(f, kTile2, kSum2, i == 0);
+    if (!kAlias) add_tile_sum<D, HB, GT>(f, kTileSum, kSum2, i == 0);
   }
   float* pa = partA + (int64_t)blockIdx.x * 2 * m * D;
-  store_sum<D, MP>(f, kSum1, reinterpret_cast<float*>(s_q), pa, m, 1.f);
-  store_sum<D, MP>(f, kSum2, reinterpret_cast<float*>(s_q), pa + m * D, m, scale);
+  store_sum<D, MP, HB>(f, kSum1, reinterpret_cast<float*>(s_q), pa, m, 1.f);
+  store_sum<D, MP, HB>(f, kSum2, reinterpret_cast<float*>(s_q), pa + m * D, m, scale);
   close_frame(f, kCols);
 }
 
 // ------------------------------------------------------------------------------------------
 // Backward column pass: dV = P3^T dO3, dK = s (dS3^T Qt + dKt_tot[l(n)] / len_l), per-CTA partials of
 // dQt = dS3 (sK).  P3 takes V's place once the scores are formed; dV and dK leave through the
-// probability buffers.
+// probability buffers.  Two blocks of landmarks take turns in them.  The products lie where the scores were: the next
+// scores are issued after everything has been read.
 template <class T, int D, int MP>
 __global__ void __launch_bounds__(kThr, 1)
 sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ dk, T* __restrict__ dv,
@@ -747,42 +831,43 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
                 const float* __restrict__ dO3, const float* __restrict__ dkt_tot, float* __restrict__ partB, TcSched sch, int m,
                 float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4, AC = acc_cols<MP, NP>();
-  constexpr uint32_t kS = 0, kG = MP, kDv = 2 * MP, kDk = kDv + 64, kTileSum = kDk + 64, kSum = kTileSum + AC, kCols = 512;
-  static_assert(kSum + 64 <= 512, "tensor memory");
+  constexpr int NX = L::NX, NB = L::NB, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1, GT = 1;
+  constexpr uint32_t kS = 0, kG = GS * MP, kDv = 0, kDk = kDv + NB * GO * 64, kTileSum = kDk + NB * GO * 64, kSum = 512 - MP, kCols = 512;
+  static_assert(L::kHBwdB == 1 && 2 * GS * MP <= kSum && kTileSum + tile_cols<1, GT>() <= kSum, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_qt = smem;
   uint8_t* s_g3 = s_qt + L::kL;
   uint8_t* s_k = s_g3 + L::kL;
   uint8_t* s_p = s_k + L::kX;               // V, then P3, then the staged dV tile
-  uint8_t* s_ds = s_p + L::kVP;             // dS3, then the staged dK tile
+  uint8_t* s_ds = s_p + L::kP;              // dS3, then the staged dK tile
   float* s_l3 = reinterpret_cast<float*>(s_ds + L::kP);
   float* s_d3 = s_l3 + MP;
   pdl_trigger();
   Frame f;
-  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_l3 + 4 * MP), sch, kCols, status, 0x5000)) return;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_d3 + MP), sch, kCols, status, 0x5000)) return;
   const T* kk = k + f.bh * sch.N * D;
   const T* vv = v + f.bh * sch.N * D;
   const uint32_t a_qt = smem_u32(s_qt), a_g3 = smem_u32(s_g3), a_k = smem_u32(s_k), a_p = smem_u32(s_p), a_ds = smem_u32(s_ds);
   InTile<T, D> rk, rv;
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
+  auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };
   rk.fetch(kk, row0(0), sch.N);
   rv.fetch(vv, row0(0), sch.N);
-  put_landmarks<D, MP, NP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
-  put_landmarks<D, MP, NP>(s_g3, dO3 + f.bh * m * D, m, 1.f);
+  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_g3, dO3 + f.bh * m * D, m, 1.f);
   if (threadIdx.x < MP) {
     s_l3[threadIdx.x] = threadIdx.x < m ? lse3[f.bh * m + threadIdx.x] * kLog2e : INFINITY;   // exp2(S - inf) = 0
     s_d3[threadIdx.x] = threadIdx.x < m ? D3[f.bh * m + threadIdx.x] : 0.f;
   }
   Segments sg(sch.seg_N, m);
   const float* rows = dkt_tot + f.bh * m * D;
-  const int c0 = f.group * NC, d0 = f.group * ND;
+  const int d0 = f.group * ND;
   rk.put(s_k);
   rv.put(s_p);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
-    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_p, a_g3);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_p, a_g3);
     umma_commit_elect(f.bars + 0);
   }
   for (int i = 0; i < f.count; ++i) {
@@ -794,22 +879,28 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     }
     f.wait(0, 0x5100);
     float s[NC], g[NC];
-    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
-    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
-    tmem_ld_wait();
+    ld_scores<NB, GS>(f, kS, MP, s);
+    ld_scores<NB, GS>(f, kG, MP, g);
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      s[j] = valid ? fast_exp2(s[j] - s_l3[c0 + j]) : 0.f;
-      g[j] = s[j] * (g[j] - s_d3[c0 + j]);
+      s[j] = valid ? fast_exp2(s[j] - s_l3[col(j)]) : 0.f;
+      g[j] = s[j] * (g[j] - s_d3[col(j)]);
     }
-    put_probs<NC, MP, NP>(s_p, f.row, c0, s);
-    put_probs<NC, MP, NP>(s_ds, f.row, c0, g);
-    f.publish();
-    if (f.warp == 0) {
-      issue_rows<MP, NP>(f.tmem + kDv, a_p, a_g3);
-      issue_rows<MP, NP>(f.tmem + kDk, a_ds, a_qt);
-      issue_contract<MP, NX, NP>(f.tmem + kTileSum, a_ds, a_k);
-      umma_commit_elect(f.bars + 1);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (b > 0) {
+        f.wait(1, 0x5200);                   // the previous block's products are done: both buffers are free
+        add_tile_sum<D, 1, GT>(f, kTileSum, kSum + 64 * (b - 1), i == 0);
+      }
+      put_probs<1>(s_p, f.row, 0, f.group, s + 16 * b);
+      put_probs<1>(s_ds, f.row, 0, f.group, g + 16 * b);
+      f.publish();
+      if (f.warp == 0) {
+        issue_rows<MP, 1, GO>(f.tmem + kDv + b * GO * 64, a_p, a_g3, b);
+        issue_rows<MP, 1, GO>(f.tmem + kDk + b * GO * 64, a_ds, a_qt, b);
+        issue_contract<1, NX, GT>(f.tmem + kTileSum, a_ds, a_k);
+        umma_commit_elect(f.bars + 1);
+      }
     }
     const int l = valid ? sg.landmark_of(sch.row_offset + row) : 0;
     const float inv = scale / (float)sg.len(l);
@@ -819,13 +910,11 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
       const float4 x = *reinterpret_cast<const float4*>(rows + l * D + d0 + j);
       add[j] = x.x * inv; add[j + 1] = x.y * inv; add[j + 2] = x.z * inv; add[j + 3] = x.w * inv;
     }
-    f.wait(1, 0x5200);
+    f.wait(1, 0x5300);
     float o[ND];
-    ld<ND>(f.tmem + kDv + f.lane_base + d0, o);
-    tmem_ld_wait();
+    ld_rows<D, NB * GO>(f, kDv, o);
     stage_row<T, D>(s_p, L::kPitch, f.row, d0, o);
-    ld<ND>(f.tmem + kDk + f.lane_base + d0, o);
-    tmem_ld_wait();
+    ld_rows<D, NB * GO>(f, kDk, o);
 #pragma unroll
     for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);    // the operand carries s log2e
     stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
@@ -835,19 +924,19 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     tc_fence_after();
     copy_out<T, D>(dv + f.bh * sch.N * D, s_p, L::kPitch, row0(i), sch.N);
     copy_out<T, D>(dk + f.bh * sch.N * D, s_ds, L::kPitch, row0(i), sch.N);
-    add_tile_sum<D, MP, NP>(f, kTileSum, kSum, i == 0);
+    add_tile_sum<D, 1, GT>(f, kTileSum, kSum + 64 * (NB - 1), i == 0);
     if (more) {
       __syncthreads();                       // the staged tiles have been read
       rv.put(s_p);
       f.publish();
       if (f.warp == 0) {
-        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_k, a_qt);
-        issue_scores<D, MP, NX, NP>(f.tmem + kG, a_p, a_g3);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kG, a_p, a_g3);
         umma_commit_elect(f.bars + 0);
       }
     }
   }
-  store_sum<D, MP>(f, kSum, reinterpret_cast<float*>(s_k), partB + (int64_t)blockIdx.x * m * D, m, scale);
+  store_sum<D, MP, 1>(f, kSum, reinterpret_cast<float*>(s_k), partB + (int64_t)blockIdx.x * m * D, m, scale);
   close_frame(f, kCols);
 }
 
@@ -859,18 +948,20 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
                 const float* __restrict__ k_landmarks, const float* __restrict__ step2, const float* __restrict__ dqt_tot,
                 TcSched sch, int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NP = L::NP, NC = MP / 4, ND = D / 4;
-  constexpr uint32_t kS = 0, kG = MP, kO = 2 * MP, kCols = pow2_cols(2 * MP + 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdC, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1;
+  constexpr int GA = NB / HB * GO;           // column groups of dQ: GO for each turn
+  constexpr uint32_t kS = 0, kG = GS * MP, kO = 2 * GS * MP, kCols = pow2_cols(kO + GA * 64);
+  static_assert(kO + GA * 64 <= 512, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
   uint8_t* s_st = s_kt + L::kL;
   uint8_t* s_q = s_st + L::kL;
   uint8_t* s_g = s_q + L::kX;
   uint8_t* s_ds = s_g + L::kX;              // dS1, then the staged dQ tile
-  float* s_red = reinterpret_cast<float*>(s_ds + L::kP);
+  float* s_red = reinterpret_cast<float*>(s_ds + HB * L::kP);
   pdl_trigger();
   Frame f;
-  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile + 4 * MP), sch, kCols, status, 0x5400)) return;
+  if (!open_frame(f, smem, reinterpret_cast<uint8_t*>(s_red + 4 * kTile), sch, kCols, status, 0x5400)) return;
   const T* qq = q + f.bh * sch.N * D;
   const T* gg = d_out + f.bh * sch.N * D;
   const uint32_t a_kt = smem_u32(s_kt), a_st = smem_u32(s_st), a_q = smem_u32(s_q), a_g = smem_u32(s_g), a_ds = smem_u32(s_ds);
@@ -878,44 +969,48 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
   rq.fetch(qq, row0(0), sch.N);
   rg.fetch(gg, row0(0), sch.N);
-  put_landmarks<D, MP, NP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
-  put_landmarks<D, MP, NP>(s_st, step2 + f.bh * m * D, m, 1.f);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rg.put(s_g);
   rq.fetch(qq, row0(1), sch.N);
   rg.fetch(gg, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
-    issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
     umma_commit_elect(f.bars + 0);
   }
   Segments sg(sch.seg_N, m);
   const float* rows = dqt_tot + f.bh * m * D;
-  const int c0 = f.group * NC, d0 = f.group * ND;
+  const int d0 = f.group * ND;
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     const bool valid = row < sch.N, more = i + 1 < f.count;
     const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
     f.wait(0, 0x5500);
     float s[NC], g[NC];
-    ld<NC>(f.tmem + kS + f.lane_base + c0, s);
-    ld<NC>(f.tmem + kG + f.lane_base + c0, g);
-    tmem_ld_wait();
-    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, c0, m);   // (its barrier: the previous output tile has left s_ds)
-    put_probs<NC, MP, NP>(s_ds, f.row, c0, g);
-    if (more) {
-      rq.put(s_q);
-      rg.put(s_g);
-    }
-    f.publish();
-    if (f.warp == 0) {
-      issue_rows<MP, NP>(f.tmem + kO, a_ds, a_kt);
-      umma_commit_elect(f.bars + 1);
-      if (more) {
-        issue_scores<D, MP, NX, NP>(f.tmem + kS, a_q, a_kt);
-        issue_scores<D, MP, NX, NP>(f.tmem + kG, a_g, a_st);
-        umma_commit_elect(f.bars + 0);
+    ld_scores<NB, GS>(f, kS, MP, s);
+    ld_scores<NB, GS>(f, kG, MP, g);
+    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, m);   // (its barrier: the previous output tile has left s_ds)
+#pragma unroll
+    for (int b0 = 0; b0 < NB; b0 += HB) {
+      if (b0 > 0) f.wait(1, 0x5600);         // the previous block has been used
+#pragma unroll
+      for (int b = 0; b < HB; ++b) put_probs<HB>(s_ds, f.row, b, f.group, g + 16 * (b0 + b));
+      if (b0 == 0 && more) {
+        rq.put(s_q);
+        rg.put(s_g);
+      }
+      f.publish();
+      if (f.warp == 0) {
+        issue_rows<MP, HB, GO>(f.tmem + kO + b0 / HB * GO * 64, a_ds, a_kt, b0);
+        umma_commit_elect(f.bars + 1);
+        if (b0 == 0 && more) {
+          issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+          issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+          umma_commit_elect(f.bars + 0);
+        }
       }
     }
     if (i + 2 < f.count) {
@@ -930,10 +1025,9 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
       const float4 x = *reinterpret_cast<const float4*>(rows + l * D + d0 + j);
       add[j] = x.x * inv; add[j + 1] = x.y * inv; add[j + 2] = x.z * inv; add[j + 3] = x.w * inv;
     }
-    f.wait(1, 0x5600);
+    f.wait(1, 0x5700);
     float o[ND];
-    ld<ND>(f.tmem + kO + f.lane_base + d0, o);
-    tmem_ld_wait();
+    ld_rows<D, GA>(f, kO, o);
 #pragma unroll
     for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);
     stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);

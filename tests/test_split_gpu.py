@@ -4,8 +4,8 @@ as the yardstick: the same calls are made through both, and the split kernels ma
 from the oracle than the CUDA-core ones by more than what their operands drop.  fp32 operands keep 24
 bits in three bf16 terms; per product the dropped terms and the truncating accumulator stay below
 2^-22 = 2.4e-7, and the pseudoinverse (condition number up to a few tens here) amplifies it like it does the
-yardstick's own rounding: bound 1.5 x yardstick + 1e-6.  16-bit inputs: the results' own rounding (2^-12, 2^-9
-relative at most) dominates both; two-term operands add at most 2^-16 per element, amplified the same way:
+yardstick's own rounding: bound 1.5 x yardstick + 1e-6.  16-bit inputs: the landmark operands and the
+probabilities have the same 24 bits, the results' own rounding (2^-12, 2^-9 relative at most) dominates both sides:
 bound 1.05 x yardstick + 5e-5."""
 import pytest
 import torch
@@ -64,3 +64,29 @@ def test_moving_reference(cuda_device):
     for key in ("out", "dq", "dk", "dv", "bmat", "lse3"):
         # scores of about 100: 2^-24 of them is an error of 6e-6 in a probability, several of which meet in a gradient
         assert _rel(got[key], want[key]) <= 1e-4, (key, _rel(got[key], want[key]))
+
+
+@pytest.mark.parametrize("case", [
+    (1, 2, 128, 64, 65, 6, 0.0, 1.0, F16), (2, 4, 2000, 64, 128, 6, 0.0, 1.0, BF16), (1, 4, 2000, 64, 128, 6, 5.0, 3.0, F16),
+    (1, 4, 1500, 32, 100, 6, 0.0, 2.0, F16), (1, 4, 1000, 32, 64, 6, 0.0, 4.0, F16), (1, 4, 1500, 16, 64, 6, 0.0, 4.0, BF16),
+], ids=lambda c: "x".join(str(x) for x in c[:8]) + str(c[8])[6:])
+def test_16bit_inputs_keep_fp32_operands(cuda_device, case):
+    """The FP32 results of the forward passes (16-bit outputs would hide a loss) for 16-bit inputs, large scores among
+    them: no further from the oracle than the CUDA-core kernels, which multiply in FP32.  Every operand has 24 bits on
+    both sides; what differs is the order and rounding of the sums, bound 2 x yardstick.  (Operands of 16 bits are
+    4 to 18 x off, at scores of about 30 an error of 1e-4 in single probabilities.)"""
+    from flashnystrom_b200 import _C
+    B, H, N, D, m, J, kappa, qk, dtype = case
+    q, k, v, dO = O.make_inputs(B, H, N, D, seed=4, dtype=torch.float32)
+    q, k, v, dO = (q * qk).to(dtype), (k * qk).to(dtype), v.to(dtype), dO.to(dtype)
+    got = run_cuda(q, k, v, dO, m, J, kappa)
+    _C.set_force_generic(True)
+    try:
+        ref = run_cuda(q, k, v, dO, m, J, kappa)
+    finally:
+        _C.set_force_generic(False)
+    want = run_oracle(q, k, v, dO, m, J, kappa)
+    for key in ("bmat", "step2", "lse1", "lse3"):
+        a, b = _rel(got[key], want[key]), _rel(ref[key], want[key])
+        print(key, f"{a:.2e} {b:.2e}")
+        assert a <= 2 * b, (key, a, b)
