@@ -290,13 +290,17 @@ _plans = {}
 _MAX_PLANS = 256
 
 
-def _plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout):
+def _plan(lib, dev, B, H, N, D, m, J, dtype, kappa_star, layout):
+    """The plan of a call on `dev`.  Workspace sizes follow the SM count of the device that is current when they are
+    asked for, so that is `dev`, and every device has plans of its own."""
     if type(kappa_star) is not float and type(kappa_star) is not int:
-        return _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
-    key = (B, H, N, D, m, J, dtype, kappa_star, layout, _flags)
+        with _on_device(dev):
+            return _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
+    key = (dev.index, B, H, N, D, m, J, dtype, kappa_star, layout, _flags)
     plan = _plans.get(key)
     if plan is None:
-        plan = _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
+        with _on_device(dev):
+            plan = _Plan(lib, B, H, N, D, m, J, dtype, kappa_star, layout)
         if len(_plans) >= _MAX_PLANS:
             _plans.clear()
         _plans[key] = plan
@@ -325,7 +329,7 @@ def forward_packed(q, k, v, num_landmarks, newton_iter, kappa_star):
     if not (q.is_cuda and _is(q, shape, dtype, dev, lay) and _is(k, shape, dtype, dev, lay) and _is(v, shape, dtype, dev, lay)):
         for t, name in ((q, "q"), (k, "k"), (v, "v")):
             _check_big(t, name, shape, layout=lay)
-    plan = _plan(lib, B, H, N, D, m, J, dtype, kappa_star, lay)
+    plan = _plan(lib, dev, B, H, N, D, m, J, dtype, kappa_star, lay)
     with _on_device(dev):
         out = _empty_like_layout(q, lay)
         saved = torch.empty(plan.floats, dtype=torch.float32, device=dev)
@@ -349,11 +353,11 @@ def backward_packed(dO, q, k, v, saved, num_landmarks, newton_iter, kappa_star):
     lay = layout_of(q)
     if lay != _lib.FNB_LAYOUT_BNHD or not tc_eligible(dtype, D, m):
         lay = _lib.FNB_LAYOUT_BHND
-    if dO.is_cuda:
-        dO = _to_layout(dO, lay)
-    plan = _plan(lib, B, H, N, D, m, J, dtype, kappa_star, lay)
-    if not (dO.is_cuda and _is(q, shape, dtype, dev, lay) and _is(k, shape, dtype, dev, lay) and _is(v, shape, dtype, dev, lay)):
-        _check_big(dO, "dO", layout=lay)
+    if not dO.is_cuda:
+        _check_big(dO, "dO")
+    dO = _to_layout(dO, lay)
+    plan = _plan(lib, dev, B, H, N, D, m, J, dtype, kappa_star, lay)
+    if not (_is(q, shape, dtype, dev, lay) and _is(k, shape, dtype, dev, lay) and _is(v, shape, dtype, dev, lay)):
         for t, name in ((q, "q_s"), (k, "k_s"), (v, "v")):
             _check_big(t, name, shape, dtype, layout=lay)
     if saved.device != dev or saved.shape != (plan.floats,) or saved.dtype != torch.float32 or not saved.is_contiguous():
