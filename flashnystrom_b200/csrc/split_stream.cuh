@@ -15,7 +15,9 @@
 // of tensor memory (thread = one row x 16 columns of each block of 64 landmarks) and write the probabilities
 // back as operand tiles: K-major when they are contracted over landmarks, MN-major when over rows.
 // The next tile's rows are in flight in registers meanwhile, and its scores are issued together with
-// the products of the current tile wherever the buffers allow.  With more than 64 landmarks a probability tile
+// the products of the current tile wherever the buffers allow.  Exponentials and logarithms are expf and logf, as
+// in the CUDA-core kernels: ex2.approx of scores in units of log 2 is faster, but with the roundings of that scaling the
+// saved lse1 and the outputs were 25 to 50 % less exact.  With more than 64 landmarks a probability tile
 // is 96 KB; where that leaves no room for the rest, its two blocks take turns in one of 48 KB.
 //
 // What bounds it: the MMAs of the fp32 passes (24 per 128 x 64 x 64 product at 48 cycles each, the time
@@ -505,14 +507,14 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
   constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GS = score_groups<D, 1>(), GT = 1;
   constexpr uint32_t kS = 0, kTileSum = GS * MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
   static_assert(kSum + 64 <= 512, "tensor memory");
-  constexpr float kMove = 8.f;
+  constexpr float kMove = 6.f;                 // probabilities stay below e^6 = 403
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_qt = smem;
   uint8_t* s_k = s_qt + L::kL;
   uint8_t* s_v = s_k + L::kX;
   uint8_t* s_p = s_v + L::kX;
   float* s_red = reinterpret_cast<float*>(s_p + HB * L::kP);      // [4][128]
-  float* s_ref = s_red + 4 * kTile;                          // [MP] reference, log2 domain
+  float* s_ref = s_red + 4 * kTile;                          // [MP] reference
   float* s_alpha = s_ref + MP;
   pdl_trigger();
   Frame f;
@@ -525,7 +527,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
   auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };   // landmark of this thread's value j
   rk.fetch(kk, row0(0), sch.N);
   rv.fetch(vv, row0(0), sch.N);
-  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale);
   if (threadIdx.x < MP) s_ref[threadIdx.x] = -INFINITY;
   rk.put(s_k);
   rk.fetch(kk, row0(1), sch.N);
@@ -563,7 +565,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
         const int l = threadIdx.x;
         const float old = s_ref[l];
         const float mx = fmaxf(fmaxf(fmaxf(s_red[l], s_red[kTile + l]), fmaxf(s_red[2 * kTile + l], s_red[3 * kTile + l])), old);
-        s_alpha[l] = old == mx ? 1.f : fast_exp2(old - mx);
+        s_alpha[l] = old == mx ? 1.f : expf(old - mx);
         s_ref[l] = mx;
       }
       __syncthreads();
@@ -573,7 +575,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
     }
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      s[j] = valid ? fast_exp2(s[j] - s_ref[col(j)]) : 0.f;
+      s[j] = valid ? expf(s[j] - s_ref[col(j)]) : 0.f;
       sum[j] += s[j];
     }
 #pragma unroll
@@ -610,7 +612,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
   __syncthreads();
   if (threadIdx.x < m) {
     const int l = threadIdx.x;
-    part_max[slot * m + l] = s_ref[l] * kLn2;
+    part_max[slot * m + l] = s_ref[l];
     part_sum[slot * m + l] = (s_red[l] + s_red[kTile + l]) + (s_red[2 * kTile + l] + s_red[3 * kTile + l]);
   }
   close_frame(f, kCols);
@@ -642,7 +644,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
   auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };
   rq.fetch(qq, row0(0), sch.N);
-  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale);
   put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rq.fetch(qq, row0(1), sch.N);
@@ -668,7 +670,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
     float sum = 0.f;
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      s[j] = fast_exp2(s[j] - mx);
+      s[j] = expf(s[j] - mx);
       sum += s[j];
     }
 #pragma unroll
@@ -687,7 +689,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
     }
     if (i + 2 < f.count) rq.fetch(qq, row0(i + 2), sch.N);
     sum = (s_max[f.row] + s_max[kTile + f.row]) + (s_max[2 * kTile + f.row] + s_max[3 * kTile + f.row]);
-    if (f.group == 0 && row < sch.N) lse1[f.bh * sch.N + row] = (mx + log2f(sum)) * kLn2;
+    if (f.group == 0 && row < sch.N) lse1[f.bh * sch.N + row] = mx + logf(sum);
     const float inv = 1.f / sum;
     f.wait(1, 0x4600);
     float o[ND];
@@ -704,13 +706,13 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
 }
 
 // The softmax-1 Jacobian of a tile from its scores s and dP1 = dO step2^T (both in registers; s becomes
-// P1 and g becomes dS1): P1 = exp2(S - lse1 log2e), D1 = rowsum(P1 o dP1), dS1 = P1 o (dP1 - D1).
+// P1 and g becomes dS1): P1 = exp(S - lse1), D1 = rowsum(P1 o dP1), dS1 = P1 o (dP1 - D1).
 template <int NC>
-__device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse2, bool valid, int m) {
+__device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse, bool valid, int m) {
   float d1 = 0.f;
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
-    s[j] = (valid && (j >> 4) * 64 + f.group * 16 + (j & 15) < m) ? fast_exp2(s[j] - lse2) : 0.f;
+    s[j] = (valid && (j >> 4) * 64 + f.group * 16 + (j & 15) < m) ? expf(s[j] - lse) : 0.f;
     d1 = fmaf(s[j], g[j], d1);
   }
   s_red[f.group * kTile + f.row] = d1;
@@ -753,7 +755,7 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
   rq.fetch(qq, row0(0), sch.N);
   rg.fetch(gg, row0(0), sch.N);
-  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale);
   put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rg.put(s_g);
@@ -768,12 +770,12 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     const bool valid = row < sch.N, more = i + 1 < f.count;
-    const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
+    const float lse = valid ? lse1[f.bh * sch.N + row] : 0.f;
     f.wait(0, 0x4900);
     float s[NC], g[NC];
     ld_scores<NB, GS>(f, kS, MP, s);
     ld_scores<NB, GS>(f, kG, MP, g);
-    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, m);
+    softmax1_jacobian<NC>(f, s_red, s, g, lse, valid, m);
 #pragma unroll
     for (int b0 = 0; b0 < NB; b0 += HB) {
 #pragma unroll
@@ -853,10 +855,10 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
   auto col = [&](int j) { return (j >> 4) * 64 + f.group * 16 + (j & 15); };
   rk.fetch(kk, row0(0), sch.N);
   rv.fetch(vv, row0(0), sch.N);
-  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_qt, q_landmarks + f.bh * m * D, m, scale);
   put_landmarks<D, MP>(s_g3, dO3 + f.bh * m * D, m, 1.f);
   if (threadIdx.x < MP) {
-    s_l3[threadIdx.x] = threadIdx.x < m ? lse3[f.bh * m + threadIdx.x] * kLog2e : INFINITY;   // exp2(S - inf) = 0
+    s_l3[threadIdx.x] = threadIdx.x < m ? lse3[f.bh * m + threadIdx.x] : INFINITY;   // exp(S - inf) = 0
     s_d3[threadIdx.x] = threadIdx.x < m ? D3[f.bh * m + threadIdx.x] : 0.f;
   }
   Segments sg(sch.seg_N, m);
@@ -883,7 +885,7 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     ld_scores<NB, GS>(f, kG, MP, g);
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
-      s[j] = valid ? fast_exp2(s[j] - s_l3[col(j)]) : 0.f;
+      s[j] = valid ? expf(s[j] - s_l3[col(j)]) : 0.f;
       g[j] = s[j] * (g[j] - s_d3[col(j)]);
     }
 #pragma unroll
@@ -916,7 +918,7 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     stage_row<T, D>(s_p, L::kPitch, f.row, d0, o);
     ld_rows<D, NB * GO>(f, kDk, o);
 #pragma unroll
-    for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);    // the operand carries s log2e
+    for (int j = 0; j < ND; ++j) o[j] += add[j];    // (the operand carries s)
     stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
     if (more) rk.put(s_k);
     tc_fence_before();
@@ -969,7 +971,7 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
   auto row0 = [&](int i) { return (int64_t)(f.first + i) * kTile; };
   rq.fetch(qq, row0(0), sch.N);
   rg.fetch(gg, row0(0), sch.N);
-  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale * kLog2e);
+  put_landmarks<D, MP>(s_kt, k_landmarks + f.bh * m * D, m, scale);
   put_landmarks<D, MP>(s_st, step2 + f.bh * m * D, m, 1.f);
   rq.put(s_q);
   rg.put(s_g);
@@ -987,12 +989,12 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     const bool valid = row < sch.N, more = i + 1 < f.count;
-    const float lse2 = valid ? lse1[f.bh * sch.N + row] * kLog2e : 0.f;
+    const float lse = valid ? lse1[f.bh * sch.N + row] : 0.f;
     f.wait(0, 0x5500);
     float s[NC], g[NC];
     ld_scores<NB, GS>(f, kS, MP, s);
     ld_scores<NB, GS>(f, kG, MP, g);
-    softmax1_jacobian<NC>(f, s_red, s, g, lse2, valid, m);   // (its barrier: the previous output tile has left s_ds)
+    softmax1_jacobian<NC>(f, s_red, s, g, lse, valid, m);   // (its barrier: the previous output tile has left s_ds)
 #pragma unroll
     for (int b0 = 0; b0 < NB; b0 += HB) {
       if (b0 > 0) f.wait(1, 0x5600);         // the previous block has been used
@@ -1029,7 +1031,7 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
     float o[ND];
     ld_rows<D, GA>(f, kO, o);
 #pragma unroll
-    for (int j = 0; j < ND; ++j) o[j] = fmaf(o[j], kLn2, add[j]);
+    for (int j = 0; j < ND; ++j) o[j] += add[j];
     stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
     tc_fence_before();
     __syncthreads();
