@@ -70,7 +70,9 @@ struct Plan {
 };
 
 // ---- terms ---------------------------------------------------------------------------------
-template <int NT>
+// kSat: values past the largest bf16 (3.39e38; an fp32 value may be up to 3.40e38) take it as their first term and stay finite;
+// infinities and NaN become NaN in the later terms.
+template <int NT, bool kSat = false>
 __device__ __forceinline__ void split8(const float* v, uint4* w) {
   uint32_t* o = reinterpret_cast<uint32_t*>(w);
 #pragma unroll
@@ -78,7 +80,9 @@ __device__ __forceinline__ void split8(const float* v, uint4* w) {
     float a = v[2 * p], b = v[2 * p + 1];
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      const uint32_t x = pack2<bf16>(a, b);
+      uint32_t x;
+      if (kSat && t == 0) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(x) : "f"(b), "f"(a));
+      else x = pack2<bf16>(a, b);
       o[4 * t + p] = x;
       if (t + 1 < NT) {
         a -= __uint_as_float(x << 16);
@@ -123,7 +127,7 @@ struct InTile {
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] = to_f<T>(e[i]);
         uint4 w[NX];
-        split8<NX>(x, w);
+        split8<NX, std::is_same<T, float>::value>(x, w);
 #pragma unroll
         for (int t = 0; t < NX; ++t) *reinterpret_cast<uint4*>(tile + t * kBlk + off) = w[t];
       }
@@ -145,7 +149,7 @@ __device__ __forceinline__ void put_landmarks(uint8_t* op, const float* src, int
       x[4] = b.x * mul; x[5] = b.y * mul; x[6] = b.z * mul; x[7] = b.w * mul;
     }
     uint4 w[kTerms];
-    split8<kTerms>(x, w);
+    split8<kTerms, true>(x, w);
 #pragma unroll
     for (int t = 0; t < kTerms; ++t) *reinterpret_cast<uint4*>(op + t * (MP * 128) + sw128_offset(r, ch)) = w[t];
   }
