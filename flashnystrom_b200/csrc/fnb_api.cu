@@ -508,7 +508,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       mx::FwdParams mp;
       mp.qt = a.q_landmarks; mp.kt = a.k_landmarks; mp.k2 = a.k2; mp.lse2 = a.lse2; mp.iterates = a.ns_iterates;
       mp.k2inv = a.k2_inv; mp.scratch = reinterpret_cast<uint8_t*>(w.pinv); mp.m = p.m; mp.D = p.D; mp.J = p.J;
-      mp.kappa = a.shape.kappa_star; mp.status = a.device_status;
+      mp.kappa = a.shape.kappa_star; mp.status = a.device_status; mp.test_drop = sch_fc.test_drop;
       if (int rc = set_smem(mx::mx_fwd_kernel, mx::kSmem, max_smem, "mid_fwd")) return rc;
       mx::mx_fwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, ns_stream>>>(mp);
       if (L.end("mid_fwd")) return L.status;
@@ -668,7 +668,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       constexpr size_t smem = sx::Plan<T, D, MPc>::kFwdC;
       if (int rc2 = set_smem(kern, smem, max_smem, "sx_fwd_c")) return rc2;
       launch_pdl(kern, dim3((unsigned)(p.BH * sch.nchunk)), dim3(sx::kThr), smem, st, (const T*)a.q, (T*)a.out, a.lse1,
-                 a.k_landmarks, a.step2, sch, p.m, scale, a.device_status);
+                 a.k_landmarks, a.step2, sch_fc, p.m, scale, a.device_status);
       return L.end("sx_fwd_c");
     });
   }

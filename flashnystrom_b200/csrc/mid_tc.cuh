@@ -9,7 +9,7 @@
 // memory stages, K in chunks of 64, in whichever orientation the product needs (an image serves as left or
 // right operand, plain or transposed, by the pieces that are copied and the descriptor they are read
 // with).  CTA `rank` of the pair forms the 64 output columns [64 rank, 64 rank + 64) of every product; the
-// terms of the right operand are stacked along N, so a K step of 16 is three MMAs,
+// terms of the right operand are stacked along N, so a K step of 16 is three MMAs (four in the second chunk),
 //     x0 [y0 | y1 | y2],  x1 [y0 | y1],  x2 [y0],
 // into column groups by weight that the epilogue adds, small ones first.  x0 y0 has one group per chunk: the
 // tensor core truncates when it adds, and with a single group fp32 dQ and dK were up to 30 % less precise
@@ -57,8 +57,9 @@ constexpr size_t kBwdScratchBytes = (size_t)kBwdImgs * kImg + (size_t)kBwdF32s *
 enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
 
 struct Shared {
-  uint64_t full[kStages], empty[kStages], done[2], ready;
+  uint64_t full[kStages], empty[kStages], done[2], ready, drain;
   uint32_t tmem_slot;
+  uint32_t fills;           // stages filled by the copying warp, written when it is through
   int abort_word;
 };
 
@@ -175,12 +176,14 @@ struct Role {
   uint32_t rphase;
   // copy / issue: position in the ring
   int stage;
-  uint32_t sphase, fills;   // fills: eight bits per stage (newton_iter <= 20: at most 160 fills of a stage)
+  uint32_t sphase, fills;   // fills: stages filled so far, in ring order
+  bool drop;                // test only: this CTA never issues one of its fills, so that a wait runs out
   // compute: accumulator row, column segment of 16 (over both blocks), completion parities
   int row, seg;
   uint32_t dphase[2];
 
-  __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status) {
+  __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status, bool drop_fill) {
+    drop = drop_fill;
     sh = s; ring = r; out = r + (size_t)kStages * kStageBytes; red = rd; rank = rk; lane = threadIdx.x & 31;
     tmem = s->tmem_slot;
     ab = Abort{&s->abort_word, status};
@@ -252,20 +255,27 @@ struct Role {
     if (R == kProducer) {
       if (lane == 0) {
         for (int kc = 0; kc < kchunks; ++kc) {
-          if (!mbar_wait(&sh->empty[stage], sphase ^ 1u, ab, 0x6010)) failed = true;
-          if (!failed) mbar_expect_tx(&sh->full[stage], kStageBytes);
+          if (!failed && !mbar_wait(&sh->empty[stage], sphase ^ 1u, ab, 0x6010)) failed = true;
+          if (drop && fills == 2) failed = true;         // fault injection on the host's request
+          const bool fill = !failed, meet = pend && (fx || fy);
           const uint32_t l = smem_u32(ring) + stage * kStageBytes, r = l + kBlockBytes;
-          if (!fx && !failed) load_left<LT>(l, X, kc);
-          if (!fy && !failed) load_right<RT>(r, Y, kc);
-          if (pend && (fx || fy)) {
-            if (!wait_cluster(&sh->ready, rphase, ab, 0x6011)) failed = true;
+          if (fill) {
+            mbar_expect_tx(&sh->full[stage], kStageBytes);
+            ++fills;
+            if (!fx) load_left<LT>(l, X, kc);
+            if (!fy) load_right<RT>(r, Y, kc);
+          }
+          if (meet) {
+            if (!failed && !wait_cluster(&sh->ready, rphase, ab, 0x6011)) failed = true;
             fence_proxy_async_all();
             rphase ^= 1u;
             pend = false;
           }
-          if (fx && !failed) load_left<LT>(l, X, kc);
-          if (fy && !failed) load_right<RT>(r, Y, kc);
-          if (!failed) fills += 1u << (8 * stage);       // (counts modulo 256: only the parity is used)
+          // (also after that wait has given up: the stage's barrier counts on all of its bytes, and the drain on the barrier)
+          if (fill) {
+            if (fx) load_left<LT>(l, X, kc);
+            if (fy) load_right<RT>(r, Y, kc);
+          }
           advance();
         }
       }
@@ -371,13 +381,7 @@ struct Role {
   }
   __device__ void close() {
     ensure();
-    if (R == kProducer && lane == 0) {      // (only after a wait gave up can a copy still be in flight here)
-#pragma unroll
-      for (int s = 0; s < kStages; ++s) {
-        const uint32_t n = (fills >> (8 * s)) & 0xffu;
-        if (failed && n) mbar_drain(&sh->full[s], (n - 1) & 1u);
-      }
-    }
+    if (R == kProducer && lane == 0) sh->fills = fills;
   }
 };
 
@@ -442,6 +446,7 @@ struct FwdParams {
   int m, D, J;
   float kappa;
   int* status;
+  int test_drop;                          // test only: CTA 0 never issues one fill
 };
 
 template <int R>
@@ -591,6 +596,7 @@ struct BwdParams {
   int64_t N;
   int head, tail;             // run dO3 / D3 / dK2inv; run the pseudoinverse backward and what follows
   int* status;
+  int test_drop;
 };
 
 template <int R>
@@ -873,7 +879,7 @@ __device__ __forceinline__ void run_role(Shared* sh, uint8_t* ring, float* red, 
   Role<R> r;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  r.open(sh, ring, red, (int)rank, p.status);
+  r.open(sh, ring, red, (int)rank, p.status, p.test_drop && blockIdx.x == 0);
   prog(r, p, (int64_t)(blockIdx.x >> 1));
 }
 template <class P, class Prog>
@@ -887,6 +893,7 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
     for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
     mbar_init(&sh->done[0], 1);
     mbar_init(&sh->done[1], 1);
+    mbar_init(&sh->drain, 1);
     mbar_init(&sh->ready, 2 * (kComputeWarps + 2));
     sh->abort_word = 0;
     fence_mbar_init();
@@ -907,6 +914,21 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
   const uint32_t tmem = sh->tmem_slot;
   tc_fence_before();
   __syncthreads();
+  // After a wait gave up, in whichever role, copies and products may still be running.  They end before the memory they
+  // write is given back; nothing is issued any more, so each stage's last fill and one more commit cover them.
+  if (sh->abort_word) {
+    if (threadIdx.x == 0) {
+      for (uint32_t s = 0; s < kStages; ++s) {
+        const uint32_t n = (sh->fills + kStages - 1 - s) / kStages;    // fills of stage s
+        if (n) mbar_drain(&sh->full[s], (n - 1) & 1u);
+      }
+    }
+    if (threadIdx.x == 32 * (kComputeWarps + 1)) {
+      umma_commit(&sh->drain);
+      mbar_drain(&sh->drain, 0);
+    }
+    __syncthreads();
+  }
   cluster_sync_all();          // nobody arrives on this CTA's barriers any more
   if (warp == 0) tmem_dealloc(tmem, 512);
 }

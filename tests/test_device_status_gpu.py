@@ -36,6 +36,34 @@ def test_bounded_wait_expires_and_the_context_stays_usable(cuda_device):
     assert e["out"] <= 2e-3 and max(e["dq"], e["dk"], e["dv"]) <= 1e-2, e
 
 
+@pytest.mark.parametrize("D,m,dtype,where", [
+    (128, 100, torch.float16, 0x60),      # the pseudoinverse kernel for more than 64 landmarks: one fill of its ring is never issued
+    (32, 64, torch.bfloat16, 0x46),       # the split-precision output pass: the products of its last tile are never announced
+])
+def test_bounded_waits_of_the_other_kernels(cuda_device, D, m, dtype, where):
+    """The same for kernels whose own copies and products may be in flight when a wait gives up: they end before the memory
+    they write is given back, and the call after that is right."""
+    from flashnystrom_b200 import _C
+    q, k, v, dO = O.make_inputs(1, 2, 1024, D, seed=12, dtype=dtype)
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    _C.check_device_status()
+    _C.set_wait_limit_ms(5)
+    _C.set_test_drop_load(True)
+    try:
+        _C.forward(qd, kd, vd, m, 6)
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="wait timed out") as e:
+            _C.check_device_status()
+    finally:
+        _C.set_test_drop_load(False)
+        _C.set_wait_limit_ms(1500)
+    assert f"status 0x0100{where:02x}" in str(e.value)
+    cu = run_cuda(q, k, v, dO, m, 6, 0.0)
+    ref = run_oracle(q, k, v, dO, m, 6, 0.0)
+    for key in ("out", "dq", "dk", "dv"):
+        assert errs(cu, ref, [key])[key] <= (3e-2 if dtype == torch.bfloat16 else 1e-2), key
+
+
 def _peaked_inputs(dtype, N=16384, m=16, D=64, seed=21, qmul=0.5, kmul=3.0):
     """Softmax-3 with a large share of a landmark's mass on one key: the queries of every segment
     share a direction (so the landmark has a component along it) and one key per segment points the
