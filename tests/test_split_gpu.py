@@ -111,3 +111,48 @@ def test_fp32_row_sums(cuda_device, B, H, N, D, m):
             err[generic] += _rel(got, want) ** 2
     print(err)
     assert err[False] <= 1.15 ** 2 * err[True]
+
+
+def test_fp32_values_past_the_largest_bf16(cuda_device):
+    """A value that rounds to infinity in bf16, under a weight of e^-60: finite on the CUDA cores, and here."""
+    from flashnystrom_b200 import _C
+    N, D, m, n = 256, 64, 8, 77
+    q, k, v, dO = O.make_inputs(1, 1, N, D, seed=3, dtype=torch.float32)
+    q = 0.1 * q + 0.5
+    k = 0.1 * k
+    k[0, 0, n] -= 15.0                       # scores of about -60 with every landmark query
+    v[0, 0, n, ::2], v[0, 0, n, 1::2] = 3.4e38, -3.4e38
+    got = run_cuda(q, k, v, dO, m, 6, 0.0)
+    _C.set_force_generic(True)
+    try:
+        ref = run_cuda(q, k, v, dO, m, 6, 0.0)
+    finally:
+        _C.set_force_generic(False)
+    want = run_oracle(q, k, v, dO, m, 6, 0.0)
+    for key in ("bmat", "out"):
+        assert torch.isfinite(ref[key]).all() and torch.isfinite(got[key]).all()
+        # a score of 60 is off by about 60 * 2^-22, which the pseudoinverse amplifies some tens of times
+        assert _rel(got[key], want[key]) <= 1e-3, key
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("dtype,D,m", [(F32, 64, 32), (F16, 32, 64), (BF16, 64, 100)])
+def test_infinities_and_nan_stay_where_the_fp32_kernels_have_them(cuda_device, bad, dtype, D, m):
+    """One bad element of V reaches its own column of the output and no other; one of Q or K reaches every output of its
+    slice and nothing of the next slice.  What is finite on the CUDA cores is finite here, and the other way round."""
+    from flashnystrom_b200 import _C
+    for which in range(3):
+        t = list(O.make_inputs(1, 2, 300, D, seed=13, dtype=F32))
+        t[which][0, 0, 150, 5] = bad
+        q, k, v, _ = (x.to(dtype).cuda() for x in t)
+        got = _C.forward(q, k, v, m, 6)[0]
+        _C.set_force_generic(True)
+        try:
+            ref = _C.forward(q, k, v, m, 6)[0]
+        finally:
+            _C.set_force_generic(False)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(ref))
+        assert torch.isfinite(got[0, 1]).all()
+        assert torch.isfinite(got[0, 0]).all(0).sum() == (D - 1 if which == 2 else 0)
+    torch.cuda.synchronize()
+    _C.check_device_status()
