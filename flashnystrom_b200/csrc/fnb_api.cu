@@ -249,13 +249,17 @@ static int check_shape(const fnb_shape* s) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Clusters of the pseudoinverse kernels for more than 64 landmarks that a launch has, and scratch areas that they work in:
+// no more than run at once (two SMs each).
+static int64_t mid_slots(int64_t BH) { return std::max<int64_t>(1, std::min<int64_t>(BH, current_sm_count() / 2)); }
+
 struct FwdWs {
   float *land_partial, *part_acc, *part_max, *part_sum, *pinv;
   void *qt16, *kt16, *st16;   // 16-bit operand copies for the tensor-core kernels
   float* st_scale;            // [BH] power-of-two normalisation of the step2 copy
   size_t bytes;
 };
-static FwdWs carve_fwd(const Plan& p, void* base) {
+static FwdWs carve_fwd(const Plan& p, uint32_t flags, void* base) {
   char* b = (char*)base;
   size_t off = 0;
   auto take = [&](size_t nfloat) { float* r = (float*)(b + off); off += align256(nfloat * sizeof(float)); return r; };
@@ -264,8 +268,8 @@ static FwdWs carve_fwd(const Plan& p, void* base) {
   w.part_acc = take((size_t)p.BH * p.nchunk * p.m * p.D);
   w.part_max = take((size_t)p.BH * p.nchunk * p.m);
   w.part_sum = take((size_t)p.BH * p.nchunk * p.m);
-  // the images of mid_tc.cuh are the larger need (the CUDA-core kernel takes kPinvFwdBufs m x m matrices)
-  w.pinv = take(p.m > ns::kN ? (size_t)p.BH * (mx::kFwdScratchBytes / sizeof(float)) : 0);
+  w.pinv = take(p.m <= ns::kN ? 0 : (flags & FNB_FLAG_FORCE_GENERIC) ? (size_t)p.BH * kPinvFwdBufs * p.m * p.m
+                                                                    : (size_t)mid_slots(p.BH) * (mx::kFwdScratchBytes / sizeof(float)));
   const int MP = p.m <= 64 ? 64 : 128;
   const size_t op16 = ((size_t)p.BH * MP * p.D + 1) / 2;   // 16-bit elements, counted in floats
   w.qt16 = take(op16); w.kt16 = take(op16); w.st16 = take(op16);
@@ -282,7 +286,7 @@ struct BwdWs {
   float* tile_scale;          // [BH][ceil(N / 128)]: factor the column pass stored each dS' tile with
   size_t bytes;
 };
-static BwdWs carve_bwd(const Plan& p, void* base) {
+static BwdWs carve_bwd(const Plan& p, uint32_t flags, void* base) {
   char* b = (char*)base;
   size_t off = 0;
   auto take = [&](size_t nfloat) { float* r = (float*)(b + off); off += align256(nfloat * sizeof(float)); return r; };
@@ -290,11 +294,12 @@ static BwdWs carve_bwd(const Plan& p, void* base) {
   const size_t md = (size_t)p.BH * p.m * p.D, mm = (size_t)p.BH * p.m * p.m;
   w.partA = take((size_t)p.nchunk * 2 * md);
   w.partB = take((size_t)p.nchunk * md);
-  w.dstep2 = take(md); w.dkt_a = take(md); w.dO3 = take(md);
+  const bool generic_pinv = p.m > ns::kN && (flags & FNB_FLAG_FORCE_GENERIC), small = p.m <= ns::kN;   // (mid_tc.cuh has what it needs in its scratch)
+  w.dstep2 = take(generic_pinv ? md : 0); w.dkt_a = take(generic_pinv || small ? md : 0); w.dO3 = take(md);
   w.dqt_ns = take(md); w.dkt_tot = take(md); w.dqt_tot = take(md);
   w.D3 = take((size_t)p.BH * p.m);
-  w.G = take(mm); w.dK2 = take(mm);
-  w.pinv = take(p.m > ns::kN ? (size_t)p.BH * (mx::kBwdScratchBytes / sizeof(float)) : 0);
+  w.G = take(generic_pinv || small ? mm : 0); w.dK2 = take(generic_pinv || small ? mm : 0);
+  w.pinv = take(small ? 0 : generic_pinv ? kPinvBwdBufs * mm : (size_t)mid_slots(p.BH) * (mx::kBwdScratchBytes / sizeof(float)));
   const int MP = p.m <= 64 ? 64 : 128;
   const size_t op16 = ((size_t)p.BH * MP * p.D + 1) / 2;
   for (int i = 0; i < 8; ++i) w.op16[i] = take(op16);
@@ -344,6 +349,32 @@ static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+// Grid of a kernel of mid_tc.cuh (its shared-memory size is set): a cluster of two CTAs per slice, up to as many as the
+// device can hold at once.  A cluster needs both its SMs in one GPC, which the occupancy call knows.
+static unsigned mid_grid(const void* kern, int64_t slices, int device) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> fit;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_pair(kern, device);
+  auto it = fit.find(key);
+  if (it == fit.end()) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * 1024); cfg.blockDim = dim3(mx::kThr); cfg.dynamicSmemBytes = mx::kSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
+    it = fit.emplace(key, n).first;
+  }
+  const int64_t slots = mid_slots(slices);
+  return 2 * (unsigned)(it->second > 0 ? std::min<int64_t>(slots, it->second) : slots);
+}
+template <class P> static unsigned mid_grid(void (*kern)(P), int64_t slices, int device) {
+  return mid_grid(reinterpret_cast<const void*>(kern), slices, device);
 }
 
 // The Newton-Schulz kernels for num_landmarks <= 64 run on the tensor cores (three-term bf16
@@ -510,7 +541,8 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       mp.k2inv = a.k2_inv; mp.scratch = reinterpret_cast<uint8_t*>(w.pinv); mp.m = p.m; mp.D = p.D; mp.J = p.J;
       mp.kappa = a.shape.kappa_star; mp.status = a.device_status; mp.test_drop = sch_fc.test_drop;
       if (int rc = set_smem(mx::mx_fwd_kernel, mx::kSmem, max_smem, "mid_fwd")) return rc;
-      mx::mx_fwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, ns_stream>>>(mp);
+      mp.BH = p.BH;
+      mx::mx_fwd_kernel<<<mid_grid(mx::mx_fwd_kernel, p.BH, a.device), mx::kThr, mx::kSmem, ns_stream>>>(mp);
       if (L.end("mid_fwd")) return L.status;
     } else {
     ns::NsFwdParams np;
@@ -901,11 +933,14 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
     if (int rc = set_smem(mx::mx_bwd_kernel, mx::kSmem, max_smem, "mid_bwd")) return rc;
     mp.head = 1; mp.tail = side_mid ? 0 : 1;
     L.begin();
-    mx::mx_bwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, st>>>(mp);
+    mp.BH = p.BH;
+    // (two launches hand dL/dK2inv over in the scratch: each slice then keeps an area of its own)
+    const unsigned mid_ctas = side_mid ? 2 * (unsigned)p.BH : mid_grid(mx::mx_bwd_kernel, p.BH, a.device);
+    mx::mx_bwd_kernel<<<mid_ctas, mx::kThr, mx::kSmem, st>>>(mp);
     if (L.end("mid_bwd")) return L.status;
     if (side_mid) {
       mp.head = 0; mp.tail = 1;
-      mx::mx_bwd_kernel<<<(unsigned)(2 * p.BH), mx::kThr, mx::kSmem, fork.begin()>>>(mp);
+      mx::mx_bwd_kernel<<<mid_ctas, mx::kThr, mx::kSmem, fork.begin()>>>(mp);
       fork.end();
     }
     if (use_tc) {
@@ -1051,8 +1086,8 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
 }
 
 
-static size_t fwd_ws_total(const fnb_shape& s) { return carve_fwd(plan_of(s), nullptr).bytes; }
-static size_t bwd_ws_total(const fnb_shape& s) { return carve_bwd(plan_of(s), nullptr).bytes; }
+static size_t fwd_ws_total(const fnb_shape& s) { return carve_fwd(plan_of(s), s.flags, nullptr).bytes; }
+static size_t bwd_ws_total(const fnb_shape& s) { return carve_bwd(plan_of(s), s.flags, nullptr).bytes; }
 
 }  // namespace fnb
 
@@ -1129,7 +1164,7 @@ int fnb_forward(const fnb_fwd_args* a) {
   if (int rc = device_limits(a->device, &max_smem, &cc, &sms)) return rc;
   cudaStream_t st = (cudaStream_t)a->stream;
   Plan p = plan_of(a->shape);
-  FwdWs w = carve_fwd(p, a->workspace);
+  FwdWs w = carve_fwd(p, a->shape.flags, a->workspace);
   switch (a->shape.dtype) {
     case FNB_F32: return forward_impl<float>(*a, p, w, max_smem, sms, st, true);
     case FNB_F16: return forward_impl<__half>(*a, p, w, max_smem, sms, st, true);
@@ -1151,7 +1186,7 @@ int fnb_backward(const fnb_bwd_args* a) {
   if (int rc = device_limits(a->device, &max_smem, &cc, &sms)) return rc;
   cudaStream_t st = (cudaStream_t)a->stream;
   Plan p = plan_of(a->shape);
-  BwdWs w = carve_bwd(p, a->workspace);
+  BwdWs w = carve_bwd(p, a->shape.flags, a->workspace);
   switch (a->shape.dtype) {
     case FNB_F32: return backward_impl<float>(*a, p, w, max_smem, sms, st, true);
     case FNB_F16: return backward_impl<__half>(*a, p, w, max_smem, sms, st, true);
@@ -1203,7 +1238,7 @@ int fnb_sp_forward(const fnb_fwd_args* a, const fnb_sp_info* sp) {
   if (int rc = device_limits(a->device, &max_smem, &cc, &sms)) return rc;
   cudaStream_t st = (cudaStream_t)a->stream;
   Plan p = plan_of(a->shape);
-  FwdWs w = carve_fwd(p, a->workspace);
+  FwdWs w = carve_fwd(p, a->shape.flags, a->workspace);
   SpCtx S;
   S.stage = sp->stage; S.rank = sp->rank; S.world = sp->world; S.N_global = sp->seq_len_global; S.xfer = sp->xfer;
   switch (a->shape.dtype) {
@@ -1228,7 +1263,7 @@ int fnb_sp_backward(const fnb_bwd_args* a, const fnb_sp_info* sp) {
   if (int rc = device_limits(a->device, &max_smem, &cc, &sms)) return rc;
   cudaStream_t st = (cudaStream_t)a->stream;
   Plan p = plan_of(a->shape);
-  BwdWs w = carve_bwd(p, a->workspace);
+  BwdWs w = carve_bwd(p, a->shape.flags, a->workspace);
   SpCtx S;
   S.stage = sp->stage; S.rank = sp->rank; S.world = sp->world; S.N_global = sp->seq_len_global; S.xfer = sp->xfer;
   switch (a->shape.dtype) {
@@ -1240,7 +1275,7 @@ int fnb_sp_backward(const fnb_bwd_args* a, const fnb_sp_info* sp) {
 
 size_t fnb_debug_pinv_workspace_bytes(int64_t bh, int32_t m) {
   if (bh <= 0 || m < 1 || m > kMaxM) return 0;
-  return align256(m > ns::kN ? (size_t)bh * mx::kBwdScratchBytes + 256 : (size_t)bh * kPinvBwdBufs * m * m * sizeof(float));
+  return align256(std::max(m > ns::kN ? (size_t)mid_slots(bh) * mx::kBwdScratchBytes + 256 : 0, (size_t)bh * kPinvBwdBufs * m * m * sizeof(float)));
 }
 // the images are copied in bulk: 16-byte aligned wherever the caller's workspace starts
 static uint8_t* pinv_scratch(void* ws) {
@@ -1276,7 +1311,8 @@ int fnb_debug_pinv_forward(int64_t bh, int32_t m, int32_t J, float kappa, const 
     mp.k2 = const_cast<float*>(k2);      // (given softmaxed: only read)
     mp.iterates = ns_iterates; mp.k2inv = k2_inv; mp.scratch = pinv_scratch(workspace); mp.m = m; mp.J = J; mp.kappa = kappa;
     FNB_CUDA(cudaFuncSetAttribute(mx::mx_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
-    mx::mx_fwd_kernel<<<(unsigned)(2 * bh), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
+    mp.BH = bh;
+    mx::mx_fwd_kernel<<<mid_grid(mx::mx_fwd_kernel, bh, device), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
   } else if (m <= ns::kN) {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_fwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kFwdSmem));
@@ -1307,7 +1343,8 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
     mp.k2 = k2; mp.iterates = ns_iterates; mp.G = d_k2_inv; mp.dK2 = d_k2; mp.scratch = pinv_scratch(workspace); mp.m = m; mp.J = J;
     mp.kappa = kappa; mp.tail = 1;
     FNB_CUDA(cudaFuncSetAttribute(mx::mx_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
-    mx::mx_bwd_kernel<<<(unsigned)(2 * bh), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
+    mp.BH = bh;
+    mx::mx_bwd_kernel<<<mid_grid(mx::mx_bwd_kernel, bh, device), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
   } else if (m <= ns::kN) {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_bwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kBwdSmem));

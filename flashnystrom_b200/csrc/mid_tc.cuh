@@ -47,7 +47,8 @@ constexpr size_t kSmem = (size_t)kStages * kStageBytes + kBlockBytes + kRedFloat
 constexpr int kAccCols = 256;                  // tensor-memory columns of one accumulator
 constexpr int kF32 = kMaxM * kMaxM;            // floats of one FP32 scratch matrix
 
-// per-slice scratch: images, then FP32 matrices
+// scratch of a cluster: images, then FP32 matrices.  A launch has at most as many clusters as run at once; each walks slices
+// gridDim.x / 2 apart and works in one scratch area, so that the scratch stays in L2 and does not grow with the slices.
 enum FwdImg { kFK2, kFA, kFZ0, kFZ1, kFM, kFV, kFT, kFwdImgs };
 constexpr size_t kFwdScratchBytes = (size_t)kFwdImgs * kImg + kF32 * sizeof(float);
 enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBdZ0, kBdZ1, kBM, kBV, kBT, kBdT, kBdV, kBdM, kBwdImgs };
@@ -442,7 +443,8 @@ __device__ inline Norms norms(const float* A, int m, float* red) {
 struct FwdParams {
   const float* qt; const float* kt;       // [BH][m][D]; null: k2 is given (softmaxed)
   float* k2; float* lse2; float* iterates; float* k2inv;
-  uint8_t* scratch;                       // [BH][kFwdScratchBytes]
+  uint8_t* scratch;                       // [gridDim.x / 2][kFwdScratchBytes]
+  int64_t BH;
   int m, D, J;
   float kappa;
   int* status;
@@ -453,7 +455,7 @@ template <int R>
 __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int64_t bh) {
   constexpr bool C = R == kCompute;
   const int m = p.m, D = p.D, mm = m * m;
-  uint8_t* base = p.scratch + bh * (int64_t)kFwdScratchBytes;
+  uint8_t* base = p.scratch + (int64_t)(blockIdx.x >> 1) * kFwdScratchBytes;
   auto img = [&](int i) { return base + (size_t)i * kImg; };
   float* a32 = reinterpret_cast<float*>(base + (size_t)kFwdImgs * kImg);
   float* k2 = p.k2 + bh * mm;
@@ -590,7 +592,8 @@ struct BwdParams {
   float* dqt_ns; float* dkt_tot; float* rows_k;   // [BH][m][D]; rows_k (scale * dkt_tot / segment length) may be null
   const float* G;             // debug entry: dL/dk2inv given, dK2 wanted
   float* dK2;
-  uint8_t* scratch;           // [BH][kBwdScratchBytes]
+  uint8_t* scratch;           // [gridDim.x / 2][kBwdScratchBytes]
+  int64_t BH;
   int m, D, J;
   float kappa, scale;
   int64_t N;
@@ -604,7 +607,7 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
   constexpr bool C = R == kCompute;
   const int m = p.m, D = p.D, mm = m * m, md = m * D, J = p.J;
   const bool ridge = p.kappa > 0.f;
-  uint8_t* base = p.scratch + bh * (int64_t)kBwdScratchBytes;
+  uint8_t* base = p.scratch + (int64_t)(blockIdx.x >> 1) * kBwdScratchBytes;
   auto img = [&](int i) { return base + (size_t)i * kImg; };
   auto f32 = [&](int i) { return reinterpret_cast<float*>(base + (size_t)kBwdImgs * kImg) + (size_t)i * kF32; };
   const float* k2 = p.k2 + bh * mm;
@@ -880,7 +883,14 @@ __device__ __forceinline__ void run_role(Shared* sh, uint8_t* ring, float* red, 
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   r.open(sh, ring, red, (int)rank, p.status, p.test_drop && blockIdx.x == 0);
-  prog(r, p, (int64_t)(blockIdx.x >> 1));
+  for (int64_t bh = blockIdx.x >> 1;;) {
+    prog(r, p, bh);
+    bh += gridDim.x >> 1;
+    if (bh >= p.BH) break;
+    __syncwarp();
+    __syncthreads();
+    cluster_sync_all();        // neither CTA copies from this slice's images any more
+  }
 }
 template <class P, class Prog>
 __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) {
