@@ -363,6 +363,8 @@ def backward_packed(dO, q, k, v, saved, num_landmarks, newton_iter, kappa_star):
     if saved.device != dev or saved.shape != (plan.floats,) or saved.dtype != torch.float32 or not saved.is_contiguous():
         _check_big(saved, "saved tensors", (plan.floats,), torch.float32)
         raise RuntimeError("saved tensors are on another device than dO")
+    if saved.data_ptr() & 15:      # (a saved-tensor hook may hand it back anywhere; its parts lie at 256-byte steps)
+        saved = saved.clone()
     with _on_device(dev):
         dq, dk, dv = (_empty_like_layout(dO, lay) for _ in range(3))
         ws = torch.empty(plan.bwd_ws, dtype=torch.uint8, device=dev)

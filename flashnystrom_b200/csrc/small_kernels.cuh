@@ -645,7 +645,12 @@ __global__ void __launch_bounds__(kThreads) landmark_finalize_kernel(LandmarkFin
       }
       const float f = p.scale / (float)sg.len(l);
       val = make_float4(val.x * f, val.y * f, val.z * f, val.w * f);
-      *reinterpret_cast<float4*>((which ? p.kt : p.qt) + (bh * m + l) * D + d) = val;
+      float* dst = (which ? p.kt : p.qt) + (bh * m + l) * D + d;
+      if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        *reinterpret_cast<float4*>(dst) = val;
+      } else {                               // (the caller's saved tensors need no more than their type's alignment)
+        dst[0] = val.x; dst[1] = val.y; dst[2] = val.z; dst[3] = val.w;
+      }
     }
     if (which == 0 && p.qt16)
       *reinterpret_cast<uint2*>(reinterpret_cast<char*>(p.qt16) + ((size_t)bh * p.MP * D + (size_t)l * D + d) * 2) =

@@ -138,15 +138,24 @@ struct InTile {
 // (m x D) FP32 landmark matrix times mul -> three term tiles of [MP rows x 128 B], rows >= m zero
 template <int D, int MP>
 __device__ __forceinline__ void put_landmarks(uint8_t* op, const float* src, int m, float mul) {
+  const bool aligned = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
   for (int idx = threadIdx.x; idx < MP * D / 8; idx += kThr) {
     const int r = idx / (D / 8), ch = idx % (D / 8);
     float x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] = 0.f;
     if (r < m) {
-      const float4 a = *reinterpret_cast<const float4*>(src + r * D + ch * 8), b = *reinterpret_cast<const float4*>(src + r * D + ch * 8 + 4);
-      x[0] = a.x * mul; x[1] = a.y * mul; x[2] = a.z * mul; x[3] = a.w * mul;
-      x[4] = b.x * mul; x[5] = b.y * mul; x[6] = b.z * mul; x[7] = b.w * mul;
+      const float* e = src + r * D + ch * 8;
+      if (aligned) {
+        const float4 a = *reinterpret_cast<const float4*>(e), b = *reinterpret_cast<const float4*>(e + 4);
+        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+        x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+      } else {                               // (the caller's saved tensors need no more than their type's alignment)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = e[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] *= mul;
     }
     uint4 w[kTerms];
     split8<kTerms, true>(x, w);

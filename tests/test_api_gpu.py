@@ -201,3 +201,84 @@ def test_head_split_layout_matches_contiguous(cuda_device):
     # fp32 (CUDA-core path): the view is accepted by the module only through a copy; the op itself refuses it
     with pytest.raises(RuntimeError, match="contiguous"):
         _C.forward(*(t.float().transpose(1, 2).contiguous().transpose(1, 2) for t in (q, k, v)), 40, 6)
+
+
+def _shifted(t):
+    """A contiguous copy of t that starts four bytes past a 16-byte boundary."""
+    buf = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+    assert buf.data_ptr() % 16 == 0
+    return buf[1:1 + t.numel()].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("dtype,D,m,names", [
+    (torch.float16, 64, 100, ("qt", "kt", "step2", "bmat")), (torch.bfloat16, 32, 128, ("qt", "kt", "step2", "bmat")),
+    (torch.float32, 128, 70, ("qt", "kt", "step2", "bmat")), (torch.float32, 64, 64, ("step2",)), (torch.float16, 32, 40, ("step2",)),
+])
+def test_saved_tensors_need_only_their_types_alignment(cuda_device, dtype, D, m, names):
+    """FP32 saved tensors that the backward took at any four-byte boundary (views into a larger buffer, say)."""
+    from flashnystrom_b200 import _C
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 2, 300, D, seed=5, dtype=dtype))
+    res = _C.forward(q, k, v, m, 4)
+    place = dict(qt=3, kt=4, step2=6, bmat=12)
+    want = _C.backward(dO, *res[1:13], v, res[0], m, 4)
+    for n in names:
+        res[place[n]] = _shifted(res[place[n]])
+    got = _C.backward(dO, *res[1:13], v, res[0], m, 4)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,D,m", [(torch.float16, 64, 100), (torch.float32, 32, 70), (torch.bfloat16, 16, 65)])
+def test_landmark_outputs_need_only_their_types_alignment(cuda_device, dtype, D, m):
+    """The same for the landmarks that a forward call of the C ABI writes (more than 64 of them)."""
+    import ctypes
+    from flashnystrom_b200 import _C, _lib
+    q, k, v, _ = (t.cuda() for t in O.make_inputs(1, 2, 300, D, seed=6, dtype=dtype))
+    lib, dev, J = _lib.load(), q.device, 4
+    want = _C.forward(q, k, v, m, J)
+    t = [torch.empty_like(x) for x in (want[0], want[7])] + [_shifted(want[i]) for i in (3, 4)]
+    t[2].zero_(), t[3].zero_()
+    t += [torch.empty_like(want[i]) for i in (11, 8, 10, 5, 12, 9, 6)]
+    shape = _C._shape_struct(1, 2, 300, D, m, J, dtype, 0.0)
+    ws = torch.empty(lib.fnb_fwd_workspace_bytes(ctypes.byref(shape)), dtype=torch.uint8, device=dev)
+    args = _lib.FwdArgs(shape, *[x.data_ptr() for x in (q, k, v, *t)], ws.data_ptr(), ws.numel(), dev.index,
+                        torch.cuda.current_stream(dev).cuda_stream, _C._status(dev).data_ptr())
+    _lib.check(lib.fnb_forward(ctypes.byref(args)))
+    torch.cuda.synchronize()
+    _C.check_device_status()
+    for a, b in zip(t, [want[i] for i in (0, 7, 3, 4, 11, 8, 10, 5, 12, 9, 6)]):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,D,m", [(torch.bfloat16, 32, 64), (torch.float16, 64, 100), (torch.float16, 128, 100), (torch.float32, 64, 64),
+                                       (torch.float32, 64, 100)])
+@pytest.mark.parametrize("split_heads", [False, True])
+def test_autograd_function_matches_the_extension_calls(cuda_device, dtype, D, m, split_heads):
+    """What users call keeps its FP32 tensors in one buffer; the extension's forward() and backward() have one each."""
+    from flashnystrom_b200 import _C, flash_nystrom_attention
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(2, 3, 300, D, seed=7, dtype=dtype))
+    res = _C.forward(q, k, v, m, 5, 5.0)
+    want = [res[0], *_C.backward(dO, *res[1:13], v, res[0], m, 5, True, 5.0)]
+    x = [q.clone(), k.clone(), v.clone()]
+    if split_heads and _C.tc_eligible(dtype, D, m):
+        x = [t.transpose(1, 2).contiguous().transpose(1, 2) for t in x]
+    x = [t.requires_grad_(True) for t in x]
+    out = flash_nystrom_attention(*x, num_landmarks=m, newton_iter=5, kappa_star=5.0)
+    out.backward(dO)
+    for a, b in zip([out, *(t.grad for t in x)], want):
+        assert torch.equal(a, b)
+
+
+def test_saved_tensor_hooks_may_move_the_buffer(cuda_device):
+    """Saved tensors that come back from a hook at another address, and not 16-byte aligned."""
+    from flashnystrom_b200 import flash_nystrom_attention
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 2, 300, 64, seed=8, dtype=torch.float32))
+    grads = []
+    for unpack in (lambda t: t, lambda t: _shifted(t) if t.dim() == 1 else t.clone()):
+        x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            out = flash_nystrom_attention(*x, num_landmarks=32)
+        out.backward(dO)
+        grads.append([t.grad for t in x])
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
