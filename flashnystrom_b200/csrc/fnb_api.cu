@@ -1275,7 +1275,7 @@ int fnb_sp_backward(const fnb_bwd_args* a, const fnb_sp_info* sp) {
 
 size_t fnb_debug_pinv_workspace_bytes(int64_t bh, int32_t m) {
   if (bh <= 0 || m < 1 || m > kMaxM) return 0;
-  return align256(std::max(m > ns::kN ? (size_t)mid_slots(bh) * mx::kBwdScratchBytes + 256 : 0, (size_t)bh * kPinvBwdBufs * m * m * sizeof(float)));
+  return align256(m > ns::kN ? (size_t)mid_slots(bh) * mx::kBwdScratchBytes + 256 : (size_t)bh * kPinvBwdBufs * m * m * sizeof(float));
 }
 // the images are copied in bulk: 16-byte aligned wherever the caller's workspace starts
 static uint8_t* pinv_scratch(void* ws) {
@@ -1305,7 +1305,7 @@ int fnb_debug_pinv_forward(int64_t bh, int32_t m, int32_t J, float kappa, const 
                                   (int)nstc::kFwdSmem));
     nstc::ns_pinv_fwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kFwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, k2_inv, m, J, kappa, nullptr);
-  } else if (m > ns::kN && ns_on_tensor_cores(0)) {
+  } else if (m > ns::kN) {
     mx::FwdParams mp;
     memset(&mp, 0, sizeof(mp));
     mp.k2 = const_cast<float*>(k2);      // (given softmaxed: only read)
@@ -1313,13 +1313,11 @@ int fnb_debug_pinv_forward(int64_t bh, int32_t m, int32_t J, float kappa, const 
     FNB_CUDA(cudaFuncSetAttribute(mx::mx_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
     mp.BH = bh;
     mx::mx_fwd_kernel<<<mid_grid(mx::mx_fwd_kernel, bh, device), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
-  } else if (m <= ns::kN) {
+  } else {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_fwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kFwdSmem));
     ns::ns_pinv_fwd_debug_kernel<<<(unsigned)bh, kThreads, ns::kFwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, k2_inv, m, J, kappa);
-  } else {
-    pinv_fwd_debug_kernel<<<(unsigned)bh, kThreads, 0, (cudaStream_t)stream>>>(k2, ns_iterates, k2_inv, (float*)workspace, m, J, kappa);
   }
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
@@ -1337,7 +1335,7 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
                                   (int)nstc::kBwdSmem));
     nstc::ns_pinv_bwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa, nullptr, nullptr, nullptr);
-  } else if (m > ns::kN && ns_on_tensor_cores(0)) {
+  } else if (m > ns::kN) {
     mx::BwdParams mp;
     memset(&mp, 0, sizeof(mp));
     mp.k2 = k2; mp.iterates = ns_iterates; mp.G = d_k2_inv; mp.dK2 = d_k2; mp.scratch = pinv_scratch(workspace); mp.m = m; mp.J = J;
@@ -1345,13 +1343,11 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
     FNB_CUDA(cudaFuncSetAttribute(mx::mx_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mx::kSmem));
     mp.BH = bh;
     mx::mx_bwd_kernel<<<mid_grid(mx::mx_bwd_kernel, bh, device), mx::kThr, mx::kSmem, (cudaStream_t)stream>>>(mp);
-  } else if (m <= ns::kN) {
+  } else {
     FNB_CUDA(cudaFuncSetAttribute(ns::ns_pinv_bwd_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)ns::kBwdSmem));
     ns::ns_pinv_bwd_debug_kernel<<<(unsigned)bh, kThreads, ns::kBwdSmem, (cudaStream_t)stream>>>(
         k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa);
-  } else {
-    pinv_bwd_debug_kernel<<<(unsigned)bh, kThreads, 0, (cudaStream_t)stream>>>(k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa);
   }
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
@@ -1463,11 +1459,14 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
   using H = __half;
   const KernelEntry ks[] = {
       {"landmark_partial<half>", (const void*)landmark_partial_kernel<H, true, 8>, kThreads, 0},
+      {"landmark_partial<half,1 warp>", (const void*)landmark_partial_kernel<H, true, 1>, kThreads, 0},
       {"ns_fwd_tc", (const void*)nstc::ns_fwd_tc_kernel, nstc::kNsTcThreads, nstc::kFwdSmem},
       {"conv_residual<half>", (const void*)conv_residual_kernel<H>, kThreads, conv_smem_bytes(64, 3)},
       {"conv_dw_partial<half,2>", (const void*)conv_dw_partial_kernel<H, 2>, kThreads, conv_smem_bytes(64, 3)},
       {"tc_fwd_b<half,64,64>", (const void*)tc::tc_fwd_b_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdBSmem<64, 64>::kBytes},
       {"combine_slab", (const void*)combine_slab_kernel<kSlabMaxChunks>, kThreads, combine_slab_smem(64)},
+      {"combine_slab<2>", (const void*)combine_slab_kernel<2>, kThreads, combine_slab_smem(64)},
+      {"combine_slab<10>", (const void*)combine_slab_kernel<10>, kThreads, combine_slab_smem(64)},
       {"tc_fwd_c<half,64,64>", (const void*)tc::tc_fwd_c_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdCSmem<64, 64>::kBytes},
       {"tc_bwd_a<half,64,64>", (const void*)tc::tc_bwd_a_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdASmem<64, 64>::kBytes},
       {"reduce_chunks", (const void*)reduce_chunks_kernel, kThreads, 0},
@@ -1481,6 +1480,13 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
       {"tc_bwd_a<half,128,64>", (const void*)tc::tc_bwd_a_kernel<H, 128, 64>, tc::kTcThreads, tc::BwdASmem<128, 64>::kBytes},
       {"tc_bwd_b<half,128,64>", (const void*)tc::tc_bwd_b_kernel<H, 128, 64>, tc::kTcThreads, tc::BwdBSmem<128, 64>::kBytes},
       {"tc_rows_inplace<half,128,64>", (const void*)tc::tc_rows_inplace_kernel<H, 128, 64>, tc::RowsSmem<128, 64>::kThreads, tc::RowsSmem<128, 64>::kBytes},
+      {"mx_fwd", (const void*)mx::mx_fwd_kernel, mx::kThr, mx::kSmem},
+      {"mx_bwd", (const void*)mx::mx_bwd_kernel, mx::kThr, mx::kSmem},
+      {"sx_fwd_b<float,64,64>", (const void*)sx::sx_fwd_b_kernel<float, 64, 64>, sx::kThr, (size_t)sx::Plan<float, 64, 64>::kFwdB},
+      {"sx_fwd_c<float,64,64>", (const void*)sx::sx_fwd_c_kernel<float, 64, 64>, sx::kThr, (size_t)sx::Plan<float, 64, 64>::kFwdC},
+      {"sx_bwd_a<float,64,64>", (const void*)sx::sx_bwd_a_kernel<float, 64, 64>, sx::kThr, (size_t)sx::Plan<float, 64, 64>::kBwdA},
+      {"sx_bwd_b<float,64,64>", (const void*)sx::sx_bwd_b_kernel<float, 64, 64>, sx::kThr, (size_t)sx::Plan<float, 64, 64>::kBwdB},
+      {"sx_bwd_c<float,64,64>", (const void*)sx::sx_bwd_c_kernel<float, 64, 64>, sx::kThr, (size_t)sx::Plan<float, 64, 64>::kBwdC},
   };
   int n = 0;
   for (const KernelEntry& k : ks) {

@@ -356,23 +356,6 @@ __global__ void __launch_bounds__(kThreads) mid_fwd_kernel(MidFwdParams p) {
                p.scratch + bh * (size_t)kPinvFwdBufs * m * m, m, p.J, p.kappa, sm);
 }
 
-__global__ void __launch_bounds__(kThreads)
-pinv_fwd_debug_kernel(const float* k2, float* iterates, float* k2inv, float* scratch, int m, int J, float kappa) {
-  __shared__ float sm[kGemmSmemFloats];
-  const int64_t bh = blockIdx.x;
-  pinv_forward(k2 + bh * m * m, iterates + bh * (size_t)(J + 1) * m * m, k2inv + bh * m * m,
-               scratch + bh * (size_t)kPinvFwdBufs * m * m, m, J, kappa, sm);
-}
-
-__global__ void __launch_bounds__(kThreads)
-pinv_bwd_debug_kernel(const float* k2, const float* iterates, const float* G, float* dK2,
-                      float* scratch, int m, int J, float kappa) {
-  __shared__ float sm[kGemmSmemFloats];
-  const int64_t bh = blockIdx.x;
-  pinv_backward(k2 + bh * m * m, iterates + bh * (size_t)(J + 1) * m * m, G + bh * m * m,
-                dK2 + bh * m * m, scratch + bh * (size_t)kPinvBwdBufs * m * m, m, J, kappa, sm);
-}
-
 // ------------------------------------------------------------------------------------------
 struct MidBwdParams {
   const float* partA;        // [BH][nchunk][2][m][D]: dstep2 and dKt partials of the row pass
