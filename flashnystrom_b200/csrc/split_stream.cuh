@@ -178,15 +178,16 @@ __device__ __forceinline__ void put_probs(uint8_t* tile, int r, int b, int group
 }
 
 // ---- products (warp-uniform; one elected lane issues) ------------------------------------------------
-// The tensor core truncates when it adds to an accumulator.  So the small partial products go first, and the K steps
-// of the leading one may be spread over G accumulators of their own (column groups of the result's width), which the
-// epilogue adds in FP32.
-// scores (128 x MP) = X (128 x D) L^T, groups MP columns apart
-template <int D, int G> __host__ __device__ constexpr int score_groups() { return G < D / 16 ? G : D / 16; }
-template <int D, int MP, int NX, int G>
+// The tensor core truncates when it adds to an accumulator.  So the small partial products go first, and where it
+// shows, the K steps of the leading one are spread over G accumulators of their own (column groups 64 apart), which the
+// epilogue adds in FP32.  With everything in one accumulator the output and dV of fp32 calls were 1.2 to 1.4 times as far
+// from the oracle as with the CUDA-core kernels, with the groups below 0.5 to 1.03 times, for 3 % of the passes'
+// time; spreading the scores' K steps as well changed nothing but the time (680 -> 695 us for a training
+// pass, B=1, H=16, N=16384, D=64, m=64).
+// scores (128 x MP) = X (128 x D) L^T
+template <int D, int MP, int NX>
 __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l) {
   constexpr uint32_t idesc = make_idesc<bf16>(kTile, MP, false, false);
-  constexpr int K = D / 16, GE = score_groups<D, G>();
   bool acc = false;
 #pragma unroll
   for (int s = kTerms - 1; s >= 0; --s)
@@ -195,16 +196,13 @@ __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l)
       const int j = s - i;
       if (j < 0 || j >= kTerms) continue;
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const int g = s == 0 ? k * GE / K : 0;
-        const bool first = g > 0 && (k - 1) * GE / K != g;
-        umma_elect(d + g * MP, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc,
-                   g > 0 ? !first : acc);
+      for (int k = 0; k < D / 16; ++k) {
+        umma_elect(d, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc, acc);
         acc = true;
       }
     }
 }
-// rows (128 x D) = P L over the HB blocks of landmarks from blk on, which the tile p holds; groups 64 columns apart.
+// rows (128 x D) = P L over the HB blocks of landmarks from blk on, which the tile p holds.
 // This product and the next always run with N = 64, the width of a swizzled block: for a smaller head_dim the columns
 // past D hold nothing and are never read.
 template <int MP, int HB, int G>
@@ -227,7 +225,7 @@ __device__ __forceinline__ void issue_rows(uint32_t d, uint32_t p, uint32_t l, i
       }
     }
 }
-// tile sum (landmarks x D) = P^T X (128 x D), groups 64 columns apart.
+// tile sum (landmarks x D) = P^T X (128 x D).
 // A tile of one block: two terms of P are stacked along M (lanes 0..63 and 64..127, added when the sum is read); the
 // one partial product that this cannot place, x2 * X0, goes to the 64 columns behind the groups, lanes 64..127.
 // A tile of two blocks: the lanes are the landmarks.
@@ -401,23 +399,11 @@ __device__ __forceinline__ void copy_out(T* slice, const uint8_t* stage, int pit
       *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(slice + (r0 + row) * D) + v * 16) = *reinterpret_cast<const uint4*>(stage + row * pitch + v * 16);
   }
 }
-// the sum of G column groups (`stride` apart) of this thread's row, 16 columns of each of NB blocks of 64
-template <int NB, int G>
-__device__ __forceinline__ void ld_scores(const Frame& f, uint32_t at, int stride, float* v) {
-  const uint32_t a = f.tmem + at + f.lane_base + f.group * 16;
+// the scores of this thread's row, 16 columns of each of NB blocks of 64
+template <int NB>
+__device__ __forceinline__ void ld_scores(const Frame& f, uint32_t at, float* v) {
 #pragma unroll
-  for (int b = 0; b < NB; ++b) ld<16>(a + b * 64, v + 16 * b);
-#pragma unroll
-  for (int g = 1; g < G; ++g)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      float x[16];
-      ld<16>(a + g * stride + b * 64, x);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 16; ++j) v[16 * b + j] += x[j];
-    }
-  tmem_ld_wait();
+  for (int b = 0; b < NB; ++b) ld<16>(f.tmem + at + f.lane_base + f.group * 16 + b * 64, v + 16 * b);
 }
 // the sum of G column groups (64 apart) of this thread's row, its quarter of the D result columns
 template <int D, int G>
@@ -517,8 +503,8 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
                 float* __restrict__ part_acc, float* __restrict__ part_max, float* __restrict__ part_sum, TcSched sch,
                 int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GS = score_groups<D, 1>(), GT = 1;
-  constexpr uint32_t kS = 0, kTileSum = GS * MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GT = 2;
+  constexpr uint32_t kS = 0, kTileSum = MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
   static_assert(kSum + 64 <= 512, "tensor memory");
   constexpr float kMove = 6.f;                 // probabilities stay below e^6 = 403
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -546,7 +532,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
   rk.fetch(kk, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
     umma_commit_elect(f.bars + 0);
   }
   float sum[NC];
@@ -556,7 +542,8 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
     const bool valid = row0(i) + f.row < sch.N;
     f.wait(0, 0x4100);
     float s[NC];
-    ld_scores<NB, GS>(f, kS, MP, s);
+    ld_scores<NB>(f, kS, s);
+    tmem_ld_wait();
     bool over = false;
 #pragma unroll
     for (int j = 0; j < NC; ++j) over = over || (s[j] - s_ref[col(j)] > kMove);   // (a NaN score never raises it)
@@ -600,7 +587,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
       issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_v);
       umma_commit_elect(f.bars + 1);
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -638,8 +625,8 @@ __global__ void __launch_bounds__(kThr, 1)
 sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict__ lse1, const float* __restrict__ k_landmarks,
                 const float* __restrict__ step2, TcSched sch, int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdC, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1;
-  constexpr uint32_t kS = 0, kO = GS * MP, kCols = pow2_cols(kO + GO * 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdC, NC = 16 * NB, ND = D / 4, GO = 4;
+  constexpr uint32_t kS = 0, kO = MP, kCols = pow2_cols(kO + GO * 64);
   static_assert(kO + GO * 64 <= 512, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
@@ -663,14 +650,15 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
   rq.fetch(qq, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
     umma_commit_elect(f.bars + 0);
   }
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     f.wait(0, 0x4500);
     float s[NC];
-    ld_scores<NB, GS>(f, kS, MP, s);
+    ld_scores<NB>(f, kS, s);
+    tmem_ld_wait();
     float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
@@ -680,12 +668,13 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
     s_max[f.group * kTile + f.row] = mx;
     __syncthreads();                         // (also: the previous output tile has left the staging buffer)
     mx = fmaxf(fmaxf(s_max[f.row], s_max[kTile + f.row]), fmaxf(s_max[2 * kTile + f.row], s_max[3 * kTile + f.row]));
-    float sum = 0.f;
+    float part[4] = {0.f, 0.f, 0.f, 0.f};    // (four short chains: less rounding, and less latency)
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
       s[j] = expf(s[j] - mx);
-      sum += s[j];
+      part[j & 3] += s[j];
     }
+    float sum = (part[0] + part[1]) + (part[2] + part[3]);
 #pragma unroll
     for (int b = 0; b < NB; ++b) put_probs<HB>(s_p, f.row, b, f.group, s + 16 * b);
     rq.put(s_q);
@@ -696,7 +685,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
       issue_rows<MP, HB, GO>(f.tmem + kO, a_p, a_st, 0);
       if (!(sch.test_drop && blockIdx.x == 0 && i + 1 == f.count)) umma_commit_elect(f.bars + 1);   // fault injection on the host's request
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
+        issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -722,12 +711,13 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
 // P1 and g becomes dS1): P1 = exp(S - lse1), D1 = rowsum(P1 o dP1), dS1 = P1 o (dP1 - D1).
 template <int NC>
 __device__ __forceinline__ void softmax1_jacobian(const Frame& f, float* s_red, float* s, float* g, float lse, bool valid, int m) {
-  float d1 = 0.f;
+  float part[4] = {0.f, 0.f, 0.f, 0.f};      // (four short chains: less rounding, and less latency)
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     s[j] = (valid && (j >> 4) * 64 + f.group * 16 + (j & 15) < m) ? expf(s[j] - lse) : 0.f;
-    d1 = fmaf(s[j], g[j], d1);
+    part[j & 3] = fmaf(s[j], g[j], part[j & 3]);
   }
+  float d1 = (part[0] + part[1]) + (part[2] + part[3]);
   s_red[f.group * kTile + f.row] = d1;
   __syncthreads();
   d1 = (s_red[f.row] + s_red[kTile + f.row]) + (s_red[2 * kTile + f.row] + s_red[3 * kTile + f.row]);
@@ -746,11 +736,11 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
                 const float* __restrict__ k_landmarks, const float* __restrict__ step2, float* __restrict__ partA, TcSched sch,
                 int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdA, NC = 16 * NB, GS = score_groups<D, 1>(), GT = 1;
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdA, NC = 16 * NB, GT = NB == 1 ? 3 : 2;
   constexpr bool kAlias = HB < NB;
-  constexpr uint32_t kS = 0, kG = GS * MP, kTileSum = kAlias ? 0 : 2 * GS * MP, kTileCols = tile_cols<HB, GT>();
+  constexpr uint32_t kS = 0, kG = MP, kTileSum = kAlias ? 0 : 2 * MP, kTileCols = tile_cols<HB, GT>();
   constexpr uint32_t kSum1 = 512 - 2 * sum_cols<MP, HB>(), kSum2 = kSum1 + sum_cols<MP, HB>(), kCols = 512;
-  static_assert(kTileSum + kTileCols <= kSum1 && 2 * GS * MP <= kSum1, "tensor memory");
+  static_assert(kTileSum + kTileCols <= kSum1 && 2 * MP <= kSum1, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
   uint8_t* s_st = s_kt + L::kL;
@@ -776,8 +766,8 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
   rg.fetch(gg, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
-    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+    issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX>(f.tmem + kG, a_g, a_st);
     umma_commit_elect(f.bars + 0);
   }
   for (int i = 0; i < f.count; ++i) {
@@ -786,8 +776,9 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
     const float lse = valid ? lse1[f.bh * sch.N + row] : 0.f;
     f.wait(0, 0x4900);
     float s[NC], g[NC];
-    ld_scores<NB, GS>(f, kS, MP, s);
-    ld_scores<NB, GS>(f, kG, MP, g);
+    ld_scores<NB>(f, kS, s);
+    ld_scores<NB>(f, kG, g);
+    tmem_ld_wait();
     softmax1_jacobian<NC>(f, s_red, s, g, lse, valid, m);
 #pragma unroll
     for (int b0 = 0; b0 < NB; b0 += HB) {
@@ -810,7 +801,7 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
       if (f.warp == 0) {
         issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_q);
         umma_commit_elect(f.bars + 2);
-        if (more && !kAlias) issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+        if (more && !kAlias) issue_scores<D, MP, NX>(f.tmem + kG, a_g, a_st);
       }
       if (b0 == 0 && i + 2 < f.count) rg.fetch(gg, row0(i + 2), sch.N);
       f.wait(2, 0x4b00);                     // dS1 (and, after the last block, Q) have been used
@@ -821,8 +812,8 @@ sx_bwd_a_kernel(const T* __restrict__ q, const T* __restrict__ d_out, const floa
       if (i + 2 < f.count) rq.fetch(qq, row0(i + 2), sch.N);
       f.publish();
       if (f.warp == 0) {
-        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
-        if (kAlias) issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+        issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+        if (kAlias) issue_scores<D, MP, NX>(f.tmem + kG, a_g, a_st);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -846,9 +837,9 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
                 const float* __restrict__ dO3, const float* __restrict__ dkt_tot, float* __restrict__ partB, TcSched sch, int m,
                 float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1, GT = 1;
-  constexpr uint32_t kS = 0, kG = GS * MP, kDv = 0, kDk = kDv + NB * GO * 64, kTileSum = kDk + NB * GO * 64, kSum = 512 - MP, kCols = 512;
-  static_assert(L::kHBwdB == 1 && 2 * GS * MP <= kSum && kTileSum + tile_cols<1, GT>() <= kSum, "tensor memory");
+  constexpr int NX = L::NX, NB = L::NB, NC = 16 * NB, ND = D / 4, GV = 4 / NB / NB;   // GV: column groups of dV
+  constexpr uint32_t kS = 0, kG = MP, kDv = 0, kDk = kDv + NB * GV * 64, kTileSum = kDk + NB * 64, kSum = 512 - MP, kCols = 512;
+  static_assert(L::kHBwdB == 1 && 2 * MP <= kSum && kTileSum + tile_cols<1, 1>() <= kSum, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_qt = smem;
   uint8_t* s_g3 = s_qt + L::kL;
@@ -881,8 +872,8 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
   rv.put(s_p);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
-    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_p, a_g3);
+    issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX>(f.tmem + kG, a_p, a_g3);
     umma_commit_elect(f.bars + 0);
   }
   for (int i = 0; i < f.count; ++i) {
@@ -894,8 +885,9 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     }
     f.wait(0, 0x5100);
     float s[NC], g[NC];
-    ld_scores<NB, GS>(f, kS, MP, s);
-    ld_scores<NB, GS>(f, kG, MP, g);
+    ld_scores<NB>(f, kS, s);
+    ld_scores<NB>(f, kG, g);
+    tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < NC; ++j) {
       s[j] = valid ? expf(s[j] - s_l3[col(j)]) : 0.f;
@@ -905,15 +897,15 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     for (int b = 0; b < NB; ++b) {
       if (b > 0) {
         f.wait(1, 0x5200);                   // the previous block's products are done: both buffers are free
-        add_tile_sum<D, 1, GT>(f, kTileSum, kSum + 64 * (b - 1), i == 0);
+        add_tile_sum<D, 1, 1>(f, kTileSum, kSum + 64 * (b - 1), i == 0);
       }
       put_probs<1>(s_p, f.row, 0, f.group, s + 16 * b);
       put_probs<1>(s_ds, f.row, 0, f.group, g + 16 * b);
       f.publish();
       if (f.warp == 0) {
-        issue_rows<MP, 1, GO>(f.tmem + kDv + b * GO * 64, a_p, a_g3, b);
-        issue_rows<MP, 1, GO>(f.tmem + kDk + b * GO * 64, a_ds, a_qt, b);
-        issue_contract<1, NX, GT>(f.tmem + kTileSum, a_ds, a_k);
+        issue_rows<MP, 1, GV>(f.tmem + kDv + b * GV * 64, a_p, a_g3, b);
+        issue_rows<MP, 1, 1>(f.tmem + kDk + b * 64, a_ds, a_qt, b);
+        issue_contract<1, NX, 1>(f.tmem + kTileSum, a_ds, a_k);
         umma_commit_elect(f.bars + 1);
       }
     }
@@ -927,9 +919,9 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     }
     f.wait(1, 0x5300);
     float o[ND];
-    ld_rows<D, NB * GO>(f, kDv, o);
+    ld_rows<D, NB * GV>(f, kDv, o);
     stage_row<T, D>(s_p, L::kPitch, f.row, d0, o);
-    ld_rows<D, NB * GO>(f, kDk, o);
+    ld_rows<D, NB>(f, kDk, o);
 #pragma unroll
     for (int j = 0; j < ND; ++j) o[j] += add[j];    // (the operand carries s)
     stage_row<T, D>(s_ds, L::kPitch, f.row, d0, o);
@@ -939,14 +931,14 @@ sx_bwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, T* __restrict_
     tc_fence_after();
     copy_out<T, D>(dv + f.bh * sch.N * D, s_p, L::kPitch, row0(i), sch.N);
     copy_out<T, D>(dk + f.bh * sch.N * D, s_ds, L::kPitch, row0(i), sch.N);
-    add_tile_sum<D, 1, GT>(f, kTileSum, kSum + 64 * (NB - 1), i == 0);
+    add_tile_sum<D, 1, 1>(f, kTileSum, kSum + 64 * (NB - 1), i == 0);
     if (more) {
       __syncthreads();                       // the staged tiles have been read
       rv.put(s_p);
       f.publish();
       if (f.warp == 0) {
-        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
-        issue_scores<D, MP, NX, GS>(f.tmem + kG, a_p, a_g3);
+        issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX>(f.tmem + kG, a_p, a_g3);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -963,9 +955,9 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
                 const float* __restrict__ k_landmarks, const float* __restrict__ step2, const float* __restrict__ dqt_tot,
                 TcSched sch, int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdC, NC = 16 * NB, ND = D / 4, GS = score_groups<D, 1>(), GO = 1;
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHBwdC, NC = 16 * NB, ND = D / 4, GO = 4 * HB / NB;
   constexpr int GA = NB / HB * GO;           // column groups of dQ: GO for each turn
-  constexpr uint32_t kS = 0, kG = GS * MP, kO = 2 * GS * MP, kCols = pow2_cols(kO + GA * 64);
+  constexpr uint32_t kS = 0, kG = MP, kO = 2 * MP, kCols = pow2_cols(kO + GA * 64);
   static_assert(kO + GA * 64 <= 512, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
@@ -992,8 +984,8 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
   rg.fetch(gg, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
-    issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+    issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX>(f.tmem + kG, a_g, a_st);
     umma_commit_elect(f.bars + 0);
   }
   Segments sg(sch.seg_N, m);
@@ -1005,8 +997,9 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
     const float lse = valid ? lse1[f.bh * sch.N + row] : 0.f;
     f.wait(0, 0x5500);
     float s[NC], g[NC];
-    ld_scores<NB, GS>(f, kS, MP, s);
-    ld_scores<NB, GS>(f, kG, MP, g);
+    ld_scores<NB>(f, kS, s);
+    ld_scores<NB>(f, kG, g);
+    tmem_ld_wait();
     softmax1_jacobian<NC>(f, s_red, s, g, lse, valid, m);   // (its barrier: the previous output tile has left s_ds)
 #pragma unroll
     for (int b0 = 0; b0 < NB; b0 += HB) {
@@ -1022,8 +1015,8 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
         issue_rows<MP, HB, GO>(f.tmem + kO + b0 / HB * GO * 64, a_ds, a_kt, b0);
         umma_commit_elect(f.bars + 1);
         if (b0 == 0 && more) {
-          issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
-          issue_scores<D, MP, NX, GS>(f.tmem + kG, a_g, a_st);
+          issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+          issue_scores<D, MP, NX>(f.tmem + kG, a_g, a_st);
           umma_commit_elect(f.bars + 0);
         }
       }

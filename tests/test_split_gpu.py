@@ -1,12 +1,10 @@
 """The split-precision tensor-core passes (fp32 with up to 64 landmarks; 16-bit inputs of head_dim 16 / 32, and of
 head_dim 64 with more than 64 landmarks) against the float64 oracle, with the FP32 CUDA-core kernels
 as the yardstick: the same calls are made through both, and the split kernels may not be further
-from the oracle than the CUDA-core ones by more than what their operands drop.  fp32 operands keep 24
-bits in three bf16 terms; per product the dropped terms and the truncating accumulator stay below
-2^-22 = 2.4e-7, and the pseudoinverse (condition number up to a few tens here) amplifies it like it does the
-yardstick's own rounding: bound 1.5 x yardstick + 1e-6.  16-bit inputs: the landmark operands and the
-probabilities have the same 24 bits, the results' own rounding (2^-12, 2^-9 relative at most) dominates both sides:
-bound 1.05 x yardstick + 5e-5."""
+from the oracle than the CUDA-core ones by more than what the pseudoinverse (condition number up to a few tens
+here, on other kernels too when the CUDA cores are forced) makes of the last places: bound 1.5 x yardstick + 1e-6.  16-bit
+inputs: the results' own rounding (2^-12, 2^-9 relative at most) dominates both sides: bound 1.05 x yardstick + 5e-5.  What
+these bounds cannot see, the exactness of the passes themselves, has tests of its own below."""
 import pytest
 import torch
 
@@ -156,3 +154,36 @@ def test_infinities_and_nan_stay_where_the_fp32_kernels_have_them(cuda_device, b
         assert torch.isfinite(got[0, 0]).all(0).sum() == (D - 1 if which == 2 else 0)
     torch.cuda.synchronize()
     _C.check_device_status()
+
+
+@pytest.mark.parametrize("B,H,N,D,m,qk", [(1, 4, 1024, 64, 32, 64 ** -0.25), (2, 2, 4096, 64, 64, 1.0), (1, 4, 3000, 32, 33, 1.0), (1, 8, 700, 64, 48, 2.0),
+                                           (1, 8, 2000, 16, 64, 1.0), (4, 16, 128, 64, 64, 1.0), (1, 2, 20000, 64, 64, 1.0)])
+def test_fp32_passes_are_as_exact_as_the_cuda_cores(cuda_device, B, H, N, D, m, qk):
+    """What the passes make of the landmark tensors that the call itself saved, against the same in 64 bits, so that the
+    pseudoinverse's error is no part of it; four seeds.  Bound 1.15 x the CUDA-core kernels' error, for the spread between
+    seeds.  (With each product in one accumulator of the tensor core, which truncates, the output and dV are 1.2 to 1.4 x
+    as far off.)"""
+    from flashnystrom_b200 import _C
+    s = float(torch.tensor(D ** -0.25, dtype=F32))
+    err = {}
+    for seed in range(4):
+        q, k, v, dO = (t.cuda() for t in O.make_inputs(B, H, N, D, seed=seed, dtype=F32))
+        q, k = q * qk, k * qk
+        for generic in (False, True):
+            _C.set_force_generic(generic)
+            try:
+                got = run_cuda(q, k, v, dO, m, 6)
+            finally:
+                _C.set_force_generic(False)
+            x = {key: t.double() for key, t in got.items()}
+            s1, s3 = (q.double() * s) @ x["kt"].transpose(-2, -1), x["qt"] @ (k.double() * s).transpose(-2, -1)
+            p1, p3 = torch.softmax(s1, -1), torch.softmax(s3, -1)
+            d_o3 = x["k2inv"].transpose(-2, -1) @ (p1.transpose(-2, -1) @ dO.double())
+            want = dict(lse1=torch.logsumexp(s1, -1), lse3=torch.logsumexp(s3, -1), bmat=p3 @ v.double(), out=p1 @ x["step2"],
+                        dv=p3.transpose(-2, -1) @ d_o3)
+            for key, w in want.items():
+                err[key, generic] = err.get((key, generic), 0.0) + float((x[key] - w).norm() / w.norm()) ** 2
+    for key in want:
+        print(key, f"{(err[key, False] / 4) ** 0.5:.2e} {(err[key, True] / 4) ** 0.5:.2e} {(err[key, False] / err[key, True]) ** 0.5:.2f}")
+    for key in want:
+        assert err[key, False] <= 1.15 ** 2 * err[key, True], key
