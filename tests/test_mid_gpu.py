@@ -2,8 +2,9 @@
 CUDA-core kernels as the yardstick.  FP32 inputs run the same streaming passes on both sides, so only these stages
 differ.  Operands keep 24 bits in three bf16 terms.  The accumulator truncates: the eight K steps of a product lose up
 to 8 * 2^-24, all in one direction, where the yardstick's 128 rounded additions lose about sqrt(128) / 2 * 2^-24
-= 6 * 2^-24 in either direction; both are amplified alike by the iterations, but a bias adds up over the terms of the
-sums that follow (up to sqrt(64) = 8 times) where rounding averages out: bound 8 x yardstick + 1e-6."""
+= 6 * 2^-24 in either direction; both are amplified alike by the iterations: bound 2 x yardstick for what these stages
+form.  A bias adds up over the terms of the sums that follow (up to sqrt(64) = 8 times) where rounding averages out:
+bound 8 x yardstick for the outputs and gradients."""
 import pytest
 import torch
 
@@ -38,18 +39,27 @@ def test_against_cuda_core_stages(cuda_device, B, H, N, D, m, J, kappa):
     for key in ("K2", "lse2", "k2inv", "step2", "out", "dq", "dk", "dv"):
         a, b = _rel(pick(got[key]), want[key]), _rel(pick(ref[key]), want[key])
         print(key, f"{a:.2e} {b:.2e}")
-        assert a <= 8 * b + 1e-6, (key, a, b)
+        assert a <= (2 if key in ("K2", "lse2", "k2inv", "step2") else 8) * b, (key, a, b)
 
 
-@pytest.mark.parametrize("BH", [2, 37, 38])     # beside the column passes up to a quarter of 148 SMs, in line above
-@pytest.mark.parametrize("D", [64, 128])
-def test_beside_the_column_passes(cuda_device, BH, D):
-    """The same slice comes out the same whatever runs beside it; fp16 results are within one rounding of the sums."""
-    m, J, N = 96, 6, 700
-    q, k, v, dO = O.make_inputs(1, BH, N, D, seed=11, dtype=torch.float16)
-    got = run_cuda(q, k, v, dO, m, J, 5.0)
-    again = run_cuda(q, k, v, dO, m, J, 5.0)
-    want = run_oracle(q[:, -1:], k[:, -1:], v[:, -1:], dO[:, -1:], m, J, 5.0)
-    for key, bound in (("out", 2e-3), ("dq", 1e-2), ("dk", 1e-2), ("dv", 1e-2)):
-        assert torch.equal(got[key], again[key]), key
-        assert O.rel_max(got[key][:, -1:].cpu(), want[key]) <= bound, key
+@pytest.mark.parametrize("D,m,dtype", [(64, 96, torch.float16), (128, 96, torch.float16), (64, 65, torch.bfloat16), (32, 128, torch.float16)])
+def test_beside_the_column_passes(cuda_device, D, m, dtype):
+    """Up to a quarter of the SMs' worth of slices the pseudoinverse kernels run beside the column passes, above in line, and
+    with more slices than clusters a cluster walks several.  The FP32 matrices of a slice do not depend on any of it,
+    bit for bit; what the column passes make of them differs by the order of their chunks, one rounding of the result."""
+    from flashnystrom_b200 import _C
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    J, N, few = 6, 700, sms // 4
+    q, k, v, dO = O.make_inputs(1, sms + 5, N, D, seed=11, dtype=dtype)
+    runs = [run_cuda(*(t[:, :BH] for t in (q, k, v, dO)), m, J, 5.0) for BH in (few, few, few + 1, sms + 5)]
+    want = run_oracle(q[:, few - 1:few], k[:, few - 1:few], v[:, few - 1:few], dO[:, few - 1:few], m, J, 5.0)
+    eps = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
+    for r in runs[1:]:
+        for key in ("qt", "kt", "K2", "lse2", "iterates", "k2inv"):
+            assert torch.equal(r[key][:, :few], runs[0][key]), key
+        for key in ("out", "dq", "dk", "dv"):
+            a, b = r[key][:, :few].float(), runs[0][key].float()
+            assert float((a - b).norm() / b.norm()) <= eps, key
+            assert O.rel_max(r[key][:, few - 1:few].cpu(), want[key]) <= (2 if key == "out" else 10) * eps, key
+    for key in ("out", "dq", "dk", "dv"):
+        assert torch.equal(runs[0][key], runs[1][key]), key
