@@ -485,9 +485,9 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
   if (S.run(0)) {
     {
       L.begin();
-      // One warp per item where an item is at most 32 KB, the whole CTA above.  Measured (us, CTA / warp): B=32, H=16,
-      // N=2000, D=64 (4 KB items) 404 / 66, B=1, H=7, N=50001, m=33 (24 KB) 32 / 25, B=2, H=8, N=16384, D=128, m=128 (32 KB)
-      // 37 / 32, B=4, H=16, N=16384, D=128 (64 KB, and fewer than two items per warp) 93 / 103.
+      // One warp per item where an item is at most 32 KB, the whole CTA above (the sums are the same).  Measured (us, CTA / warp):
+      // B=32, H=16, N=2000, D=64 (4 KB items) 404 / 94, B=1, H=7, N=50001, m=33 (24 KB) 32 / 22, B=2, H=8, N=16384, D=128,
+      // m=128 (32 KB) 37 / 36; at B=4, H=16, N=16384, D=128 (64 KB) there are fewer than two items per warp.
       const int64_t items = 2 * p.BH * p.m * lmC, seg = seg_N / p.m;
       if (items > 0x7fffffff) return fail(FNB_ERR_INVALID_ARGUMENT, "too many pooling items (%lld)", (long long)items);
       const bool by_warp = (seg + lmC - 1) / lmC * p.D * (int64_t)sizeof(T) <= 32 * 1024;
@@ -649,7 +649,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
       cp.acc_bh_stride = (int64_t)nchunk_b * p.m * p.D; cp.acc_chunk_stride = (int64_t)p.m * p.D;
       cp.vec_bh_stride = (int64_t)nchunk_b * p.m; cp.vec_chunk_stride = p.m;
     }
-    if ((use_tc || use_sx) && p.D % 16 == 0) {
+    if (use_tc || use_sx) {
       // the tensor-core output passes pack their own operand copies: merge + step2 only, spread over
       // D / 16 CTAs per slice
       CombineSlabParams sp2;

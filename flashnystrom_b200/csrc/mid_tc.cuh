@@ -21,9 +21,10 @@
 //
 // What bounds it: the latency of a phase, about 9000 cycles with one product (result block out to L2 2000-2400,
 // meeting the peer 800, first chunk in 1550, MMAs 2400, accumulator out and split 2300), not the 144 KB a CTA copies
-// per product.  Clusters of four or eight that copied FP32 operands and split them in every CTA took, on a B200 at
-// B=2, H=8 (us, before / now): forward D=128, J=8 with ridge 326 / 216, D=64, J=6 without 234 / 160; backward
-// 651 / 439 and 478 / 310; per iteration 37 / 19 and 70 / 37.
+// per product (ncu: tensor pipe active 13 to 18 %, DRAM idle).  Clusters of four or eight that copied FP32 operands and split
+// them in every CTA took, on a B200 at B=2, H=8 (us, before / now): forward D=128, J=8 with ridge 326 / 222, D=64, J=6 without
+// 234 / 164; backward 651 / 443 and 478 / 316; per iteration 37 / 19 and 70 / 37.  One to eight slices of head_dim 128,
+// training pass: 705 .. 820 / 526 .. 643.
 #pragma once
 #include "common.cuh"
 #include "small_kernels.cuh"

@@ -20,13 +20,13 @@
 // saved lse1 and the outputs were 25 to 50 % less exact.  With more than 64 landmarks a probability tile
 // is 96 KB; where that leaves no room for the rest, its two blocks take turns in one of 48 KB.
 //
-// What bounds it: the MMAs of the fp32 passes (24 per 128 x 64 x 64 product at 48 cycles each, the time
-// their operands take through shared memory; a tile of the column pass of the backward needs 128 of
-// them) and, for 16-bit inputs, the exp / split / store work on the probabilities, each in turn with the
-// other for want of room for a second set of buffers.  Measured on a B200, us per launch, against the
-// CUDA-core kernels of generic_kernels.cuh (fwd_b, fwd_c, bwd_a, bwd_b, bwd_c):
-//   fp32, B=1, H=16, N=16384, D=64, m=64    1135, 574, 1996, 1948, 863  ->  78, 64, 117, 130, 95
-//   bf16, B=2, H=8,  N=8192,  D=64, m=128    727, 431, 1319, 1379, 713  ->  41, 37,  50,  60, 46
+// What bounds it: no unit, but the phases of a tile in turn (input split, score MMAs, exponentials and split of the
+// probabilities, MMAs, results out), which one CTA per SM cannot overlap much for want of room for a second set of buffers.
+// fp32, shape below: tensor pipe active 17 to 26 % (about 36 cycles per 128 x 64 x 16 MMA, whose operands come out of
+// shared memory; the column pass of the backward issues 128 of them per tile), issue slots 35 to 43 %, DRAM 14 to 20 %.
+// Measured on a B200, us per launch, against the CUDA-core kernels of generic_kernels.cuh (fwd_b, fwd_c, bwd_a, bwd_b, bwd_c):
+//   fp32, B=1, H=16, N=16384, D=64, m=64    1135, 574, 1996, 1948, 863  ->  95, 70, 129, 143, 103
+//   bf16, B=2, H=8,  N=8192,  D=64, m=128    727, 431, 1319, 1379, 713  ->  60, 50,  69, 101,  64
 #pragma once
 #include <type_traits>
 #include "common.cuh"
