@@ -182,12 +182,15 @@ __device__ __forceinline__ void put_probs(uint8_t* tile, int r, int b, int group
 // shows, the K steps of the leading one are spread over G accumulators of their own (column groups 64 apart), which the
 // epilogue adds in FP32.  With everything in one accumulator the output and dV of fp32 calls were 1.2 to 1.4 times as far
 // from the oracle as with the CUDA-core kernels, with the groups below 0.5 to 1.03 times, for 3 % of the passes'
-// time; spreading the scores' K steps as well changed nothing but the time (680 -> 695 us for a training
-// pass, B=1, H=16, N=16384, D=64, m=64).
-// scores (128 x MP) = X (128 x D) L^T
-template <int D, int MP, int NX>
+// time.  The scores have two groups in the forward passes of more than 64 landmarks, where lse3 was 1.2 times as far off
+// at scores of about 10 without; elsewhere that changed nothing but the time (680 -> 695 us for a training pass,
+// fp32, B=1, H=16, N=16384, D=64, m=64).
+// scores (128 x MP) = X (128 x D) L^T, groups MP columns apart
+template <int D, int MP, int NX, int G = 1>
 __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l) {
   constexpr uint32_t idesc = make_idesc<bf16>(kTile, MP, false, false);
+  constexpr int K = D / 16;
+  static_assert(G <= K, "a group has a K step at least");
   bool acc = false;
 #pragma unroll
   for (int s = kTerms - 1; s >= 0; --s)
@@ -196,8 +199,11 @@ __device__ __forceinline__ void issue_scores(uint32_t d, uint32_t x, uint32_t l)
       const int j = s - i;
       if (j < 0 || j >= kTerms) continue;
 #pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        umma_elect(d, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc, acc);
+      for (int k = 0; k < K; ++k) {
+        const int g = s == 0 ? k * G / K : 0;
+        const bool first = g > 0 && (k - 1) * G / K != g;
+        umma_elect(d + g * MP, smem_desc_sw128(x + i * kBlk + k * 32, 16, 1024), smem_desc_sw128(l + j * (MP * 128) + k * 32, 16, 1024), idesc,
+                   g > 0 ? !first : acc);
         acc = true;
       }
     }
@@ -399,11 +405,22 @@ __device__ __forceinline__ void copy_out(T* slice, const uint8_t* stage, int pit
       *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(slice + (r0 + row) * D) + v * 16) = *reinterpret_cast<const uint4*>(stage + row * pitch + v * 16);
   }
 }
-// the scores of this thread's row, 16 columns of each of NB blocks of 64
-template <int NB>
+// the scores of this thread's row, 16 columns of each of NB blocks of 64, the sum of G column groups
+template <int NB, int G = 1>
 __device__ __forceinline__ void ld_scores(const Frame& f, uint32_t at, float* v) {
+  const uint32_t a = f.tmem + at + f.lane_base + f.group * 16;
 #pragma unroll
-  for (int b = 0; b < NB; ++b) ld<16>(f.tmem + at + f.lane_base + f.group * 16 + b * 64, v + 16 * b);
+  for (int b = 0; b < NB; ++b) ld<16>(a + b * 64, v + 16 * b);
+#pragma unroll
+  for (int g = 1; g < G; ++g)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      float x[16];
+      ld<16>(a + g * (NB * 64) + b * 64, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[16 * b + j] += x[j];
+    }
 }
 // the sum of G column groups (64 apart) of this thread's row, its quarter of the D result columns
 template <int D, int G>
@@ -503,8 +520,8 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
                 float* __restrict__ part_acc, float* __restrict__ part_max, float* __restrict__ part_sum, TcSched sch,
                 int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GT = 2;
-  constexpr uint32_t kS = 0, kTileSum = MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdB, NC = 16 * NB, GS = NB == 2 && D > 16 ? 2 : 1, GT = 2;
+  constexpr uint32_t kS = 0, kTileSum = GS * MP, kSum = kTileSum + tile_cols<HB, GT>(), kCols = pow2_cols(kSum + 64);
   static_assert(kSum + 64 <= 512, "tensor memory");
   constexpr float kMove = 6.f;                 // probabilities stay below e^6 = 403
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -532,7 +549,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
   rk.fetch(kk, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
     umma_commit_elect(f.bars + 0);
   }
   float sum[NC];
@@ -542,7 +559,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
     const bool valid = row0(i) + f.row < sch.N;
     f.wait(0, 0x4100);
     float s[NC];
-    ld_scores<NB>(f, kS, s);
+    ld_scores<NB, GS>(f, kS, s);
     tmem_ld_wait();
     bool over = false;
 #pragma unroll
@@ -587,7 +604,7 @@ sx_fwd_b_kernel(const T* __restrict__ k, const T* __restrict__ v, const float* _
       issue_contract<HB, NX, GT>(f.tmem + kTileSum, a_p, a_v);
       umma_commit_elect(f.bars + 1);
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX>(f.tmem + kS, a_k, a_qt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_k, a_qt);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -625,8 +642,8 @@ __global__ void __launch_bounds__(kThr, 1)
 sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict__ lse1, const float* __restrict__ k_landmarks,
                 const float* __restrict__ step2, TcSched sch, int m, float scale, int* status) {
   using L = Plan<T, D, MP>;
-  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdC, NC = 16 * NB, ND = D / 4, GO = 4;
-  constexpr uint32_t kS = 0, kO = MP, kCols = pow2_cols(kO + GO * 64);
+  constexpr int NX = L::NX, NB = L::NB, HB = L::kHFwdC, NC = 16 * NB, ND = D / 4, GS = NB == 2 && D > 16 ? 2 : 1, GO = 4;
+  constexpr uint32_t kS = 0, kO = GS * MP, kCols = pow2_cols(kO + GO * 64);
   static_assert(kO + GO * 64 <= 512, "tensor memory");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* s_kt = smem;
@@ -650,14 +667,14 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
   rq.fetch(qq, row0(1), sch.N);
   f.publish();
   if (f.warp == 0) {
-    issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+    issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
     umma_commit_elect(f.bars + 0);
   }
   for (int i = 0; i < f.count; ++i) {
     const int64_t row = row0(i) + f.row;
     f.wait(0, 0x4500);
     float s[NC];
-    ld_scores<NB>(f, kS, s);
+    ld_scores<NB, GS>(f, kS, s);
     tmem_ld_wait();
     float mx = -INFINITY;
 #pragma unroll
@@ -685,7 +702,7 @@ sx_fwd_c_kernel(const T* __restrict__ q, T* __restrict__ out, float* __restrict_
       issue_rows<MP, HB, GO>(f.tmem + kO, a_p, a_st, 0);
       if (!(sch.test_drop && blockIdx.x == 0 && i + 1 == f.count)) umma_commit_elect(f.bars + 1);   // fault injection on the host's request
       if (i + 1 < f.count) {
-        issue_scores<D, MP, NX>(f.tmem + kS, a_q, a_kt);
+        issue_scores<D, MP, NX, GS>(f.tmem + kS, a_q, a_kt);
         umma_commit_elect(f.bars + 0);
       }
     }
@@ -1051,7 +1068,7 @@ sx_bwd_c_kernel(const T* __restrict__ q, const T* __restrict__ d_out, T* __restr
 // 16 .. 64 and up to 128 landmarks (head_dim 64 with up to 64 landmarks has 16-bit kernels of its own, which are
 // asked first).  The line lies where the term tiles of one 128-row tile and both landmark operands stop fitting into
 // shared memory: three terms of a 128-landmark or head_dim-128 operand pair take 96 .. 192 KB alone.  They are
-// faster than the CUDA-core kernels from one tile on (B=1, H=4, N=1024, m=32, fp32: 143 -> 76 us for the five).
+// faster than the CUDA-core kernels from one tile on (B=1, H=4, N=1024, m=32, fp32: 143 -> 79 us for the five).
 inline bool supported(int dtype, int D, int m, uint32_t flags) {
   if ((flags & FNB_FLAG_FORCE_GENERIC) || D > 64) return false;
   return dtype == FNB_F32 ? m <= 64 : m <= 128;

@@ -71,7 +71,8 @@ def test_moving_reference(cuda_device):
 def test_16bit_inputs_keep_fp32_operands(cuda_device, case):
     """The FP32 results of the forward passes (16-bit outputs would hide a loss) for 16-bit inputs, large scores among
     them: no further from the oracle than the CUDA-core kernels, which multiply in FP32.  Every operand has 24 bits on
-    both sides; what differs is the order and rounding of the sums, bound 2 x yardstick.  (Operands of 16 bits are
+    both sides; what differs is the order and rounding of the sums: bound 1.15 x yardstick, for the spread of a few slices;
+    2 x for step2, whose pseudoinverse comes from other kernels too when the CUDA cores are forced.  (Operands of 16 bits are
     4 to 18 x off, at scores of about 30 an error of 1e-4 in single probabilities.)"""
     from flashnystrom_b200 import _C
     B, H, N, D, m, J, kappa, qk, dtype = case
@@ -87,7 +88,7 @@ def test_16bit_inputs_keep_fp32_operands(cuda_device, case):
     for key in ("bmat", "step2", "lse1", "lse3"):
         a, b = _rel(got[key], want[key]), _rel(ref[key], want[key])
         print(key, f"{a:.2e} {b:.2e}")
-        assert a <= 2 * b, (key, a, b)
+        assert a <= (2 if key == "step2" else 1.15) * b, (key, a, b)
 
 
 @pytest.mark.parametrize("B,H,N,D,m", [(1, 4, 1024, 64, 32), (2, 2, 4096, 64, 64), (1, 8, 2000, 16, 64), (1, 4, 3000, 32, 33)])
