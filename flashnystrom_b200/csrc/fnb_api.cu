@@ -553,7 +553,7 @@ static int forward_impl(const fnb_fwd_args& a, const Plan& p, const FwdWs& w, in
     np.qt_out = a.q_landmarks; np.kt_out = a.k_landmarks;
     if (ns_on_tensor_cores(a.shape.flags)) {
       if (int rc = set_smem(nstc::ns_fwd_tc_kernel, nstc::kFwdSmem, max_smem, "ns_fwd")) return rc;
-      nstc::ns_fwd_tc_kernel<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kFwdSmem, ns_stream>>>(np, a.device_status);
+      nstc::ns_fwd_tc_kernel<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kFwdSmem, ns_stream>>>(nstc::FwdParams{np, false}, a.device_status);
     } else {
       if (int rc = set_smem(ns::ns_fwd_kernel, ns::kFwdSmem, max_smem, "ns_fwd")) return rc;
       ns::ns_fwd_kernel<<<(unsigned)p.BH, kThreads, ns::kFwdSmem, ns_stream>>>(np);
@@ -886,18 +886,21 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       np.m = p.m; np.D = p.D; np.J = p.J; np.kappa = a.shape.kappa_star;
       np.rows_k = use_tc ? w.rows_k : nullptr; np.N = seg_N; np.scale = scale;
       if (p.J >= 1 && ns_on_tensor_cores(a.shape.flags)) {
-        auto ns_kern = p.D == 128 ? nstc::ns_bwd_tc_kernel<2> : nstc::ns_bwd_tc_kernel<1>;
-        if (int rc = set_smem(ns_kern, nstc::kBwdSmem, max_smem, "ns_bwd")) return rc;
-        nstc::BwdHeadParams hp{};
+        if (int rc = set_smem(nstc::ns_bwd_tc_kernel, nstc::kBwdSmem, max_smem, "ns_bwd")) return rc;
+        nstc::BwdParams bp{};
+        nstc::BwdHeadParams& hp = bp.h;
+        bp.p = np;
+        const int finish = p.D == 128 ? 2 : 1;       // 64 columns of the landmarks at a time
         if (fused_mid) {
           hp.partA = fused_pa; hp.nchunk = fused_pa_chunks; hp.k2inv = a.k2_inv; hp.bmat = a.bmat;
           hp.dkt_a = w.dkt_a; hp.D3 = side_ns ? nullptr : w.D3; hp.do3n = do3n; hp.do3_scale = w.do3_scale;
           hp.qt16 = qt16; hp.qt_mul = scale * tc::kLog2e; hp.dtype = a.shape.dtype; hp.MP = MP;
         }
         if (side_ns)
-          ns_kern<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kBwdSmem, ns_stream>>>(np, hp, a.device_status);
+          nstc::ns_bwd_tc_kernel<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kBwdSmem, ns_stream>>>(bp, finish, a.device_status);
         else
-          launch_pdl(ns_kern, dim3((unsigned)p.BH), dim3(nstc::kNsTcThreads), nstc::kBwdSmem, st, np, hp, a.device_status);
+          launch_pdl(nstc::ns_bwd_tc_kernel, dim3((unsigned)p.BH), dim3(nstc::kNsTcThreads), nstc::kBwdSmem, st, bp, finish,
+                     a.device_status);
       } else {
         if (int rc = set_smem(ns::ns_bwd_kernel, ns::kBwdSmem, max_smem, "ns_bwd")) return rc;
         ns::ns_bwd_kernel<<<(unsigned)p.BH, kThreads, ns::kBwdSmem, st>>>(np);
@@ -1301,10 +1304,12 @@ int fnb_debug_pinv_forward(int64_t bh, int32_t m, int32_t J, float kappa, const 
   DeviceGuard g(device);
   if (!g.ok) return fail(FNB_ERR_CUDA, "cannot select CUDA device %d", device);
   if (m <= ns::kN && ns_on_tensor_cores(0)) {
-    FNB_CUDA(cudaFuncSetAttribute(nstc::ns_pinv_fwd_tc_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)nstc::kFwdSmem));
-    nstc::ns_pinv_fwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kFwdSmem, (cudaStream_t)stream>>>(
-        k2, ns_iterates, k2_inv, m, J, kappa, nullptr);
+    nstc::FwdParams fp{};
+    fp.k2_given = true;
+    fp.p.k2 = const_cast<float*>(k2);    // (given softmaxed: only read)
+    fp.p.iterates = ns_iterates; fp.p.k2inv = k2_inv; fp.p.m = m; fp.p.J = J; fp.p.kappa = kappa;
+    FNB_CUDA(raise_smem(reinterpret_cast<const void*>(nstc::ns_fwd_tc_kernel), nstc::kFwdSmem));
+    nstc::ns_fwd_tc_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kFwdSmem, (cudaStream_t)stream>>>(fp, nullptr);
   } else if (m > ns::kN) {
     mx::FwdParams mp;
     memset(&mp, 0, sizeof(mp));
@@ -1331,10 +1336,11 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
   DeviceGuard g(device);
   if (!g.ok) return fail(FNB_ERR_CUDA, "cannot select CUDA device %d", device);
   if (m <= ns::kN && ns_on_tensor_cores(0)) {
-    FNB_CUDA(cudaFuncSetAttribute(nstc::ns_pinv_bwd_tc_debug_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)nstc::kBwdSmem));
-    nstc::ns_pinv_bwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(
-        k2, ns_iterates, d_k2_inv, d_k2, (float*)workspace, m, J, kappa, nullptr, nullptr, nullptr);
+    nstc::BwdParams bp{};
+    bp.p.k2 = k2; bp.p.iterates = ns_iterates; bp.p.G = d_k2_inv; bp.p.spill = (float*)workspace;
+    bp.p.m = m; bp.p.D = ns::kN; bp.p.J = J; bp.p.kappa = kappa; bp.dK2 = d_k2;
+    FNB_CUDA(raise_smem(reinterpret_cast<const void*>(nstc::ns_bwd_tc_kernel), nstc::kBwdSmem));
+    nstc::ns_bwd_tc_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, 0, nullptr);
   } else if (m > ns::kN) {
     mx::BwdParams mp;
     memset(&mp, 0, sizeof(mp));
@@ -1421,10 +1427,12 @@ int fnb_debug_ns_bwd_step(int64_t bh, int32_t m, const float* k2, const float* z
   if (!g.ok) return fail(FNB_ERR_CUDA, "cannot select CUDA device %d", device);
   int max_smem = 0, cc = 0, sms = 0;
   if (int rc = device_limits(device, &max_smem, &cc, &sms)) return rc;
-  if (int rc = set_smem(nstc::ns_pinv_bwd_tc_debug_kernel, nstc::kBwdSmem, max_smem, "ns_pinv_bwd")) return rc;
+  if (int rc = set_smem(nstc::ns_bwd_tc_kernel, nstc::kBwdSmem, max_smem, "ns_pinv_bwd")) return rc;
   // one iteration of the product kernel's loop (J = 1, no ridge), stopped in front of the Z0 tail
-  nstc::ns_pinv_bwd_tc_debug_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(
-      k2, z_j, d_z_next, nullptr, nullptr, m, 1, 0.f, nullptr, d_z_out, d_k2_acc);
+  nstc::BwdParams bp{};
+  bp.p.k2 = k2; bp.p.iterates = z_j; bp.p.G = d_z_next; bp.p.m = m; bp.p.D = ns::kN; bp.p.J = 1;
+  bp.step_dz = d_z_out; bp.step_da = d_k2_acc;
+  nstc::ns_bwd_tc_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, -1, nullptr);
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
 }
@@ -1470,8 +1478,7 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
       {"tc_fwd_c<half,64,64>", (const void*)tc::tc_fwd_c_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdCSmem<64, 64>::kBytes},
       {"tc_bwd_a<half,64,64>", (const void*)tc::tc_bwd_a_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdASmem<64, 64>::kBytes},
       {"reduce_chunks", (const void*)reduce_chunks_kernel, kThreads, 0},
-      {"ns_bwd_tc", (const void*)nstc::ns_bwd_tc_kernel<1>, nstc::kNsTcThreads, nstc::kBwdSmem},
-      {"ns_bwd_tc_d128", (const void*)nstc::ns_bwd_tc_kernel<2>, nstc::kNsTcThreads, nstc::kBwdSmem},
+      {"ns_bwd_tc", (const void*)nstc::ns_bwd_tc_kernel, nstc::kNsTcThreads, nstc::kBwdSmem},
       {"colpass_operands", (const void*)colpass_operands_kernel, kThreads, (size_t)kColpassOperandSmem},
       {"tc_bwd_b<half,64,64>", (const void*)tc::tc_bwd_b_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdBSmem<64, 64>::kBytes},
       {"tc_rows_inplace<half,64,64>", (const void*)tc::tc_rows_inplace_kernel<H, 64, 64>, tc::kTcThreads, tc::RowsSmem<64, 64>::kBytes},

@@ -1,28 +1,42 @@
-// Newton-Schulz pseudoinverse on the sm_100a tensor cores with FP32-equivalent arithmetic.
+// Newton-Schulz pseudoinverse on the sm_100a tensor cores with FP32-equivalent arithmetic (up to 64 landmarks).
 //
-// Every 64 x 64 FP32 matrix of the iteration is kept in shared memory as three bf16 tiles
-// x = x0 + x1 + x2 (each term the bf16 rounding of what the previous terms left over: 24
-// significant bits together, the FP32 exponent range), stored in the order (x1, x0, x2) so that
-// both (x1, x0) and (x0, x2) are contiguous.  A product needs the partial products x_i * y_j with
-// i + j <= 2 (the others are below 2^-24 relative).  tcgen05.mma takes as long for M = 128 as for
-// M = 64 and only 1.4x as long for N = 128 as for N = 64, so the terms are stacked along both
-// dimensions and a product is two MMAs per 16-wide K step instead of six:
-//     [x1; x0] * [y1 | y0]  -> accumulator columns   0..127   (x1y1, x1y0 | x0y1, x0y0)
-//     [x0; x2] * [y0 | y2]  -> accumulator columns 128..255   (x0y0*, x0y2 | x2y0, x2y2*)
-// (* not used).  Rows 0..63 of the stacked left operand land in TMEM lanes 0..63, rows 64..127 in
-// lanes 64..127, so the epilogue adds the wanted 64-column blocks inside each lane and then the
-// two lane halves through a small shared-memory exchange between partner warps.  The tiles use
-// the 128-byte swizzle ([64 rows x 128 B]); a matrix stored row-major serves as either operand,
-// plain or transposed, by choosing the K-major or the MN-major shared-memory descriptor, so no
-// transposed copies exist.  One CTA per (b,h) slice: 8 compute warps (256 threads) and a ninth
-// warp whose first lane issues the MMAs.  After the exchange every compute thread owns 16
-// consecutive columns of one row, applies the step's affine map and writes the next operand
-// tiles; when its tiles are written it arrives on a "ready" mbarrier the issuing thread waits on.
-// Independent products of a step are issued together with two commits, so the epilogue of the
-// first group overlaps the MMAs of the second.  A wait that gives up (bounded, 1.5 s) marks the
-// call failed in the status word; control flow never depends on it, so no barrier is missed.
-// The set-up and the tail of the algorithm (softmax, ridge, norms, Z0 and its gradient) are the
-// FP32 CUDA-core code of ns_kernels.cuh, run on FP32 staging buffers that alias the tile slots.
+// Arithmetic.  The iteration Z' = Z (13 I - M (15 I - M (7 I - M))) / 4, M = A Z, is run in its residual form: with
+// R = I - M the polynomial is 4 (I + R (I + R / 2)^2), so
+//     R = I - A Z,   Y = Z R,   W = I + R + R^2 / 4,   Z' = Z + Y W.
+// That is four products as before, but three dependent steps in place of four (Y and W go side by side), and
+// nothing cancels near convergence: the error of K2inv against 64 bits is 0.5 to 0.8 of the nested form's.  The
+// backward is that of this form (below); gradients do not depend on which form is differentiated.
+//
+// Products.  Every 64 x 64 FP32 matrix is kept in shared memory as three bf16 tiles x = x0 + x1 + x2 (each term the
+// bf16 rounding of what the previous terms left over: 24 significant bits together, the FP32 exponent range), stored in
+// the order (x1, x0, x2) so that (x1, x0) and (x0, x2) are both contiguous.  A product needs the partial products x_i y_j with
+// i + j <= 2 (the others are below 2^-24 relative).  The terms are stacked along M and N, two MMAs of 128 x 128 per
+// 16-wide K step into the SAME 128 accumulator columns:
+//     [x1; x0] * [y1 | y0], then [x0; x2] * [y0 | y2]
+//     lanes  0..63:  columns 0..63 = x1 y1 + x0 y0,  columns 64..127 = x1 y0 + x0 y2
+//     lanes 64..127: columns 0..63 = x0 y1 + x2 y0,  columns 64..127 = not used (x0 y0 once more)
+// All K steps of the first pair come first, so the leading partial product is added to four times, onto a
+// small value.  An epilogue thread reads 32 (lanes 64..127) or 64 columns, and the two lane halves are added through
+// shared memory between partner warps.  The tiles use the 128-byte swizzle ([64 rows x 128 B]); a matrix stored row-major
+// serves as either operand, plain or transposed, through the K-major or the MN-major descriptor.
+//
+// Roles.  One CTA per (b,h) slice: 8 compute warps and a ninth warp that issues the MMAs (warp-uniform code, one elected lane;
+// with a single lane in the role every descriptor went through vector registers and the kernels were slower than
+// what they replaced).  After the
+// exchange every compute thread owns 16 consecutive columns of one row, applies the step's affine map and writes
+// the next operand tiles, then arrives on a "ready" mbarrier that the issuing thread waits on; groups of MMAs are
+// committed to "done" mbarriers.  A wait that gives up (bounded, 1.5 s) marks the call failed in the status word;
+// control flow never depends on it, so no barrier is missed.
+//
+// With m <= 48 the K steps past m are left out, with m <= 32 also the epilogues of the warps whose 32 x 32 block is empty:
+// what lies there in the tiles is never read.
+//
+// What bounds it: the latency of a step (issue and eight MMAs about 1000 cycles, accumulator out, lane halves added, split and
+// stored about 1000), three of them per iteration in the forward; in the backward, where eight products run beside the
+// chain, shared-memory bandwidth (an MMA reads 8 KB per 65 cycles, an epilogue moves 56 KB).  Instructions come from a cold
+// cache the first time round: 5 us of the forward, 15 of the backward.  Measured (us, nested form with one accumulator per
+// partial product / this, J = 6): 32 slices, m = 64 forward 45 / 43, backward 76 / 66; m = 32 43 / 35 and 66 / 48;
+// 512 slices 162 / 117 and 310 / 283; 64 slices of head_dim 128 with the ridge (then on the CUDA cores) 74 / 52 and 121 / 90.
 #pragma once
 #include "ns_kernels.cuh"
 #include "small_kernels.cuh"
@@ -40,264 +54,49 @@ using ns::Norms;
 constexpr int kTileBytes = kN * 128;        // one bf16 term of a matrix
 constexpr int kSet = 3 * kTileBytes;        // the three terms of a matrix, order (x1, x0, x2)
 constexpr int kTerm0 = kTileBytes, kTerm1 = 0, kTerm2 = 2 * kTileBytes;
-constexpr int kXchBytes = kN * kN * 4;      // FP32 exchange buffer between the lane halves, one per accumulator
-constexpr int kFwdSlots = 7, kBwdSlots = 8;
-constexpr size_t kFwdSmem = (size_t)kFwdSlots * kSet + kXchBytes + 1024;
-constexpr size_t kBwdSmem = (size_t)kBwdSlots * kSet + 2 * kXchBytes + 1024;
-constexpr uint32_t kFwdTmemCols = 256, kBwdTmemCols = 512;
-constexpr uint32_t kAcc0 = 0, kAcc1 = 256;  // TMEM column of the two accumulators
-
-// Optional phase timestamps of CTA 0 (profiling builds only).
-#ifdef FNB_NS_TRACE
-__device__ unsigned long long g_ns_span[2 * 64];   // per-CTA kernel entry / exit times
-__device__ unsigned long long g_ns_trace[160];
-__device__ int g_ns_trace_n;
-#define NS_TRACE()                                                                                  \
-  do {                                                                                              \
-    if (blockIdx.x == 0 && threadIdx.x == 0 && g_ns_trace_n < 160) g_ns_trace[g_ns_trace_n++] = global_ns(); \
-  } while (0)
-#ifdef FNB_NS_TRACE_FINE
-#define NS_TRACE2() NS_TRACE()
-#else
-#define NS_TRACE2() do {} while (0)
-#endif
-#else
-#define NS_TRACE() do {} while (0)
-#define NS_TRACE2() do {} while (0)
-#endif
-
-struct Ctx {
-  uint8_t* base;        // 1024-byte aligned start of the tile slots
-  float4* xch;          // exchange buffers: [accumulator][4][256 threads]
-  uint64_t* bar;        // two completion barriers (MMA groups -> compute warps)
-  uint64_t* ready;      // operand tiles written (one arrival per compute warp -> issuing thread)
-  uint32_t phase[2];    // parity the next wait on each completion barrier uses
-  uint32_t rphase;      // parity the next wait on `ready` uses
-  bool failed;          // a wait of this thread gave up
-  uint32_t tmem;        // base address of the allocated tensor memory
-  Abort ab;
-  // epilogue role of this thread: TMEM lane 32*quarter + lane holds row `row` of the lane half
-  // `part`; after the exchange the thread owns columns col0 .. col0+15 of that row
-  int row, part, c32, col0, pair_bar;
-  uint32_t lane_off;
-  __device__ __forceinline__ uint8_t* slot(int i) const { return base + (size_t)i * kSet; }
-  __device__ __forceinline__ uint32_t slot_addr(int i) const { return smem_u32(base) + (uint32_t)i * kSet; }
-};
-
-// ---- FP32 -> three bf16 terms ---------------------------------------------------------------
-// 8 consecutive values of row r, columns 8*chunk .. 8*chunk+7 -> one 16-byte chunk per term
-__device__ __forceinline__ void split_store8(uint8_t* set, int r, int chunk, const float* v) {
-  uint32_t w0[4], w1[4], w2[4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    float a = v[2 * p], b = v[2 * p + 1];
-    w0[p] = pack2<__nv_bfloat16>(a, b);            // low half = a, high half = b
-    a -= __uint_as_float(w0[p] << 16);
-    b -= __uint_as_float(w0[p] & 0xffff0000u);
-    w1[p] = pack2<__nv_bfloat16>(a, b);
-    a -= __uint_as_float(w1[p] << 16);
-    b -= __uint_as_float(w1[p] & 0xffff0000u);
-    w2[p] = pack2<__nv_bfloat16>(a, b);
-  }
-  const uint32_t off = sw128_offset(r, chunk);
-  *reinterpret_cast<uint4*>(set + kTerm0 + off) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-  *reinterpret_cast<uint4*>(set + kTerm1 + off) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-  *reinterpret_cast<uint4*>(set + kTerm2 + off) = make_uint4(w2[0], w2[1], w2[2], w2[3]);
-}
-// 16 values: columns col0 .. col0+15 of row r
-__device__ __forceinline__ void split_store16(uint8_t* set, int r, int col0, const float* v) {
-  split_store8(set, r, (col0 >> 3), v);
-  split_store8(set, r, (col0 >> 3) + 1, v + 8);
-}
-
-// whole-matrix conversions: thread t handles row t >> 2, columns 16*(t & 3) .. +15
-// dense global [rows x cols] matrix with row stride ld -> registers, zero beyond rows / cols
-__device__ __forceinline__ void load_global16(const float* g, int rows, int cols, int ld, float* v) {
-  const int r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
-  if (((ld | cols) & 3) == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int cc = c0 + 4 * q;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < rows && cc < cols) x = *reinterpret_cast<const float4*>(g + (size_t)r * ld + cc);
-      v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = (r < rows && c0 + i < cols) ? g[(size_t)r * ld + c0 + i] : 0.f;
-  }
-}
-__device__ __forceinline__ void store_set16(uint8_t* set, const float* v) {
-  split_store16(set, threadIdx.x >> 2, (threadIdx.x & 3) * 16, v);
-}
-__device__ __forceinline__ void store_buf16(float* X, const float* v) {
-  float* dst = X + (threadIdx.x >> 2) * kLd + (threadIdx.x & 3) * 16;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-    *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-}
-// padded FP32 shared buffer (row stride kLd) -> tile set
-__device__ __forceinline__ void convert_buf(uint8_t* set, const float* X) {
-  const int r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
-  float v[16];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float4 x = *reinterpret_cast<const float4*>(X + r * kLd + c0 + 4 * q);
-    v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
-  }
-  split_store16(set, r, c0, v);
-}
-
-// ---- products -------------------------------------------------------------------------------
-// An operand is a tile set plus how the product reads it:
-//   left operand  X (M x K):  plain = K-major,  transposed (X^T as left operand) = MN-major
-//   right operand Y (K x N):  plain = MN-major, transposed (Y^T as right operand) = K-major
-struct Operand { uint32_t addr; bool mn; };
-__device__ __forceinline__ Operand left(uint32_t set) { return {set, false}; }
-__device__ __forceinline__ Operand left_t(uint32_t set) { return {set, true}; }
-__device__ __forceinline__ Operand right(uint32_t set) { return {set, true}; }
-__device__ __forceinline__ Operand right_t(uint32_t set) { return {set, false}; }
-
-// descriptor of two stacked term tiles starting `first` bytes into the set, K step k
-__device__ __forceinline__ uint64_t pair_desc(const Operand& o, int first, int k) {
-  const uint32_t tile = o.addr + (uint32_t)first;
-  return o.mn ? smem_desc_sw128(tile + k * 2048, kTileBytes, 1024)   // 16 rows of K per step; the second
-                                                                     // 64-wide block is the next tile
-              : smem_desc_sw128(tile + k * 32, 16, 1024);            // 32 bytes of K per step; rows 64..127
-                                                                     // continue into the next tile
-}
-// accumulator at TMEM address d (256 columns) (+)= a * b
-__device__ __forceinline__ void issue_product(uint32_t d, Operand a, Operand b, bool accumulate) {
-  const uint32_t idesc = make_idesc<__nv_bfloat16>(128, 128, a.mn, b.mn);
-  uint32_t acc = accumulate ? 1u : 0u;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    umma(d, pair_desc(a, 0, k), pair_desc(b, 0, k), idesc, acc);                          // [x1;x0] [y1|y0]
-    umma(d + 128, pair_desc(a, kTileBytes, k), pair_desc(b, kTileBytes, k), idesc, acc);  // [x0;x2] [y0|y2]
-    acc = 1u;
-  }
-}
+constexpr int kFwdSlots = 4, kBwdSlots = 9;
+constexpr size_t kFwdSmem = (size_t)kFwdSlots * kSet + 1024;   // 97 KB: two slices per SM
+constexpr size_t kBwdSmem = (size_t)kBwdSlots * kSet + 1024;
+static_assert(kBuf * (int)sizeof(float) <= kSet, "an FP32 staging buffer has to fit a slot");
+constexpr uint32_t kAccCols = 128;
+constexpr uint32_t kFwdTmemCols = 2 * kAccCols, kBwdTmemCols = 4 * kAccCols;
+constexpr int kMaxBars = 8;
 
 constexpr int kComputeThreads = 256;
 constexpr int kNsTcThreads = kComputeThreads + 32;
 __device__ __forceinline__ bool is_compute() { return threadIdx.x < kComputeThreads; }
-__device__ __forceinline__ bool is_issuer() { return threadIdx.x == kComputeThreads; }
 
-// compute side: my operand tiles (and my reads of the accumulators) are done
-__device__ __forceinline__ void tiles_ready(Ctx& c) {
-  fence_proxy_async();
-  tc_fence_before();
-  mbar_arrive_warp(c.ready);
-}
-// compute side: wait for MMA group g (0 or 1) of the current batch
-__device__ __forceinline__ void wait_group(Ctx& c, int g, int where) {
-  NS_TRACE2();
-  if (!mbar_wait(c.bar + g, c.phase[g], c.ab, where)) c.failed = true;
-  c.phase[g] ^= 1u;
-  tc_fence_after();
-  NS_TRACE2();
-}
-// issuing thread: wait for the operands, issue two groups of products, one commit each
-template <class IssueA, class IssueB>
-__device__ __forceinline__ void mma_batch(Ctx& c, int where, IssueA issue_a, IssueB issue_b) {
-  if (!c.failed && !mbar_wait(c.ready, c.rphase, c.ab, where)) c.failed = true;
-  c.rphase ^= 1u;
-  if (c.failed) return;
-  tc_fence_after();
-  issue_a();
-  umma_commit(c.bar);
-  issue_b();
-  umma_commit(c.bar + 1);
-}
-template <class Issue>
-__device__ __forceinline__ void mma_single(Ctx& c, int where, Issue issue) {
-  if (!c.failed && !mbar_wait(c.ready, c.rphase, c.ab, where)) c.failed = true;
-  c.rphase ^= 1u;
-  if (c.failed) return;
-  tc_fence_after();
-  issue();
-  umma_commit(c.bar);
-}
-
-// Result of the accumulator at TMEM column `col`: after the call v[0..15] holds columns
-// c.col0 .. c.col0+15 of row c.row.  Every thread must call (warp-wide TMEM loads, pair barriers).
-__device__ __forceinline__ void acc_result(const Ctx& c, uint32_t col, float* v) {
-  float s[32], t[32], u[32];
-  const uint32_t a = c.tmem + col + c.lane_off;
-  tmem_ld32(a, s);                                // lanes 0..63: x1y1 ; lanes 64..127: x0y1
-  tmem_ld32(a + 64, t);                           //              x1y0 ;                x0y0
-  tmem_ld32(a + (c.part ? 128 : 192), u);         //              x0y2 ;                x2y0
-  tmem_ld_wait();
-#pragma unroll
-  for (int i = 0; i < 32; ++i) s[i] = (s[i] + t[i]) + u[i];
-  NS_TRACE2();
-  // Hand the 16 columns the partner finalises over, take the partner's share of mine (part is
-  // warp-uniform; the two branches keep every register index a constant).  A buffer is written again only
-  // after another batch of products has completed, which every warp's arrival precedes: one barrier is enough.
-  float4* x = c.xch + (col == kAcc0 ? 0 : kXchBytes / 16) + threadIdx.x;
-  const float4* y = c.xch + (col == kAcc0 ? 0 : kXchBytes / 16) + (threadIdx.x ^ 64);
-  if (c.part == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) x[q * 256] = make_float4(s[16 + 4 * q], s[17 + 4 * q], s[18 + 4 * q], s[19 + 4 * q]);
-    named_barrier(c.pair_bar, 64);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 w = y[q * 256];
-      v[4 * q] = s[4 * q] + w.x; v[4 * q + 1] = s[4 * q + 1] + w.y;
-      v[4 * q + 2] = s[4 * q + 2] + w.z; v[4 * q + 3] = s[4 * q + 3] + w.w;
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) x[q * 256] = make_float4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
-    named_barrier(c.pair_bar, 64);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 w = y[q * 256];
-      v[4 * q] = s[16 + 4 * q] + w.x; v[4 * q + 1] = s[17 + 4 * q] + w.y;
-      v[4 * q + 2] = s[18 + 4 * q] + w.z; v[4 * q + 3] = s[19 + 4 * q] + w.w;
-    }
-  }
-  NS_TRACE2();
-}
-
-// v[i] = s * v[i] + (diagonal ? d : 0), diagonal restricted to the leading m x m block
-__device__ __forceinline__ void affine(const Ctx& c, float* v, float s, float d, int m) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = s * v[i] + ((c.col0 + i == c.row && c.row < m) ? d : 0.f);
-}
-// this thread's row segment, restricted to the leading rows x cols block -> dense global matrix
-__device__ __forceinline__ void store_global16(const Ctx& c, float* g, const float* v, int rows, int cols, int ld) {
-  if (c.row >= rows) return;
-  if (((ld | cols) & 3) == 0) {
-#pragma unroll
-    for (int i = 0; i < 16; i += 4)
-      if (c.col0 + i < cols)
-        *reinterpret_cast<float4*>(g + (size_t)c.row * ld + c.col0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (c.col0 + i < cols) g[(size_t)c.row * ld + c.col0 + i] = v[i];
-  }
-}
-__device__ __forceinline__ void store_row16(const Ctx& c, float* X, const float* v) {
-#pragma unroll
-  for (int i = 0; i < 16; i += 4)
-    *reinterpret_cast<float4*>(X + c.row * kLd + c.col0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-}
-
-// common set-up / teardown of the kernels below (called by all 288 threads)
 struct Shared {
-  uint64_t bar[2];
-  uint64_t ready;
+  uint64_t done[kMaxBars];    // MMA groups complete (issuing warp -> compute warps)
+  uint64_t ready[kMaxBars];   // operand tiles written, accumulators read (one arrival per compute warp -> issuing warp)
   uint32_t tmem_slot;
   int abort_word;
 };
-__device__ __forceinline__ void ctx_open(Ctx& c, Shared& sh, uint8_t* dyn, int slots, int* status, uint32_t cols) {
+
+struct Ctx {
+  uint8_t* base;        // 1024-byte aligned start of the tile slots
+  uint32_t smem;        // the same as a shared-memory address
+  Shared* sh;
+  uint32_t parity;      // bit b: parity of the next wait on done[b] (compute) or ready[b] (issuer)
+  bool failed;          // a wait of this thread gave up
+  uint32_t tmem;        // base address of the allocated tensor memory
+  Abort ab;
+  // epilogue role of this thread: TMEM lane 32 * quarter + lane holds row `row` of the lane half `part`; after
+  // the exchange the thread owns columns col0 .. col0 + 15 of that row
+  int row, part, col0, c32, pair_bar;
+  uint32_t lane_addr;   // TMEM offset of the thread's 32 columns
+  float trunc;          // see fetch()
+  bool act;             // this warp's 32 x 32 block of an m x m matrix has something in it (it is never read otherwise)
+  __device__ __forceinline__ uint32_t slot(int i) const { return smem + i * kSet; }
+  __device__ __forceinline__ float* stage(int i) const { return reinterpret_cast<float*>(base + i * kSet); }
+};
+
+// common set-up / teardown of the kernels below (called by all 288 threads)
+__device__ __forceinline__ void ctx_open(Ctx& c, Shared& sh, uint8_t* dyn, int* status, uint32_t cols, int m) {
   c.base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
-  c.xch = reinterpret_cast<float4*>(c.base + (size_t)slots * kSet);
-  c.bar = sh.bar;
-  c.ready = &sh.ready;
-  c.phase[0] = c.phase[1] = c.rphase = 0;
+  c.smem = smem_u32(c.base);
+  c.sh = &sh;
+  c.parity = 0;
   c.failed = false;
   c.ab.flag = &sh.abort_word;
   c.ab.status = status;
@@ -307,12 +106,15 @@ __device__ __forceinline__ void ctx_open(Ctx& c, Shared& sh, uint8_t* dyn, int s
   c.c32 = half * 32;
   c.col0 = c.c32 + 16 * c.part;
   c.pair_bar = 1 + (quarter & 1) + 2 * half;      // warps w and w ^ 2 share a barrier
-  c.lane_off = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c.c32;
+  c.lane_addr = ((uint32_t)(quarter * 32) << 16) + (uint32_t)c.c32;
+  c.act = (quarter & 1) * 32 < m && c.c32 < m;
+  c.trunc = (float)((m + 15) / 16) * 0x1p-26f;
   if (threadIdx.x == 0) {
     sh.abort_word = 0;
-    mbar_init(&sh.bar[0], 1);
-    mbar_init(&sh.bar[1], 1);
-    mbar_init(&sh.ready, kComputeThreads / 32);
+    for (int i = 0; i < kMaxBars; ++i) {
+      mbar_init(&sh.done[i], 1);
+      mbar_init(&sh.ready[i], kComputeThreads / 32);
+    }
     fence_mbar_init();
   }
   if (threadIdx.x < 32) {
@@ -330,86 +132,297 @@ __device__ __forceinline__ void ctx_close(Ctx& c, uint32_t cols) {
   if (threadIdx.x < 32) tmem_dealloc(c.tmem, cols);
 }
 
-// ---------------------------------------------------------------------------------------------
-// Forward.  Slots: 0 A, 1 Z, 2 M, 3 nU = M - 7I, 4 V, 5 qT = T / 4, 6 K2 (ridge only).
-// FP32 staging (K2, A) aliases slots 2..4; in: K2 (softmaxed, padded) in staging buffer 0.
-__device__ __forceinline__ float* fwd_staging(const Ctx& c) { return reinterpret_cast<float*>(c.slot(2)); }
-
-// issuing thread: the products of the forward in the order the compute warps consume them
-__device__ inline void pinv_forward_issue(Ctx& c, int J, float kappa, bool scores) {
-  const uint32_t sA = c.slot_addr(0), sZ = c.slot_addr(1), sM = c.slot_addr(2), sU = c.slot_addr(3),
-                 sV = c.slot_addr(4), sT = c.slot_addr(5), sK2 = c.slot_addr(6);
-  const uint32_t acc0 = c.tmem + kAcc0;
-  if (scores) mma_single(c, 0x20ff, [&] { issue_product(acc0, left(sA), right_t(sZ), false); });   // Qt Kt^T
-  for (int j = 0; j < J; ++j) {
-    mma_single(c, 0x2100, [&] { issue_product(acc0, left(sA), right(sZ), false); });
-    mma_single(c, 0x2101, [&] { issue_product(acc0, left(sM), right(sU), false); });
-    mma_single(c, 0x2102, [&] { issue_product(acc0, left(sM), right(sV), false); });
-    mma_single(c, 0x2103, [&] { issue_product(acc0, left(sZ), right(sT), false); });
+// ---- FP32 <-> three bf16 terms ---------------------------------------------------------------
+// (Shared memory is accessed by 32-bit addresses: the slots are picked at run time, and generic accesses cost more.)
+__device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+// 8 consecutive values of row r, columns 8*chunk .. 8*chunk+7 -> one 16-byte chunk per term
+__device__ __forceinline__ void split_store8(uint32_t set, int r, int chunk, const float* v) {
+  uint32_t w0[4], w1[4], w2[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float a = v[2 * p], b = v[2 * p + 1];
+    w0[p] = pack2<__nv_bfloat16>(a, b);            // low half = a, high half = b
+    a -= __uint_as_float(w0[p] << 16);
+    b -= __uint_as_float(w0[p] & 0xffff0000u);
+    w1[p] = pack2<__nv_bfloat16>(a, b);
+    a -= __uint_as_float(w1[p] << 16);
+    b -= __uint_as_float(w1[p] & 0xffff0000u);
+    w2[p] = pack2<__nv_bfloat16>(a, b);
   }
-  if (kappa > 0.f) mma_single(c, 0x2104, [&] { issue_product(acc0, left(sZ), right_t(sK2), false); });
+  const uint32_t at = set + sw128_offset(r, chunk);
+  sts128(at + kTerm0, w0[0], w0[1], w0[2], w0[3]);
+  sts128(at + kTerm1, w1[0], w1[1], w1[2], w1[3]);
+  sts128(at + kTerm2, w2[0], w2[1], w2[2], w2[3]);
+}
+// this thread's 16 columns of its row
+__device__ __forceinline__ void put_row16(const Ctx& c, uint32_t set, const float* v) {
+  split_store8(set, c.row, c.col0 >> 3, v);
+  split_store8(set, c.row, (c.col0 >> 3) + 1, v + 8);
+}
+// the sum of the three terms, smallest first (the FP32 value the tile was made from)
+__device__ __forceinline__ void get_row16(const Ctx& c, uint32_t set, float* v) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t off = sw128_offset(c.row, (c.col0 >> 3) + h);
+    uint32_t w0[4], w1[4], w2[4];
+    *reinterpret_cast<uint4*>(w0) = lds128(set + kTerm0 + off);
+    *reinterpret_cast<uint4*>(w1) = lds128(set + kTerm1 + off);
+    *reinterpret_cast<uint4*>(w2) = lds128(set + kTerm2 + off);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      v[8 * h + 2 * p] = __uint_as_float(w0[p] << 16) + (__uint_as_float(w1[p] << 16) + __uint_as_float(w2[p] << 16));
+      v[8 * h + 2 * p + 1] = __uint_as_float(w0[p] & 0xffff0000u) +
+                             (__uint_as_float(w1[p] & 0xffff0000u) + __uint_as_float(w2[p] & 0xffff0000u));
+    }
+  }
 }
 
-// compute warps
-__device__ inline void pinv_forward_tc(Ctx& c, float* red, float* iterates, float* k2inv, int m, int J,
-                                       float kappa) {
-  float* bK2 = fwd_staging(c);
-  float* bA = bK2 + kBuf;
-  const int mm_ = m * m;
-  const float* A = bK2;
-  if (kappa > 0.f) {
-    Norms nk = ns::norms(bK2, m, red);
-    const float lam = nk.n1 * nk.ninf / kappa;
-    ns::mm<ns::TN>(bK2, bK2, [&](int r, int cc, float acc) { bA[r * kLd + cc] = acc + ((r == cc && r < m) ? lam : 0.f); });
-    A = bA;
-    convert_buf(c.slot(6), bK2);
-  }
-  Norms na = ns::norms(A, m, red);
-  const float cden = fmaxf(na.n1 * na.ninf, 1e-12f);
-  // v: the iterate of the last step, in the layout of the epilogue.  It goes to global memory while the next
-  // product runs (in front of that product the store took 1300 of the 9300 cycles of an iteration).
-  float v[16];
-  // Z0 = A^T / cden
+// ---- global / staging accesses ---------------------------------------------------------------
+// Whole-matrix tile loads: thread t handles row t >> 2 and the 8-column chunks (t & 3) and (t & 3) + 4, so that four
+// adjacent lanes cover 128 consecutive bytes.
+__device__ __forceinline__ void load_chunk8(const float* g, int r, int chunk, int rows, int cols, int ld, float* v) {
+  const int c0 = 8 * chunk;
+  if (((ld | cols) & 3) == 0) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = A[(c.col0 + i) * kLd + c.row] / cden;
-  split_store16(c.slot(1), c.row, c.col0, v);
-  convert_buf(c.slot(0), A);
-  NS_TRACE();
-  for (int j = 0; j < J; ++j) {
-    NS_TRACE();
-    tiles_ready(c);
-    if (!c.failed) store_global16(c, iterates + (size_t)j * mm_, v, m, m, m);
-    wait_group(c, 0, 0x2110);
-    acc_result(c, kAcc0, v);
-    split_store16(c.slot(2), c.row, c.col0, v);
-    affine(c, v, 1.f, -7.f, m);
-    split_store16(c.slot(3), c.row, c.col0, v);
-    tiles_ready(c);
-    wait_group(c, 0, 0x2111);
-    acc_result(c, kAcc0, v);
-    affine(c, v, 1.f, 15.f, m);
-    split_store16(c.slot(4), c.row, c.col0, v);
-    tiles_ready(c);
-    wait_group(c, 0, 0x2112);
-    acc_result(c, kAcc0, v);
-    affine(c, v, -0.25f, 3.25f, m);
-    split_store16(c.slot(5), c.row, c.col0, v);
-    tiles_ready(c);
-    wait_group(c, 0, 0x2113);
-    acc_result(c, kAcc0, v);
-    split_store16(c.slot(1), c.row, c.col0, v);
+    for (int q = 0; q < 2; ++q) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < rows && c0 + 4 * q < cols) x = *reinterpret_cast<const float4*>(g + (size_t)r * ld + c0 + 4 * q);
+      v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (r < rows && c0 + i < cols) ? g[(size_t)r * ld + c0 + i] : 0.f;
   }
-  NS_TRACE();
-  if (kappa > 0.f) tiles_ready(c);
-  if (!c.failed) {
-    store_global16(c, iterates + (size_t)J * mm_, v, m, m, m);
-    if (!(kappa > 0.f)) store_global16(c, k2inv, v, m, m, m);
+}
+// dense global [rows x cols] matrix with row stride ld -> registers, zero beyond rows / cols
+__device__ __forceinline__ void load_tile16(const float* g, int rows, int cols, int ld, float* v) {
+  load_chunk8(g, threadIdx.x >> 2, threadIdx.x & 3, rows, cols, ld, v);
+  load_chunk8(g, threadIdx.x >> 2, (threadIdx.x & 3) + 4, rows, cols, ld, v + 8);
+}
+__device__ __forceinline__ void put_tile16(uint32_t set, const float* v) {
+  split_store8(set, threadIdx.x >> 2, threadIdx.x & 3, v);
+  split_store8(set, threadIdx.x >> 2, (threadIdx.x & 3) + 4, v + 8);
+}
+// the same elements -> / <- a padded FP32 staging buffer (row stride kLd)
+__device__ __forceinline__ void stage_tile16(float* X, const float* v) {
+  float* d = X + (threadIdx.x >> 2) * kLd + (threadIdx.x & 3) * 8;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<float4*>(d + (q & 1) * 4 + (q >> 1) * 32) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+// this thread's 16 columns of its row: global, staging
+__device__ __forceinline__ void load_row16(const Ctx& c, const float* g, int rows, int cols, int ld, float* v) {
+  load_chunk8(g, c.row, c.col0 >> 3, rows, cols, ld, v);
+  load_chunk8(g, c.row, (c.col0 >> 3) + 1, rows, cols, ld, v + 8);
+}
+__device__ __forceinline__ void store_row16(const Ctx& c, float* g, const float* v, int rows, int cols, int ld) {
+  if (c.row >= rows) return;
+  if (((ld | cols) & 3) == 0) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 4)
+      if (c.col0 + i < cols)
+        *reinterpret_cast<float4*>(g + (size_t)c.row * ld + c.col0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (c.col0 + i < cols) g[(size_t)c.row * ld + c.col0 + i] = v[i];
   }
-  if (kappa > 0.f) {
-    // k2inv = Z_J K2^T
-    wait_group(c, 0, 0x2114);
-    acc_result(c, kAcc0, v);
-    if (!c.failed) store_global16(c, k2inv, v, m, m, m);
+}
+__device__ __forceinline__ void stage_row16(const Ctx& c, float* X, const float* v) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4)
+    *reinterpret_cast<float4*>(X + c.row * kLd + c.col0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+}
+__device__ __forceinline__ void unstage_row16(const Ctx& c, const float* X, float* v) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(X + c.row * kLd + c.col0 + i);
+    v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+  }
+}
+// the same for the transposed matrix
+__device__ __forceinline__ void unstage_col16(const Ctx& c, const float* X, float* v) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = X[(c.col0 + i) * kLd + c.row];
+}
+// d on the diagonal of the leading m x m block
+__device__ __forceinline__ void add_diag(const Ctx& c, float* v, float d, int m) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] += (c.col0 + i == c.row && c.row < m) ? d : 0.f;
+}
+
+// ---- products -------------------------------------------------------------------------------
+// accumulator at TMEM address d (128 columns) (+)= a * b over nk K steps of 16.  Operands are tile sets:
+//   left operand  X (M x K):  plain = K-major,  transposed (X^T as left operand) = MN-major
+//   right operand Y (K x N):  plain = MN-major, transposed (Y^T as right operand) = K-major
+// Warp-uniform code, one elected lane issues: the eight MMAs are one block of assembly, so that the election happens once
+// and the descriptors stay in uniform registers (750 cycles per product when each MMA elected and its strides were run-time
+// values).
+template <bool AT, bool BT>
+__device__ __forceinline__ void issue_product(uint32_t d, uint32_t a, uint32_t b, bool accumulate, uint32_t nk) {
+  // K-major: rows 64..127 continue into the next tile, 16 of K are 32 bytes; MN-major: the second 64-wide block is
+  // the next tile, 16 of K are 16 rows
+  const uint64_t da = smem_desc_sw128(a, AT ? kTileBytes : 16, 1024), db = smem_desc_sw128(b, BT ? 16 : kTileBytes, 1024);
+  constexpr uint32_t idesc = make_idesc<__nv_bfloat16>(128, 128, AT, !BT);
+  constexpr int sa = AT ? 2048 / 16 : 2, sb = BT ? 2 : 2048 / 16, t = kTileBytes / 16;
+  // first the (x1, x0) (y1, y0) tiles over all of K, then (x0, x2) (y0, y2)
+  asm volatile(
+      "{\n\t.reg .pred e, e1, e2, e3, p, q;\n\t.reg .b64 x, y;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "setp.gt.and.u32 e1, %5, 1, e;\n\tsetp.gt.and.u32 e2, %5, 2, e;\n\tsetp.gt.and.u32 e3, %5, 3, e;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "add.s64 x, %1, %6;\n\tadd.s64 y, %2, %7;\n\t"
+      "@e1 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, x, %6;\n\tadd.s64 y, y, %7;\n\t"
+      "@e2 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, x, %6;\n\tadd.s64 y, y, %7;\n\t"
+      "@e3 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, %1, %8;\n\tadd.s64 y, %2, %8;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, x, %6;\n\tadd.s64 y, y, %7;\n\t"
+      "@e1 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, x, %6;\n\tadd.s64 y, y, %7;\n\t"
+      "@e2 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t"
+      "add.s64 x, x, %6;\n\tadd.s64 y, y, %7;\n\t"
+      "@e3 tcgen05.mma.cta_group::1.kind::f16 [%0], x, y, %3, q;\n\t}"
+      ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(nk), "n"(sa), "n"(sb), "n"(t)
+      : "memory");
+}
+
+// compute side: my operand tiles (and my reads of the accumulators) are done
+__device__ __forceinline__ void arrive_ready(Ctx& c, int b) {
+  fence_proxy_async();
+  tc_fence_before();
+  mbar_arrive_warp(c.sh->ready + b);
+}
+// issuing warp (all lanes, so that its control flow and operands stay warp-uniform)
+__device__ __forceinline__ void wait_ready(Ctx& c, int b, int where) {
+  const bool ok = c.failed || mbar_wait(c.sh->ready + b, (c.parity >> b) & 1u, c.ab, where);
+  if (!__all_sync(0xffffffffu, ok)) c.failed = true;
+  c.parity ^= 1u << b;
+  tc_fence_after();
+}
+__device__ __forceinline__ void wait_done(Ctx& c, int b, int where) {
+  if (!mbar_wait(c.sh->done + b, (c.parity >> b) & 1u, c.ab, where)) c.failed = true;
+  c.parity ^= 1u << b;
+  tc_fence_after();
+}
+
+// The tensor core truncates when it adds to an accumulator; the leading partial product is added to once per K step and
+// loses about an eighth of an ulp each time on the average, which `trunc` (a share of the value) gives back on its way to the
+// small ones.  Without it K2inv and dQ of fp32 calls were up to 1.28 and 1.24 times as far from the oracle as with one add fewer
+// per product, with it 0.83 to 0.98 and 0.90 to 0.99 times.
+constexpr float kTruncScores = 0x1p-25f;    // below half an ulp of any value: exact sums stay exact
+// This thread's share of the accumulator at TMEM column `col`, before the two lane halves are added: 16 columns that it
+// keeps and 16 that its partner finalises.  Every thread of a warp must call.
+__device__ __forceinline__ void fetch(const Ctx& c, uint32_t col, float trunc, float* keep, float* send) {
+  const uint32_t a = c.tmem + col + c.lane_addr, ak = a + 16 * c.part, as = a + 16 - 16 * c.part;
+  tmem_ld16(ak, keep);
+  tmem_ld16(as, send);
+  if (c.part == 0) {
+    float x[16], y[16];
+    tmem_ld16(ak + kN, x);
+    tmem_ld16(as + kN, y);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      keep[i] += fmaf(trunc, keep[i], x[i]);
+      send[i] += fmaf(trunc, send[i], y[i]);
+    }
+  } else {
+    tmem_ld_wait();
+  }
+}
+// Adds the two lane halves.  `set`: a slot that no product reads and no thread but this pair's touches in the rows and
+// columns of the pair (the slot the result goes to, usually): each half hands over through a term of its own.
+__device__ __forceinline__ void exchange(const Ctx& c, uint32_t set, const float* keep, const float* send, float* v) {
+  const uint32_t x = set + c.part * kTileBytes, y = set + (1 - c.part) * kTileBytes;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    sts128(x + sw128_offset(c.row, (c.c32 >> 3) + q), __float_as_uint(send[4 * q]), __float_as_uint(send[4 * q + 1]),
+           __float_as_uint(send[4 * q + 2]), __float_as_uint(send[4 * q + 3]));
+  named_barrier(c.pair_bar, 64);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 w = lds128(y + sw128_offset(c.row, (c.c32 >> 3) + q));
+    v[4 * q] = keep[4 * q] + __uint_as_float(w.x); v[4 * q + 1] = keep[4 * q + 1] + __uint_as_float(w.y);
+    v[4 * q + 2] = keep[4 * q + 2] + __uint_as_float(w.z); v[4 * q + 3] = keep[4 * q + 3] + __uint_as_float(w.w);
+  }
+  named_barrier(c.pair_bar, 64);
+}
+
+// the two together: the accumulator at `col` once done[b] has completed; nothing where `act` is false
+__device__ __forceinline__ void take(Ctx& c, int b, uint32_t col, uint32_t set, bool act, float* v, float trunc) {
+  wait_done(c, b, 0x2100 + b);
+  if (act) {
+    float keep[16], send[16];
+    fetch(c, col, trunc, keep, send);
+    exchange(c, set, keep, send, v);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Forward.  Products in order (s):
+//   -2        scores Qt Kt^T (head_dim 128: two products, 64 columns each)    slots 0, 1 (2, 3)
+//   -1        K2^T K2 (ridge only)                                            slot 2
+//   4j, ...   R = I - A Z | Y = Z R | W = I + R + R R / 4 | Z' = Z + Y W      A 0, Z 1, R and W 2, Y 3
+//   4J        k2inv = Z K2^T (ridge only)                                     K2 in slot 0
+// Even s: accumulator 0, odd s: accumulator 1.  Y is formed before W: Z is in registers too, so its slot
+// stays free, and W goes over R.  FP32 staging of K2, then A: slot 3.
+// Two slices per SM (97 KB, 256 TMEM columns, 112 registers): the epilogues of one run beside the products of the other.
+constexpr int kFwdStage = 3;
+struct FwdParams {
+  ns::NsFwdParams p;
+  bool k2_given;        // p.k2 holds the softmaxed matrix: no scores, no softmax
+};
+
+__device__ inline void fwd_issue(Ctx& c, const FwdParams& f) {
+  const bool ridge = f.p.kappa > 0.f;
+  const uint32_t nk = (f.p.m + 15) / 16, acc0 = c.tmem, acc1 = c.tmem + kAccCols;
+  if (!f.k2_given) {
+    wait_ready(c, 0, 0x2100);
+    if (c.failed) return;
+    issue_product<false, true>(acc0, c.slot(0), c.slot(1), false, 4);
+    if (f.p.D > kN) issue_product<false, true>(acc0, c.slot(2), c.slot(3), true, 4);
+    umma_commit_elect(c.sh->done);
+  }
+  if (ridge) {
+    wait_ready(c, 0, 0x2101);
+    if (c.failed) return;
+    issue_product<true, false>(acc1, c.slot(2), c.slot(2), false, nk);
+    umma_commit_elect(c.sh->done + 1);
+  }
+#pragma unroll 1
+  for (int j = 0; j < f.p.J; ++j) {
+    wait_ready(c, 0, 0x2102);
+    if (c.failed) return;
+    issue_product<false, false>(acc0, c.slot(0), c.slot(1), false, nk);    // A Z
+    umma_commit_elect(c.sh->done);
+    wait_ready(c, 0, 0x2103);
+    if (c.failed) return;
+    issue_product<false, false>(acc1, c.slot(1), c.slot(2), false, nk);    // Z R
+    umma_commit_elect(c.sh->done + 1);
+    issue_product<false, false>(acc0, c.slot(2), c.slot(2), false, nk);    // R R
+    umma_commit_elect(c.sh->done);
+    wait_ready(c, 0, 0x2104);
+    if (c.failed) return;
+    issue_product<false, false>(acc1, c.slot(3), c.slot(2), false, nk);    // Y W
+    umma_commit_elect(c.sh->done + 1);
+  }
+  if (ridge) {
+    wait_ready(c, 0, 0x2105);
+    if (c.failed) return;
+    issue_product<false, true>(acc0, c.slot(1), c.slot(0), false, nk);     // Z K2^T
+    umma_commit_elect(c.sh->done);
   }
 }
 
@@ -460,348 +473,176 @@ __device__ inline void softmax16(float* X, const ns::NsFwdParams& p, int64_t bh)
   ns::ns_sync();
 }
 
-// Scores S2 = Qt Kt^T for head_dim 64 as one split product (Qt in slot 0, Kt in slot 1, both
-// overwritten afterwards), then the FP32 row softmax.
-__device__ inline void s2_softmax_tc(Ctx& c, const ns::NsFwdParams& p, int64_t bh) {
-  const int m = p.m, D = p.D;
-  float q[16], k[16], v[16];
+// The landmarks as tiles: Qt in slots 0 (and 2 for head_dim 128), Kt in slots 1 (and 3).
+__device__ __forceinline__ void fwd_landmarks(Ctx& c, const ns::NsFwdParams& p, int64_t bh) {
+  const int m = p.m, D = p.D, r = threadIdx.x >> 2;
+  float q[16], k[16];
   if (p.land) {
-    pooled_row16(p.land, 0, p.BH, bh, m, p.C, p.seg_N, p.scale, q);
-    pooled_row16(p.land, 1, p.BH, bh, m, p.C, p.seg_N, p.scale, k);
-    const int r = threadIdx.x >> 2, c0 = (threadIdx.x & 3) * 16;
-    if (r < m) {
-      float4* dq = reinterpret_cast<float4*>(p.qt_out + (bh * m + r) * D + c0);
-      float4* dk = reinterpret_cast<float4*>(p.kt_out + (bh * m + r) * D + c0);
+    // raw segment sums of the pooling pass, [2][BH][m][C][64]: scale * sum / length, and FP32 copies to global memory
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        dq[i] = make_float4(q[4 * i], q[4 * i + 1], q[4 * i + 2], q[4 * i + 3]);
-        dk[i] = make_float4(k[4 * i], k[4 * i + 1], k[4 * i + 2], k[4 * i + 3]);
+    for (int i = 0; i < 16; ++i) { q[i] = 0.f; k[i] = 0.f; }
+    if (r < m) {
+      const size_t off = ((size_t)bh * m + r) * p.C * kN, which = (size_t)p.BH * m * p.C * kN;
+      const int c0 = (threadIdx.x & 3) * 8;
+      for (int ch = 0; ch < p.C; ++ch) {
+        const float* src = p.land + off + (size_t)ch * kN + c0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int o = (j & 1) * 4 + (j >> 1) * 32;
+          const float4 x = *reinterpret_cast<const float4*>(src + o), y = *reinterpret_cast<const float4*>(src + which + o);
+          q[4 * j] += x.x; q[4 * j + 1] += x.y; q[4 * j + 2] += x.z; q[4 * j + 3] += x.w;
+          k[4 * j] += y.x; k[4 * j + 1] += y.y; k[4 * j + 2] += y.z; k[4 * j + 3] += y.w;
+        }
+      }
+      const float f = p.scale / (float)Segments(p.seg_N, m).len(r);
+      float* dq = p.qt_out + ((size_t)bh * m + r) * kN + c0;
+      float* dk = p.kt_out + ((size_t)bh * m + r) * kN + c0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int o = (j & 1) * 4 + (j >> 1) * 32;
+#pragma unroll
+        for (int i = 4 * j; i < 4 * j + 4; ++i) { q[i] *= f; k[i] *= f; }
+        *reinterpret_cast<float4*>(dq + o) = make_float4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
+        *reinterpret_cast<float4*>(dk + o) = make_float4(k[4 * j], k[4 * j + 1], k[4 * j + 2], k[4 * j + 3]);
       }
     }
-  } else {
-    load_global16(p.qt + bh * m * D, m, D, D, q);
-    load_global16(p.kt + bh * m * D, m, D, D, k);
+    put_tile16(c.slot(0), q);
+    put_tile16(c.slot(1), k);
+    return;
   }
-  store_set16(c.slot(0), q);
-  store_set16(c.slot(1), k);
-  tiles_ready(c);
-  wait_group(c, 0, 0x210f);
-  acc_result(c, kAcc0, v);
-  store_row16(c, fwd_staging(c), v);
-  ns::ns_sync();
-  softmax16(fwd_staging(c), p, bh);
+#pragma unroll 1
+  for (int h = 0; h < (D > kN ? 2 : 1); ++h) {
+    const int cols = min(D, kN);
+    load_tile16(p.qt + bh * m * D + h * kN, m, cols, D, q);
+    load_tile16(p.kt + bh * m * D + h * kN, m, cols, D, k);
+    put_tile16(c.slot(2 * h), q);
+    put_tile16(c.slot(2 * h + 1), k);
+  }
 }
 
-__global__ void __launch_bounds__(kNsTcThreads, 1) ns_fwd_tc_kernel(ns::NsFwdParams p, int* status) {
-  extern __shared__ uint8_t dyn_smem[];
-  __shared__ float red[ns::kRedFloats];
-  __shared__ Shared sh;
-  Ctx c;
-  ctx_open(c, sh, dyn_smem, kFwdSlots, status, kFwdTmemCols);
-  const int64_t bh = blockIdx.x;
-  const int m = p.m;
-  const bool scores_tc = p.D == kN;
-  if (is_compute()) {
-    NS_TRACE();
-    if (scores_tc) s2_softmax_tc(c, p, bh);
-    else ns::s2_softmax(fwd_staging(c), p, bh);
-    NS_TRACE();
-    pinv_forward_tc(c, red, p.iterates + bh * (size_t)(p.J + 1) * m * m, p.k2inv + bh * m * m, m, p.J, p.kappa);
-  } else if (is_issuer()) {
-    pinv_forward_issue(c, p.J, p.kappa, scores_tc);
-  }
-  ctx_close(c, kFwdTmemCols);
-}
-
-__global__ void __launch_bounds__(kNsTcThreads, 1)
-ns_pinv_fwd_tc_debug_kernel(const float* k2, float* iterates, float* k2inv, int m, int J, float kappa,
-                            int* status) {
-  extern __shared__ uint8_t dyn_smem[];
-  __shared__ float red[ns::kRedFloats];
-  __shared__ Shared sh;
-  Ctx c;
-  ctx_open(c, sh, dyn_smem, kFwdSlots, status, kFwdTmemCols);
-  const int64_t bh = blockIdx.x;
-  if (is_compute()) {
-    ns::load_mat(fwd_staging(c), k2 + bh * m * m, m);
+__device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams& f, int64_t bh) {
+  const ns::NsFwdParams& p = f.p;
+  const int m = p.m, J = p.J, mm_ = m * m;
+  const bool ridge = p.kappa > 0.f;
+  const int last = 4 * J + (ridge ? 1 : 0);
+  float* X = c.stage(kFwdStage);
+  float* iterates = p.iterates + bh * (size_t)(J + 1) * mm_;
+  float* k2 = p.k2 + bh * mm_;
+  float z[16], r[16], v[16];       // Z_j, R and the value in hand
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { r[i] = 0.f; v[i] = 0.f; }
+  if (f.k2_given) {
+    load_tile16(k2, m, m, m, v);
+    stage_tile16(X, v);
     ns::ns_sync();
-    pinv_forward_tc(c, red, iterates + bh * (size_t)(J + 1) * m * m, k2inv + bh * m * m, m, J, kappa);
-  } else if (is_issuer()) {
-    pinv_forward_issue(c, J, kappa, false);
+  } else {
+    fwd_landmarks(c, p, bh);
+    arrive_ready(c, 0);
   }
+#pragma unroll 1
+  for (int s = f.k2_given ? -1 : -2; s < last; ++s) {
+    if (s == -1 && !ridge) continue;                       // A = K2
+    if (s == -1 || s == 0) {
+      // X = K2 (s = -1) or A: its norms, then K2 as an operand, or A and Z0
+      const Norms n = ns::norms(X, m, red);
+      unstage_row16(c, X, v);
+      if (s == -1) {
+        r[0] = n.n1 * n.ninf / p.kappa;                    // lambda
+        put_row16(c, c.slot(2), v);
+      } else {
+        const float cden = fmaxf(n.n1 * n.ninf, 1e-12f);
+        put_row16(c, c.slot(0), v);
+        unstage_col16(c, X, z);                            // Z0 = A^T / cden
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z[i] /= cden;
+        put_row16(c, c.slot(1), z);
+      }
+      arrive_ready(c, 0);
+      if (s == 0 && c.act && !c.failed) store_row16(c, iterates, z, m, m, m);
+    }
+    if (s >= 0 && s < 4 * J) {
+      // one iteration; R, then Y and W, then Z'
+      take(c, 0, 0, c.slot(2), c.act, v, c.trunc);
+      if (c.act) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) r[i] = -v[i];
+        add_diag(c, r, 1.f, m);
+        put_row16(c, c.slot(2), r);
+      }
+      arrive_ready(c, 0);
+      take(c, 1, kAccCols, c.slot(3), c.act, v, c.trunc);
+      if (c.act) put_row16(c, c.slot(3), v);
+      take(c, 0, 0, c.slot(2), c.act, v, c.trunc);
+      if (c.act) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = fmaf(0.25f, v[i], r[i]);
+        add_diag(c, v, 1.f, m);
+        put_row16(c, c.slot(2), v);
+      }
+      arrive_ready(c, 0);
+      s += 3;
+      const bool end = s == 4 * J - 1;
+      if (ridge && end) load_row16(c, k2, m, m, m, r);      // (R is dead; K2 is the last product's operand)
+      take(c, 1, kAccCols, c.slot(1), c.act, v, c.trunc);
+      if (c.act) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z[i] += v[i];
+        put_row16(c, c.slot(1), z);
+        if (ridge && end) put_row16(c, c.slot(0), r);
+      }
+      if (!end || ridge) arrive_ready(c, 0);
+      if (c.act && !c.failed) {
+        store_row16(c, iterates + (size_t)((s >> 2) + 1) * mm_, z, m, m, m);
+        if (end && !ridge) store_row16(c, p.k2inv + bh * mm_, z, m, m, m);
+      }
+      continue;
+    }
+    // scores (s = -2), K2^T K2 (s = -1), k2inv (s = 4J)
+    take(c, s & 1, (s & 1) * kAccCols, c.slot(s == -1 ? 0 : 2), c.act, v, s == -2 ? kTruncScores : c.trunc);
+    if (s == 4 * J) {
+      if (c.act && !c.failed) store_row16(c, p.k2inv + bh * mm_, v, m, m, m);
+      break;
+    }
+    if (!c.act) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = 0.f;
+    }
+    if (s == -1) add_diag(c, v, r[0], m);
+    stage_row16(c, X, v);
+    ns::ns_sync();
+    if (s == -2) softmax16(X, p, bh);
+  }
+}
+
+__global__ void __launch_bounds__(kNsTcThreads, 2) ns_fwd_tc_kernel(FwdParams f, int* status) {
+  extern __shared__ uint8_t dyn_smem[];
+  __shared__ float red[ns::kRedFloats];
+  __shared__ Shared sh;
+  Ctx c;
+  ctx_open(c, sh, dyn_smem, status, kFwdTmemCols, f.p.m);
+  if (is_compute()) fwd_compute(c, red, f, blockIdx.x);
+  else fwd_issue(c, f);
   ctx_close(c, kFwdTmemCols);
 }
 
 // ---------------------------------------------------------------------------------------------
-// Backward.  Slots: 0 A, 1 Z_j, 2 dZ (gradient w.r.t. Z_{j+1}), 3 M, 4 nU = M - 7I,
-// 5 ndT = -dT, 6 V then qT = T / 4, 7 dV then dM.  Two TMEM accumulators.  Per iteration, with
-// dT = Z^T dZ / 4, dV = -M^T dT, dU = -M^T dV:
-//   batch 1:  M = A Z                         | ndT = -(Z^T dZ) / 4
-//   batch 2:  V = 15 I + M nU                 | dV  = M^T ndT
-//   batch 3:  dM = ndT V^T + dV nU^T + M^T dV | qT = (13 I - M V) / 4
-//   batch 4:  dZ' = dZ qT^T + A^T dM          | dA += dM Z^T   (dA lives in registers)
-// The epilogue of the group left of the bar runs while the group right of it is still in the
-// tensor core.  The next iterate is fetched into registers a whole iteration ahead.  With the
-// ridge the FP32 set-up (K2, A, Z_J, dZ_J) is staged in slots 5..7; after the loop the tail
-// works in FP32 buffers at the start of the slot area.  A last batch (head_dim 64 only) forms the
-// landmark gradients dqt_ns = dS2 Kt and dS2^T Qt from slots 5 (dS2), 6 (Kt), 7 (Qt); head_dim 128
-// runs it twice, once per 64 columns of Kt and Qt.
-constexpr int kBwdStageSlot = 5;
-__device__ __forceinline__ float* bwd_stage(const Ctx& c, int i) {
-  return reinterpret_cast<float*>(c.slot(kBwdStageSlot)) + (size_t)i * kBuf;
-}
-__device__ __forceinline__ float* bwd_tail(const Ctx& c, int i) {
-  return reinterpret_cast<float*>(c.base) + (size_t)i * kBuf;
-}
-
-// issuing thread
-__device__ inline void pinv_backward_issue(Ctx& c, int J, int finish, bool head) {
-  if (head) {
-    // dO3 = K2inv^T dstep2 | dK2inv = dstep2 Bmat^T   (slots 3 K2inv, 4 dstep2, 6 Bmat)
-    const uint32_t sKi = c.slot_addr(3), sDs = c.slot_addr(4), sBm = c.slot_addr(6);
-    mma_batch(c, 0x21f0, [&] { issue_product(c.tmem + kAcc0, left_t(sKi), right(sDs), false); },
-              [&] { issue_product(c.tmem + kAcc1, left(sDs), right_t(sBm), false); });
-  }
-  const uint32_t sA = c.slot_addr(0), sZ = c.slot_addr(1), sdZ = c.slot_addr(2), sM = c.slot_addr(3),
-                 sU = c.slot_addr(4), sdT = c.slot_addr(5), sV = c.slot_addr(6), sT = c.slot_addr(6),
-                 sdV = c.slot_addr(7), sdM = c.slot_addr(7);
-  const uint32_t acc0 = c.tmem + kAcc0, acc1 = c.tmem + kAcc1;
-  for (int j = J - 1; j >= 0; --j) {
-    mma_batch(c, 0x2200, [&] { issue_product(acc0, left(sA), right(sZ), false); },
-              [&] { issue_product(acc1, left_t(sZ), right(sdZ), false); });
-    mma_batch(c, 0x2201, [&] { issue_product(acc0, left(sM), right(sU), false); },
-              [&] { issue_product(acc1, left_t(sM), right(sdT), false); });
-    mma_batch(c, 0x2202,
-              [&] {
-                issue_product(acc1, left(sdT), right_t(sV), false);
-                issue_product(acc1, left(sdV), right_t(sU), true);
-                issue_product(acc1, left_t(sM), right(sdV), true);
-              },
-              [&] { issue_product(acc0, left(sM), right(sV), false); });
-    mma_batch(c, 0x2203,
-              [&] {
-                issue_product(acc0, left(sdZ), right_t(sT), false);
-                issue_product(acc0, left_t(sA), right(sdM), true);
-              },
-              [&] { issue_product(acc1, left(sdM), right_t(sZ), false); });
-  }
-  for (int half = 0; half < finish; ++half) {
-    const uint32_t sS = c.slot_addr(5), sK = c.slot_addr(6), sQ = c.slot_addr(7);
-    mma_batch(c, 0x2204, [&] { issue_product(acc0, left(sS), right(sK), false); },
-              [&] { issue_product(acc1, left_t(sS), right(sQ), false); });
-  }
-}
-
-// compute warps.  Requires J >= 1.  Returns dK2 (padded FP32 buffer); K2 is left in bwd_tail(c, 0).
-// before_tail() runs between the iterations and the FP32 tail (a place to start global loads
-// whose latency the tail hides).
-template <class BeforeTail>
-__device__ __forceinline__ float* pinv_backward_tc(Ctx& c, float* red, const float* k2g, const float* iterates,
-                                                   const float* G, float* spill, int m, int J, float kappa,
-                                                   BeforeTail before_tail, float* znext, const float* a,
-                                                   float* step_dz = nullptr, float* step_da = nullptr) {
-  // G == nullptr: dL/dk2inv is already in place (slot 2 without the ridge, staging buffer 3 with it)
-  // znext, a: Z_{J-1} and K2 as load_global16 gives them (fetched by the caller ahead of its own products)
-  const int mm_ = m * m;
-  if (kappa > 0.f) {
-    float* bK2 = bwd_stage(c, 0);
-    float* bA = bwd_stage(c, 1);
-    float* bZ = bwd_stage(c, 2);
-    float* bdZ = bwd_stage(c, 3);
-    ns::load_mat(bK2, k2g, m);
-    if (G) ns::load_mat(bdZ, G, m);
-    ns::ns_sync();
-    Norms nk = ns::norms(bK2, m, red);
-    const float lam = nk.n1 * nk.ninf / kappa;
-    ns::mm<ns::TN>(bK2, bK2, [&](int r, int cc, float acc) { bA[r * kLd + cc] = acc + ((r == cc && r < m) ? lam : 0.f); });
-    ns::load_mat(bZ, iterates + (size_t)J * mm_, m);
-    ns::ns_sync();
-    // dK2_a = G^T Z_J -> global spill; dZ_J = G K2
-    ns::mm<ns::TN>(bdZ, bZ, [&](int r, int cc, float acc) { if (r < m && cc < m) spill[r * m + cc] = acc; });
-    ns::mm<ns::NN>(bdZ, bK2, [&](int r, int cc, float acc) { bdZ[r * kLd + cc] = acc; });
-    convert_buf(c.slot(0), bA);
-    convert_buf(c.slot(2), bdZ);
-  } else {
-    // A = K2 and dZ_J = G go straight from global memory into their tiles
-    if (G) {
-      float g[16];
-      load_global16(G, m, m, m, g);
-      store_set16(c.slot(2), g);
-    }
-    store_set16(c.slot(0), a);
-  }
-  store_set16(c.slot(1), znext);
-  NS_TRACE();
-  float v[16], dA[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) dA[i] = 0.f;
-  for (int j = J - 1; j >= 0; --j) {
-    tiles_ready(c);
-    // next iterate; in the last iteration K2 for the FP32 tail instead
-    load_global16(j > 0 ? iterates + (size_t)(j - 1) * mm_ : k2g, m, m, m, znext);
-    wait_group(c, 0, 0x2210);
-    acc_result(c, kAcc0, v);
-    split_store16(c.slot(3), c.row, c.col0, v);
-    affine(c, v, 1.f, -7.f, m);
-    split_store16(c.slot(4), c.row, c.col0, v);
-    wait_group(c, 1, 0x2220);
-    acc_result(c, kAcc1, v);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
-    split_store16(c.slot(5), c.row, c.col0, v);
-    NS_TRACE();
-    tiles_ready(c);
-    wait_group(c, 0, 0x2211);
-    acc_result(c, kAcc0, v);
-    affine(c, v, 1.f, 15.f, m);
-    split_store16(c.slot(6), c.row, c.col0, v);
-    wait_group(c, 1, 0x2221);
-    acc_result(c, kAcc1, v);
-    split_store16(c.slot(7), c.row, c.col0, v);
-    NS_TRACE();
-    tiles_ready(c);
-    wait_group(c, 0, 0x2212);
-    acc_result(c, kAcc1, v);
-    split_store16(c.slot(7), c.row, c.col0, v);      // dM over dV: every product reading dV is done
-    wait_group(c, 1, 0x2222);
-    acc_result(c, kAcc0, v);
-    affine(c, v, -0.25f, 3.25f, m);
-    split_store16(c.slot(6), c.row, c.col0, v);      // qT over V
-    NS_TRACE();
-    tiles_ready(c);
-    wait_group(c, 0, 0x2213);
-    acc_result(c, kAcc0, v);
-    if (j > 0) split_store16(c.slot(2), c.row, c.col0, v);
-    wait_group(c, 1, 0x2223);
-    // every product of this iteration is complete: all tiles are free
-    if (j == 0) store_row16(c, bwd_tail(c, 2), v);
-    acc_result(c, kAcc1, v);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dA[i] += v[i];
-    if (j > 0) store_set16(c.slot(1), znext);
-    NS_TRACE();
-  }
-  if (step_dz) {
-    // isolation hook: hand back dL/dZ_0 and the dL/dA accumulated over the iterations, skip the tail
-    ns::ns_sync();
-    if (!c.failed) {
-      ns::store_mat(step_dz, bwd_tail(c, 2), m);
-      store_global16(c, step_da, dA, m, m, m);
-    }
-    return nullptr;
-  }
-  before_tail();
-  store_row16(c, bwd_tail(c, 3), dA);
-  float* bK2 = bwd_tail(c, 0);
-  float* bA = bwd_tail(c, 1);
-  store_buf16(bK2, znext);
-  ns::ns_sync();
-  NS_TRACE();
-  const float* A = bK2;
-  if (kappa > 0.f) {
-    Norms nk = ns::norms(bK2, m, red);
-    const float lam = nk.n1 * nk.ninf / kappa;
-    ns::mm<ns::TN>(bK2, bK2, [&](int r, int cc, float acc) { bA[r * kLd + cc] = acc + ((r == cc && r < m) ? lam : 0.f); });
-    A = bA;
-  }
-  return ns::pinv_backward_tail(bK2, A, bwd_tail(c, 2), bwd_tail(c, 3), bwd_tail(c, 4), bwd_tail(c, 5), red, spill,
-                                m, kappa);
-}
-
-__global__ void __launch_bounds__(kNsTcThreads, 1)
-ns_pinv_bwd_tc_debug_kernel(const float* k2, const float* iterates, const float* G, float* dK2, float* spill,
-                            int m, int J, float kappa, int* status, float* step_dz, float* step_da) {
-  extern __shared__ uint8_t dyn_smem[];
-  __shared__ float red[ns::kRedFloats];
-  __shared__ Shared sh;
-  Ctx c;
-  ctx_open(c, sh, dyn_smem, kBwdSlots, status, kBwdTmemCols);
-  const int64_t bh = blockIdx.x;
-  if (is_compute()) {
-    // step hook: one iteration (J = 1) whose "iterates" is the single matrix Z_j per slice
-    const float* its = step_dz ? iterates + bh * (size_t)m * m : iterates + bh * (size_t)(J + 1) * m * m;
-    float z[16], a[16];
-    load_global16(its + (size_t)(J - 1) * m * m, m, m, m, z);
-    load_global16(k2 + bh * m * m, m, m, m, a);
-    float* out = pinv_backward_tc(c, red, k2 + bh * m * m, its, G + bh * m * m, spill + bh * m * m, m, J, kappa, [] {}, z, a,
-                                  step_dz ? step_dz + bh * m * m : nullptr, step_da ? step_da + bh * m * m : nullptr);
-    if (out && !c.failed) ns::store_mat(dK2 + bh * m * m, out, m);
-  } else if (is_issuer()) {
-    pinv_backward_issue(c, J, false, false);
-  }
-  ctx_close(c, kBwdTmemCols);
-}
-
-// Softmax-2 Jacobian and the landmark gradients after the pseudoinverse backward, for head_dim 64
-// and 128: dqt_ns = dS2 Kt and dkt_tot = dkt_a + dS2^T Qt as one more batch of split products per
-// 64 columns of the landmarks.
-// bK2, dK2: padded FP32 buffers inside the tail area (slots 0..4); slots 5..7 take the operands.
-struct FinishOperands { float kt[16], qt[16], da[16]; };
-// global loads of the finishing step for columns [64 half, 64 half + 64); the first half is issued
-// early so that its latency hides behind the tail
-__device__ __forceinline__ void finish_load(const Ctx& c, const ns::NsBwdParams& p, int64_t bh, int half,
-                                            FinishOperands& f) {
-  const int m = p.m, D = p.D, md = m * D;
-  load_global16(p.kt + bh * md + half * kN, m, kN, D, f.kt);
-  load_global16(p.qt + bh * md + half * kN, m, kN, D, f.qt);
-  // dkt_a for the row segment this thread finalises
-  const float* src = p.dkt_a + bh * md + (size_t)c.row * D + half * kN + c.col0;
-#pragma unroll
-  for (int i = 0; i < 16; i += 4) {
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c.row < m) x = *reinterpret_cast<const float4*>(src + i);
-    f.da[i] = x.x; f.da[i + 1] = x.y; f.da[i + 2] = x.z; f.da[i + 3] = x.w;
-  }
-}
-template <int NH>
-__device__ inline void ns_bwd_finish_tc(Ctx& c, const ns::NsBwdParams& p, int64_t bh, const float* bK2, float* dK2,
-                                        FinishOperands& f) {
-  const int m = p.m, D = p.D, md = m * D, t = threadIdx.x;
-  // softmax-2 Jacobian in place: dS2 = K2 o (dK2 - rowsum(dK2 o K2))
-  const int w = t >> 5, lane = t & 31;
-  for (int r = w; r < kN; r += kComputeThreads / 32) {
-    float a0 = dK2[r * kLd + lane], a1 = dK2[r * kLd + lane + 32];
-    float k0 = bK2[r * kLd + lane], k1 = bK2[r * kLd + lane + 32];
-    float s = a0 * k0 + a1 * k1;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    dK2[r * kLd + lane] = k0 * (a0 - s);
-    dK2[r * kLd + lane + 32] = k1 * (a1 - s);
-  }
-  ns::ns_sync();
-  convert_buf(c.slot(5), dK2);
-#pragma unroll
-  for (int half = 0; half < NH; ++half) {
-    // every product that read slots 6 and 7 has been waited for below
-    if (half > 0) finish_load(c, p, bh, half, f);
-    store_set16(c.slot(6), f.kt);
-    store_set16(c.slot(7), f.qt);
-    tiles_ready(c);
-    const size_t off = (size_t)bh * md + half * kN;
-    float v[16];
-    wait_group(c, 0, 0x2214);
-    acc_result(c, kAcc0, v);
-    if (!c.failed) store_global16(c, p.dqt_ns + off, v, m, kN, D);
-    wait_group(c, 1, 0x2224);
-    acc_result(c, kAcc1, v);
-    if (c.failed) return;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] += f.da[i];
-    store_global16(c, p.dkt_tot + off, v, m, kN, D);
-    if (p.rows_k && c.row < m) {
-      Segments sg(p.N, m);
-      const float fk = p.scale / (float)sg.len(c.row);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] *= fk;
-      store_global16(c, p.rows_k + off, v, m, kN, D);
-    }
-  }
-}
-
-// Head of the fused backward middle stage (head_dim 64): reduce the per-CTA partials of the
-// softmax-1 pass, then dO3 = K2inv^T dstep2 (-> D3, normalised 16-bit copy for the column pass) and
-// dK2inv = dstep2 Bmat^T, which lands where the pseudoinverse backward expects dL/dk2inv.
+// Backward.  With R = I - A Z, W = I + R + R^2 / 4, Y = Z R, Z' = Z + Y W and G = dL/dZ':
+//     dY = G W^T,  H = Y^T G / 4 (= dW / 4),  D = -dL/dR = -(Z^T dY + H R^T + R^T H + 4 H)
+//     dL/dZ = G + dY R^T + A^T D,  dL/dA += D Z^T
+// Three dependent steps per iteration (four in the nested form), and R, W, Y of the next lower iterate are formed
+// beside them.  Slots: A 0, Z_j and Z_{j-1} 1 and 2, R_j and R_{j-1} 3 and 4, G_j (then D) and G_{j-1} 5 and 6, W (then dY) 7,
+// Y (then H) 8.  Per iteration, in the order the products are issued (accumulator, done barrier):
+//     dY (3, 0) | H (2, 1) | R_{j-1} (1, 2) | D = Z^T dY + H R^T + R^T H (0, 3) | dY R^T (3)
+//     | R_{j-1}^2 (1, 4) | + A^T D (3, 5) | Z_{j-1} R_{j-1} (2, 6) | D Z^T (0, 7)
+// so that the products (11 of about 520 cycles) keep the tensor core busy while the epilogues run.  dL/dA is
+// summed in registers before the lane halves are added.  j = J is a prologue that only forms R, W, Y of Z_{J-1}.
+// Before it: dO3 = K2inv^T dstep2 and dK2inv = dstep2 Bmat^T of the fused middle stage, and with the ridge A = K2^T K2 +
+// lambda I, dZ_J = dK2inv K2 and dL/dK2 = dK2inv^T Z_J.  After it: the norm terms of Z0, the ridge, the softmax-2
+// Jacobian, and dqt_ns = dS2 Kt, dkt_tot = dkt_a + dS2^T Qt, 64 columns at a time.
+//
+// Head of the fused middle stage (head_dim 64):
 struct BwdHeadParams {
-  const float* partA;         // [BH][nchunk][2][m][D]: dstep2 partials, dKt partials
+  const float* partA;         // [BH][nchunk][2][m][D]: dstep2 partials, dKt partials (null: G is given)
   int nchunk;
   const float* k2inv; const float* bmat;
   float* dkt_a;               // [BH][m][D] out
@@ -814,155 +655,494 @@ struct BwdHeadParams {
   float qt_mul;
   int dtype, MP;
 };
+struct BwdParams {
+  ns::NsBwdParams p;
+  BwdHeadParams h;
+  float* dK2;                 // [BH][m][m]: stop there (pseudoinverse alone)
+  float* step_dz;             // [BH][m][m] each: stop after the iterations with dL/dZ_0 and dL/dA
+  float* step_da;             //   (p.iterates then is Z_0 alone)
+};
 
-__device__ inline void bwd_head_tc(Ctx& c, float* red, const ns::NsBwdParams& p, const BwdHeadParams& h, int64_t bh) {
-  const int m = p.m, D = p.D, md = m * D, t = threadIdx.x;
-  const int r = t >> 2, c0 = (t & 3) * 16;
-  NS_TRACE();
-  // reduce the partials: this thread owns row r, columns c0 .. c0+15 of both sums
-  float ds[16], dk[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) { ds[i] = 0.f; dk[i] = 0.f; }
-  if (r < m) {
-    const float* base = h.partA + bh * (int64_t)h.nchunk * 2 * md + (size_t)r * D + c0;
-    constexpr int CB = 3;
-    for (int ch0 = 0; ch0 < h.nchunk; ch0 += CB) {
-      float4 x[CB][4], y[CB][4];
-#pragma unroll
-      for (int i = 0; i < CB; ++i) {
-        const int ch = min(ch0 + i, h.nchunk - 1);
-        const float4* s0 = reinterpret_cast<const float4*>(base + (size_t)ch * 2 * md);
-        const float4* s1 = reinterpret_cast<const float4*>(base + (size_t)ch * 2 * md + md);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { x[i][q] = s0[q]; y[i][q] = s1[q]; }
-      }
-#pragma unroll
-      for (int i = 0; i < CB; ++i)
-        if (ch0 + i < h.nchunk) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            ds[4 * q] += x[i][q].x; ds[4 * q + 1] += x[i][q].y; ds[4 * q + 2] += x[i][q].z; ds[4 * q + 3] += x[i][q].w;
-            dk[4 * q] += y[i][q].x; dk[4 * q + 1] += y[i][q].y; dk[4 * q + 2] += y[i][q].z; dk[4 * q + 3] += y[i][q].w;
-          }
-        }
-    }
-    float4* out = reinterpret_cast<float4*>(h.dkt_a + bh * md + (size_t)r * D + c0);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) out[q] = make_float4(dk[4 * q], dk[4 * q + 1], dk[4 * q + 2], dk[4 * q + 3]);
+// Steps outside the iterations, which share one body.  kNorms comes with no accumulator first (K2), with the ridge again for
+// the Gram matrix.
+enum BwdStep { kNorms, kHeadO3, kHeadG, kRidgeG, kRidgeK2, kSumDA, kTailK2, kDQ, kDK };
+
+// issuing warp.  ready barriers: 0 G and W (also the head's operands, and those of the tail), 1 Y (also K2), 2 Z_{j-1}
+// (also A), 3 dY (also dK2inv), 4 H, 5 R_{j-1}, 6 D.
+__device__ inline void bwd_issue(Ctx& c, const BwdParams& f, int finish) {
+  const bool ridge = f.p.kappa > 0.f, head = f.h.partA != nullptr;
+  const int J = f.p.J;
+  const uint32_t nk = (f.p.m + 15) / 16, acc0 = c.tmem, acc1 = acc0 + kAccCols, acc2 = acc1 + kAccCols, acc3 = acc2 + kAccCols;
+  auto commit = [&](int b) { umma_commit_elect(c.sh->done + b); };
+  if (ridge) {
+    wait_ready(c, 1, 0x2201);
+    if (c.failed) return;
+    issue_product<true, false>(acc1, c.slot(4), c.slot(4), false, nk);                 // K2^T K2
+    commit(3);
   }
-  NS_TRACE();
-  store_set16(c.slot(4), ds);
-  {
-    float ki[16], bm[16];
-    load_global16(h.k2inv + bh * m * m, m, m, m, ki);
-    load_global16(h.bmat + bh * md, m, D, D, bm);
-    store_set16(c.slot(3), ki);
-    store_set16(c.slot(6), bm);
+  if (head) {
+    wait_ready(c, 0, 0x2200);
+    if (c.failed) return;
+    issue_product<true, false>(acc3, c.slot(7), c.slot(8), false, nk);                 // K2inv^T dstep2
+    commit(0);
+    issue_product<false, true>(acc0, c.slot(8), c.slot(6), false, 4);                  // dstep2 Bmat^T (K is the head_dim)
+    commit(1);
   }
-  tiles_ready(c);
-  NS_TRACE();
-  // operands of this thread's share of the epilogue: Bmat segment for D3, Qt row for the copy
-  float bseg[16], qrow[16];
-  {
-    const float* src = h.bmat + bh * md + (size_t)c.row * D + c.col0;
-#pragma unroll
-    for (int i = 0; i < 16; i += 4) {
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c.row < m) x = *reinterpret_cast<const float4*>(src + i);
-      bseg[i] = x.x; bseg[i + 1] = x.y; bseg[i + 2] = x.z; bseg[i + 3] = x.w;
-    }
+  if (ridge) {
+    wait_ready(c, 3, 0x2203);
+    if (c.failed) return;
+    issue_product<false, false>(acc3, c.slot(6), c.slot(4), false, nk);                // dK2inv K2
+    commit(5);
+    issue_product<true, false>(acc0, c.slot(6), c.slot(2), false, nk);                 // dK2inv^T Z_J
+    commit(7);
   }
-  load_global16(p.qt + bh * md, m, D, D, qrow);
-  float v[16];
-  wait_group(c, 0, 0x21f1);
-  acc_result(c, kAcc0, v);                       // dO3
-  float d3 = 0.f, amax = 0.f;
-#pragma unroll
-  for (int i = 0; i < 16; ++i) { d3 = fmaf(v[i], bseg[i], d3); amax = fmaxf(amax, fabsf(v[i])); }
-  float* do3f = bwd_tail(c, 0);                  // FP32 dO3 until the scale is known (slots 0, 1 are still free)
-  store_row16(c, do3f, v);
-  // red: [0..255] D3 partials (4 per row), [256..263] per-warp maxima
-  red[c.row * 4 + (c.c32 >> 5) * 2 + c.part] = d3;
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((t & 31) == 0) red[256 + (t >> 5)] = amax;
-  wait_group(c, 1, 0x21f2);
-  acc_result(c, kAcc1, v);                       // dK2inv
-  if (p.kappa > 0.f) store_row16(c, bwd_stage(c, 3), v);
-  else split_store16(c.slot(2), c.row, c.col0, v);
-  ns::ns_sync();
-  float cmax = red[256];
-#pragma unroll
-  for (int w = 1; w < kComputeThreads / 32; ++w) cmax = fmaxf(cmax, red[256 + w]);
-  const float sc = pow2_scale(cmax), inv_sc = 1.f / sc;
-  if (h.D3) {
-  if (t == 0) h.do3_scale[bh] = sc;
-  if (t < m) h.D3[bh * m + t] = (red[4 * t] + red[4 * t + 1]) + (red[4 * t + 2] + red[4 * t + 3]);
-  {
-    // 16-bit copies, rows >= m zero: dO3 / scale and qt_mul * Qt
-    const size_t ob = (size_t)bh * h.MP * D;
-    uint32_t w0[8], w1[8];
-#pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      const float a = (r < m) ? do3f[r * kLd + c0 + i] * inv_sc : 0.f;
-      const float b = (r < m) ? do3f[r * kLd + c0 + i + 1] * inv_sc : 0.f;
-      w0[i >> 1] = h.dtype == 1 ? pack2<__half>(a, b) : pack2<__nv_bfloat16>(a, b);
-      w1[i >> 1] = h.dtype == 1 ? pack2<__half>(qrow[i] * h.qt_mul, qrow[i + 1] * h.qt_mul)
-                                : pack2<__nv_bfloat16>(qrow[i] * h.qt_mul, qrow[i + 1] * h.qt_mul);
+#pragma unroll 1
+  for (int j = J; j >= 0; --j) {
+    const int par = (J - 1 - j) & 1;
+    const bool main_part = j < J, prime = j > 0;
+    const uint32_t z = c.slot(1 + par), zn = c.slot(2 - par), r = c.slot(3 + par), rn = c.slot(4 - par), g = c.slot(5 + par);
+    if (main_part) {
+      wait_ready(c, 0, 0x2210);
+      if (c.failed) return;
+      issue_product<false, true>(acc3, g, c.slot(7), false, nk);                       // G W^T
+      commit(0);
+      wait_ready(c, 1, 0x2211);
+      if (c.failed) return;
+      issue_product<true, false>(acc2, c.slot(8), g, false, nk);                       // Y^T G
+      commit(1);
     }
-    if (r < h.MP) {
-      uint4* d0 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(h.do3n) + ob + (size_t)r * D + c0);
-      uint4* d1 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(h.qt16) + ob + (size_t)r * D + c0);
-      d0[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]); d0[1] = make_uint4(w0[4], w0[5], w0[6], w0[7]);
-      d1[0] = make_uint4(w1[0], w1[1], w1[2], w1[3]); d1[1] = make_uint4(w1[4], w1[5], w1[6], w1[7]);
+    if (prime) {
+      wait_ready(c, 2, 0x2212);
+      if (c.failed) return;
+      issue_product<false, false>(acc1, c.slot(0), zn, false, nk);                     // A Z'
+      commit(2);
+    }
+    if (main_part) {
+      wait_ready(c, 3, 0x2213);
+      if (c.failed) return;
+      issue_product<true, false>(acc0, z, c.slot(7), false, nk);                       // Z^T dY
+      wait_ready(c, 4, 0x2214);
+      if (c.failed) return;
+      issue_product<false, true>(acc0, c.slot(8), r, true, nk);                        // + H R^T
+      issue_product<true, false>(acc0, r, c.slot(8), true, nk);                        // + R^T H
+      commit(3);
+      issue_product<false, true>(acc3, c.slot(7), r, false, nk);                       // dY R^T
+    }
+    if (prime) {
+      wait_ready(c, 5, 0x2215);
+      if (c.failed) return;
+      issue_product<false, false>(acc1, rn, rn, false, nk);                            // R'^2
+      commit(4);
+    }
+    if (main_part) {
+      wait_ready(c, 6, 0x2216);
+      if (c.failed) return;
+      issue_product<true, false>(acc3, c.slot(0), g, true, nk);                        // + A^T D
+      commit(5);
+    }
+    if (prime) {
+      issue_product<false, false>(acc2, zn, rn, false, nk);                            // Z' R'
+      commit(6);
+    }
+    if (main_part) {
+      issue_product<false, true>(acc0, g, z, false, nk);                               // D Z^T
+      commit(7);
     }
   }
+  if (finish < 0) return;
+  if (ridge) {
+    wait_ready(c, 0, 0x2220);
+    if (c.failed) return;
+    issue_product<false, false>(acc3, c.slot(6), c.slot(5), false, nk);                // K2 dA
+    issue_product<false, true>(acc3, c.slot(6), c.slot(5), true, nk);                  // + K2 dA^T
+    commit(0);
   }
-  ns::ns_sync();   // do3f (slots 0, 1) is free again
-  NS_TRACE();
+#pragma unroll 1
+  for (int half = 0; half < finish; ++half) {
+    wait_ready(c, 0, 0x2221);
+    if (c.failed) return;
+    issue_product<false, false>(acc0, c.slot(5), c.slot(6), false, nk);                // dS2 Kt
+    commit(0);
+    issue_product<true, false>(acc1, c.slot(5), c.slot(7), false, nk);                 // dS2^T Qt
+    commit(1);
+  }
 }
 
-// NH: batches of the finishing step = head_dim / 64 for head_dim 64 and 128 (the instantiation with
-// NH = 1 also serves the smaller head dims, whose finishing step runs on the CUDA cores)
-template <int NH>
-__global__ void __launch_bounds__(kNsTcThreads, 1)
-ns_bwd_tc_kernel(ns::NsBwdParams p, BwdHeadParams h, int* status) {
+// compute warps.  finish: batches of 64 columns of the landmark gradients; 0: stop at dL/dK2, -1: after the iterations.
+__device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams& f, int64_t bh, int finish) {
+  const ns::NsBwdParams& p = f.p;
+  const BwdHeadParams& h = f.h;
+  const int m = p.m, D = p.D, J = p.J, mm_ = m * m, t = threadIdx.x;
+  const int64_t md = (int64_t)m * D;
+  const bool ridge = p.kappa > 0.f, head = h.partA != nullptr;
+  const float* iterates = p.iterates + bh * (size_t)(f.step_dz ? 1 : J + 1) * mm_;
+  float* X = c.stage(3);
+  float v[16], g[16], hd[16], r[16], da_keep[16], da_send[16], z[16];
+  float lam = 0.f;
+  Norms nrm;
+  // ---- operands ----
+  load_tile16(iterates + (size_t)(J - 1) * mm_, m, m, m, z);
+  load_tile16(p.k2 + bh * mm_, m, m, m, r);
+  if (ridge) load_tile16(iterates + (size_t)J * mm_, m, m, m, hd);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) { g[i] = 0.f; da_keep[i] = 0.f; da_send[i] = 0.f; }
+  if (!head) load_row16(c, p.G + bh * mm_, m, m, m, g);
+  put_tile16(c.slot(1), z);
+  put_tile16(c.slot(ridge ? 4 : 0), r);
+  if (ridge) put_tile16(c.slot(2), hd);
+  arrive_ready(c, ridge ? 1 : 2);
+  stage_tile16(X, r);
+  if (!head) put_row16(c, c.slot(ridge ? 6 : 5), g);
+  if (!head && ridge) arrive_ready(c, 3);
+  if (ridge) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) g[i] = 0.f;       // dL/dZ_J = G K2 is added to it
+  }
+  if (J > 1) load_tile16(iterates + (size_t)(J - 2) * mm_, m, m, m, z);
+  if (head) {
+    // reduce the partials of the first row pass: dstep2 -> slot 8, dkt_a -> global
+    float ds[16], dk[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) { ds[i] = 0.f; dk[i] = 0.f; }
+    const int row = t >> 2, c0 = (t & 3) * 8;
+    if (row < m) {
+      const float* src = h.partA + bh * (int64_t)h.nchunk * 2 * md + (size_t)row * kN + c0;
+#pragma unroll 2
+      for (int ch = 0; ch < h.nchunk; ++ch, src += 2 * md) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int o = (q & 1) * 4 + (q >> 1) * 32;
+          const float4 x = *reinterpret_cast<const float4*>(src + o), y = *reinterpret_cast<const float4*>(src + md + o);
+          ds[4 * q] += x.x; ds[4 * q + 1] += x.y; ds[4 * q + 2] += x.z; ds[4 * q + 3] += x.w;
+          dk[4 * q] += y.x; dk[4 * q + 1] += y.y; dk[4 * q + 2] += y.z; dk[4 * q + 3] += y.w;
+        }
+      }
+      float* out = h.dkt_a + bh * md + (size_t)row * kN + c0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4*>(out + (q & 1) * 4 + (q >> 1) * 32) = make_float4(dk[4 * q], dk[4 * q + 1], dk[4 * q + 2], dk[4 * q + 3]);
+    }
+    put_tile16(c.slot(8), ds);
+    load_tile16(h.k2inv + bh * mm_, m, m, m, v);
+    load_tile16(h.bmat + bh * md, m, kN, kN, ds);
+    put_tile16(c.slot(7), v);
+    put_tile16(c.slot(6), ds);
+    arrive_ready(c, 0);
+  }
+  ns::ns_sync();                                     // X is complete
+
+#pragma unroll 1
+  for (int phase = 0; phase < 2; ++phase) {
+    // ---- before and after the iterations ----
+    int step = phase ? kSumDA : kNorms;
+    bool first = true;                                 // the first kNorms has no accumulator
+    int half = 0;
+#pragma unroll 1
+    for (;;) {
+      // global operands of this step or of the batch after it, ahead of the wait
+      if (step == kHeadO3 && h.D3) load_row16(c, p.qt + bh * md, m, kN, kN, hd);
+      if (step == kDQ) load_row16(c, p.dkt_a + bh * md + half * kN, m, min(D, kN), D, z);
+      if (step == kSumDA || step == kDQ) {
+        const int hn = step == kDQ ? half + 1 : 0;
+        if (hn < finish) {
+          load_tile16(p.kt + bh * md + hn * kN, m, min(D, kN), D, hd);
+          load_tile16(p.qt + bh * md + hn * kN, m, min(D, kN), D, r);
+        }
+      }
+      // slot that the result goes to (or a free one to add the lane halves in), accumulator, done barrier
+      int dst, acc, done;
+      switch (step) {
+        case kNorms: dst = 0; acc = 1; done = 3; break;
+        case kHeadO3: dst = 5; acc = 3; done = 0; break;
+        case kHeadG: dst = ridge ? 6 : 5; acc = 0; done = 1; break;
+        case kRidgeG: dst = 5; acc = 3; done = 5; break;
+        case kRidgeK2: dst = 6; acc = 0; done = 7; break;
+        case kTailK2: dst = 4; acc = 3; done = 0; break;
+        case kDQ: dst = 8; acc = 0; done = 0; break;
+        case kDK: dst = 4; acc = 1; done = 1; break;
+        default: dst = 7; acc = 0; done = -1; break;   // kSumDA: in registers
+      }
+      // (results of the head and of the last batch have head_dim columns)
+      const bool act = (step == kHeadO3 || step == kDQ || step == kDK) ? (c.row & 32) < m : c.act;
+      if (step == kNorms && first) {
+      } else {
+        if (done >= 0) wait_done(c, done, 0x2210 + step);
+        if (act) {
+          float keep[16], send[16];
+          if (step == kSumDA) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) { keep[i] = da_keep[i]; send[i] = da_send[i]; }
+          } else {
+            fetch(c, acc * kAccCols, c.trunc, keep, send);
+          }
+          exchange(c, c.slot(dst), keep, send, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        }
+      }
+      int next = -1, arrive = -1;
+      bool jacobian = false;
+      switch (step) {
+        case kNorms:
+          if (!first) {
+            add_diag(c, v, lam, m);
+            put_row16(c, c.slot(0), v);
+            stage_row16(c, X, v);
+            arrive_ready(c, 2);
+            ns::ns_sync();
+          }
+          nrm = ns::norms(X, m, red);
+          if (first && ridge) { lam = nrm.n1 * nrm.ninf / p.kappa; next = kNorms; }
+          else next = head ? kHeadO3 : ridge ? kRidgeG : -1;
+          first = false;
+          break;
+        case kHeadO3: {
+          next = kHeadG;
+          if (!h.D3) break;
+          // dO3: its row sums with Bmat, and the 16-bit operands of the column pass, dO3 / scale and qt_mul * Qt (rows
+          // past m are zero)
+          float b[16], d3 = 0.f, amax = 0.f;
+          get_row16(c, c.slot(6), b);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) { d3 = fmaf(v[i], b[i], d3); amax = fmaxf(amax, fabsf(v[i])); }
+          red[c.row * 4 + (c.col0 >> 4)] = d3;
+          for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+          if ((t & 31) == 0) red[4 * kN + (t >> 5)] = amax;
+          ns::ns_sync();
+          float cmax = red[4 * kN];
+#pragma unroll
+          for (int w = 1; w < kComputeThreads / 32; ++w) cmax = fmaxf(cmax, red[4 * kN + w]);
+          const float sc = pow2_scale(cmax), inv_sc = 1.f / sc;
+          if (t == 0) h.do3_scale[bh] = sc;
+          if (t < m) h.D3[bh * m + t] = (red[4 * t] + red[4 * t + 1]) + (red[4 * t + 2] + red[4 * t + 3]);
+          uint32_t w0[8], w1[8];
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            const float x = v[i] * inv_sc, y = v[i + 1] * inv_sc, q0 = hd[i] * h.qt_mul, q1 = hd[i + 1] * h.qt_mul;
+            w0[i >> 1] = h.dtype == 1 ? pack2<__half>(x, y) : pack2<__nv_bfloat16>(x, y);
+            w1[i >> 1] = h.dtype == 1 ? pack2<__half>(q0, q1) : pack2<__nv_bfloat16>(q0, q1);
+          }
+          const size_t off = ((size_t)bh * h.MP + c.row) * kN + c.col0;
+          uint4* d0 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(h.do3n) + off);
+          uint4* d1 = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(h.qt16) + off);
+          d0[0] = make_uint4(w0[0], w0[1], w0[2], w0[3]); d0[1] = make_uint4(w0[4], w0[5], w0[6], w0[7]);
+          d1[0] = make_uint4(w1[0], w1[1], w1[2], w1[3]); d1[1] = make_uint4(w1[4], w1[5], w1[6], w1[7]);
+          break;
+        }
+        case kHeadG:
+          if (act) put_row16(c, c.slot(dst), v);
+          if (ridge) { arrive = 3; next = kRidgeG; }
+          else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) g[i] = v[i];
+          }
+          break;
+        case kRidgeG:
+#pragma unroll
+          for (int i = 0; i < 16; ++i) g[i] = v[i];
+          if (act) put_row16(c, c.slot(dst), v);
+          next = kRidgeK2;
+          break;
+        case kRidgeK2:
+          if (act && !c.failed) store_row16(c, p.spill + bh * mm_, v, m, m, m);
+          break;
+        case kSumDA: {
+          if (f.step_dz) {
+            if (!c.failed) {
+              store_row16(c, f.step_dz + bh * mm_, g, m, m, m);
+              store_row16(c, f.step_da + bh * mm_, v, m, m, m);
+            }
+            break;
+          }
+          // Z0 = A^T / c, c = ||A||_1 ||A||_inf (first-occurrence maxima): g = dL/dZ_0, v = dL/dA of the iterations
+          float gt[16], a[16], part = 0.f;
+          stage_row16(c, X, g);
+          if (c.act) get_row16(c, c.slot(0), a);
+          else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) a[i] = 0.f;
+          }
+          ns::ns_sync();
+          unstage_col16(c, X, gt);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) part = fmaf(gt[i], a[i], part);
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          if ((t & 31) == 0) red[4 * kN + (t >> 5)] = part;
+          ns::ns_sync();
+          float S = 0.f;
+#pragma unroll
+          for (int w = 0; w < kComputeThreads / 32; ++w) S += red[4 * kN + w];
+          const float craw = nrm.n1 * nrm.ninf, cden = fmaxf(craw, 1e-12f);
+          const bool clamped = !(craw > 1e-12f);
+          const float col_term = clamped ? 0.f : -S * nrm.ninf / (cden * cden);
+          const float row_term = clamped ? 0.f : -S * nrm.n1 / (cden * cden);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float sg = a[i] > 0.f ? 1.f : (a[i] < 0.f ? -1.f : 0.f);
+            float x = v[i] + gt[i] / cden;
+            if (c.col0 + i == nrm.jc) x += sg * col_term;
+            if (c.row == nrm.ir) x += sg * row_term;
+            v[i] = (c.row < m && c.col0 + i < m) ? x : 0.f;
+            g[i] = a[i];
+          }
+          if (ridge) {
+            // dL/dK2 = (what kRidgeK2 left) + K2 (dA + dA^T)
+            put_row16(c, c.slot(5), v);
+            load_row16(c, p.k2 + bh * mm_, m, m, m, g);
+            put_row16(c, c.slot(6), g);
+            arrive = 0;
+            next = kTailK2;
+          } else {
+            jacobian = true;
+          }
+          break;
+        }
+        case kTailK2: {
+          float e[16];
+          load_row16(c, p.spill + bh * mm_, m, m, m, e);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = (c.row < m && c.col0 + i < m) ? v[i] + e[i] : 0.f;
+          jacobian = true;
+          break;
+        }
+        case kDQ:
+          if (!c.failed) store_row16(c, p.dqt_ns + bh * md + half * kN, v, m, min(D, kN), D);
+          next = kDK;
+          break;
+        default: {                                       // kDK
+          const int64_t off = bh * md + half * kN;
+          ++half;
+          if (c.failed) break;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] += z[i];
+          store_row16(c, p.dkt_tot + off, v, m, min(D, kN), D);
+          if (p.rows_k && c.row < m) {
+            Segments sg(p.N, m);
+            const float fk = p.scale / (float)sg.len(c.row);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] *= fk;
+            store_row16(c, p.rows_k + off, v, m, min(D, kN), D);
+          }
+          break;
+        }
+      }
+      if (jacobian && f.dK2) {
+        if (!c.failed) store_row16(c, f.dK2 + bh * mm_, v, m, m, m);
+        jacobian = false;
+      } else if (jacobian) {
+        // softmax-2: dS2 = K2 o (dK2 - rowsum(dK2 o K2)); g holds K2
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s = fmaf(v[i], g[i], s);
+        red[c.row * 4 + (c.col0 >> 4)] = s;
+        ns::ns_sync();
+        s = (red[4 * c.row] + red[4 * c.row + 1]) + (red[4 * c.row + 2] + red[4 * c.row + 3]);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = g[i] * (v[i] - s);
+        put_row16(c, c.slot(5), v);
+      }
+      if (jacobian || (step == kDK && half < finish)) {
+        put_tile16(c.slot(6), hd);                       // Kt, Qt
+        put_tile16(c.slot(7), r);
+        arrive = 0;
+        next = kDQ;
+      }
+      if (arrive >= 0) arrive_ready(c, arrive);
+      if (next < 0) break;
+      step = next;
+    }
+    if (phase) break;
+
+    // ---- the iterations; j = J only forms R, W, Y of Z_{J-1}, j = 0 needs none ----
+#pragma unroll 1
+    for (int j = J; j >= 0; --j) {
+      const int par = (J - 1 - j) & 1;
+      const bool main_part = j < J, prime = j > 0;
+      if (main_part) {
+        if (prime) {
+          put_tile16(c.slot(2 - par), z);                // Z_{j-1}: every product that read this slot is complete
+          arrive_ready(c, 2);
+          if (j > 1) load_tile16(iterates + (size_t)(j - 2) * mm_, m, m, m, z);
+        }
+        take(c, 0, 3 * kAccCols, c.slot(7), c.act, v, c.trunc);   // dY
+        if (c.act) put_row16(c, c.slot(7), v);
+        arrive_ready(c, 3);
+        take(c, 1, 2 * kAccCols, c.slot(8), c.act, v, c.trunc);   // H
+        if (c.act) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) { v[i] *= 0.25f; hd[i] = v[i]; }
+          put_row16(c, c.slot(8), v);
+        }
+        arrive_ready(c, 4);
+      }
+      if (prime) {
+        take(c, 2, kAccCols, c.slot(4 - par), c.act, v, c.trunc); // R of the next lower iterate
+        if (c.act) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = -v[i];
+          add_diag(c, r, 1.f, m);
+          put_row16(c, c.slot(4 - par), r);
+        }
+        arrive_ready(c, 5);
+      }
+      if (main_part) {
+        take(c, 3, 0, c.slot(5 + par), c.act, v, c.trunc);        // D
+        if (c.act) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = -fmaf(4.f, hd[i], v[i]);
+          put_row16(c, c.slot(5 + par), v);
+        }
+        arrive_ready(c, 6);
+      }
+      if (prime) {
+        take(c, 4, kAccCols, c.slot(7), c.act, v, c.trunc);       // W
+        if (c.act) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = fmaf(0.25f, v[i], r[i]);
+          add_diag(c, v, 1.f, m);
+          put_row16(c, c.slot(7), v);
+        }
+        if (!main_part) arrive_ready(c, 0);
+      }
+      if (main_part) {
+        take(c, 5, 3 * kAccCols, c.slot(6 - par), c.act, v, c.trunc);   // G
+        if (c.act) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) g[i] += v[i];
+          if (prime) put_row16(c, c.slot(6 - par), g);
+        }
+        if (prime) arrive_ready(c, 0);
+      }
+      if (prime) {
+        take(c, 6, 2 * kAccCols, c.slot(8), c.act, v, c.trunc);   // Y
+        if (c.act) put_row16(c, c.slot(8), v);
+        arrive_ready(c, 1);
+      }
+      if (main_part) {
+        wait_done(c, 7, 0x2107);                         // dL/dA
+        if (c.act) {
+          float keep[16], send[16];
+          fetch(c, 0, c.trunc, keep, send);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) { da_keep[i] += keep[i]; da_send[i] += send[i]; }
+        }
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kNsTcThreads, 1) ns_bwd_tc_kernel(BwdParams f, int finish, int* status) {
   extern __shared__ uint8_t dyn_smem[];
-#ifdef FNB_NS_TRACE
-  if (threadIdx.x == 0 && blockIdx.x < 64) g_ns_span[2 * blockIdx.x] = global_ns();
-#endif
   __shared__ float red[ns::kRedFloats];
   __shared__ Shared sh;
   Ctx c;
-  NS_TRACE();
   pdl_trigger();
-  ctx_open(c, sh, dyn_smem, kBwdSlots, status, kBwdTmemCols);
+  ctx_open(c, sh, dyn_smem, status, kBwdTmemCols, f.p.m);
   pdl_wait();
-  NS_TRACE();
-  const int64_t bh = blockIdx.x;
-  const int m = p.m, mm_ = m * m;
-  const int finish_tc = p.D == NH * kN ? NH : 0;   // batches of the finishing step
-  const bool head = h.partA != nullptr;      // fused middle stage (head_dim 64 only)
-  if (is_compute()) {
-    float z[16], a[16];
-    load_global16(p.iterates + (bh * (size_t)(p.J + 1) + p.J - 1) * mm_, m, m, m, z);
-    load_global16(p.k2 + bh * mm_, m, m, m, a);
-    if (head) bwd_head_tc(c, red, p, h, bh);
-    FinishOperands fo;
-    float* dK2 = pinv_backward_tc(c, red, p.k2 + bh * mm_, p.iterates + bh * (size_t)(p.J + 1) * mm_,
-                                  head ? nullptr : p.G + bh * mm_,
-                                  p.spill + bh * mm_, m, p.J, p.kappa, [&] { if (finish_tc) finish_load(c, p, bh, 0, fo); }, z, a);
-    NS_TRACE();
-    if (finish_tc) ns_bwd_finish_tc<NH>(c, p, bh, bwd_tail(c, 0), dK2, fo);
-    else if (!c.failed) ns::ns_bwd_finish(p, bh, bwd_tail(c, 0), dK2);
-    NS_TRACE();
-  } else if (is_issuer()) {
-    pinv_backward_issue(c, p.J, finish_tc, head);
-  }
+  if (is_compute()) bwd_compute(c, red, f, blockIdx.x, finish);
+  else bwd_issue(c, f, finish);
   ctx_close(c, kBwdTmemCols);
-  NS_TRACE();
-#ifdef FNB_NS_TRACE
-  if (threadIdx.x == 0 && blockIdx.x < 64) g_ns_span[2 * blockIdx.x + 1] = global_ns();
-#endif
 }
 
 }  // namespace nstc

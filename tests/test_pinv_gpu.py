@@ -61,6 +61,34 @@ def test_pinv_forward_and_backward(cuda_device, m, J, kappa):
         assert O.rel_max(dk2, ref[0]) < 5e-4, "d_k2"
 
 
+@pytest.mark.parametrize("D", [16, 64, 128])
+@pytest.mark.parametrize("m", [15, 17, 31, 32, 47, 48, 49, 63, 64])
+@pytest.mark.parametrize("kappa", [0.0, 5.0])
+def test_tensor_core_pinv_no_less_precise_than_cuda_cores(cuda_device, m, D, kappa):
+    """Edges of the 16-wide K steps and of the 32 x 32 blocks, the three head_dim forms of the scores and of the landmark
+    gradients.  Both kernels against the oracle in float64 on the same landmarks and incoming gradients; the bound is twice
+    the CUDA cores' own error (three bf16 terms hold an FP32 value, accumulation has FP32's rounding) plus one FP32 ulp."""
+    from flashnystrom_b200 import _C
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 3, 4 * m + 5, D, seed=m + D, dtype=torch.float32))
+    err = {}
+    for generic in (False, True):
+        _C.set_force_generic(generic)
+        try:
+            r = _C.forward(q, k, v, m, 6, kappa)
+            g = _C.backward(dO, *r[1:13], v, r[0], m, 6, True, kappa)
+        finally:
+            _C.set_force_generic(False)
+        _C.check_device_status()
+        with torch.device("cuda"):
+            d = [t.double() for t in (q, k, v, dO)]
+            f = O.forward(*d[:3], m, 6, kappa)
+            f.update(O.backward(*d, m, 6, kappa, fwd=f))
+        got = {"K2": r[11], "k2inv": r[5], "dq": g[0], "dk": g[1]}
+        err[generic] = {n: float((t.double() - f[n]).norm() / f[n].norm()) for n, t in got.items()}
+    for n in err[True]:
+        assert err[False][n] <= 2 * err[True][n] + 2.0 ** -23, (n, err)
+
+
 def test_pinv_same_call_twice_is_bit_identical(cuda_device):
     from flashnystrom_b200 import _C
     k2 = _softmax_matrix(4, 64, seed=1).cuda()
