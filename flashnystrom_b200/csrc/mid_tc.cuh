@@ -1,6 +1,6 @@
 // Landmark-sized stages for 64 < num_landmarks <= 128 on the sm_100a tensor cores, FP32-equivalent: a
 // thread-block cluster of two CTAs per (b,h) slice works through the softmax-2, ridge and Newton-Schulz
-// products (forward and exact backward) of mid_kernels.cuh.
+// products (forward and exact backward).
 //
 // Every matrix that is an operand exists once as an "image" in global memory (it stays in L2): three bf16
 // terms x = x0 + x1 + x2 (24 significant bits), padded with zeros to 128 x 128, already in the 128-byte
@@ -19,12 +19,12 @@
 // `ready` barriers; operands that are older than the last phase are copied ahead of it.  All waits are
 // bounded; control flow never depends on them.
 //
-// What bounds it: the latency of a phase, about 9000 cycles with one product (result block out to L2 2000-2400,
-// meeting the peer 800, first chunk in 1550, MMAs 2400, accumulator out and split 2300), not the 144 KB a CTA copies
-// per product (ncu: tensor pipe active 13 to 18 %, DRAM idle).  Clusters of four or eight that copied FP32 operands and split
-// them in every CTA took, on a B200 at B=2, H=8 (us, before / now): forward D=128, J=8 with ridge 326 / 222, D=64, J=6 without
-// 234 / 164; backward 651 / 443 and 478 / 316; per iteration 37 / 19 and 70 / 37.  One to eight slices of head_dim 128,
-// training pass: 705 .. 820 / 526 .. 643.
+// The iteration runs in its residual form (ns_tc_kernels.cuh): with R = I - A Z three dependent phases in place of four.
+//
+// What bounds it: shared-memory bandwidth under the products (an MMA set of a K step reads 24 KB and its copies write 9, 2350 of
+// ideally 1670 cycles per product) and what a phase waits for: the result block out to L2 (put 1600, publish 2300), the peer,
+// the first chunk in (1550).  Measured at B=2, H=8, m=128 (us, nested form issued by one lane / this): forward D=128, J=8 with
+// ridge 222 / 205, D=64, J=6 without 164 / 152; backward 447 / 408 and 318 / 289.
 #pragma once
 #include "common.cuh"
 #include "small_kernels.cuh"
@@ -50,16 +50,20 @@ constexpr int kF32 = kMaxM * kMaxM;            // floats of one FP32 scratch mat
 
 // scratch of a cluster: images, then FP32 matrices.  A launch has at most as many clusters as run at once; each walks slices
 // gridDim.x / 2 apart and works in one scratch area, so that the scratch stays in L2 and does not grow with the slices.
-enum FwdImg { kFK2, kFA, kFZ0, kFZ1, kFM, kFV, kFT, kFwdImgs };
+enum FwdImg { kFK2, kFA, kFZ0, kFZ1, kFR, kFW, kFY, kFwdImgs };
 constexpr size_t kFwdScratchBytes = (size_t)kFwdImgs * kImg + kF32 * sizeof(float);
-enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBdZ0, kBdZ1, kBM, kBV, kBT, kBdT, kBdV, kBdM, kBwdImgs };
+enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBZ2, kBG0, kBG1, kBR0, kBR1, kBW, kBY, kBdY, kBH, kBwdImgs };
 enum BwdF32 { kGA, kGdZ, kGdK, kGg, kBwdF32s };
 constexpr size_t kBwdScratchBytes = (size_t)kBwdImgs * kImg + (size_t)kBwdF32s * kF32 * sizeof(float);
+
+// Share of a leading partial product that its truncating additions (three per group of four K steps) have lost on the average.
+// Given back, K2inv is 0.45 to 0.98 times as far from the oracle as in the nested form, without it up to 1.17 times.
+constexpr float kTrunc = 0x1.8p-25f;
 
 enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
 
 struct Shared {
-  uint64_t full[kStages], empty[kStages], done[2], ready, drain;
+  uint64_t full[kStages], empty[kStages], done[2], released[2], ready, drain;
   uint32_t tmem_slot;
   uint32_t fills;           // stages filled by the copying warp, written when it is through
   int abort_word;
@@ -164,6 +168,76 @@ __device__ __forceinline__ void set_row(float* g, int c0, int cols, bool row_ok,
   }
 }
 
+// The MMAs of one K chunk (64): warp-uniform code, one elected lane issues.  One block of assembly, so that the election
+// happens once and the descriptors stay in uniform registers: issued from a single lane an MMA took 103 cycles, a product
+// 2900, and the issuing warp bounded the backward.  d: accumulator, l: left chunk, r: right chunk.
+template <bool LT, bool RT>
+__device__ __forceinline__ void issue_chunk(uint32_t d, uint32_t l, uint32_t r, bool second, bool accumulate) {
+  const uint64_t a = LT ? smem_desc_sw128(l, kTermBytes / 2, 1024) : smem_desc_sw128(l, 16, 1024);
+  const uint64_t b = RT ? smem_desc_sw128(r, 16, 1024) : smem_desc_sw128(r, kTermBytes / 2, 1024);
+  constexpr uint32_t i192 = make_idesc<__nv_bfloat16>(128, 192, LT, !RT), i128 = make_idesc<__nv_bfloat16>(128, 128, LT, !RT),
+                     i64 = make_idesc<__nv_bfloat16>(128, 64, LT, !RT);
+  constexpr int sa = LT ? 2048 / 16 : 2, sb = RT ? 2 : 2048 / 16, ta = kTermBytes / 16, tb = kTermBytes / 32;
+  if (!second) {
+    asm volatile(
+          "{\n\t.reg .pred e, p, q;\n\t.reg .b64 a0, a1, a2, b, b1;\n\t.reg .b32 d1, d2, d3;\n\t"
+          "elect.sync _|e, 0xffffffff;\n\t"
+          "setp.ne.b32 p, %3, 0;\n\t"
+          "setp.eq.b32 q, %3, %3;\n\t"
+          "add.u32 d1, %0, 64;\n\tadd.u32 d2, %0, 128;\n\tadd.u32 d3, %0, 192;\n\t"
+          "mov.b64 a0, %1;\n\tadd.s64 a1, %1, %9;\n\tadd.s64 a2, a1, %9;\n\tmov.b64 b, %2;\n\tadd.s64 b1, %2, %10;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b, %4, p;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b, %4, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b, %4, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b, %4, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "}"
+          ::"r"(d), "l"(a), "l"(b), "r"(accumulate ? 1u : 0u), "r"(i192), "r"(i128), "r"(i64), "n"(sa), "n"(sb), "n"(ta), "n"(tb)
+          : "memory");
+  } else {
+    // b1: the second term of the right operand, its columns 0..127 then being y1 | y2
+    asm volatile(
+          "{\n\t.reg .pred e, p, q;\n\t.reg .b64 a0, a1, a2, b, b1;\n\t.reg .b32 d1, d2, d3;\n\t"
+          "elect.sync _|e, 0xffffffff;\n\t"
+          "setp.ne.b32 p, %3, 0;\n\t"
+          "setp.eq.b32 q, %3, %3;\n\t"
+          "add.u32 d1, %0, 64;\n\tadd.u32 d2, %0, 128;\n\tadd.u32 d3, %0, 192;\n\t"
+          "mov.b64 a0, %1;\n\tadd.s64 a1, %1, %9;\n\tadd.s64 a2, a1, %9;\n\tmov.b64 b, %2;\n\tadd.s64 b1, %2, %10;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d3], a0, b, %6, p;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a0, b1, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\tadd.s64 b1, b1, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d3], a0, b, %6, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a0, b1, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\tadd.s64 b1, b1, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d3], a0, b, %6, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a0, b1, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "add.s64 a0, a0, %7;\n\tadd.s64 a1, a1, %7;\n\tadd.s64 a2, a2, %7;\n\tadd.s64 b, b, %8;\n\tadd.s64 b1, b1, %8;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d3], a0, b, %6, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a0, b1, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d1], a1, b, %5, q;\n\t"
+          "@e tcgen05.mma.cta_group::1.kind::f16 [d2], a2, b, %6, q;\n\t"
+          "}"
+          ::"r"(d), "l"(a), "l"(b), "r"(accumulate ? 1u : 0u), "r"(i192), "r"(i128), "r"(i64), "n"(sa), "n"(sb), "n"(ta), "n"(tb)
+          : "memory");
+  }
+}
+
 // One role's walk through the program.
 template <int R>
 struct Role {
@@ -183,6 +257,7 @@ struct Role {
   // compute: accumulator row, column segment of 16 (over both blocks), completion parities
   int row, seg;
   uint32_t dphase[2];
+  uint32_t relphase[2];     // issue: parity of the next wait on released[]
 
   __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status, bool drop_fill) {
     drop = drop_fill;
@@ -191,7 +266,7 @@ struct Role {
     ab = Abort{&s->abort_word, status};
     failed = pend = false;
     rphase = sphase = fills = 0; stage = 0;
-    dphase[0] = dphase[1] = 0;
+    dphase[0] = dphase[1] = relphase[0] = relphase[1] = 0;
     const int w = threadIdx.x >> 5;
     row = (w & 3) * 32 + lane;
     seg = rank * 4 + (w >> 2);
@@ -202,7 +277,9 @@ struct Role {
     if (R == kCompute && read_peer && !pend) __threadfence();
     if (!pend) return;
     pend = false;
-    if (R == kCompute || lane == 0) {
+    if (R == kIssuer) {
+      settle(wait_cluster(&sh->ready, rphase, ab, 0x6000 + R));
+    } else if (R == kCompute || lane == 0) {
       if (!wait_cluster(&sh->ready, rphase, ab, 0x6000 + R)) failed = true;
       if (R == kProducer) fence_proxy_async_all();
       if (R == kCompute && read_peer) __threadfence();
@@ -282,42 +359,23 @@ struct Role {
         }
       }
     } else if (R == kIssuer) {
-      if (lane == 0) {
-        ensure();
-        const uint32_t d = tmem + acc * kAccCols;
-        for (int kc = 0; kc < kchunks; ++kc) {
-          if (!failed && !mbar_wait(&sh->full[stage], sphase, ab, 0x6020)) failed = true;
-          if (!failed) {
-            tc_fence_after();
-            const uint32_t l = smem_u32(ring) + stage * kStageBytes, r = l + kBlockBytes;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t b = RT ? smem_desc_sw128(r + k * 32, 16, 1024) : smem_desc_sw128(r + k * 2048, kTermBytes / 2, 1024);
-              // the tile of the second term of the right operand, its columns 0..127 then being y1 | y2
-              const uint64_t b1 = b + ((kTermBytes / 2) >> 4);
-              uint64_t a[3];
-#pragma unroll
-              for (int t = 0; t < 3; ++t) {
-                const uint32_t lt = l + t * kTermBytes;
-                a[t] = LT ? smem_desc_sw128(lt + k * 2048, kTermBytes / 2, 1024) : smem_desc_sw128(lt + k * 32, 16, 1024);
-              }
-              if (kc == 0) {
-                umma(d, a[0], b, make_idesc<__nv_bfloat16>(128, 192, LT, !RT), (accumulate || k > 0) ? 1u : 0u);
-              } else {
-                umma(d + 192, a[0], b, make_idesc<__nv_bfloat16>(128, 64, LT, !RT), (accumulate || k > 0) ? 1u : 0u);
-                umma(d + 64, a[0], b1, make_idesc<__nv_bfloat16>(128, 128, LT, !RT), 1u);
-              }
-              umma(d + 64, a[1], b, make_idesc<__nv_bfloat16>(128, 128, LT, !RT), 1u);
-              umma(d + 128, a[2], b, make_idesc<__nv_bfloat16>(128, 64, LT, !RT), 1u);
-            }
-            umma_commit(&sh->empty[stage]);
-          }
-          advance();
+      ensure();
+      const uint32_t d = tmem + acc * kAccCols;
+      for (int kc = 0; kc < kchunks; ++kc) {
+        settle(failed || mbar_wait(&sh->full[stage], sphase, ab, 0x6020));
+        if (!failed) {
+          tc_fence_after();
+          const uint32_t l = smem_u32(ring) + stage * kStageBytes;
+          issue_chunk<LT, RT>(d, l, l + kBlockBytes, kc > 0, accumulate);
+          umma_commit_elect(&sh->empty[stage]);
         }
-      } else {
-        if (pend) { pend = false; rphase ^= 1u; }
+        advance();
       }
     }
+  }
+  // issue: the warp goes on as one
+  __device__ __forceinline__ void settle(bool ok) {
+    if (!__all_sync(0xffffffffu, ok)) failed = true;
   }
   __device__ __forceinline__ void advance() {
     if (++stage == kStages) { stage = 0; sphase ^= 1u; }
@@ -342,11 +400,11 @@ struct Role {
     for (int t = 0; t < 3; ++t) bulk_load(dst + t * (kTermBytes / 2), src + t * kTermBytes, kTermBytes / 2, &sh->full[stage]);
   }
   __device__ __forceinline__ void commit(int g) {
-    if (R == kIssuer && lane == 0 && !failed) umma_commit(&sh->done[g]);
+    if (R == kIssuer && !failed) umma_commit_elect(&sh->done[g]);
   }
   // compute: the 16 values of this thread (row, columns 16 seg ..) of accumulator acc once group g is complete;
   // kchunks as in product()
-  __device__ __forceinline__ void result(int g, int acc, float* v, int kchunks = 2) {
+  __device__ __forceinline__ void result(int g, int acc, float* v, int kchunks = 2, float trunc = kTrunc) {
     if (!mbar_wait(&sh->done[g], dphase[g], ab, 0x6030 + g)) failed = true;
     dphase[g] ^= 1u;
     __syncwarp();
@@ -366,7 +424,22 @@ struct Role {
       for (int i = 0; i < 16; ++i) v[i] += y[i];
     }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] += x[i];
+    for (int i = 0; i < 16; ++i) v[i] += fmaf(trunc, v[i], x[i]);
+  }
+  // An accumulator that is used again within a phase: the compute warps release it once it has been read, the issuing
+  // warp waits for that (as often as it is released).
+  __device__ __forceinline__ void release(int acc) {
+    if (R == kCompute) {
+      tc_fence_before();
+      mbar_arrive_warp(&sh->released[acc]);
+    }
+  }
+  __device__ __forceinline__ void reuse(int acc) {
+    if (R == kIssuer) {
+      settle(failed || mbar_wait(&sh->released[acc], relphase[acc], ab, 0x6040 + acc));
+      relphase[acc] ^= 1u;
+      tc_fence_after();
+    }
   }
   __device__ __forceinline__ int col0() const { return 16 * seg; }
   __device__ __forceinline__ void add_diag(float* v, float d, int m) const {
@@ -466,14 +539,14 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
   float v[16];
   if (p.qt) {
     if (C) {
-      r.convert(p.qt + bh * m * D, m, D, img(kFM));
-      r.convert(p.kt + bh * m * D, m, D, img(kFV));
+      r.convert(p.qt + bh * m * D, m, D, img(kFR));
+      r.convert(p.kt + bh * m * D, m, D, img(kFW));
     }
     r.publish(true);
-    r.template product<false, true>(img(kFM), true, img(kFV), true, (D + 63) / 64, 0, false);
+    r.template product<false, true>(img(kFR), true, img(kFW), true, (D + 63) / 64, 0, false);
     r.commit(0);
     if (C) {
-      r.result(0, 0, v, (D + 63) / 64);
+      r.result(0, 0, v, (D + 63) / 64, 0.f);
       set_row<16>(k2 + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
     }
     r.publish(true);
@@ -532,45 +605,49 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
     set_row<16>(iterates + (size_t)row * m, 16 * s, m, row < m, v);
   }
   r.publish(true);
+  // R = I - A Z, then Y = Z R and W = I + R + R^2 / 4 side by side, then Z' = Z + Y W
+  float z[16], rv[16];
+  if (C) {
+    r.ensure();
+    get_row<16>(iterates + (size_t)r.row * m, r.col0(), m, r.row < m, z);
+  }
   for (int j = 0; j < p.J; ++j) {
     uint8_t* Z = img(kFZ0 + (j & 1));
     uint8_t* Zn = img(kFZ0 + ((j + 1) & 1));
-    float mv[16];
-    r.template product<false, false>(A, false, Z, true, 2, 0, false);           // M = A Z
+    r.template product<false, false>(A, j == 0, Z, true, 2, 0, false);
     r.commit(0);
     if (C) {
-      r.result(0, 0, mv);
-      r.put(img(kFM), mv);
-    }
-    r.publish(false);
-    r.template product<false, false>(img(kFM), true, img(kFM), true, 2, 0, false);
-    r.commit(0);
-    if (C) {
-      r.result(0, 0, v);                                                        // V = 15 I - M (7 I - M)
+      r.result(0, 0, rv);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, mv[i], v[i]);
-      r.add_diag(v, 15.f, m);
-      r.put(img(kFV), v);
+      for (int i = 0; i < 16; ++i) rv[i] = -rv[i];
+      r.add_diag(rv, 1.f, m);
+      r.put(img(kFR), rv);
     }
     r.publish(false);
-    r.template product<false, false>(img(kFM), false, img(kFV), true, 2, 0, false);
+    r.template product<false, false>(Z, false, img(kFR), true, 2, 0, false);
     r.commit(0);
+    r.template product<false, false>(img(kFR), true, img(kFR), true, 2, 1, false);
+    r.commit(1);
     if (C) {
-      r.result(0, 0, v);                                                        // T / 4 = (13 I - M V) / 4
+      r.result(0, 0, v);
+      r.put(img(kFY), v);
+      r.result(1, 1, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
-      r.add_diag(v, 3.25f, m);
-      r.put(img(kFT), v);
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(0.25f, v[i], rv[i]);
+      r.add_diag(v, 1.f, m);
+      r.put(img(kFW), v);
     }
     r.publish(false);
-    r.template product<false, false>(Z, false, img(kFT), true, 2, 0, false);    // Z' = Z T / 4
+    r.template product<false, false>(img(kFY), true, img(kFW), true, 2, 0, false);
     r.commit(0);
     if (C) {
       r.result(0, 0, v);
-      r.put(Zn, v);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) z[i] += v[i];
+      if (j < p.J - 1 || p.kappa > 0.f) r.put(Zn, z);
       const bool ok = r.row < m && !r.failed;
-      set_row<16>(iterates + (size_t)(j + 1) * mm + (size_t)r.row * m, r.col0(), m, ok, v);
-      if (j == p.J - 1 && !(p.kappa > 0.f)) set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, ok, v);
+      set_row<16>(iterates + (size_t)(j + 1) * mm + (size_t)r.row * m, r.col0(), m, ok, z);
+      if (j == p.J - 1 && !(p.kappa > 0.f)) set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, ok, z);
     }
     r.publish(false);
   }
@@ -615,22 +692,22 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
   const float* iterates = p.iterates + bh * (int64_t)(J + 1) * mm;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool own_d = r.rank * 64 < D;          // this CTA has columns of an (m x D) result
-  uint8_t* Gi = ridge ? img(kBdM) : img(kBdZ0 + (J & 1));   // dL/dk2inv; without the ridge it is dL/dZ_J
+  uint8_t* Gi = ridge ? img(kBH) : img(kBG0 + (J & 1));     // dL/dk2inv; without the ridge it is dL/dZ_J
   float v[16];
   if (p.head) {
     const float* dstep2 = p.sums + bh * 2 * md;
     float* dO3 = p.dO3 + bh * md;
     if (C) {
-      r.convert(p.k2inv + bh * mm, m, m, img(kBM));
-      r.convert(dstep2, m, D, img(kBT));
-      r.convert(p.bmat + bh * md, m, D, img(kBV));
+      r.convert(p.k2inv + bh * mm, m, m, img(kBR0));
+      r.convert(dstep2, m, D, img(kBR1));
+      r.convert(p.bmat + bh * md, m, D, img(kBW));
     }
     r.publish(true);
     if (own_d) {
-      r.template product<true, false>(img(kBM), true, img(kBT), true, 2, 0, false);       // dO3 = K2inv^T dstep2
+      r.template product<true, false>(img(kBR0), true, img(kBR1), true, 2, 0, false);     // dO3 = K2inv^T dstep2
       r.commit(0);
     }
-    r.template product<false, true>(img(kBT), true, img(kBV), true, (D + 63) / 64, 1, false);   // dK2inv = dstep2 Bmat^T
+    r.template product<false, true>(img(kBR1), true, img(kBW), true, (D + 63) / 64, 1, false);  // dK2inv = dstep2 Bmat^T
     r.commit(1);
     if (C) {
       if (own_d) {
@@ -639,6 +716,7 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
       }
       r.result(1, 1, v, (D + 63) / 64);
       r.put(Gi, v);
+      set_row<16>(f32(kGdZ) + (size_t)r.row * m, r.col0(), m, r.row < m, v);     // (read back by this thread, maybe in a launch of its own)
     }
     r.publish(true);
     if (C) {
@@ -658,16 +736,19 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
   if (C) {
     if (p.G) r.convert(p.G + bh * mm, m, m, Gi);
     r.convert(k2, m, m, img(kBK2));
-    r.convert(iterates + (size_t)(J - 1) * mm, m, m, img(kBZ0 + ((J - 1) & 1)));
-    if (ridge) r.convert(iterates + (size_t)J * mm, m, m, img(kBT));
+    r.convert(iterates + (size_t)(J - 1) * mm, m, m, img(kBZ0 + (J - 1) % 3));
+    if (J > 1) r.convert(iterates + (size_t)(J - 2) * mm, m, m, img(kBZ0 + (J - 2) % 3));
+    if (ridge) r.convert(iterates + (size_t)J * mm, m, m, img(kBY));
   }
   r.publish(true);
   const uint8_t* A = img(kBK2);
   const float* A32 = k2;
+  float g[16];                                    // dL/dZ of the iterate above
+  if (C && !ridge) get_row<16>((p.G ? p.G + bh * mm : f32(kGdZ)) + (size_t)r.row * m, r.col0(), m, r.row < m, g);
   if (ridge) {
     r.template product<true, false>(img(kBK2), true, img(kBK2), true, 2, 0, false);
     r.commit(0);
-    r.template product<true, false>(Gi, true, img(kBT), true, 2, 1, false);          // G^T Z_J
+    r.template product<true, false>(Gi, true, img(kBY), true, 2, 1, false);          // G^T Z_J
     r.commit(1);
     if (C) {
       const Norms nk = norms(k2, m, r.red);
@@ -682,86 +763,125 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
     r.template product<false, false>(Gi, false, img(kBK2), false, 2, 0, false);      // dL/dZ_J = G K2
     r.commit(0);
     if (C) {
-      r.result(0, 0, v);
-      r.put(img(kBdZ0 + (J & 1)), v);
+      r.result(0, 0, g);
+      r.put(img(kBG0 + (J & 1)), g);
     }
     r.publish(false);
     A = img(kBA);
     A32 = f32(kGA);
   }
-  // Per iteration, with dT = Z^T dZ / 4, dV = -M^T dT, dU = -M^T dV and U = 7 I - M:
-  //   1:  M = A Z                                       | ndT = -Z^T dZ / 4
-  //   2:  V = 15 I - 7 M + M M                          | dV = M^T ndT
-  //   3:  dM = ndT V^T + dV M^T + M^T dV - 7 dV         | qT = (13 I - M V) / 4
-  //   4:  dZ' = dZ qT^T + A^T dM                        | dA += dM Z^T  (registers)
-  float dA[16];
+  // Per iteration, with R = I - A Z, W = I + R + R^2 / 4, Y = Z R, Z' = Z + Y W and G = dL/dZ':
+  //   1:  dY = G W^T | H = Y^T G / 4 | R of the next lower iterate
+  //   2:  D = -(Z^T dY + H R^T + R^T H + 4 H) (over G) | its R^2, for W
+  //   3:  its Y | dL/dZ = G + dY R^T + A^T D | dL/dA += D Z^T (registers, read in the next phase)
+  // j = J only forms R, W, Y of Z_{J-1}.  Z_{j-2} is converted in phase 2: three images, since the one it goes to was last
+  // copied in the phase before.
+  float dA[16], rv[16], hd[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) dA[i] = 0.f;
-  for (int j = J - 1; j >= 0; --j) {
-    uint8_t* Z = img(kBZ0 + (j & 1));
-    uint8_t* dZ = img(kBdZ0 + ((j + 1) & 1));
-    float mv[16], dv[16];
-    r.template product<false, false>(A, j == J - 1, Z, j == J - 1, 2, 0, false);
-    r.commit(0);
-    r.template product<true, false>(Z, false, dZ, true, 2, 1, false);
-    r.commit(1);
-    if (C) {
-      r.ensure();
-      if (j > 0) r.convert(iterates + (size_t)(j - 1) * mm, m, m, img(kBZ0 + ((j + 1) & 1)));
-      r.result(0, 0, mv);
-      r.put(img(kBM), mv);
-      r.result(1, 1, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
-      r.put(img(kBdT), v);
+  for (int j = J; j >= 0; --j) {
+    const bool main_part = j < J, prime = j > 0;
+    uint8_t *Z = img(kBZ0 + j % 3), *Zn = img(kBZ0 + (j + 2) % 3);
+    uint8_t *Rj = img(kBR0 + (j & 1)), *Rn = img(kBR0 + ((j + 1) & 1)), *G = img(kBG0 + ((j + 1) & 1)), *Gn = img(kBG0 + (j & 1));
+    if (main_part) {
+      r.template product<false, true>(G, true, img(kBW), true, 2, 1, false);
+      r.commit(1);
+      if (j < J - 1) r.reuse(0);
+      r.template product<true, false>(img(kBY), true, G, true, 2, 0, false);
+      r.commit(0);
+      if (prime) r.reuse(1);
     }
-    r.publish(j > 0);
-    r.template product<false, false>(img(kBM), true, img(kBM), true, 2, 0, false);
-    r.commit(0);
-    r.template product<true, false>(img(kBM), true, img(kBdT), true, 2, 1, false);
-    r.commit(1);
-    if (C) {
-      r.result(0, 0, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, mv[i], v[i]);
-      r.add_diag(v, 15.f, m);
-      r.put(img(kBV), v);
-      r.result(1, 1, dv);
-      r.put(img(kBdV), dv);
+    if (prime) {
+      r.template product<false, false>(A, !main_part, Zn, true, 2, 1, false);
+      r.commit(1);
     }
-    r.publish(false);
-    r.template product<false, false>(img(kBM), false, img(kBV), true, 2, 0, false);
-    r.commit(0);
-    r.template product<false, true>(img(kBdT), false, img(kBV), true, 2, 1, false);
-    r.template product<false, true>(img(kBdV), true, img(kBM), false, 2, 1, true);
-    r.template product<true, false>(img(kBM), false, img(kBdV), true, 2, 1, true);
-    r.commit(1);
     if (C) {
-      r.result(0, 0, v);
+      if (main_part) {
+        if (j < J - 1) {
+          r.result(0, 0, v);
+          r.release(0);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] *= -0.25f;
-      r.add_diag(v, 3.25f, m);
-      r.put(img(kBT), v);
-      r.result(1, 1, v);
+          for (int i = 0; i < 16; ++i) dA[i] += v[i];
+        }
+        r.result(1, 1, v);
+        if (prime) r.release(1);
+        r.put(img(kBdY), v);
+        r.result(0, 0, hd);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fmaf(-7.f, dv[i], v[i]);
-      r.put(img(kBdM), v);
+        for (int i = 0; i < 16; ++i) hd[i] *= 0.25f;
+        r.put(img(kBH), hd);
+      }
+      if (prime) {
+        r.result(1, 1, rv);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) rv[i] = -rv[i];
+        r.add_diag(rv, 1.f, m);
+        r.put(Rn, rv);
+      }
     }
     r.publish(false);
-    r.template product<false, true>(dZ, false, img(kBT), true, 2, 0, false);
-    r.template product<true, false>(A, false, img(kBdM), true, 2, 0, true);
-    r.commit(0);
-    r.template product<false, true>(img(kBdM), true, Z, false, 2, 1, false);
-    r.commit(1);
-    if (C) {
-      r.result(0, 0, v);
-      if (j > 0) r.put(img(kBdZ0 + (j & 1)), v);
-      else set_row<16>(f32(kGdZ) + (size_t)r.row * m, r.col0(), m, r.row < m, v);
-      r.result(1, 1, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) dA[i] += v[i];
+    if (main_part) {
+      r.template product<true, false>(Z, false, img(kBdY), true, 2, 0, false);
+      r.template product<false, true>(img(kBH), true, Rj, false, 2, 0, true);
+      r.template product<true, false>(Rj, false, img(kBH), true, 2, 0, true);
+      r.commit(0);
     }
-    r.publish(j == 0);
+    if (prime) {
+      r.template product<false, false>(Rn, true, Rn, true, 2, 1, false);
+      r.commit(1);
+    }
+    if (main_part) {
+      if (C) {
+        r.ensure(false);
+        if (j > 1) r.convert(iterates + (size_t)(j - 2) * mm, m, m, img(kBZ0 + (j + 1) % 3));
+        r.result(0, 0, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = -fmaf(4.f, hd[i], v[i]);
+        r.put(G, v);
+      }
+      r.publish(false);
+    }
+    if (C && prime) {
+      r.result(1, 1, v);
+      if (main_part) r.release(1);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(0.25f, v[i], rv[i]);
+      r.add_diag(v, 1.f, m);
+      r.put(img(kBW), v);
+    }
+    if (prime) {
+      r.template product<false, false>(Zn, false, Rn, !main_part, 2, 0, false);
+      r.commit(0);
+    }
+    if (main_part) {
+      if (prime) r.reuse(1);
+      r.template product<false, true>(img(kBdY), false, Rj, false, 2, 1, false);
+      r.template product<true, false>(A, false, G, true, 2, 1, true);
+      r.commit(1);
+      if (prime) r.reuse(0);
+      r.template product<false, true>(G, true, Z, false, 2, 0, false);
+      r.commit(0);
+    }
+    if (C) {
+      if (prime) {
+        r.result(0, 0, v);
+        if (main_part) r.release(0);
+        r.put(img(kBY), v);
+      }
+      if (main_part) {
+        r.result(1, 1, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) g[i] += v[i];
+        if (prime) r.put(Gn, g);
+        else {
+          set_row<16>(f32(kGdZ) + (size_t)r.row * m, r.col0(), m, r.row < m, g);
+          r.result(0, 0, v);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) dA[i] += v[i];
+        }
+      }
+    }
+    r.publish(j > 1 || j == 0);
   }
   // Z0 = A^T / c with c = ||A||_1 ||A||_inf; S = sum_{a,b} dZ0[a,b] A[b,a]
   if (C) {
@@ -814,10 +934,10 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
         const int cc = 16 * s + i;
         v[i] = (row < m && cc < m) ? __ldcg(out32 + (size_t)row * m + cc) + __ldcg(out32 + (size_t)cc * m + row) : 0.f;
       }
-      put16(img(kBT), row, s, v);
+      put16(img(kBY), row, s, v);
     }
     r.publish(true);
-    r.template product<false, false>(img(kBK2), false, img(kBT), true, 2, 0, false);
+    r.template product<false, false>(img(kBK2), false, img(kBY), true, 2, 0, false);
     r.commit(0);
     if (C) {
       r.result(0, 0, v);
@@ -843,16 +963,16 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
 #pragma unroll
       for (int q = 0; q < 4; ++q) x[q] = k[q] * (x[q] - s);
-      put_row(img(kBM), row, lane, x);
+      put_row(img(kBR0), row, lane, x);
     }
-    r.convert(p.kt + bh * md, m, D, img(kBV));
-    r.convert(p.qt + bh * md, m, D, img(kBdV));
+    r.convert(p.kt + bh * md, m, D, img(kBW));
+    r.convert(p.qt + bh * md, m, D, img(kBdY));
   }
   r.publish(true);
   if (own_d) {
-    r.template product<false, false>(img(kBM), true, img(kBV), true, 2, 0, false);
+    r.template product<false, false>(img(kBR0), true, img(kBW), true, 2, 0, false);
     r.commit(0);
-    r.template product<true, false>(img(kBM), true, img(kBdV), true, 2, 1, false);
+    r.template product<true, false>(img(kBR0), true, img(kBdY), true, 2, 1, false);
     r.commit(1);
     if (C) {
       const size_t off = (size_t)bh * md + (size_t)r.row * D;
@@ -904,6 +1024,8 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
     for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
     mbar_init(&sh->done[0], 1);
     mbar_init(&sh->done[1], 1);
+    mbar_init(&sh->released[0], kComputeWarps);
+    mbar_init(&sh->released[1], kComputeWarps);
     mbar_init(&sh->drain, 1);
     mbar_init(&sh->ready, 2 * (kComputeWarps + 2));
     sh->abort_word = 0;
@@ -934,8 +1056,8 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
         if (n) mbar_drain(&sh->full[s], (n - 1) & 1u);
       }
     }
-    if (threadIdx.x == 32 * (kComputeWarps + 1)) {
-      umma_commit(&sh->drain);
+    if (warp == kComputeWarps + 1) {
+      umma_commit_elect(&sh->drain);       // (from the lane that issued)
       mbar_drain(&sh->drain, 0);
     }
     __syncthreads();

@@ -61,6 +61,14 @@ def test_pinv_forward_and_backward(cuda_device, m, J, kappa):
         assert O.rel_max(dk2, ref[0]) < 5e-4, "d_k2"
 
 
+@pytest.mark.parametrize("m", [33, 65, 127, 128])
+@pytest.mark.parametrize("J,kappa", [(1, 0.0), (2, 0.0), (3, 0.0), (1, 5.0), (2, 5.0)])
+def test_pinv_few_iterations(cuda_device, m, J, kappa):
+    """One to three iterations: the backward forms R, W and Y one iterate ahead and (past 64 landmarks) rotates three images
+    of the iterates.  Bounds as in test_pinv_forward_and_backward."""
+    test_pinv_forward_and_backward(cuda_device, m, J, kappa)
+
+
 @pytest.mark.parametrize("D", [16, 64, 128])
 @pytest.mark.parametrize("m", [15, 17, 31, 32, 47, 48, 49, 63, 64])
 @pytest.mark.parametrize("kappa", [0.0, 5.0])
