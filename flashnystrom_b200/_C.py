@@ -34,6 +34,7 @@ def set_force_generic(on: bool):
     """Route 16-bit inputs through the CUDA-core FP32 kernels too (verification aid)."""
     global _flags
     _flags = (_flags | _lib.FNB_FLAG_FORCE_GENERIC) if on else (_flags & ~_lib.FNB_FLAG_FORCE_GENERIC)
+    native().set_flags(_flags)
 
 
 def set_test_drop_load(on: bool):
@@ -41,6 +42,7 @@ def set_test_drop_load(on: bool):
     a bounded device-side wait runs out (see FNB_FLAG_TEST_DROP_LOAD)."""
     global _flags
     _flags = (_flags | _lib.FNB_FLAG_TEST_DROP_LOAD) if on else (_flags & ~_lib.FNB_FLAG_TEST_DROP_LOAD)
+    native().set_flags(_flags)
 
 
 def set_wait_limit_ms(ms: int, device=0):
@@ -263,6 +265,40 @@ def _print_bwd_debug(dev, **tensors):
         print(f"[FNB_BWD_DEBUG] {name}: absmax={st['absmax']:.4e} absmean={st['absmean']:.4e} "
               f"nonfinite={st['nonfinite']}")
     check_device_status(dev)
+
+
+# ---- the eager path ---------------------------------------------------------------------------------------
+_native = None
+
+
+def native():
+    """The C++ module that the eager calls go through."""
+    global _native
+    if _native is None:
+        mod = _lib.native()
+        mod.set_flags(_flags)
+        mod.set_debug(lambda dO, dq, dk, dv, step2, k2inv: _print_bwd_debug(dO.device, dO=dO, dQ=dq, dK=dk, dV=dv, step2=step2,
+                                                                            k2inv=k2inv))
+        _native = mod
+    return _native
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def being_transformed():
+    """A trace or a functorch transform is under way."""
+    return torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
+
+
+def attention(q, k, v, num_landmarks, newton_iter, kappa_star, weight=None):
+    """Attention (and the convolution residual) through the C++ module, differentiable; None for a call that is not plainly one of
+    plain tensors and numbers, which then takes the autograd functions of flash_nystrom.py."""
+    if (type(q) in _PLAIN and type(k) in _PLAIN and type(v) in _PLAIN and type(num_landmarks) is int and type(newton_iter) is int
+            and (type(kappa_star) is float or type(kappa_star) is int) and (weight is None or type(weight) in _PLAIN)
+            and not being_transformed()):
+        return native().attention(q, k, v, num_landmarks, newton_iter, kappa_star, weight, _status(q.device))
+    return None
 
 
 # ---- the autograd function's path -----------------------------------------------------------------------

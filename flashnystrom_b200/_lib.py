@@ -4,11 +4,13 @@ The shared library is built in-tree (flashnystrom_b200/lib/).  Loading never fal
 another implementation: if the library is missing and cannot be built, import of the
 compute entry points raises."""
 import ctypes as C
+import importlib.util
 import os
 import threading
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libflashnystrom_b200.so")
+NATIVE_PATH = os.path.join(_PKG, "lib", "_native.so")
 
 FNB_F32, FNB_F16, FNB_BF16 = 0, 1, 2
 FNB_FLAG_FORCE_GENERIC = 1
@@ -142,6 +144,27 @@ def load(build_if_missing=True):
             fn.argtypes = args
         _lib = lib
         return lib
+
+
+_native = None
+
+
+def native():
+    """The C++ module of the eager path (csrc/native.cpp), built first if it is absent."""
+    global _native
+    if _native is not None:
+        return _native
+    load()
+    with _lock:
+        if _native is None:
+            if not os.path.exists(NATIVE_PATH):
+                from . import build as _build
+                _build.build_native()
+            spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _native = module
+    return _native
 
 
 def last_error():

@@ -7,6 +7,16 @@ import torch.nn.functional as F
 from . import _C
 from .nystrom_config import NystromConfig
 
+_LINEAR_FORWARD = nn.Linear.forward
+_ANY_GLOBAL_HOOK = torch.nn.modules.module._has_any_global_hook
+
+
+def _plain_linear(p):
+    """p is torch's own bias-free linear and nothing watches or changes what it does."""
+    return (type(p) is nn.Linear and p.bias is None and "forward" not in p.__dict__ and type(p.weight) is nn.Parameter
+            and not (p._forward_hooks or p._forward_pre_hooks or p._backward_hooks or p._backward_pre_hooks))
+
+
 # The reference sets HAS_CUDA when its extension imports (flash_nystrom/__init__.py:38-46).  Here
 # the library is the only implementation: the flag says whether it can run on this machine.
 HAS_CUDA = bool(torch.cuda.is_available())
@@ -92,6 +102,10 @@ def flash_nystrom_attention(q, k, v, num_landmarks=64, newton_iter=6, conv_weigh
         from . import _ops
         out = _ops.attention_via_ops(q, k, v, num_landmarks, newton_iter, kappa_star)
     else:
+        out = _C.attention(q, k, v, num_landmarks, newton_iter, kappa_star,
+                           conv_weight if conv_weight is not None and conv_kernel_size > 0 else None)
+        if out is not None:
+            return out
         out = FlashNystromFunction.apply(q, k, v, num_landmarks, newton_iter, fast_dk2inv,
                                          kappa_star, use_tc_pinv)
     if conv_weight is not None and conv_kernel_size > 0:
@@ -125,7 +139,28 @@ class FlashNystromAttention(nn.Module):
         else:
             self.conv_weight = None
 
+    def _native_forward(self, x):
+        """The whole block through the C++ module, or None: projections that are more than four plain linears, and calls
+        that something traces or transforms, take the way below."""
+        cfg, conv = self.config, self.conv_weight
+        if not (type(x) is torch.Tensor and x.is_cuda and torch._C._len_torch_function_stack() == 0
+                and not _C.being_transformed() and nn.Linear.forward is _LINEAR_FORWARD and not _ANY_GLOBAL_HOOK()
+                and _plain_linear(self.q_proj) and _plain_linear(self.k_proj) and _plain_linear(self.v_proj)
+                and _plain_linear(self.out_proj) and type(cfg.num_landmarks) is int and type(cfg.newton_iter) is int
+                and (type(cfg.kappa_star) is float or type(cfg.kappa_star) is int)):
+            return None
+        if conv is None or cfg.conv_kernel_size <= 0:
+            conv = None
+        elif type(conv) is not nn.Parameter:
+            return None
+        return _C.native().module_forward(x, self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.out_proj.weight,
+                                          self.heads, cfg.num_landmarks, cfg.newton_iter, cfg.kappa_star, conv, _C._status(x.device))
+
     def forward(self, x):
+        if not torch.compiler.is_compiling():
+            y = self._native_forward(x)
+            if y is not None:
+                return y
         B, N, _ = x.shape
         H, D = self.heads, self.head_dim
         # Head-split views of the projection outputs, no transposing copies: where the tensor-core
