@@ -252,6 +252,31 @@ __device__ __forceinline__ void unstage_col16(const Ctx& c, const float* X, floa
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = X[(c.col0 + i) * kLd + c.row];
 }
+// A staged matrix -> the leading rows x cols block of a dense global matrix, whole sectors per instruction.  (From the
+// accumulator layout, 32 rows of 16 bytes per instruction, the store of an iterate kept the warps for 1700 cycles, this takes 400.)
+__device__ __forceinline__ void store_staged(const float* X, float* g, int rows, int cols, int ld) {
+  if (((ld | cols) & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
+    const int r = threadIdx.x >> 2;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = 16 * q + 4 * (threadIdx.x & 3);
+      if (r < rows && c < cols) *reinterpret_cast<float4*>(g + (size_t)r * ld + c) = *reinterpret_cast<const float4*>(X + r * kLd + c);
+    }
+  } else {
+#pragma unroll 4
+    for (int i = 0; i < 8; ++i) {
+      const int r = (threadIdx.x >> 5) + 8 * i, c = threadIdx.x & 31;
+      if (r < rows && c < cols) g[(size_t)r * ld + c] = X[r * kLd + c];
+      if (r < rows && c + 32 < cols) g[(size_t)r * ld + c + 32] = X[r * kLd + c + 32];
+    }
+  }
+}
+// x / c with rc = 1 / c: a product and one correction of its remainder (Markstein 1990), correctly rounded but for results near
+// the underflow threshold
+__device__ __forceinline__ float div_by(float x, float c, float rc) {
+  const float q = x * rc;
+  return fmaf(fmaf(-q, c, x), rc, q);
+}
 // d on the diagonal of the leading m x m block
 __device__ __forceinline__ void add_diag(const Ctx& c, float* v, float d, int m) {
 #pragma unroll
@@ -454,22 +479,11 @@ __device__ inline void softmax16(float* X, const ns::NsFwdParams& p, int64_t bh)
   sum = part[0];
   sum += __shfl_xor_sync(0xffffffffu, sum, 2);
   sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  const float rsum = 1.f / sum;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) row[4 * i + k] = r < m ? v[i] / sum : 0.f;
+  for (int i = 0; i < 16; ++i) row[4 * i + k] = r < m ? div_by(v[i], sum, rsum) : 0.f;
   __syncwarp();                              // a row's four lanes are in one warp
-  if (r < m) {
-    const int c0 = 16 * k;
-    float* g = p.k2 + bh * m * m + (size_t)r * m + c0;
-    if ((m & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (c0 + 4 * q < m) *reinterpret_cast<float4*>(g + 4 * q) = *reinterpret_cast<const float4*>(row + c0 + 4 * q);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) if (c0 + i < m) g[i] = row[c0 + i];
-    }
-    if (k == 0) p.lse2[bh * m + r] = mx + logf(sum);
-  }
+  if (r < m && k == 0) p.lse2[bh * m + r] = mx + logf(sum);
   ns::ns_sync();
 }
 
@@ -530,7 +544,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
   float* k2 = p.k2 + bh * mm_;
   float z[16], r[16], v[16];       // Z_j, R and the value in hand
 #pragma unroll
-  for (int i = 0; i < 16; ++i) { r[i] = 0.f; v[i] = 0.f; }
+  for (int i = 0; i < 16; ++i) { r[i] = 0.f; v[i] = 0.f; }       // (inactive warps keep zeros)
   if (f.k2_given) {
     load_tile16(k2, m, m, m, v);
     stage_tile16(X, v);
@@ -550,18 +564,25 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
         r[0] = n.n1 * n.ninf / p.kappa;                    // lambda
         put_row16(c, c.slot(2), v);
       } else {
-        const float cden = fmaxf(n.n1 * n.ninf, 1e-12f);
+        const float cden = fmaxf(n.n1 * n.ninf, 1e-12f), rcden = 1.f / cden;
         put_row16(c, c.slot(0), v);
         unstage_col16(c, X, z);                            // Z0 = A^T / cden
 #pragma unroll
-        for (int i = 0; i < 16; ++i) z[i] /= cden;
+        for (int i = 0; i < 16; ++i) z[i] = div_by(z[i], cden, rcden);
         put_row16(c, c.slot(1), z);
       }
       arrive_ready(c, 0);
-      if (s == 0 && c.act && !c.failed) store_row16(c, iterates, z, m, m, m);
+      // to global memory beside the product: K2 first, Z0 (staged over it) below
+      if (!f.k2_given && !c.failed && (s == -1 || !ridge)) store_staged(X, k2, m, m, m);
+      if (s == 0) {
+        ns::ns_sync();
+        stage_row16(c, X, z);
+      }
     }
     if (s >= 0 && s < 4 * J) {
-      // one iteration; R, then Y and W, then Z'
+      // one iteration; R, then Y and W, then Z'.  Z_j is staged in X (slot 3, free until Y) and leaves while the product runs.
+      ns::ns_sync();
+      if (!c.failed) store_staged(X, iterates + (size_t)(s >> 2) * mm_, m, m, m);
       take(c, 0, 0, c.slot(2), c.act, v, c.trunc);
       if (c.act) {
 #pragma unroll
@@ -591,16 +612,23 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
         if (ridge && end) put_row16(c, c.slot(0), r);
       }
       if (!end || ridge) arrive_ready(c, 0);
-      if (c.act && !c.failed) {
-        store_row16(c, iterates + (size_t)((s >> 2) + 1) * mm_, z, m, m, m);
-        if (end && !ridge) store_row16(c, p.k2inv + bh * mm_, z, m, m, m);
+      stage_row16(c, X, z);
+      if (end) {
+        ns::ns_sync();
+        if (!c.failed) {
+          store_staged(X, iterates + (size_t)J * mm_, m, m, m);
+          if (!ridge) store_staged(X, p.k2inv + bh * mm_, m, m, m);
+        }
       }
       continue;
     }
     // scores (s = -2), K2^T K2 (s = -1), k2inv (s = 4J)
     take(c, s & 1, (s & 1) * kAccCols, c.slot(s == -1 ? 0 : 2), c.act, v, s == -2 ? kTruncScores : c.trunc);
     if (s == 4 * J) {
-      if (c.act && !c.failed) store_row16(c, p.k2inv + bh * mm_, v, m, m, m);
+      ns::ns_sync();
+      stage_row16(c, X, v);
+      ns::ns_sync();
+      if (!c.failed) store_staged(X, p.k2inv + bh * mm_, m, m, m);
       break;
     }
     if (!c.act) {
@@ -777,7 +805,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
   const bool ridge = p.kappa > 0.f, head = h.partA != nullptr;
   const float* iterates = p.iterates + bh * (size_t)(f.step_dz ? 1 : J + 1) * mm_;
   float* X = c.stage(3);
-  float v[16], g[16], hd[16], r[16], da_keep[16], da_send[16], z[16];
+  float v[16], g[16], da_keep[16], da_send[16], z[16], hd[16], r[16];
   float lam = 0.f;
   Norms nrm;
   // ---- operands ----
@@ -841,12 +869,17 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
     for (;;) {
       // global operands of this step or of the batch after it, ahead of the wait
       if (step == kHeadO3 && h.D3) load_row16(c, p.qt + bh * md, m, kN, kN, hd);
-      if (step == kDQ) load_row16(c, p.dkt_a + bh * md + half * kN, m, min(D, kN), D, z);
-      if (step == kSumDA || step == kDQ) {
-        const int hn = step == kDQ ? half + 1 : 0;
-        if (hn < finish) {
-          load_tile16(p.kt + bh * md + hn * kN, m, min(D, kN), D, hd);
-          load_tile16(p.qt + bh * md + hn * kN, m, min(D, kN), D, r);
+      if (step == kDQ) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {                    // dkt_a, as store_staged walks a matrix
+          const int rr = t >> 2, cc = 16 * q + 4 * (t & 3);
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (rr < m && cc < min(D, kN)) x = *reinterpret_cast<const float4*>(p.dkt_a + bh * md + (size_t)rr * D + half * kN + cc);
+          z[4 * q] = x.x; z[4 * q + 1] = x.y; z[4 * q + 2] = x.z; z[4 * q + 3] = x.w;
+        }
+        if (half + 1 < finish) {
+          load_tile16(p.kt + bh * md + (half + 1) * kN, m, min(D, kN), D, hd);
+          load_tile16(p.qt + bh * md + (half + 1) * kN, m, min(D, kN), D, r);
         }
       }
       // slot that the result goes to (or a free one to add the lane halves in), accumulator, done barrier
@@ -973,14 +1006,14 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           float S = 0.f;
 #pragma unroll
           for (int w = 0; w < kComputeThreads / 32; ++w) S += red[4 * kN + w];
-          const float craw = nrm.n1 * nrm.ninf, cden = fmaxf(craw, 1e-12f);
+          const float craw = nrm.n1 * nrm.ninf, cden = fmaxf(craw, 1e-12f), rcden = 1.f / cden;
           const bool clamped = !(craw > 1e-12f);
           const float col_term = clamped ? 0.f : -S * nrm.ninf / (cden * cden);
           const float row_term = clamped ? 0.f : -S * nrm.n1 / (cden * cden);
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float sg = a[i] > 0.f ? 1.f : (a[i] < 0.f ? -1.f : 0.f);
-            float x = v[i] + gt[i] / cden;
+            float x = v[i] + div_by(gt[i], cden, rcden);
             if (c.col0 + i == nrm.jc) x += sg * col_term;
             if (c.row == nrm.ir) x += sg * row_term;
             v[i] = (c.row < m && c.col0 + i < m) ? x : 0.f;
@@ -1007,23 +1040,28 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           break;
         }
         case kDQ:
-          if (!c.failed) store_row16(c, p.dqt_ns + bh * md + half * kN, v, m, min(D, kN), D);
+          stage_row16(c, c.stage(1), v);
+          ns::ns_sync();
+          if (!c.failed) store_staged(c.stage(1), p.dqt_ns + bh * md + half * kN, m, min(D, kN), D);
           next = kDK;
           break;
         default: {                                       // kDK
-          const int64_t off = bh * md + half * kN;
-          ++half;
-          if (c.failed) break;
+          stage_row16(c, c.stage(2), v);
+          ns::ns_sync();
+          const int rr = t >> 2;
+          const float fk = p.rows_k ? p.scale / (float)Segments(p.N, m).len(min(rr, m - 1)) : 0.f;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] += z[i];
-          store_row16(c, p.dkt_tot + off, v, m, min(D, kN), D);
-          if (p.rows_k && c.row < m) {
-            Segments sg(p.N, m);
-            const float fk = p.scale / (float)sg.len(c.row);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] *= fk;
-            store_row16(c, p.rows_k + off, v, m, min(D, kN), D);
+          for (int q = 0; q < 4; ++q) {
+            const int cc = 16 * q + 4 * (t & 3);
+            if (rr < m && cc < min(D, kN) && !c.failed) {
+              float4 x = *reinterpret_cast<const float4*>(c.stage(2) + rr * kLd + cc);
+              x.x += z[4 * q]; x.y += z[4 * q + 1]; x.z += z[4 * q + 2]; x.w += z[4 * q + 3];
+              const size_t off = (size_t)bh * md + (size_t)rr * D + half * kN + cc;
+              *reinterpret_cast<float4*>(p.dkt_tot + off) = x;
+              if (p.rows_k) *reinterpret_cast<float4*>(p.rows_k + off) = make_float4(x.x * fk, x.y * fk, x.z * fk, x.w * fk);
+            }
           }
+          ++half;
           break;
         }
       }
@@ -1094,6 +1132,10 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           put_row16(c, c.slot(5 + par), v);
         }
         arrive_ready(c, 6);
+        if (!prime && finish > 0) {                      // the first operands of the landmark gradients, ahead of time
+          load_tile16(p.kt + bh * md, m, min(D, kN), D, hd);
+          load_tile16(p.qt + bh * md, m, min(D, kN), D, r);
+        }
       }
       if (prime) {
         take(c, 4, kAccCols, c.slot(7), c.act, v, c.trunc);       // W
