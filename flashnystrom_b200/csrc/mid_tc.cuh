@@ -2,7 +2,8 @@
 // thread-block cluster of two CTAs per (b,h) slice works through the softmax-2, ridge and Newton-Schulz
 // products (forward and exact backward).
 //
-// Every matrix that is an operand exists once as an "image" in global memory (it stays in L2): three bf16
+// Outside the forward iteration, which keeps its operands on the chip (fwd_program), every matrix that is an operand exists
+// once as an "image" in global memory (it stays in L2): three bf16
 // terms x = x0 + x1 + x2 (24 significant bits), padded with zeros to 128 x 128, already in the 128-byte
 // swizzle the tensor core reads, [64-column block][term][128 rows x 128 B].  The epilogue that forms a result
 // splits it once and writes its image; a consumer's operands are plain bulk copies into a ring of shared-
@@ -21,10 +22,12 @@
 //
 // The iteration runs in its residual form (ns_tc_kernels.cuh): with R = I - A Z three dependent phases in place of four.
 //
-// What bounds it: shared-memory bandwidth under the products (an MMA set of a K step reads 24 KB and its copies write 9, 2350 of
-// ideally 1670 cycles per product) and what a phase waits for: the result block out to L2 (put 1600, publish 2300), the peer,
-// the first chunk in (1550).  Measured at B=2, H=8, m=128 (us, nested form issued by one lane / this): forward D=128, J=8 with
-// ridge 222 / 205, D=64, J=6 without 164 / 152; backward 447 / 408 and 318 / 289.
+// What bounds it: forward, the products of an iteration (four, 2400 cycles each: shared-memory bandwidth, an MMA set of a K step
+// reads 24 KB) and between them the way of a result through registers, split and shared memory (2500 cycles, three times);
+// backward, the same with what a phase waits for: copies out of L2 (9 KB per K step), the result block out to it (put 1600,
+// publish 2300), the peer, the first chunk in (1550).  Measured at B=2, H=8, m=128 (us): forward D=128, J=8 with
+// ridge 222 with four products in a row, 205 in residual form through L2, 128 with the operands on the chip; D=64, J=6 without
+// 164, 152, 94; backward 447 / 408 and 318 / 289.
 #pragma once
 #include "common.cuh"
 #include "small_kernels.cuh"
@@ -43,14 +46,14 @@ constexpr int kStages = 2;
 constexpr int kStageBytes = kBlockBytes + kBlockBytes / 2;   // left chunk (128 x 64) and right chunk (64 x 64), all terms
 constexpr int kComputeWarps = 16;
 constexpr int kThr = 32 * (kComputeWarps + 2);
-constexpr int kRedFloats = 17 * kMaxM;
-constexpr size_t kSmem = (size_t)kStages * kStageBytes + kBlockBytes + kRedFloats * sizeof(float) + 128 + 1024;
+constexpr int kRedFloats = 64 * kMaxM;          // 17 kMaxM for norms(); the forward iteration stages 64 columns of an iterate
+constexpr size_t kSmem = (size_t)kStages * kStageBytes + kBlockBytes + kRedFloats * sizeof(float) + 256 + 1024;
 constexpr int kAccCols = 256;                  // tensor-memory columns of one accumulator
 constexpr int kF32 = kMaxM * kMaxM;            // floats of one FP32 scratch matrix
 
 // scratch of a cluster: images, then FP32 matrices.  A launch has at most as many clusters as run at once; each walks slices
 // gridDim.x / 2 apart and works in one scratch area, so that the scratch stays in L2 and does not grow with the slices.
-enum FwdImg { kFK2, kFA, kFZ0, kFZ1, kFR, kFW, kFY, kFwdImgs };
+enum FwdImg { kFK2, kFA, kFZ0, kFR, kFW, kFwdImgs };
 constexpr size_t kFwdScratchBytes = (size_t)kFwdImgs * kImg + kF32 * sizeof(float);
 enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBZ2, kBG0, kBG1, kBR0, kBR1, kBW, kBY, kBdY, kBH, kBwdImgs };
 enum BwdF32 { kGA, kGdZ, kGdK, kGg, kBwdF32s };
@@ -64,7 +67,11 @@ enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
 
 struct Shared {
   uint64_t full[kStages], empty[kStages], done[2], released[2], ready, drain;
+  // forward iteration: products complete in both CTAs; result blocks written here; blocks that came from the peer; slots loaded
+  uint64_t both[2], put, came[3], loaded[3];
   uint32_t tmem_slot;
+  uint32_t loads[3];        // loads of each slot, written when the issuing warp is through
+  uint32_t inbound[4][3];   // copies that the peer has sent here, likewise
   uint32_t fills;           // stages filled by the copying warp, written when it is through
   int abort_word;
 };
@@ -171,13 +178,15 @@ __device__ __forceinline__ void set_row(float* g, int c0, int cols, bool row_ok,
 // The MMAs of one K chunk (64): warp-uniform code, one elected lane issues.  One block of assembly, so that the election
 // happens once and the descriptors stay in uniform registers: issued from a single lane an MMA took 103 cycles, a product
 // 2900, and the issuing warp bounded the backward.  d: accumulator, l: left chunk, r: right chunk.
-template <bool LT, bool RT>
+// RS: bytes between the terms of the right chunk.
+template <bool LT, bool RT, int RS = kTermBytes / 2>
 __device__ __forceinline__ void issue_chunk(uint32_t d, uint32_t l, uint32_t r, bool second, bool accumulate) {
   const uint64_t a = LT ? smem_desc_sw128(l, kTermBytes / 2, 1024) : smem_desc_sw128(l, 16, 1024);
-  const uint64_t b = RT ? smem_desc_sw128(r, 16, 1024) : smem_desc_sw128(r, kTermBytes / 2, 1024);
+  const uint64_t b = RT ? smem_desc_sw128(r, 16, 1024) : smem_desc_sw128(r, RS, 1024);
+  static_assert(!RT || RS == 64 * 128, "the rows of all terms are one operand");
   constexpr uint32_t i192 = make_idesc<__nv_bfloat16>(128, 192, LT, !RT), i128 = make_idesc<__nv_bfloat16>(128, 128, LT, !RT),
                      i64 = make_idesc<__nv_bfloat16>(128, 64, LT, !RT);
-  constexpr int sa = LT ? 2048 / 16 : 2, sb = RT ? 2 : 2048 / 16, ta = kTermBytes / 16, tb = kTermBytes / 32;
+  constexpr int sa = LT ? 2048 / 16 : 2, sb = RT ? 2 : 2048 / 16, ta = kTermBytes / 16, tb = RS / 16;
   if (!second) {
     asm volatile(
           "{\n\t.reg .pred e, p, q;\n\t.reg .b64 a0, a1, a2, b, b1;\n\t.reg .b32 d1, d2, d3;\n\t"
@@ -258,6 +267,7 @@ struct Role {
   int row, seg;
   uint32_t dphase[2];
   uint32_t relphase[2];     // issue: parity of the next wait on released[]
+  uint32_t bphase[2], pphase, cphase[3], lphase[3], loads[3], sent[3];     // forward iteration: parities, loads and copies issued
 
   __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status, bool drop_fill) {
     drop = drop_fill;
@@ -266,7 +276,8 @@ struct Role {
     ab = Abort{&s->abort_word, status};
     failed = pend = false;
     rphase = sphase = fills = 0; stage = 0;
-    dphase[0] = dphase[1] = relphase[0] = relphase[1] = 0;
+    dphase[0] = dphase[1] = relphase[0] = relphase[1] = bphase[0] = bphase[1] = pphase = 0;
+    for (int i = 0; i < 3; ++i) cphase[i] = lphase[i] = loads[i] = sent[i] = 0;
     const int w = threadIdx.x >> 5;
     row = (w & 3) * 32 + lane;
     seg = rank * 4 + (w >> 2);
@@ -407,6 +418,9 @@ struct Role {
   __device__ __forceinline__ void result(int g, int acc, float* v, int kchunks = 2, float trunc = kTrunc) {
     if (!mbar_wait(&sh->done[g], dphase[g], ab, 0x6030 + g)) failed = true;
     dphase[g] ^= 1u;
+    take(acc, v, kchunks, trunc);
+  }
+  __device__ __forceinline__ void take(int acc, float* v, int kchunks = 2, float trunc = kTrunc) const {
     __syncwarp();
     tc_fence_after();
     const uint32_t a = tmem + (uint32_t)acc * kAccCols + ((uint32_t)(row & ~31) << 16) + (uint32_t)((seg & 3) * 16);
@@ -441,6 +455,102 @@ struct Role {
       tc_fence_after();
     }
   }
+  // ---- forward iteration: operands stay in four blocks of shared memory ("slots", where ring and staging are otherwise)
+  __device__ __forceinline__ uint32_t slot(int i) const { return smem_u32(ring) + i * kBlockBytes; }
+  // every product issued before is complete in both CTAs
+  __device__ __forceinline__ void wait_both(int g) {
+    const bool ok = mbar_wait(&sh->both[g], bphase[g], ab, 0x6050 + g);
+    if (R == kIssuer) settle(failed || ok);
+    else if (!ok) failed = true;
+    bphase[g] ^= 1u;
+  }
+  __device__ __forceinline__ void commit_both(int g) {
+    if (!failed)
+      asm volatile(
+          "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+          "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+          ::"r"(smem_u32(&sh->both[g])), "h"((uint16_t)3)
+          : "memory");
+  }
+  // compute: this thread's 16 values -> its place in slot i
+  __device__ __forceinline__ void put_slot(int i, const float* v) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint4 w[3];
+      sx::split8<3>(v + 8 * c, w);
+      uint8_t* p = ring + (size_t)i * kBlockBytes + sw128_offset(row, (seg & 3) * 2 + c);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) *reinterpret_cast<uint4*>(p + t * kTermBytes) = w[t];
+    }
+    fence_proxy_async();
+  }
+  // for the issuing warp: the blocks put so far are there
+  __device__ __forceinline__ void announce() {
+    tc_fence_before();
+    mbar_arrive_warp(&sh->put);
+  }
+  // the block put into slot `from` -> slot `to` of the peer.  The four warps that hold the same 32 rows have them copied in bulk
+  // by one thread: stored from the registers (32 rows x 16 B per instruction) a block took 3000 cycles.
+  __device__ __forceinline__ void send(int from, int to, int what) {
+    const int q = (threadIdx.x >> 5) & 3;
+    named_barrier(2 + q, 128);
+    if (threadIdx.x < 128 && lane == 0 && !failed) {
+      uint32_t dst, bar;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(slot(to) + q * 4096), "r"(rank ^ 1));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&sh->came[what])), "r"(rank ^ 1));
+      asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(3 * 4096) : "memory");
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(dst + t * kTermBytes), "r"(slot(from) + q * 4096 + t * kTermBytes), "r"(4096), "r"(bar) : "memory");
+      ++sent[what];
+    }
+  }
+  // this thread's 16 values -> staged row (64 columns, 16-byte words swizzled); after a barrier of the four warps of these
+  // rows (send() has one), the staged rows -> an (m x m) matrix.  Stored from the accumulator layout (32 rows x 16 B per
+  // instruction) an iterate took 3500 cycles, and everything behind it waited.
+  __device__ __forceinline__ void stage_rows(const float* v) {
+    float4* dst = reinterpret_cast<float4*>(red) + row * 16;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dst[((seg & 3) * 4 + q) ^ (row & 15)] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  }
+  __device__ __forceinline__ void store_rows(float* g, int m) const {
+    const int w = threadIdx.x >> 5, c = lane & 15;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int rr = (w & 3) * 32 + (w >> 2) * 8 + 2 * i + (lane >> 4);
+      const float4 x = reinterpret_cast<const float4*>(red)[rr * 16 + (c ^ (rr & 15))];
+      const float v[4] = {x.x, x.y, x.z, x.w};
+      set_row<4>(g + (size_t)rr * m, rank * 64 + 4 * c, m, rr < m && !failed, v);
+    }
+  }
+  __device__ __forceinline__ void row_sync() { named_barrier(2 + ((threadIdx.x >> 5) & 3), 128); }
+  // issue
+  __device__ __forceinline__ void wait_put() {
+    settle(failed || mbar_wait(&sh->put, pphase, ab, 0x6060));
+    pphase ^= 1u;
+    tc_fence_after();
+  }
+  __device__ __forceinline__ void wait_came(int what) {
+    settle(failed || wait_cluster(&sh->came[what], cphase[what], ab, 0x6070 + what));
+    cphase[what] ^= 1u;
+  }
+  __device__ __forceinline__ void wait_loaded(int l) {
+    settle(failed || mbar_wait(&sh->loaded[l], lphase[l], ab, 0x6080 + l));
+    lphase[l] ^= 1u;
+  }
+  // may the next load be issued?  (lane 0 issues it)
+  __device__ __forceinline__ bool begin_load(int l, uint32_t bytes) {
+    if (drop && loads[0] + loads[1] + loads[2] == 2) failed = true;     // fault injection on the host's request
+    if (failed) return false;
+    ++loads[l];
+    if (lane == 0) mbar_expect_tx(&sh->loaded[l], bytes);
+    return lane == 0;
+  }
+  template <bool RT = false, int RS = kTermBytes>
+  __device__ __forceinline__ void chunk(int acc, uint32_t left, uint32_t right, bool second) {
+    if (!failed) issue_chunk<false, RT, RS>(tmem + acc * kAccCols, left, right, second, false);
+  }
   __device__ __forceinline__ int col0() const { return 16 * seg; }
   __device__ __forceinline__ void add_diag(float* v, float d, int m) const {
 #pragma unroll
@@ -457,6 +567,14 @@ struct Role {
   __device__ void close() {
     ensure();
     if (R == kProducer && lane == 0) sh->fills = fills;
+    if (R == kIssuer && lane == 0)
+      for (int i = 0; i < 3; ++i) sh->loads[i] = loads[i];
+    if (R == kCompute && threadIdx.x < 128 && lane == 0)       // (the peer counts on these copies until they have arrived)
+      for (int i = 0; i < 3; ++i) {
+        uint32_t at;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&sh->inbound[threadIdx.x >> 5][i])), "r"(rank ^ 1));
+        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at), "r"(sent[i]) : "memory");
+      }
   }
 };
 
@@ -605,57 +723,123 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
     set_row<16>(iterates + (size_t)row * m, 16 * s, m, row < m, v);
   }
   r.publish(true);
-  // R = I - A Z, then Y = Z R and W = I + R + R^2 / 4 side by side, then Z' = Z + Y W
+  // R = I - A Z, then Y = Z R and W = I + R + R^2 / 4 side by side, then Z' = Z + Y W.  All operands are on the chip: a
+  // block of 64 columns is left operand (K) and right operand (columns) from the same place, a CTA's own block needs no
+  // exchange, and the products begin with it; the peer's block, needed on the left only, arrives behind them from the peer's
+  // shared memory.  So no phase waits for the L2.  Slots: 0, 1 hold Z, then Y (own block, peer's); 2, 3 hold R
+  // (W in 2), and before that the two blocks of A, which come from its image while Z' is formed.  A slot is written again
+  // after the products that read it are complete in BOTH CTAs (commits arrive in both).
+  constexpr bool I = R == kIssuer;
+  const bool ridge = p.kappa > 0.f;
+  const int own = r.rank, peer = r.rank ^ 1;
+  enum { kFromR, kFromY, kFromZ };
+  constexpr uint32_t half = kTermBytes / 2;       // 64 rows of a block
   float z[16], rv[16];
-  if (C) {
-    r.ensure();
-    get_row<16>(iterates + (size_t)r.row * m, r.col0(), m, r.row < m, z);
+  r.ensure();
+  if (C) get_row<16>(iterates + (size_t)r.row * m, r.col0(), m, r.row < m, z);
+  auto load_A = [&](int b) {
+    if (r.begin_load(b, kBlockBytes)) bulk_load(r.slot(2 + b), A + (size_t)b * kBlockBytes, kBlockBytes, &r.sh->loaded[b]);
+  };
+  if (I) {
+    fence_proxy_async_all();
+    if (r.begin_load(2, 2 * kBlockBytes)) {
+      bulk_load(r.slot(0), img(kFZ0) + (size_t)own * kBlockBytes, kBlockBytes, &r.sh->loaded[2]);
+      bulk_load(r.slot(1), img(kFZ0) + (size_t)peer * kBlockBytes, kBlockBytes, &r.sh->loaded[2]);
+    }
+    load_A(1);
+    load_A(0);
   }
   for (int j = 0; j < p.J; ++j) {
-    uint8_t* Z = img(kFZ0 + (j & 1));
-    uint8_t* Zn = img(kFZ0 + ((j + 1) & 1));
-    r.template product<false, false>(A, j == 0, Z, true, 2, 0, false);
-    r.commit(0);
+    const bool more = j + 1 < p.J;
+    if (I) {
+      if (j == 0) r.wait_loaded(2);
+      else r.wait_put();
+      r.wait_loaded(1);
+      tc_fence_after();
+      r.chunk(0, r.slot(3), r.slot(0) + half, false);
+      r.wait_loaded(0);
+      r.chunk(0, r.slot(2), r.slot(0), true);
+      r.commit_both(0);
+      r.wait_put();                                  // R
+      r.wait_both(0);
+      if (j > 0) r.wait_came(kFromZ);
+      r.chunk(0, r.slot(0), r.slot(2) + own * half, false);
+      r.chunk(0, r.slot(1), r.slot(2) + peer * half, true);
+      r.commit_both(0);
+      r.chunk(1, r.slot(2), r.slot(2) + own * half, false);
+      r.wait_came(kFromR);
+      r.chunk(1, r.slot(3), r.slot(2) + peer * half, true);
+      r.commit_both(1);
+      r.wait_put();                                  // Y and W
+      r.wait_both(0);
+      r.wait_both(1);
+      r.chunk(0, r.slot(0), r.slot(2) + own * half, false);
+      if (more) load_A(1);
+      r.wait_came(kFromY);
+      r.chunk(0, r.slot(1), r.slot(2) + peer * half, true);
+      r.commit_both(0);
+      r.wait_both(0);
+      if (more) {
+        load_A(0);
+      } else if (ridge && r.begin_load(0, kBlockBytes)) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int x = 0; x < 3; ++x)
+            bulk_load(r.slot(2) + (b * 3 + x) * half, img(kFK2) + (size_t)b * kBlockBytes + x * kTermBytes + own * half, half, &r.sh->loaded[0]);
+      }
+    }
     if (C) {
-      r.result(0, 0, rv);
+      r.wait_both(0);
+      r.take(0, rv);
 #pragma unroll
       for (int i = 0; i < 16; ++i) rv[i] = -rv[i];
       r.add_diag(rv, 1.f, m);
-      r.put(img(kFR), rv);
-    }
-    r.publish(false);
-    r.template product<false, false>(Z, false, img(kFR), true, 2, 0, false);
-    r.commit(0);
-    r.template product<false, false>(img(kFR), true, img(kFR), true, 2, 1, false);
-    r.commit(1);
-    if (C) {
-      r.result(0, 0, v);
-      r.put(img(kFY), v);
-      r.result(1, 1, v);
+      r.put_slot(2, rv);
+      r.announce();
+      r.send(2, 3, kFromR);
+      r.wait_both(0);
+      r.take(0, v);
+      r.put_slot(0, v);
+      r.send(0, 1, kFromY);
+      r.wait_both(1);
+      r.take(1, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = fmaf(0.25f, v[i], rv[i]);
       r.add_diag(v, 1.f, m);
-      r.put(img(kFW), v);
-    }
-    r.publish(false);
-    r.template product<false, false>(img(kFY), true, img(kFW), true, 2, 0, false);
-    r.commit(0);
-    if (C) {
-      r.result(0, 0, v);
+      r.put_slot(2, v);
+      r.announce();
+      r.wait_both(0);
+      r.take(0, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) z[i] += v[i];
-      if (j < p.J - 1 || p.kappa > 0.f) r.put(Zn, z);
-      const bool ok = r.row < m && !r.failed;
-      set_row<16>(iterates + (size_t)(j + 1) * mm + (size_t)r.row * m, r.col0(), m, ok, z);
-      if (j == p.J - 1 && !(p.kappa > 0.f)) set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, ok, z);
+      if (more || ridge) {
+        r.put_slot(0, z);
+        r.announce();
+        r.stage_rows(z);
+        r.send(0, 1, kFromZ);
+      } else {
+        r.stage_rows(z);
+        r.row_sync();
+        r.store_rows(k2inv, m);
+      }
+      r.store_rows(iterates + (size_t)(j + 1) * mm, m);
     }
-    r.publish(false);
   }
-  if (p.kappa > 0.f) {
-    r.template product<false, true>(img(kFZ0 + (p.J & 1)), true, img(kFK2), false, 2, 0, false);   // Z_J K2^T
-    r.commit(0);
+  if (ridge) {                                       // K2inv = Z_J K2^T
+    if (I) {
+      r.wait_put();
+      r.wait_loaded(0);
+      tc_fence_after();
+      r.template chunk<true, kTermBytes / 2>(0, r.slot(0), r.slot(2) + own * 3 * half, false);
+      r.wait_came(kFromZ);
+      r.template chunk<true, kTermBytes / 2>(0, r.slot(1), r.slot(2) + peer * 3 * half, true);
+      r.commit_both(0);
+      r.wait_both(0);
+    }
     if (C) {
-      r.result(0, 0, v);
+      r.wait_both(0);
+      r.take(0, v);
       set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
     }
   }
@@ -1018,7 +1202,7 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~(uintptr_t)1023);
   float* red = reinterpret_cast<float*>(ring + (size_t)kStages * kStageBytes + kBlockBytes);
   Shared* sh = reinterpret_cast<Shared*>(red + kRedFloats);
-  static_assert(sizeof(Shared) <= 128, "barriers");
+  static_assert(sizeof(Shared) <= 256, "barriers");
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&sh->full[s], 1); mbar_init(&sh->empty[s], 1); }
@@ -1027,6 +1211,14 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
     mbar_init(&sh->released[0], kComputeWarps);
     mbar_init(&sh->released[1], kComputeWarps);
     mbar_init(&sh->drain, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&sh->both[i], 2);
+    mbar_init(&sh->put, kComputeWarps);
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&sh->came[i], 4);
+      mbar_init(&sh->loaded[i], 1);
+      sh->loads[i] = 0;
+      for (int q = 0; q < 4; ++q) sh->inbound[q][i] = 0;
+    }
     mbar_init(&sh->ready, 2 * (kComputeWarps + 2));
     sh->abort_word = 0;
     fence_mbar_init();
@@ -1055,6 +1247,8 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
         const uint32_t n = (sh->fills + kStages - 1 - s) / kStages;    // fills of stage s
         if (n) mbar_drain(&sh->full[s], (n - 1) & 1u);
       }
+      for (int i = 0; i < 3; ++i)
+        if (sh->loads[i]) mbar_drain(&sh->loaded[i], (sh->loads[i] - 1) & 1u);
     }
     if (warp == kComputeWarps + 1) {
       umma_commit_elect(&sh->drain);       // (from the lane that issued)
@@ -1062,7 +1256,17 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
     }
     __syncthreads();
   }
-  cluster_sync_all();          // nobody arrives on this CTA's barriers any more
+  cluster_sync_all();          // nobody arrives on this CTA's barriers any more, or copies into its memory
+  if (sh->abort_word && threadIdx.x == 0)      // (copies on their way: their last phase, with the arrivals of those who gave up before)
+    for (int i = 0; i < 3; ++i) {
+      uint32_t n = 0;
+      for (int q = 0; q < 4; ++q) n = max(n, sh->inbound[q][i]);
+      for (int q = 0; q < 4; ++q)
+        if (sh->inbound[q][i] < n) mbar_arrive(&sh->came[i]);
+      if (n) mbar_drain(&sh->came[i], (n - 1) & 1u);
+    }
+  __syncwarp();
+  cluster_sync_all();
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
