@@ -26,8 +26,8 @@
 // reads 24 KB) and between them the way of a result through registers, split and shared memory (2500 cycles, three times);
 // backward, the same with what a phase waits for: copies out of L2 (9 KB per K step), the result block out to it (put 1600,
 // publish 2300), the peer, the first chunk in (1550).  Measured at B=2, H=8, m=128 (us): forward D=128, J=8 with
-// ridge 222 with four products in a row, 205 in residual form through L2, 128 with the operands on the chip; D=64, J=6 without
-// 164, 152, 94; backward 447 / 408 and 318 / 289.
+// ridge 222 with four products in a row, 205 in residual form through L2, 123 with the operands on the chip; D=64, J=6 without
+// 164, 152, 95; backward 447 / 408 and 318 / 289.
 #pragma once
 #include "common.cuh"
 #include "small_kernels.cuh"
@@ -53,7 +53,7 @@ constexpr int kF32 = kMaxM * kMaxM;            // floats of one FP32 scratch mat
 
 // scratch of a cluster: images, then FP32 matrices.  A launch has at most as many clusters as run at once; each walks slices
 // gridDim.x / 2 apart and works in one scratch area, so that the scratch stays in L2 and does not grow with the slices.
-enum FwdImg { kFK2, kFA, kFZ0, kFR, kFW, kFwdImgs };
+enum FwdImg { kFK2, kFA, kFR, kFW, kFwdImgs };
 constexpr size_t kFwdScratchBytes = (size_t)kFwdImgs * kImg + kF32 * sizeof(float);
 enum BwdImg { kBK2, kBA, kBZ0, kBZ1, kBZ2, kBG0, kBG1, kBR0, kBR1, kBW, kBY, kBdY, kBH, kBwdImgs };
 enum BwdF32 { kGA, kGdZ, kGdK, kGg, kBwdF32s };
@@ -68,9 +68,9 @@ enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
 struct Shared {
   uint64_t full[kStages], empty[kStages], done[2], released[2], ready, drain;
   // forward iteration: products complete in both CTAs; result blocks written here; blocks that came from the peer; slots loaded
-  uint64_t both[2], put, came[3], loaded[3];
+  uint64_t both[2], put, came[3], loaded[2];
   uint32_t tmem_slot;
-  uint32_t loads[3];        // loads of each slot, written when the issuing warp is through
+  uint32_t loads[2];        // loads of each slot, written when the issuing warp is through
   uint32_t inbound[4][3];   // copies that the peer has sent here, likewise
   uint32_t fills;           // stages filled by the copying warp, written when it is through
   int abort_word;
@@ -267,7 +267,7 @@ struct Role {
   int row, seg;
   uint32_t dphase[2];
   uint32_t relphase[2];     // issue: parity of the next wait on released[]
-  uint32_t bphase[2], pphase, cphase[3], lphase[3], loads[3], sent[3];     // forward iteration: parities, loads and copies issued
+  uint32_t bphase[2], pphase, cphase[3], lphase[2], loads[2], sent[3];     // forward iteration: parities, loads and copies issued
 
   __device__ void open(Shared* s, uint8_t* r, float* rd, int rk, int* status, bool drop_fill) {
     drop = drop_fill;
@@ -277,7 +277,8 @@ struct Role {
     failed = pend = false;
     rphase = sphase = fills = 0; stage = 0;
     dphase[0] = dphase[1] = relphase[0] = relphase[1] = bphase[0] = bphase[1] = pphase = 0;
-    for (int i = 0; i < 3; ++i) cphase[i] = lphase[i] = loads[i] = sent[i] = 0;
+    lphase[0] = lphase[1] = loads[0] = loads[1] = 0;
+    for (int i = 0; i < 3; ++i) cphase[i] = sent[i] = 0;
     const int w = threadIdx.x >> 5;
     row = (w & 3) * 32 + lane;
     seg = rank * 4 + (w >> 2);
@@ -541,7 +542,7 @@ struct Role {
   }
   // may the next load be issued?  (lane 0 issues it)
   __device__ __forceinline__ bool begin_load(int l, uint32_t bytes) {
-    if (drop && loads[0] + loads[1] + loads[2] == 2) failed = true;     // fault injection on the host's request
+    if (drop && loads[0] + loads[1] == 2) failed = true;     // fault injection on the host's request
     if (failed) return false;
     ++loads[l];
     if (lane == 0) mbar_expect_tx(&sh->loaded[l], bytes);
@@ -568,7 +569,7 @@ struct Role {
     ensure();
     if (R == kProducer && lane == 0) sh->fills = fills;
     if (R == kIssuer && lane == 0)
-      for (int i = 0; i < 3; ++i) sh->loads[i] = loads[i];
+      for (int i = 0; i < 2; ++i) sh->loads[i] = loads[i];
     if (R == kCompute && threadIdx.x < 128 && lane == 0)       // (the peer counts on these copies until they have arrived)
       for (int i = 0; i < 3; ++i) {
         uint32_t at;
@@ -665,7 +666,9 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
     r.commit(0);
     if (C) {
       r.result(0, 0, v, (D + 63) / 64, 0.f);
-      set_row<16>(k2 + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
+      r.stage_rows(v);
+      r.row_sync();
+      r.store_rows(k2, m);
     }
     r.publish(true);
   }
@@ -705,24 +708,14 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
       r.result(0, 0, v);
       r.add_diag(v, nk.n1 * nk.ninf / p.kappa, m);
       r.put(img(kFA), v);
-      set_row<16>(a32 + (size_t)r.row * m, r.col0(), m, r.row < m, v);
+      r.stage_rows(v);
+      r.row_sync();
+      r.store_rows(a32, m);
     }
     r.publish(true);
     A = img(kFA);
     A32 = a32;
   }
-  if (C) {
-    r.ensure();
-    const Norms na = norms(A32, m, r.red);
-    const float c = fmaxf(na.n1 * na.ninf, 1e-12f);
-    // Z0 = A^T / c; lanes run along the rows of Z0 (the columns of A)
-    const int row = r.rank * 64 + (threadIdx.x & 63), s = threadIdx.x >> 6;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = (row < m && 16 * s + i < m) ? __ldcg(A32 + (size_t)(16 * s + i) * m + row) / c : 0.f;
-    put16(img(kFZ0), row, s, v);
-    set_row<16>(iterates + (size_t)row * m, 16 * s, m, row < m, v);
-  }
-  r.publish(true);
   // R = I - A Z, then Y = Z R and W = I + R + R^2 / 4 side by side, then Z' = Z + Y W.  All operands are on the chip: a
   // block of 64 columns is left operand (K) and right operand (columns) from the same place, a CTA's own block needs no
   // exchange, and the products begin with it; the peer's block, needed on the left only, arrives behind them from the peer's
@@ -736,24 +729,30 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
   constexpr uint32_t half = kTermBytes / 2;       // 64 rows of a block
   float z[16], rv[16];
   r.ensure();
-  if (C) get_row<16>(iterates + (size_t)r.row * m, r.col0(), m, r.row < m, z);
   auto load_A = [&](int b) {
     if (r.begin_load(b, kBlockBytes)) bulk_load(r.slot(2 + b), A + (size_t)b * kBlockBytes, kBlockBytes, &r.sh->loaded[b]);
   };
   if (I) {
     fence_proxy_async_all();
-    if (r.begin_load(2, 2 * kBlockBytes)) {
-      bulk_load(r.slot(0), img(kFZ0) + (size_t)own * kBlockBytes, kBlockBytes, &r.sh->loaded[2]);
-      bulk_load(r.slot(1), img(kFZ0) + (size_t)peer * kBlockBytes, kBlockBytes, &r.sh->loaded[2]);
-    }
     load_A(1);
     load_A(0);
+  }
+  if (C) {
+    // Z0 = A^T / c, lanes along the rows of Z0 (the columns of A)
+    const Norms na = norms(A32, m, r.red);
+    const float c = fmaxf(na.n1 * na.ninf, 1e-12f);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) z[i] = (r.row < m && r.col0() + i < m) ? __ldcg(A32 + (size_t)(r.col0() + i) * m + r.row) / c : 0.f;
+    r.put_slot(0, z);
+    r.announce();
+    r.stage_rows(z);
+    r.send(0, 1, kFromZ);
+    r.store_rows(iterates, m);
   }
   for (int j = 0; j < p.J; ++j) {
     const bool more = j + 1 < p.J;
     if (I) {
-      if (j == 0) r.wait_loaded(2);
-      else r.wait_put();
+      r.wait_put();                                  // Z
       r.wait_loaded(1);
       tc_fence_after();
       r.chunk(0, r.slot(3), r.slot(0) + half, false);
@@ -762,7 +761,7 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
       r.commit_both(0);
       r.wait_put();                                  // R
       r.wait_both(0);
-      if (j > 0) r.wait_came(kFromZ);
+      r.wait_came(kFromZ);
       r.chunk(0, r.slot(0), r.slot(2) + own * half, false);
       r.chunk(0, r.slot(1), r.slot(2) + peer * half, true);
       r.commit_both(0);
@@ -840,7 +839,10 @@ __device__ __forceinline__ void fwd_program(Role<R>& r, const FwdParams& p, int6
     if (C) {
       r.wait_both(0);
       r.take(0, v);
-      set_row<16>(k2inv + (size_t)r.row * m, r.col0(), m, r.row < m && !r.failed, v);
+      r.row_sync();                                  // the staged rows of Z_J have left
+      r.stage_rows(v);
+      r.row_sync();
+      r.store_rows(k2inv, m);
     }
   }
   r.close();
@@ -1215,8 +1217,7 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
     mbar_init(&sh->put, kComputeWarps);
     for (int i = 0; i < 3; ++i) {
       mbar_init(&sh->came[i], 4);
-      mbar_init(&sh->loaded[i], 1);
-      sh->loads[i] = 0;
+      if (i < 2) { mbar_init(&sh->loaded[i], 1); sh->loads[i] = 0; }
       for (int q = 0; q < 4; ++q) sh->inbound[q][i] = 0;
     }
     mbar_init(&sh->ready, 2 * (kComputeWarps + 2));
@@ -1247,7 +1248,7 @@ __device__ __forceinline__ void run_kernel(uint8_t* dyn, const P& p, Prog prog) 
         const uint32_t n = (sh->fills + kStages - 1 - s) / kStages;    // fills of stage s
         if (n) mbar_drain(&sh->full[s], (n - 1) & 1u);
       }
-      for (int i = 0; i < 3; ++i)
+      for (int i = 0; i < 2; ++i)
         if (sh->loads[i]) mbar_drain(&sh->loaded[i], (sh->loads[i] - 1) & 1u);
     }
     if (warp == kComputeWarps + 1) {
