@@ -35,8 +35,8 @@
 // stored about 1000), three of them per iteration in the forward; in the backward, where eight products run beside the
 // chain, shared-memory bandwidth (an MMA reads 8 KB per 65 cycles, an epilogue moves 56 KB).  Instructions come from a cold
 // cache the first time round: 5 us of the forward, 15 of the backward.  Measured (us, nested form with one accumulator per
-// partial product / this, J = 6): 32 slices, m = 64 forward 45 / 43, backward 76 / 66; m = 32 43 / 35 and 66 / 48;
-// 512 slices 162 / 117 and 310 / 283; 64 slices of head_dim 128 with the ridge (then on the CUDA cores) 74 / 52 and 121 / 90.
+// partial product / this, J = 6): 32 slices, m = 64 forward 45 / 41, backward 76 / 66; m = 32 43 / 33 and 66 / 48;
+// 512 slices 162 / 109 and 310 / 287; 64 slices of head_dim 128 with the ridge (then on the CUDA cores) 74 / 50 and 121 / 90.
 #pragma once
 #include "ns_kernels.cuh"
 #include "small_kernels.cuh"
