@@ -635,7 +635,10 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = 0.f;
     }
-    if (s == -1) add_diag(c, v, r[0], m);
+    if (s == -1) {
+      add_diag(c, v, r[0], m);
+      ns::ns_sync();                         // K2 leaves X behind its arrival for the product: every warp is through with that
+    }
     stage_row16(c, X, v);
     ns::ns_sync();
     if (s == -2) softmax16(X, p, bh);

@@ -182,3 +182,18 @@ def test_probe_occupancy_leaves_the_kernels_usable(cuda_device):
     conv_again = _C.conv_residual(v, w)
     torch.cuda.synchronize()
     assert torch.equal(first, again) and torch.equal(conv_first, conv_again)
+
+
+@pytest.mark.parametrize("dtype,m", [(torch.float16, 64), (torch.bfloat16, 63), (torch.float32, 49), (torch.float32, 33), (torch.float16, 30)])
+def test_k2_is_the_same_with_and_without_the_ridge(cuda_device, dtype, m):
+    """The forward kernel copies the softmaxed matrix out of a buffer that the ridge's Gram matrix takes next; scores and softmax
+    do not depend on the ridge, so both calls give the same bits.  Two slices per SM, several times, 4-byte copies (m not a
+    multiple of four) and 16-byte ones."""
+    from flashnystrom_b200 import _C
+    q, k, v, _ = (t.cuda() for t in O.make_inputs(37, 8, 2 * m + 1, 64, seed=m, dtype=dtype))
+    want = _C.forward(q, k, v, m, 4, 0.0)
+    for _ in range(8):
+        got = _C.forward(q, k, v, m, 4, 5.0)
+        assert torch.equal(got[11], want[11])
+        assert torch.equal(got[8], want[8])
+    _C.check_device_status()
