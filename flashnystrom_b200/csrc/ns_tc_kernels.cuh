@@ -185,11 +185,13 @@ __device__ __forceinline__ void get_row16(const Ctx& c, uint32_t set, float* v) 
 }
 
 // ---- global / staging accesses ---------------------------------------------------------------
+// (the caller's FP32 tensors need no more than their type's alignment)
+__device__ __forceinline__ bool whole16(const float* g) { return (reinterpret_cast<uintptr_t>(g) & 15u) == 0; }
 // Whole-matrix tile loads: thread t handles row t >> 2 and the 8-column chunks (t & 3) and (t & 3) + 4, so that four
 // adjacent lanes cover 128 consecutive bytes.
 __device__ __forceinline__ void load_chunk8(const float* g, int r, int chunk, int rows, int cols, int ld, float* v) {
   const int c0 = 8 * chunk;
-  if (((ld | cols) & 3) == 0) {
+  if (((ld | cols) & 3) == 0 && whole16(g)) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -224,7 +226,7 @@ __device__ __forceinline__ void load_row16(const Ctx& c, const float* g, int row
 }
 __device__ __forceinline__ void store_row16(const Ctx& c, float* g, const float* v, int rows, int cols, int ld) {
   if (c.row >= rows) return;
-  if (((ld | cols) & 3) == 0) {
+  if (((ld | cols) & 3) == 0 && whole16(g)) {
 #pragma unroll
     for (int i = 0; i < 16; i += 4)
       if (c.col0 + i < cols)
@@ -255,7 +257,7 @@ __device__ __forceinline__ void unstage_col16(const Ctx& c, const float* X, floa
 // A staged matrix -> the leading rows x cols block of a dense global matrix, whole sectors per instruction.  (From the
 // accumulator layout, 32 rows of 16 bytes per instruction, the store of an iterate kept the warps for 1700 cycles, this takes 400.)
 __device__ __forceinline__ void store_staged(const float* X, float* g, int rows, int cols, int ld) {
-  if (((ld | cols) & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15u) == 0) {
+  if (((ld | cols) & 3) == 0 && whole16(g)) {
     const int r = threadIdx.x >> 2;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {

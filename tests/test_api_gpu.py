@@ -282,3 +282,55 @@ def test_saved_tensor_hooks_may_move_the_buffer(cuda_device):
         grads.append([t.grad for t in x])
     for a, b in zip(*grads):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype,D,m,kappa", [(torch.float16, 64, 64, 5.0), (torch.float16, 64, 64, 0.0), (torch.bfloat16, 128, 32, 5.0),
+                                             (torch.float32, 64, 36, 5.0), (torch.float32, 32, 33, 5.0)])
+def test_softmaxed_matrix_and_iterates_need_only_their_types_alignment(cuda_device, dtype, D, m, kappa):
+    """Up to 64 landmarks: K2 and the iterates at any four-byte boundary, written by a forward call of the C ABI (which reads K2
+    back for the ridge) and read by the backward."""
+    import ctypes
+    from flashnystrom_b200 import _C, _lib
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 2, 300, D, seed=6, dtype=dtype))
+    lib, dev, J = _lib.load(), q.device, 4
+    want = _C.forward(q, k, v, m, J, kappa)
+    got = [t if i in (1, 2) else torch.zeros_like(t) for i, t in enumerate(want)]
+    for i in (10, 11):
+        got[i] = _shifted(got[i])
+    shape = _C._shape_struct(1, 2, 300, D, m, J, dtype, kappa)
+    ws = torch.empty(lib.fnb_fwd_workspace_bytes(ctypes.byref(shape)), dtype=torch.uint8, device=dev)
+    outputs = [got[i].data_ptr() for i in (0, 7, 3, 4, 11, 8, 10, 5, 12, 9, 6)]
+    args = _lib.FwdArgs(shape, *[x.data_ptr() for x in (q, k, v)], *outputs, ws.data_ptr(), ws.numel(), dev.index,
+                        torch.cuda.current_stream(dev).cuda_stream, _C._status(dev).data_ptr())
+    _lib.check(lib.fnb_forward(ctypes.byref(args)))
+    _C.check_device_status()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    for a, b in zip(_C.backward(dO, *got[1:13], v, got[0], m, J, True, kappa), _C.backward(dO, *want[1:13], v, want[0], m, J, True, kappa)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m,kappa", [(64, 5.0), (64, 0.0), (36, 5.0), (33, 5.0), (100, 5.0)])
+def test_pseudoinverse_entries_need_only_their_types_alignment(cuda_device, m, kappa):
+    import ctypes
+    from flashnystrom_b200 import _C, _lib
+    k2 = torch.softmax(torch.randn(2, m, m, device="cuda", generator=torch.Generator("cuda").manual_seed(m)), -1)
+    G = torch.randn(2, m, m, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    iterates, inv = _C.debug_pinv_forward(k2, 4, kappa)
+    dk2 = _C.debug_pinv_backward(k2, iterates, G, kappa)
+    lib, dev, t = _lib.load(), k2.device, {}
+    for name, x in (("k2", k2), ("G", G)):
+        t[name] = _shifted(x)
+    for name, x in (("iterates", iterates), ("inv", inv), ("dk2", dk2)):
+        t[name] = _shifted(torch.zeros_like(x))
+    ws = torch.empty(lib.fnb_debug_pinv_workspace_bytes(2, m) + 4, dtype=torch.uint8, device=dev)[4:]
+    stream, p = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream), {n: x.data_ptr() for n, x in t.items()}
+    _lib.check(lib.fnb_debug_pinv_forward(2, m, 4, kappa, p["k2"], p["iterates"], p["inv"], ws.data_ptr(), ws.numel(), dev.index, stream))
+    _lib.check(lib.fnb_debug_pinv_backward(2, m, 4, kappa, p["k2"], p["iterates"], p["G"], p["dk2"], ws.data_ptr(), ws.numel(), dev.index, stream))
+    for name, x in (("iterates", iterates), ("inv", inv), ("dk2", dk2)):
+        assert torch.equal(t[name], x), name
+    if m <= 64:
+        z, da = (_shifted(torch.zeros_like(k2)) for _ in range(2))
+        want = _C.debug_ns_bwd_step(k2, inv, G)
+        _lib.check(lib.fnb_debug_ns_bwd_step(2, m, p["k2"], p["inv"], p["G"], z.data_ptr(), da.data_ptr(), dev.index, stream))
+        assert torch.equal(z, want[0]) and torch.equal(da, want[1])
