@@ -274,10 +274,10 @@ __device__ __forceinline__ void store_staged(const float* X, float* g, int rows,
   }
 }
 // x / c with rc = 1 / c: a product and one correction of its remainder (Markstein 1990), correctly rounded but for results near
-// the underflow threshold
+// the underflow threshold.  The remainder of an infinite x or c is not a number: there the product is the quotient.
 __device__ __forceinline__ float div_by(float x, float c, float rc) {
-  const float q = x * rc;
-  return fmaf(fmaf(-q, c, x), rc, q);
+  const float q = x * rc, corrected = fmaf(fmaf(-q, c, x), rc, q);
+  return corrected == corrected ? corrected : q;
 }
 // d on the diagonal of the leading m x m block
 __device__ __forceinline__ void add_diag(const Ctx& c, float* v, float d, int m) {

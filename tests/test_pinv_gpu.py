@@ -197,3 +197,49 @@ def test_k2_is_the_same_with_and_without_the_ridge(cuda_device, dtype, m):
         assert torch.equal(got[11], want[11])
         assert torch.equal(got[8], want[8])
     _C.check_device_status()
+
+
+@pytest.mark.parametrize("m", [17, 64])
+def test_first_iterate_is_the_rounded_quotient(cuda_device, m):
+    """Z0 = A^T / (||A||_1 ||A||_inf) against torch's division on the same bits, values over 40 powers of two.  The kernel adds the norms
+    up in its own order, at most 19 additions each, and rounds their product: the divisor is within 24 units in the last place
+    of the one in float64, and one of these has to give all quotients of a matrix."""
+    from flashnystrom_b200 import _C
+    g = torch.Generator().manual_seed(m)
+    a = (torch.randn(24, m, m, generator=g) * torch.exp2(torch.rand(24, m, m, generator=g) * 40 - 30)).cuda()
+    z0 = _C.debug_pinv_forward(a, 1)[0][:, 0]
+    c = (a.abs().double().sum(1).amax(1) * a.abs().double().sum(2).amax(1)).float()
+    steps = (c.view(torch.int32)[:, None] + torch.arange(-24, 25, device="cuda", dtype=torch.int32)).view(torch.float32)
+    same = (a.transpose(1, 2)[:, None] / steps[:, :, None, None] == z0[:, None]).flatten(2).all(2)
+    assert same.any(1).all()
+
+
+@pytest.mark.parametrize("m", [17, 64])
+def test_infinite_divisor(cuda_device, m):
+    """An infinite entry, and finite ones whose norms' product overflows: zeros, and NaN for inf / inf."""
+    from flashnystrom_b200 import _C
+    a = _softmax_matrix(2, m, seed=m).cuda()
+    a[0, 3, 5] = float("inf")
+    a[1] *= 1e25
+    z0 = _C.debug_pinv_forward(a, 1)[0][:, 0]
+    assert torch.equal(z0.nan_to_num(nan=7.0), (a.transpose(1, 2) / float("inf")).nan_to_num(nan=7.0))
+
+
+@pytest.mark.parametrize("dtype,m", [(torch.float32, 17), (torch.float16, 64), (torch.float32, 64)])
+@pytest.mark.parametrize("kappa", [1e-25, 3e-20])
+def test_ridge_whose_norms_overflow(cuda_device, dtype, m, kappa):
+    """Condition numbers so small that the product of A's norms overflows: Z0 = A^T / inf = 0, and so are the other iterates and the
+    output.  What is finite of the gradients on the CUDA cores, which divide, is finite here."""
+    from flashnystrom_b200 import _C
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 2, 300, 64, seed=9, dtype=dtype))
+    finite = []
+    for generic in (False, True):
+        _C.set_force_generic(generic)
+        try:
+            r = _C.forward(q, k, v, m, 4, kappa)
+            assert not r[10].any() and not r[5].any() and not r[0].any()
+            finite.append([t.isfinite() for t in _C.backward(dO, *r[1:13], v, r[0], m, 4, True, kappa)])
+        finally:
+            _C.set_force_generic(False)
+    for a, b in zip(*finite):
+        assert torch.equal(a, b)
