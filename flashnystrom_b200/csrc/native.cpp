@@ -142,7 +142,9 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
                             const std::optional<at::Tensor>& weight, const Call& c) {
     at::Tensor saved;
     at::Tensor out = run_forward(q, k, v, c, saved);
-    variable_list keep{q, k, v, saved};
+    // (a gradient of the taps alone needs v and nothing else of the attention)
+    const bool inputs = q.requires_grad() || k.requires_grad() || v.requires_grad();
+    variable_list keep = inputs ? variable_list{v, q, k, saved} : variable_list{v};
     if (weight) {
       at::Tensor w32 = rounded_taps(*weight, v);
       out = run_conv(v, c.layout, w32, &out, false);
@@ -150,6 +152,7 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
       ctx->saved_data["weight_dtype"] = (int64_t)weight->scalar_type();
     }
     ctx->save_for_backward(keep);
+    ctx->saved_data["conv"] = weight.has_value();
     ctx->saved_data["m"] = (int64_t)c.shape.num_landmarks;
     ctx->saved_data["J"] = (int64_t)c.shape.newton_iter;
     ctx->saved_data["kappa"] = (double)c.shape.kappa_star;
@@ -158,23 +161,39 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
   }
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    variable_list kept = ctx->get_saved_variables();
-    const at::Tensor &q = kept[0], &k = kept[1], &v = kept[2];
-    at::Tensor saved = kept[3];
-    const bool conv = kept.size() > 4;
-    const int64_t m = ctx->saved_data["m"].toInt(), J = ctx->saved_data["J"].toInt();
-    const uint32_t flags = g_flags.load();
+    const variable_list kept = ctx->get_saved_variables();
+    const bool conv = ctx->saved_data["conv"].toBool(), inputs = kept.size() > 2;
+    const at::Tensor& v = kept[0];
     at::Tensor g = grads[0];
     TORCH_CHECK(g.defined() && g.is_cuda() && g.dim() == 4, "dO must be a 4D CUDA tensor (flashnystrom_b200 has no CPU path)");
     const int dtype = dtype_of(g);
     TORCH_CHECK(dtype >= 0, "Supported dtypes: float32, float16, bfloat16");
     c10::cuda::CUDAGuard guard(g.device());
-    int layout = layout_of(q);
+    const int64_t m = ctx->saved_data["m"].toInt();
+    const uint32_t flags = g_flags.load();
+    int layout = layout_of(v);
     if (layout != FNB_LAYOUT_BNHD || !takes_bnhd(dtype, g.size(3), m, flags)) layout = FNB_LAYOUT_BHND;
     g = to_layout(g, layout);
-    for (const at::Tensor* t : {&q, &k, &v})
-      TORCH_CHECK(t->scalar_type() == g.scalar_type() && t->device() == g.device() && t->sizes() == g.sizes() && layout_of(*t) == layout,
+    for (size_t i = 0; i < (inputs ? 3 : 1); ++i)
+      TORCH_CHECK(kept[i].scalar_type() == g.scalar_type() && kept[i].device() == g.device() && kept[i].sizes() == g.sizes() &&
+                      layout_of(kept[i]) == layout,
                   "a saved q, k or v does not match dO in shape, dtype, device or layout");
+    variable_list result(5);
+    if (inputs) attention_backward(ctx, kept[1], kept[2], v, kept[3], g, layout, m, flags, result);
+    if (conv) {
+      const at::Tensor& w32 = kept.back();
+      TORCH_CHECK(w32.scalar_type() == at::kFloat && w32.device() == g.device() && w32.dim() == 2 && w32.size(0) == g.size(1) && w32.is_contiguous(),
+                  "the saved convolution weights do not match dO");
+      if (ctx->needs_input_grad(2)) result[2] = run_conv(g, layout, w32, &result[2], true);
+      if (ctx->needs_input_grad(3))
+        result[3] = run_conv_dweight(v, g, layout, w32.size(1)).to((at::ScalarType)ctx->saved_data["weight_dtype"].toInt());
+    }
+    return result;
+  }
+
+  static void attention_backward(AutogradContext* ctx, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, at::Tensor saved,
+                                 const at::Tensor& g, int layout, int64_t m, uint32_t flags, variable_list& result) {
+    const int64_t J = ctx->saved_data["J"].toInt();
     const Saved parts(g.size(0) * g.size(1), g.size(2), g.size(3), m, J);
     TORCH_CHECK(saved.device() == g.device() && saved.scalar_type() == at::kFloat && saved.dim() == 1 && saved.numel() == parts.floats &&
                     saved.is_contiguous(),
@@ -202,16 +221,9 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
       py::reinterpret_borrow<py::object>(g_debug)(g, dq, dk, dv, saved.narrow(0, parts.offset[9], BH * m * D),
                                                   saved.narrow(0, parts.offset[6], BH * m * m));
     }
-    at::Tensor dw;
-    if (conv) {
-      const at::Tensor& w32 = kept[4];
-      TORCH_CHECK(w32.scalar_type() == at::kFloat && w32.device() == g.device() && w32.dim() == 2 && w32.size(0) == g.size(1) && w32.is_contiguous(),
-                  "the saved convolution weights do not match dO");
-      if (ctx->needs_input_grad(2)) dv = run_conv(g, layout, w32, &dv, true);
-      if (ctx->needs_input_grad(3))
-        dw = run_conv_dweight(v, g, layout, w32.size(1)).to((at::ScalarType)ctx->saved_data["weight_dtype"].toInt());
-    }
-    return {dq, dk, dv, dw, at::Tensor()};
+    result[0] = dq;
+    result[1] = dk;
+    result[2] = dv;
   }
 };
 

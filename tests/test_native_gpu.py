@@ -220,3 +220,23 @@ def test_module_backward_with_create_graph(cuda_device):
         if h:
             h.remove()
     assert (got[0] - got[1]).abs().max() <= 1e-2 * got[1].abs().max()
+
+
+def test_taps_alone_run_no_attention_backward(cuda_device, monkeypatch, capfd):
+    """Only the convolution's weights want a gradient: the attention's backward does not run (it would print its statistics) and
+    nothing is kept for it."""
+    from flashnystrom_b200 import flash_nystrom_attention
+    q, k, v, dO = _inputs(1, 2, 256, 64, torch.float16, False)
+    w0 = torch.randn(2, 3, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).half()
+    monkeypatch.setenv("FNB_BWD_DEBUG", "1")
+    kept, grads = [], []
+    for native in (True, False):
+        w = w0.clone().requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(tuple(t.shape)) or t, lambda t: t):
+            out = flash_nystrom_attention(q, k, v, 32, 6, conv_weight=w, conv_kernel_size=3) if native else _functions(q, k, v, 32, 6, 0.0, w)
+        out.backward(dO)
+        grads.append(w.grad)
+    assert kept == [tuple(v.shape), (2, 3)] * 2
+    assert torch.equal(*grads)
+    torch.cuda.synchronize()
+    assert "[FNB_BWD_DEBUG]" not in capfd.readouterr().out
