@@ -239,18 +239,22 @@ at::Tensor head_split(const at::Tensor& x2, const at::Tensor& w, int64_t B, int6
 }
 at::Tensor rows_of(const at::Tensor& t) { return t.transpose(1, 2).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}); }
 
+// Both nodes keep what a gradient that is wanted takes, as a torch linear does: its input for the weight's, its weight for the
+// input's.  (The rest may be changed in place, and is not held.)
+bool wants(const at::Tensor& t) { return t.requires_grad(); }
+at::Tensor kept_if(bool keep, const at::Tensor& t) { return keep ? t : at::Tensor(); }
+
 struct ProjectionsNode : torch::autograd::Function<ProjectionsNode> {
   static variable_list forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& wq, const at::Tensor& wk, const at::Tensor& wv,
                                int64_t H) {
     const int64_t B = x.size(0), N = x.size(1);
     const at::Tensor x2 = x.view({B * N, x.size(2)});
-    ctx->save_for_backward({x, wq, wk, wv});
+    ctx->save_for_backward({kept_if(wants(wq) || wants(wk) || wants(wv), x), kept_if(wants(x), wq), kept_if(wants(x), wk), kept_if(wants(x), wv)});
     return {head_split(x2, wq, B, N, H), head_split(x2, wk, B, N, H), head_split(x2, wv, B, N, H)};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    variable_list kept = ctx->get_saved_variables();
-    const at::Tensor& x = kept[0];
-    const at::Tensor x2 = x.reshape({-1, x.size(-1)});
+    const variable_list kept = ctx->get_saved_variables();
+    const at::Tensor x2 = kept[0].defined() ? kept[0].reshape({-1, kept[0].size(-1)}) : at::Tensor();
     variable_list result(5);
     at::Tensor dx;
     for (int i = 0; i < 3; ++i) {
@@ -258,7 +262,7 @@ struct ProjectionsNode : torch::autograd::Function<ProjectionsNode> {
       if (ctx->needs_input_grad(0)) dx = i == 0 ? at::mm(g, kept[1]) : at::addmm(dx, g, kept[1 + i]);
       if (ctx->needs_input_grad(1 + i)) result[1 + i] = at::mm(g.t(), x2);
     }
-    if (dx.defined()) result[0] = dx.view(x.sizes());
+    if (dx.defined()) result[0] = dx.view({grads[0].size(0), grads[0].size(2), dx.size(1)});
     return result;
   }
 };
@@ -269,19 +273,20 @@ at::Tensor project_out(const at::Tensor& o, const at::Tensor& w) {
 }
 struct OutputNode : torch::autograd::Function<OutputNode> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& o, const at::Tensor& w) {
-    ctx->save_for_backward({o, w});
+    ctx->save_for_backward({kept_if(wants(w), o), kept_if(wants(o), w)});
+    ctx->saved_data["heads"] = o.size(1);
     at::Tensor y = at::empty({o.size(0), o.size(2), w.size(0)}, o.options());
     at::Tensor flat = y.as_strided({o.size(0) * o.size(2), w.size(0)}, {w.size(0), 1});
     at::mm_out(flat, rows_of(o), w.t());
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    variable_list kept = ctx->get_saved_variables();
+    const variable_list kept = ctx->get_saved_variables();
     const at::Tensor &o = kept[0], &w = kept[1];
-    const int64_t B = o.size(0), H = o.size(1), N = o.size(2), D = o.size(3);
+    const int64_t B = grads[0].size(0), N = grads[0].size(1), H = ctx->saved_data["heads"].toInt();
     const at::Tensor g = grads[0].reshape({B * N, -1});
     variable_list result(2);
-    if (ctx->needs_input_grad(0)) result[0] = at::mm(g, w).view({B, N, H, D}).transpose(1, 2);
+    if (ctx->needs_input_grad(0)) result[0] = at::mm(g, w).view({B, N, H, w.size(1) / H}).transpose(1, 2);
     if (ctx->needs_input_grad(1)) result[1] = at::mm(g.t(), rows_of(o));
     return result;
   }

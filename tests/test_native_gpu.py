@@ -240,3 +240,33 @@ def test_taps_alone_run_no_attention_backward(cuda_device, monkeypatch, capfd):
     assert torch.equal(*grads)
     torch.cuda.synchronize()
     assert "[FNB_BWD_DEBUG]" not in capfd.readouterr().out
+
+
+@pytest.mark.parametrize("changed", ["x", "projections", "out_proj"])
+def test_module_keeps_only_what_its_gradients_take(cuda_device, changed):
+    """What no wanted gradient takes may be changed in place between forward and backward, as with four linears: x under frozen
+    projections, the projections' weights for an x without a gradient, the output's weight where it alone is trained."""
+    x0 = torch.randn(2, 100, 128, device="cuda", generator=torch.Generator("cuda").manual_seed(4)).half()
+    grads = []
+    for native in (True, False):
+        mod = _module(torch.float16)
+        h = None if native else mod.q_proj.register_forward_hook(lambda *a: None)
+        x = x0.clone()
+        if changed == "x":
+            for p in (mod.q_proj, mod.k_proj, mod.v_proj):
+                p.weight.requires_grad_(False)
+            leaf = x.requires_grad_(True)
+            x = leaf * 1
+        elif changed == "out_proj":
+            for n, p in mod.named_parameters():
+                p.requires_grad_(n == "out_proj.weight")
+        y = mod(x)
+        with torch.no_grad():
+            for t in {"x": [x], "projections": [mod.q_proj.weight, mod.k_proj.weight, mod.v_proj.weight], "out_proj": [mod.out_proj.weight]}[changed]:
+                t.add_(1)
+        y.backward(torch.ones_like(y))
+        grads.append([leaf.grad if changed == "x" else None] + [p.grad for p in mod.parameters()])
+    for a, b in zip(*grads):
+        assert (a is None) == (b is None)
+        if a is not None:
+            assert (a.double() - b.double()).abs().max() <= 4 * torch.finfo(torch.float16).eps * b.double().abs().max()
