@@ -77,10 +77,10 @@ struct Call {
   int layout;
   at::Tensor status;       // the device's status word
 };
-fnb_shape shape_of(const at::Tensor& q, int64_t m, int64_t J, double kappa, int layout, uint32_t flags) {
+fnb_shape shape_of(at::IntArrayRef sizes, int dtype, int64_t m, int64_t J, double kappa, int layout, uint32_t flags) {
   fnb_shape s{};
-  s.batch = q.size(0); s.heads = q.size(1); s.seq_len = q.size(2); s.head_dim = (int32_t)q.size(3);
-  s.num_landmarks = (int32_t)m; s.newton_iter = (int32_t)J; s.dtype = dtype_of(q);
+  s.batch = sizes[0]; s.heads = sizes[1]; s.seq_len = sizes[2]; s.head_dim = (int32_t)sizes[3];
+  s.num_landmarks = (int32_t)m; s.newton_iter = (int32_t)J; s.dtype = dtype;
   s.kappa_star = (float)kappa; s.flags = flags; s.layout = layout;
   return s;
 }
@@ -201,7 +201,7 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
     if (reinterpret_cast<uintptr_t>(saved.data_ptr()) & 15u) saved = saved.clone();   // (a saved-tensor hook may hand it back anywhere)
     const at::Tensor status = ctx->saved_data["status"].toTensor();
     fnb_bwd_args a{};
-    a.shape = shape_of(g, m, J, ctx->saved_data["kappa"].toDouble(), layout, flags);
+    a.shape = shape_of(g.sizes(), dtype_of(g), m, J, ctx->saved_data["kappa"].toDouble(), layout, flags);
     check(fnb_check_shape(&a.shape));
     at::Tensor dq = empty_in(g, layout), dk = empty_in(g, layout), dv = empty_in(g, layout);
     at::Tensor ws = bytes(fnb_bwd_workspace_bytes(&a.shape), g);
@@ -295,6 +295,24 @@ struct OutputNode : torch::autograd::Function<OutputNode> {
 bool plain(const at::Tensor& t) { return t.is_cuda() && t.layout() == at::kStrided && !at::isTensorSubclassLike(t) && !t.is_neg() && !t.is_conj(); }
 bool has_tangent(const at::Tensor& t) { return t._fw_grad(0).defined(); }
 
+// taps for B x H slices
+bool takes_taps(const at::Tensor& w, const at::Tensor& like, int64_t B, int64_t H) {
+  return plain(w) && w.device() == like.device() && at::isFloatingType(w.scalar_type()) && w.dim() == 2 && w.size(0) == H && w.size(1) % 2 == 1 &&
+         w.size(1) <= 127 && !has_tangent(w) && B * H <= 65535;
+}
+bool takes_numbers(int64_t m, int64_t J, double kappa) {
+  return m >= 1 && m <= INT32_MAX && J >= 1 && J <= INT32_MAX && std::isfinite(kappa);
+}
+
+// (without the interpreter's lock, with the tensors' device current, all of it checked)
+at::Tensor run_attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const std::optional<at::Tensor>& weight, const Call& c) {
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (weight && weight->requires_grad())))
+    return AttentionNode::apply(q, k, v, weight, c);
+  at::Tensor saved;
+  at::Tensor out = run_forward(q, k, v, c, saved);
+  return weight ? run_conv(v, c.layout, rounded_taps(*weight, v), &out, false) : out;
+}
+
 // out, or nothing where the call is not one for this path
 std::optional<at::Tensor> attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, int64_t m, int64_t J, double kappa,
                                     const std::optional<at::Tensor>& weight, const at::Tensor& status) {
@@ -303,30 +321,20 @@ std::optional<at::Tensor> attention(const at::Tensor& q, const at::Tensor& k, co
     if (!plain(*t) || t->dim() != 4 || t->scalar_type() != q.scalar_type() || t->sizes() != q.sizes() || t->device() != q.device() || has_tangent(*t))
       return std::nullopt;
   const int dtype = dtype_of(q);
-  if (dtype < 0 || q.numel() == 0 || m < 1 || m > INT32_MAX || J < 1 || J > INT32_MAX || !std::isfinite(kappa)) return std::nullopt;
+  if (dtype < 0 || q.numel() == 0 || !takes_numbers(m, J, kappa)) return std::nullopt;
   if (status.device() != q.device()) return std::nullopt;
   const uint32_t flags = g_flags.load();
-  const int64_t H = q.size(1), D = q.size(3);
   int layout = layout_of(q);
-  if (layout == FNB_LAYOUT_BNHD && !takes_bnhd(dtype, D, m, flags)) return std::nullopt;
+  if (layout == FNB_LAYOUT_BNHD && !takes_bnhd(dtype, q.size(3), m, flags)) return std::nullopt;
   if (layout == kNoLayout || layout_of(k) != layout || layout_of(v) != layout) return std::nullopt;
-  if (weight) {
-    const at::Tensor& w = *weight;
-    if (!plain(w) || w.device() != q.device() || !at::isFloatingType(w.scalar_type()) || w.dim() != 2 || w.size(0) != H || w.size(1) % 2 == 0 ||
-        w.size(1) > 127 || has_tangent(w) || q.size(0) * H > 65535)
-      return std::nullopt;
-  }
+  if (weight && !takes_taps(*weight, q, q.size(0), q.size(1))) return std::nullopt;
   for (const at::Tensor* t : {&q, &k, &v})
     if (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15u) return std::nullopt;
-  Call c{shape_of(q, m, J, kappa, layout, flags), layout, status};
+  Call c{shape_of(q.sizes(), dtype, m, J, kappa, layout, flags), layout, status};
   if (fnb_check_shape(&c.shape)) return std::nullopt;
   py::gil_scoped_release nogil;
   c10::cuda::CUDAGuard guard(q.device());
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (weight && weight->requires_grad())))
-    return AttentionNode::apply(q, k, v, weight, c);
-  at::Tensor saved;
-  at::Tensor out = run_forward(q, k, v, c, saved);
-  return weight ? run_conv(v, layout, rounded_taps(*weight, v), &out, false) : out;
+  return run_attention(q, k, v, weight, c);
 }
 
 // The module's forward: projections, attention, output projection.  The caller has seen to it that the projections are plain
@@ -340,29 +348,27 @@ std::optional<at::Tensor> module_forward(const at::Tensor& x, const at::Tensor& 
     if (!plain(*t) || t->scalar_type() != x.scalar_type() || t->device() != x.device() || !t->is_contiguous() || has_tangent(*t)) return std::nullopt;
   for (const at::Tensor* t : {&wq, &wk, &wv, &wo})
     if (t->dim() != 2 || t->size(0) != dim || t->size(1) != dim) return std::nullopt;
-  if (dim == 0 || x.numel() == 0 || H < 1 || dim % H || dtype_of(x) < 0 || !takes_bnhd(dtype_of(x), dim / H, m, g_flags.load())) return std::nullopt;
-  if (m < 1 || m > x.size(1) || J < 1 || J > 20 || !std::isfinite(kappa) || kappa < 0) return std::nullopt;   // (refused by the call itself)
-  if (conv && (!plain(*conv) || conv->device() != x.device() || conv->dim() != 2 || conv->size(0) != H || conv->size(1) % 2 == 0 || conv->size(1) > 127))
+  const uint32_t flags = g_flags.load();
+  if (dim == 0 || x.numel() == 0 || H < 1 || dim % H || dtype_of(x) < 0 || !takes_numbers(m, J, kappa) || !takes_bnhd(dtype_of(x), dim / H, m, flags))
     return std::nullopt;
-  c10::cuda::CUDAGuard guard(x.device());
-  const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || wq.requires_grad() || wk.requires_grad() || wv.requires_grad());
-  variable_list qkv;
-  {
-    py::gil_scoped_release nogil;
-    if (grad) {
-      qkv = ProjectionsNode::apply(x, wq, wk, wv, H);
-    } else {
-      at::AutoGradMode off(false);
-      const int64_t B = x.size(0), N = x.size(1);
-      const at::Tensor x2 = x.view({B * N, dim});
-      for (const at::Tensor* w : {&wq, &wk, &wv}) qkv.push_back(head_split(x2, *w, B, N, H));
-    }
-  }
-  const std::optional<at::Tensor> o = attention(qkv[0], qkv[1], qkv[2], m, J, kappa, conv, status);
-  if (!o) return std::nullopt;
+  if (status.device() != x.device() || (conv && !takes_taps(*conv, x, x.size(0), H))) return std::nullopt;
+  const int64_t B = x.size(0), N = x.size(1);
+  const int layout = H == 1 || N == 1 ? FNB_LAYOUT_BHND : FNB_LAYOUT_BNHD;      // (head-split views of one head or row are contiguous)
+  const Call c{shape_of({B, H, N, dim / H}, dtype_of(x), m, J, kappa, layout, flags), layout, status};
+  if (fnb_check_shape(&c.shape)) return std::nullopt;      // (refused further on; nothing has been formed yet)
   py::gil_scoped_release nogil;
-  if (at::GradMode::is_enabled() && (o->requires_grad() || wo.requires_grad())) return OutputNode::apply(*o, wo);
-  return project_out(*o, wo);
+  c10::cuda::CUDAGuard guard(x.device());
+  variable_list qkv;
+  if (at::GradMode::is_enabled() && (x.requires_grad() || wq.requires_grad() || wk.requires_grad() || wv.requires_grad())) {
+    qkv = ProjectionsNode::apply(x, wq, wk, wv, H);
+  } else {
+    at::AutoGradMode off(false);
+    const at::Tensor x2 = x.view({B * N, dim});
+    for (const at::Tensor* w : {&wq, &wk, &wv}) qkv.push_back(head_split(x2, *w, B, N, H));
+  }
+  const at::Tensor o = run_attention(qkv[0], qkv[1], qkv[2], conv, c);
+  if (at::GradMode::is_enabled() && (o.requires_grad() || wo.requires_grad())) return OutputNode::apply(o, wo);
+  return project_out(o, wo);
 }
 
 }  // namespace

@@ -270,3 +270,22 @@ def test_module_keeps_only_what_its_gradients_take(cuda_device, changed):
         assert (a is None) == (b is None)
         if a is not None:
             assert (a.double() - b.double()).abs().max() <= 4 * torch.finfo(torch.float16).eps * b.double().abs().max()
+
+
+def test_module_is_handed_back_before_anything_is_formed(cuda_device):
+    """What the attention would not take is seen before the projections run: more slices than the convolution has, taps of
+    another device, fewer rows than landmarks, a number of iterations out of range."""
+    from flashnystrom_b200 import _C
+    mod, many = _module(torch.float16), _module(torch.float16, m=1)
+    x = torch.randn(1, 100, 128, device="cuda").half()
+    assert mod._native_forward(x) is not None
+    host = _module(torch.float16)
+    host.conv_weight = torch.nn.Parameter(host.conv_weight.detach().cpu())
+    odd = _module(torch.float16)
+    odd.config.newton_iter = 21
+    for refused, y in ((many, torch.zeros(32768, 1, 128, device="cuda", dtype=torch.float16)), (host, x), (mod, x[:, :31]), (odd, x)):
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        assert refused._native_forward(y) is None
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+    _C.check_device_status()
