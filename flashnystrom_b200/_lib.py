@@ -10,7 +10,6 @@ import threading
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libflashnystrom_b200.so")
-NATIVE_PATH = os.path.join(_PKG, "lib", "_native.so")
 
 FNB_F32, FNB_F16, FNB_BF16 = 0, 1, 2
 FNB_FLAG_FORCE_GENERIC = 1
@@ -136,7 +135,7 @@ def load(build_if_missing=True):
             if not build_if_missing:
                 raise ImportError(f"{LIB_PATH} not found; run python -m flashnystrom_b200.build")
             from . import build as _build
-            _build.build()
+            _build.build_library(path=LIB_PATH)
         lib = C.CDLL(LIB_PATH)
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(lib, name)
@@ -150,17 +149,15 @@ _native = None
 
 
 def native():
-    """The C++ module of the eager path (csrc/native.cpp), built first if it is absent."""
+    """The C++ module of the eager path (csrc/native.cpp), built first where there is none for this source, header and torch."""
     global _native
     if _native is not None:
         return _native
     load()
     with _lock:
         if _native is None:
-            if not os.path.exists(NATIVE_PATH):
-                from . import build as _build
-                _build.build_native()
-            spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+            from . import build as _build
+            spec = importlib.util.spec_from_file_location(__package__ + "._native", _build.build_native())
             module = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(module)
             _native = module
