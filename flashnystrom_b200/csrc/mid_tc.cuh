@@ -62,6 +62,9 @@ constexpr size_t kBwdScratchBytes = (size_t)kBwdImgs * kImg + (size_t)kBwdF32s *
 // Share of a leading partial product that its truncating additions (three per group of four K steps) have lost on the average.
 // Given back, K2inv is 0.45 to 0.98 times as far from the oracle as in the nested form, without it up to 1.17 times.
 constexpr float kTrunc = 0x1.8p-25f;
+// Two and three products in one accumulator: four additions more for each (dL/dK2 1.0 times as far from 64 bits as FP32 sums are, 1.2 to
+// 1.3 times with one product's share for all).
+constexpr float kTrunc2 = 7 * kTrunc / 3, kTrunc3 = 11 * kTrunc / 3;
 
 enum { kProducer = 0, kIssuer = 1, kCompute = 2 };
 
@@ -1020,7 +1023,7 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
       if (C) {
         r.ensure(false);
         if (j > 1) r.convert(iterates + (size_t)(j - 2) * mm, m, m, img(kBZ0 + (j + 1) % 3));
-        r.result(0, 0, v);
+        r.result(0, 0, v, 2, kTrunc3);
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = -fmaf(4.f, hd[i], v[i]);
         r.put(G, v);
@@ -1055,7 +1058,7 @@ __device__ __forceinline__ void bwd_program(Role<R>& r, const BwdParams& p, int6
         r.put(img(kBY), v);
       }
       if (main_part) {
-        r.result(1, 1, v);
+        r.result(1, 1, v, 2, kTrunc2);
 #pragma unroll
         for (int i = 0; i < 16; ++i) g[i] += v[i];
         if (prime) r.put(Gn, g);

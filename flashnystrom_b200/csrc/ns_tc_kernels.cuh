@@ -348,7 +348,11 @@ __device__ __forceinline__ void wait_done(Ctx& c, int b, int where) {
 // loses about an eighth of an ulp each time on the average, which `trunc` (a share of the value) gives back on its way to the
 // small ones.  Without it K2inv and dQ of fp32 calls were up to 1.28 and 1.24 times as far from the oracle as with one add fewer
 // per product, with it 0.83 to 0.98 and 0.90 to 0.99 times.
+// A product that is added to one before adds its small terms onto the large value as well: two products in an accumulator are three
+// times as many truncating additions as one, three five times.  (With one product's share for all, dL/dK2 was 1.6 to 2.2 times as far
+// from 64 bits as FP32 sums are, with theirs 1.2 to 1.3 times; mean over 16 to 64 landmarks, J = 4 to 8.)
 constexpr float kTruncScores = 0x1p-25f;    // below half an ulp of any value: exact sums stay exact
+constexpr float kTruncHead = 4 * 0x1p-26f;  // a sum over 64 columns, however many landmarks
 // This thread's share of the accumulator at TMEM column `col`, before the two lane halves are added: 16 columns that it
 // keeps and 16 that its partner finalises.  Every thread of a warp must call.
 __device__ __forceinline__ void fetch(const Ctx& c, uint32_t col, float trunc, float* keep, float* send) {
@@ -911,7 +915,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
 #pragma unroll
             for (int i = 0; i < 16; ++i) { keep[i] = da_keep[i]; send[i] = da_send[i]; }
           } else {
-            fetch(c, acc * kAccCols, c.trunc, keep, send);
+            fetch(c, acc * kAccCols, step == kHeadG ? kTruncHead : step == kTailK2 ? 3.f * c.trunc : c.trunc, keep, send);
           }
           exchange(c, c.slot(dst), keep, send, v);
         } else {
@@ -1130,7 +1134,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         arrive_ready(c, 5);
       }
       if (main_part) {
-        take(c, 3, 0, c.slot(5 + par), c.act, v, c.trunc);        // D
+        take(c, 3, 0, c.slot(5 + par), c.act, v, 5.f * c.trunc);  // D
         if (c.act) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = -fmaf(4.f, hd[i], v[i]);
@@ -1153,7 +1157,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         if (!main_part) arrive_ready(c, 0);
       }
       if (main_part) {
-        take(c, 5, 3 * kAccCols, c.slot(6 - par), c.act, v, c.trunc);   // G
+        take(c, 5, 3 * kAccCols, c.slot(6 - par), c.act, v, 3.f * c.trunc);   // G
         if (c.act) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) g[i] += v[i];
