@@ -886,7 +886,6 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
       np.m = p.m; np.D = p.D; np.J = p.J; np.kappa = a.shape.kappa_star;
       np.rows_k = use_tc ? w.rows_k : nullptr; np.N = seg_N; np.scale = scale;
       if (p.J >= 1 && ns_on_tensor_cores(a.shape.flags)) {
-        if (int rc = set_smem(nstc::ns_bwd_tc_kernel, nstc::kBwdSmem, max_smem, "ns_bwd")) return rc;
         nstc::BwdParams bp{};
         nstc::BwdHeadParams& hp = bp.h;
         bp.p = np;
@@ -896,10 +895,12 @@ static int backward_impl(const fnb_bwd_args& a, const Plan& p, const BwdWs& w, i
           hp.dkt_a = w.dkt_a; hp.D3 = side_ns ? nullptr : w.D3; hp.do3n = do3n; hp.do3_scale = w.do3_scale;
           hp.qt16 = qt16; hp.qt_mul = scale * tc::kLog2e; hp.dtype = a.shape.dtype; hp.MP = MP;
         }
+        auto kern = nstc::bwd_kernel(bp);
+        if (int rc = set_smem(kern, nstc::kBwdSmem, max_smem, "ns_bwd")) return rc;
         if (side_ns)
-          nstc::ns_bwd_tc_kernel<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kBwdSmem, ns_stream>>>(bp, finish, a.device_status);
+          kern<<<(unsigned)p.BH, nstc::kNsTcThreads, nstc::kBwdSmem, ns_stream>>>(bp, finish, a.device_status);
         else
-          launch_pdl(nstc::ns_bwd_tc_kernel, dim3((unsigned)p.BH), dim3(nstc::kNsTcThreads), nstc::kBwdSmem, st, bp, finish,
+          launch_pdl(kern, dim3((unsigned)p.BH), dim3(nstc::kNsTcThreads), nstc::kBwdSmem, st, bp, finish,
                      a.device_status);
       } else {
         if (int rc = set_smem(ns::ns_bwd_kernel, ns::kBwdSmem, max_smem, "ns_bwd")) return rc;
@@ -1339,8 +1340,9 @@ int fnb_debug_pinv_backward(int64_t bh, int32_t m, int32_t J, float kappa, const
     nstc::BwdParams bp{};
     bp.p.k2 = k2; bp.p.iterates = ns_iterates; bp.p.G = d_k2_inv; bp.p.spill = (float*)workspace;
     bp.p.m = m; bp.p.D = ns::kN; bp.p.J = J; bp.p.kappa = kappa; bp.dK2 = d_k2;
-    FNB_CUDA(raise_smem(reinterpret_cast<const void*>(nstc::ns_bwd_tc_kernel), nstc::kBwdSmem));
-    nstc::ns_bwd_tc_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, 0, nullptr);
+    auto kern = nstc::bwd_kernel(bp);
+    FNB_CUDA(raise_smem(reinterpret_cast<const void*>(kern), nstc::kBwdSmem));
+    kern<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, 0, nullptr);
   } else if (m > ns::kN) {
     mx::BwdParams mp;
     memset(&mp, 0, sizeof(mp));
@@ -1427,12 +1429,13 @@ int fnb_debug_ns_bwd_step(int64_t bh, int32_t m, const float* k2, const float* z
   if (!g.ok) return fail(FNB_ERR_CUDA, "cannot select CUDA device %d", device);
   int max_smem = 0, cc = 0, sms = 0;
   if (int rc = device_limits(device, &max_smem, &cc, &sms)) return rc;
-  if (int rc = set_smem(nstc::ns_bwd_tc_kernel, nstc::kBwdSmem, max_smem, "ns_pinv_bwd")) return rc;
   // one iteration of the product kernel's loop (J = 1, no ridge), stopped in front of the Z0 tail
   nstc::BwdParams bp{};
   bp.p.k2 = k2; bp.p.iterates = z_j; bp.p.G = d_z_next; bp.p.m = m; bp.p.D = ns::kN; bp.p.J = 1;
   bp.step_dz = d_z_out; bp.step_da = d_k2_acc;
-  nstc::ns_bwd_tc_kernel<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, -1, nullptr);
+  auto kern = nstc::bwd_kernel(bp);
+  if (int rc = set_smem(kern, nstc::kBwdSmem, max_smem, "ns_pinv_bwd")) return rc;
+  kern<<<(unsigned)bh, nstc::kNsTcThreads, nstc::kBwdSmem, (cudaStream_t)stream>>>(bp, -1, nullptr);
   FNB_CUDA(cudaPeekAtLastError());
   return 0;
 }
@@ -1478,7 +1481,7 @@ int fnb_kernel_report(int device, fnb_kernel_info* out, int cap) {
       {"tc_fwd_c<half,64,64>", (const void*)tc::tc_fwd_c_kernel<H, 64, 64>, tc::kTcThreads, tc::FwdCSmem<64, 64>::kBytes},
       {"tc_bwd_a<half,64,64>", (const void*)tc::tc_bwd_a_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdASmem<64, 64>::kBytes},
       {"reduce_chunks", (const void*)reduce_chunks_kernel, kThreads, 0},
-      {"ns_bwd_tc", (const void*)nstc::ns_bwd_tc_kernel, nstc::kNsTcThreads, nstc::kBwdSmem},
+      {"ns_bwd_tc", (const void*)nstc::ns_bwd_tc_kernel<true>, nstc::kNsTcThreads, nstc::kBwdSmem},
       {"colpass_operands", (const void*)colpass_operands_kernel, kThreads, (size_t)kColpassOperandSmem},
       {"tc_bwd_b<half,64,64>", (const void*)tc::tc_bwd_b_kernel<H, 64, 64>, tc::kTcThreads, tc::BwdBSmem<64, 64>::kBytes},
       {"tc_rows_inplace<half,64,64>", (const void*)tc::tc_rows_inplace_kernel<H, 64, 64>, tc::kTcThreads, tc::RowsSmem<64, 64>::kBytes},

@@ -86,6 +86,7 @@ struct Ctx {
   int row, part, col0, c32, pair_bar;
   uint32_t lane_addr;   // TMEM offset of the thread's 32 columns
   float trunc;          // see fetch()
+  bool mm16, md16;      // (m x m) (forward), (m x head_dim) matrices go sixteen bytes at a time
   bool act;             // this warp's 32 x 32 block of an m x m matrix has something in it (it is never read otherwise)
   __device__ __forceinline__ uint32_t slot(int i) const { return smem + i * kSet; }
   __device__ __forceinline__ float* stage(int i) const { return reinterpret_cast<float*>(base + i * kSet); }
@@ -185,13 +186,19 @@ __device__ __forceinline__ void get_row16(const Ctx& c, uint32_t set, float* v) 
 }
 
 // ---- global / staging accesses ---------------------------------------------------------------
-// (the caller's FP32 tensors need no more than their type's alignment)
-__device__ __forceinline__ bool whole16(const float* g) { return (reinterpret_cast<uintptr_t>(g) & 15u) == 0; }
+// `vec`: sixteen bytes at a time; the caller's FP32 tensors need no more than their type's alignment.  The backward has two forms: W
+// for matrices that all lie whole on sixteen bytes, rows of (m x m) ones included, which is the usual case and has no other way
+// in its code; else (m x m) matrices go four bytes at a time and (m x head_dim) ones by their addresses.  With a look at each address
+// in one form it took 1 to 4 % longer than with none, in two forms it takes 0 to 5 % less (us, pseudoinverse alone, J = 6, none /
+// look / two forms: m = 32, 4 slices 41.0 / 41.0 / 39.0; m = 64, 32 slices 49.2 / 51.0 / 49.2, 512 slices 203 / 210 / 197).  The forward in two
+// forms took longer (m = 64, 32 slices 31.0 / 30.8 / 32.8): it asks Ctx.
+template <class... P>
+__host__ __device__ __forceinline__ bool whole16(const P*... g) { return ((reinterpret_cast<uintptr_t>(g) | ...) & 15u) == 0; }
 // Whole-matrix tile loads: thread t handles row t >> 2 and the 8-column chunks (t & 3) and (t & 3) + 4, so that four
 // adjacent lanes cover 128 consecutive bytes.
-__device__ __forceinline__ void load_chunk8(const float* g, int r, int chunk, int rows, int cols, int ld, float* v) {
+__device__ __forceinline__ void load_chunk8(const float* g, int r, int chunk, int rows, int cols, int ld, bool vec, float* v) {
   const int c0 = 8 * chunk;
-  if (((ld | cols) & 3) == 0 && whole16(g)) {
+  if (vec) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -204,9 +211,9 @@ __device__ __forceinline__ void load_chunk8(const float* g, int r, int chunk, in
   }
 }
 // dense global [rows x cols] matrix with row stride ld -> registers, zero beyond rows / cols
-__device__ __forceinline__ void load_tile16(const float* g, int rows, int cols, int ld, float* v) {
-  load_chunk8(g, threadIdx.x >> 2, threadIdx.x & 3, rows, cols, ld, v);
-  load_chunk8(g, threadIdx.x >> 2, (threadIdx.x & 3) + 4, rows, cols, ld, v + 8);
+__device__ __forceinline__ void load_tile16(const float* g, int rows, int cols, int ld, bool vec, float* v) {
+  load_chunk8(g, threadIdx.x >> 2, threadIdx.x & 3, rows, cols, ld, vec, v);
+  load_chunk8(g, threadIdx.x >> 2, (threadIdx.x & 3) + 4, rows, cols, ld, vec, v + 8);
 }
 __device__ __forceinline__ void put_tile16(uint32_t set, const float* v) {
   split_store8(set, threadIdx.x >> 2, threadIdx.x & 3, v);
@@ -220,13 +227,13 @@ __device__ __forceinline__ void stage_tile16(float* X, const float* v) {
     *reinterpret_cast<float4*>(d + (q & 1) * 4 + (q >> 1) * 32) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
 // this thread's 16 columns of its row: global, staging
-__device__ __forceinline__ void load_row16(const Ctx& c, const float* g, int rows, int cols, int ld, float* v) {
-  load_chunk8(g, c.row, c.col0 >> 3, rows, cols, ld, v);
-  load_chunk8(g, c.row, (c.col0 >> 3) + 1, rows, cols, ld, v + 8);
+__device__ __forceinline__ void load_row16(const Ctx& c, const float* g, int rows, int cols, int ld, bool vec, float* v) {
+  load_chunk8(g, c.row, c.col0 >> 3, rows, cols, ld, vec, v);
+  load_chunk8(g, c.row, (c.col0 >> 3) + 1, rows, cols, ld, vec, v + 8);
 }
-__device__ __forceinline__ void store_row16(const Ctx& c, float* g, const float* v, int rows, int cols, int ld) {
+__device__ __forceinline__ void store_row16(const Ctx& c, float* g, const float* v, int rows, int cols, int ld, bool vec) {
   if (c.row >= rows) return;
-  if (((ld | cols) & 3) == 0 && whole16(g)) {
+  if (vec) {
 #pragma unroll
     for (int i = 0; i < 16; i += 4)
       if (c.col0 + i < cols)
@@ -256,8 +263,8 @@ __device__ __forceinline__ void unstage_col16(const Ctx& c, const float* X, floa
 }
 // A staged matrix -> the leading rows x cols block of a dense global matrix, whole sectors per instruction.  (From the
 // accumulator layout, 32 rows of 16 bytes per instruction, the store of an iterate kept the warps for 1700 cycles, this takes 400.)
-__device__ __forceinline__ void store_staged(const float* X, float* g, int rows, int cols, int ld) {
-  if (((ld | cols) & 3) == 0 && whole16(g)) {
+__device__ __forceinline__ void store_staged(const float* X, float* g, int rows, int cols, int ld, bool vec) {
+  if (vec) {
     const int r = threadIdx.x >> 2;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -533,8 +540,8 @@ __device__ __forceinline__ void fwd_landmarks(Ctx& c, const ns::NsFwdParams& p, 
 #pragma unroll 1
   for (int h = 0; h < (D > kN ? 2 : 1); ++h) {
     const int cols = min(D, kN);
-    load_tile16(p.qt + bh * m * D + h * kN, m, cols, D, q);
-    load_tile16(p.kt + bh * m * D + h * kN, m, cols, D, k);
+    load_tile16(p.qt + bh * m * D + h * kN, m, cols, D, c.md16, q);
+    load_tile16(p.kt + bh * m * D + h * kN, m, cols, D, c.md16, k);
     put_tile16(c.slot(2 * h), q);
     put_tile16(c.slot(2 * h + 1), k);
   }
@@ -552,7 +559,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
 #pragma unroll
   for (int i = 0; i < 16; ++i) { r[i] = 0.f; v[i] = 0.f; }       // (inactive warps keep zeros)
   if (f.k2_given) {
-    load_tile16(k2, m, m, m, v);
+    load_tile16(k2, m, m, m, c.mm16, v);
     stage_tile16(X, v);
     ns::ns_sync();
   } else {
@@ -579,7 +586,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
       }
       arrive_ready(c, 0);
       // to global memory beside the product: K2 first, Z0 (staged over it) below
-      if (!f.k2_given && !c.failed && (s == -1 || !ridge)) store_staged(X, k2, m, m, m);
+      if (!f.k2_given && !c.failed && (s == -1 || !ridge)) store_staged(X, k2, m, m, m, c.mm16);
       if (s == 0) {
         ns::ns_sync();
         stage_row16(c, X, z);
@@ -588,7 +595,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
     if (s >= 0 && s < 4 * J) {
       // one iteration; R, then Y and W, then Z'.  Z_j is staged in X (slot 3, free until Y) and leaves while the product runs.
       ns::ns_sync();
-      if (!c.failed) store_staged(X, iterates + (size_t)(s >> 2) * mm_, m, m, m);
+      if (!c.failed) store_staged(X, iterates + (size_t)(s >> 2) * mm_, m, m, m, c.mm16);
       take(c, 0, 0, c.slot(2), c.act, v, c.trunc);
       if (c.act) {
 #pragma unroll
@@ -609,7 +616,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
       arrive_ready(c, 0);
       s += 3;
       const bool end = s == 4 * J - 1;
-      if (ridge && end) load_row16(c, k2, m, m, m, r);      // (R is dead; K2 is the last product's operand)
+      if (ridge && end) load_row16(c, k2, m, m, m, c.mm16, r);      // (R is dead; K2 is the last product's operand)
       take(c, 1, kAccCols, c.slot(1), c.act, v, c.trunc);
       if (c.act) {
 #pragma unroll
@@ -622,8 +629,8 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
       if (end) {
         ns::ns_sync();
         if (!c.failed) {
-          store_staged(X, iterates + (size_t)J * mm_, m, m, m);
-          if (!ridge) store_staged(X, p.k2inv + bh * mm_, m, m, m);
+          store_staged(X, iterates + (size_t)J * mm_, m, m, m, c.mm16);
+          if (!ridge) store_staged(X, p.k2inv + bh * mm_, m, m, m, c.mm16);
         }
       }
       continue;
@@ -634,7 +641,7 @@ __device__ __forceinline__ void fwd_compute(Ctx& c, float* red, const FwdParams&
       ns::ns_sync();
       stage_row16(c, X, v);
       ns::ns_sync();
-      if (!c.failed) store_staged(X, p.k2inv + bh * mm_, m, m, m);
+      if (!c.failed) store_staged(X, p.k2inv + bh * mm_, m, m, m, c.mm16);
       break;
     }
     if (!c.act) {
@@ -657,6 +664,8 @@ __global__ void __launch_bounds__(kNsTcThreads, 2) ns_fwd_tc_kernel(FwdParams f,
   __shared__ Shared sh;
   Ctx c;
   ctx_open(c, sh, dyn_smem, status, kFwdTmemCols, f.p.m);
+  c.md16 = whole16(f.p.qt, f.p.kt);
+  c.mm16 = (f.p.m & 3) == 0 && whole16(f.p.k2, f.p.iterates, f.p.k2inv);
   if (is_compute()) fwd_compute(c, red, f, blockIdx.x);
   else fwd_issue(c, f);
   ctx_close(c, kFwdTmemCols);
@@ -806,6 +815,7 @@ __device__ inline void bwd_issue(Ctx& c, const BwdParams& f, int finish) {
 }
 
 // compute warps.  finish: batches of 64 columns of the landmark gradients; 0: stop at dL/dK2, -1: after the iterations.
+template <bool W>
 __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams& f, int64_t bh, int finish) {
   const ns::NsBwdParams& p = f.p;
   const BwdHeadParams& h = f.h;
@@ -818,12 +828,12 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
   float lam = 0.f;
   Norms nrm;
   // ---- operands ----
-  load_tile16(iterates + (size_t)(J - 1) * mm_, m, m, m, z);
-  load_tile16(p.k2 + bh * mm_, m, m, m, r);
-  if (ridge) load_tile16(iterates + (size_t)J * mm_, m, m, m, hd);
+  load_tile16(iterates + (size_t)(J - 1) * mm_, m, m, m, W, z);
+  load_tile16(p.k2 + bh * mm_, m, m, m, W, r);
+  if (ridge) load_tile16(iterates + (size_t)J * mm_, m, m, m, W, hd);
 #pragma unroll
   for (int i = 0; i < 16; ++i) { g[i] = 0.f; da_keep[i] = 0.f; da_send[i] = 0.f; }
-  if (!head) load_row16(c, p.G + bh * mm_, m, m, m, g);
+  if (!head) load_row16(c, p.G + bh * mm_, m, m, m, W, g);
   put_tile16(c.slot(1), z);
   put_tile16(c.slot(ridge ? 4 : 0), r);
   if (ridge) put_tile16(c.slot(2), hd);
@@ -835,7 +845,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
 #pragma unroll
     for (int i = 0; i < 16; ++i) g[i] = 0.f;       // dL/dZ_J = G K2 is added to it
   }
-  if (J > 1) load_tile16(iterates + (size_t)(J - 2) * mm_, m, m, m, z);
+  if (J > 1) load_tile16(iterates + (size_t)(J - 2) * mm_, m, m, m, W, z);
   if (head) {
     // reduce the partials of the first row pass: dstep2 -> slot 8, dkt_a -> global
     float ds[16], dk[16];
@@ -860,8 +870,8 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         *reinterpret_cast<float4*>(out + (q & 1) * 4 + (q >> 1) * 32) = make_float4(dk[4 * q], dk[4 * q + 1], dk[4 * q + 2], dk[4 * q + 3]);
     }
     put_tile16(c.slot(8), ds);
-    load_tile16(h.k2inv + bh * mm_, m, m, m, v);
-    load_tile16(h.bmat + bh * md, m, kN, kN, ds);
+    load_tile16(h.k2inv + bh * mm_, m, m, m, W, v);
+    load_tile16(h.bmat + bh * md, m, kN, kN, W || c.md16, ds);
     put_tile16(c.slot(7), v);
     put_tile16(c.slot(6), ds);
     arrive_ready(c, 0);
@@ -877,7 +887,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
 #pragma unroll 1
     for (;;) {
       // global operands of this step or of the batch after it, ahead of the wait
-      if (step == kHeadO3 && h.D3) load_row16(c, p.qt + bh * md, m, kN, kN, hd);
+      if (step == kHeadO3 && h.D3) load_row16(c, p.qt + bh * md, m, kN, kN, W || c.md16, hd);
       if (step == kDQ) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {                    // dkt_a, as store_staged walks a matrix
@@ -887,8 +897,8 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           z[4 * q] = x.x; z[4 * q + 1] = x.y; z[4 * q + 2] = x.z; z[4 * q + 3] = x.w;
         }
         if (half + 1 < finish) {
-          load_tile16(p.kt + bh * md + (half + 1) * kN, m, min(D, kN), D, hd);
-          load_tile16(p.qt + bh * md + (half + 1) * kN, m, min(D, kN), D, r);
+          load_tile16(p.kt + bh * md + (half + 1) * kN, m, min(D, kN), D, W || c.md16, hd);
+          load_tile16(p.qt + bh * md + (half + 1) * kN, m, min(D, kN), D, W || c.md16, r);
         }
       }
       // slot that the result goes to (or a free one to add the lane halves in), accumulator, done barrier
@@ -987,13 +997,13 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           next = kRidgeK2;
           break;
         case kRidgeK2:
-          if (act && !c.failed) store_row16(c, p.spill + bh * mm_, v, m, m, m);
+          if (act && !c.failed) store_row16(c, p.spill + bh * mm_, v, m, m, m, W);
           break;
         case kSumDA: {
           if (f.step_dz) {
             if (!c.failed) {
-              store_row16(c, f.step_dz + bh * mm_, g, m, m, m);
-              store_row16(c, f.step_da + bh * mm_, v, m, m, m);
+              store_row16(c, f.step_dz + bh * mm_, g, m, m, m, W);
+              store_row16(c, f.step_da + bh * mm_, v, m, m, m, W);
             }
             break;
           }
@@ -1031,7 +1041,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
           if (ridge) {
             // dL/dK2 = (what kRidgeK2 left) + K2 (dA + dA^T)
             put_row16(c, c.slot(5), v);
-            load_row16(c, p.k2 + bh * mm_, m, m, m, g);
+            load_row16(c, p.k2 + bh * mm_, m, m, m, W, g);
             put_row16(c, c.slot(6), g);
             arrive = 0;
             next = kTailK2;
@@ -1042,7 +1052,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         }
         case kTailK2: {
           float e[16];
-          load_row16(c, p.spill + bh * mm_, m, m, m, e);
+          load_row16(c, p.spill + bh * mm_, m, m, m, W, e);
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = (c.row < m && c.col0 + i < m) ? v[i] + e[i] : 0.f;
           jacobian = true;
@@ -1051,7 +1061,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         case kDQ:
           stage_row16(c, c.stage(1), v);
           ns::ns_sync();
-          if (!c.failed) store_staged(c.stage(1), p.dqt_ns + bh * md + half * kN, m, min(D, kN), D);
+          if (!c.failed) store_staged(c.stage(1), p.dqt_ns + bh * md + half * kN, m, min(D, kN), D, W || c.md16);
           next = kDK;
           break;
         default: {                                       // kDK
@@ -1075,7 +1085,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         }
       }
       if (jacobian && f.dK2) {
-        if (!c.failed) store_row16(c, f.dK2 + bh * mm_, v, m, m, m);
+        if (!c.failed) store_row16(c, f.dK2 + bh * mm_, v, m, m, m, W);
         jacobian = false;
       } else if (jacobian) {
         // softmax-2: dS2 = K2 o (dK2 - rowsum(dK2 o K2)); g holds K2
@@ -1110,7 +1120,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         if (prime) {
           put_tile16(c.slot(2 - par), z);                // Z_{j-1}: every product that read this slot is complete
           arrive_ready(c, 2);
-          if (j > 1) load_tile16(iterates + (size_t)(j - 2) * mm_, m, m, m, z);
+          if (j > 1) load_tile16(iterates + (size_t)(j - 2) * mm_, m, m, m, W, z);
         }
         take(c, 0, 3 * kAccCols, c.slot(7), c.act, v, c.trunc);   // dY
         if (c.act) put_row16(c, c.slot(7), v);
@@ -1142,8 +1152,8 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
         }
         arrive_ready(c, 6);
         if (!prime && finish > 0) {                      // the first operands of the landmark gradients, ahead of time
-          load_tile16(p.kt + bh * md, m, min(D, kN), D, hd);
-          load_tile16(p.qt + bh * md, m, min(D, kN), D, r);
+          load_tile16(p.kt + bh * md, m, min(D, kN), D, W || c.md16, hd);
+          load_tile16(p.qt + bh * md, m, min(D, kN), D, W || c.md16, r);
         }
       }
       if (prime) {
@@ -1183,6 +1193,7 @@ __device__ __forceinline__ void bwd_compute(Ctx& c, float* red, const BwdParams&
   }
 }
 
+template <bool W>
 __global__ void __launch_bounds__(kNsTcThreads, 1) ns_bwd_tc_kernel(BwdParams f, int finish, int* status) {
   extern __shared__ uint8_t dyn_smem[];
   __shared__ float red[ns::kRedFloats];
@@ -1190,10 +1201,18 @@ __global__ void __launch_bounds__(kNsTcThreads, 1) ns_bwd_tc_kernel(BwdParams f,
   Ctx c;
   pdl_trigger();
   ctx_open(c, sh, dyn_smem, status, kBwdTmemCols, f.p.m);
+  c.md16 = whole16(f.p.qt, f.p.kt, f.h.bmat);
   pdl_wait();
-  if (is_compute()) bwd_compute(c, red, f, blockIdx.x, finish);
+  if (is_compute()) bwd_compute<W>(c, red, f, blockIdx.x, finish);
   else bwd_issue(c, f, finish);
   ctx_close(c, kBwdTmemCols);
+}
+
+// the form for a call
+inline auto bwd_kernel(const BwdParams& f) {
+  const ns::NsBwdParams& p = f.p;
+  return (p.m & 3) == 0 && whole16(p.qt, p.kt, p.k2, p.iterates, p.G, p.spill, f.h.k2inv, f.h.bmat, f.dK2, f.step_dz, f.step_da)
+             ? ns_bwd_tc_kernel<true> : ns_bwd_tc_kernel<false>;
 }
 
 }  // namespace nstc
