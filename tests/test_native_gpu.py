@@ -110,24 +110,36 @@ def test_transforms_and_tracing_go_to_the_autograd_functions(cuda_device):
 
 
 def test_backward_on_the_stream_of_the_forward(cuda_device):
-    """Forward and backward on a side stream, many times over, with the caller's stream busy: allocations and launches
-    belong to the side stream."""
+    """Forward and backward on a side stream while the caller's stream is busy: copies of the results that the side stream takes at once
+    are right, and the side stream is through before the caller's, so that nothing was launched on that one."""
     from flashnystrom_b200 import flash_nystrom_attention
-    q, k, v, dO = _inputs(1, 4, 2048, 64, torch.bfloat16, False)
+    host = [t.cpu().pin_memory() for t in _inputs(1, 4, 2048, 64, torch.bfloat16, False)]
+    taps = torch.randn(4, 3, dtype=torch.bfloat16).pin_memory()
 
     def step():
-        x = [t.detach().requires_grad_(True) for t in (q, k, v)]
-        out = flash_nystrom_attention(*x, num_landmarks=64)
+        q, k, v, dO = (t.to(cuda_device, non_blocking=True) for t in host)
+        w = taps.to(cuda_device, non_blocking=True)
+        x = [t.requires_grad_(True) for t in (q, k, v, w)]
+        out = flash_nystrom_attention(q, k, v, num_landmarks=64, conv_weight=w, conv_kernel_size=3)
         out.backward(dO)
-        return [out.detach()] + [t.grad for t in x]
+        return [t.clone() for t in [out.detach()] + [t.grad for t in x]]
     want = step()
-    side = torch.cuda.Stream()
-    side.wait_stream(torch.cuda.current_stream())
+    caller, side = torch.cuda.current_stream(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        held = [step() for _ in range(8)]             # (the side stream's memory, so that nothing is allocated below)
+        del held
+    torch.cuda.synchronize()
+    torch.cuda._sleep(400_000_000)                    # about 0.2 s of one thread
+    busy, done = torch.cuda.Event(), torch.cuda.Event()
+    busy.record(caller)
     with torch.cuda.stream(side):
         got = [step() for _ in range(8)]
-    torch.cuda.current_stream().wait_stream(side)
+        done.record(side)
+    done.synchronize()
+    assert not busy.query()
     for g in got:
         assert all(torch.equal(a, b) for a, b in zip(g, want))
+    caller.synchronize()
 
 
 def test_debug_statistics_are_printed(cuda_device, monkeypatch, capfd):

@@ -74,8 +74,9 @@ def test_pinv_few_iterations(cuda_device, m, J, kappa):
 @pytest.mark.parametrize("kappa", [0.0, 5.0])
 def test_tensor_core_pinv_no_less_precise_than_cuda_cores(cuda_device, m, D, kappa):
     """Edges of the 16-wide K steps and of the 32 x 32 blocks, the three head_dim forms of the scores and of the landmark
-    gradients.  Both kernels against the oracle in float64 on the same landmarks and incoming gradients; the bound is twice
-    the CUDA cores' own error (three bf16 terms hold an FP32 value, accumulation has FP32's rounding) plus one FP32 ulp."""
+    gradients.  Both kernels against the oracle in float64 on the same landmarks and incoming gradients; the bound is the CUDA
+    cores' own error plus the rounding of an FP32 result, half a unit in the last place (measured: K2inv 0.50 times the CUDA cores'
+    error in the mean and 0.91 at most, dQ 0.56 and 0.92, dK 0.57 and 0.94; K2, whose error is that rounding, 1.08 and 1.30)."""
     from flashnystrom_b200 import _C
     q, k, v, dO = (t.cuda() for t in O.make_inputs(1, 3, 4 * m + 5, D, seed=m + D, dtype=torch.float32))
     err = {}
@@ -94,7 +95,7 @@ def test_tensor_core_pinv_no_less_precise_than_cuda_cores(cuda_device, m, D, kap
         got = {"K2": r[11], "k2inv": r[5], "dq": g[0], "dk": g[1]}
         err[generic] = {n: float((t.double() - f[n]).norm() / f[n].norm()) for n, t in got.items()}
     for n in err[True]:
-        assert err[False][n] <= 2 * err[True][n] + 2.0 ** -23, (n, err)
+        assert err[False][n] <= err[True][n] + 2.0 ** -24, (n, err)
 
 
 def test_pinv_same_call_twice_is_bit_identical(cuda_device):
