@@ -9,9 +9,9 @@ graph).
         -> (dq, dk, dv)
 
 Both have fake (meta) implementations, and nystrom_fwd has its autograd formula registered, so the
-operators work under FakeTensorMode, AOT autograd and opcheck.  The eager path of the package keeps
-using the plain autograd.Function (less dispatcher overhead per call); `flash_nystrom_attention`
-switches to the operators while a compiler is tracing."""
+operators work under FakeTensorMode, AOT autograd and opcheck.  Eager calls go through the C++ module
+(csrc/native.cpp) and, where that hands them back, through the autograd functions of flash_nystrom.py (less dispatcher
+overhead per call); `flash_nystrom_attention` switches to the operators while a compiler is tracing."""
 from typing import Tuple
 
 import torch

@@ -26,8 +26,8 @@
 // reads 24 KB) and between them the way of a result through registers, split and shared memory (2500 cycles, three times);
 // backward, the same with what a phase waits for: copies out of L2 (9 KB per K step), the result block out to it (put 1600,
 // publish 2300), the peer, the first chunk in (1550).  Measured at B=2, H=8, m=128 (us): forward D=128, J=8 with
-// ridge 222 with four products in a row, 205 in residual form through L2, 123 with the operands on the chip; D=64, J=6 without
-// 164, 152, 95; backward 447 / 408 and 318 / 289.
+// ridge 222 with four products in a row, 205 in residual form through L2, 136 with the operands on the chip (121 of it behind the
+// softmax); D=64, J=6 without 164, 152, 100; backward 447 / 406 and 318 / 287.
 #pragma once
 #include "common.cuh"
 #include "small_kernels.cuh"

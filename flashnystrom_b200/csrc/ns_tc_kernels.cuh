@@ -4,8 +4,8 @@
 // R = I - M the polynomial is 4 (I + R (I + R / 2)^2), so
 //     R = I - A Z,   Y = Z R,   W = I + R + R^2 / 4,   Z' = Z + Y W.
 // That is four products as before, but three dependent steps in place of four (Y and W go side by side), and
-// nothing cancels near convergence: the error of K2inv against 64 bits is 0.5 to 0.8 of the nested form's.  The
-// backward is that of this form (below); gradients do not depend on which form is differentiated.
+// nothing cancels near convergence: the error of K2inv against 64 bits is 0.57 to 1.04 times the nested form's,
+// 0.79 in the mean (16 to 128 landmarks, J = 4 to 8, three ridges).  The backward is that of this form (below); gradients do not depend on which form is differentiated.
 //
 // Products.  Every 64 x 64 FP32 matrix is kept in shared memory as three bf16 tiles x = x0 + x1 + x2 (each term the
 // bf16 rounding of what the previous terms left over: 24 significant bits together, the FP32 exponent range), stored in
@@ -35,8 +35,8 @@
 // stored about 1000), three of them per iteration in the forward; in the backward, where eight products run beside the
 // chain, shared-memory bandwidth (an MMA reads 8 KB per 65 cycles, an epilogue moves 56 KB).  Instructions come from a cold
 // cache the first time round: 5 us of the forward, 15 of the backward.  Measured (us, nested form with one accumulator per
-// partial product / this, J = 6): 32 slices, m = 64 forward 45 / 41, backward 76 / 66; m = 32 43 / 33 and 66 / 48;
-// 512 slices 162 / 109 and 310 / 287; 64 slices of head_dim 128 with the ridge (then on the CUDA cores) 74 / 50 and 121 / 90.
+// partial product / this, J = 6): 32 slices, m = 64 forward 45 / 43, backward 76 / 66; m = 32 43 / 33 and 66 / 48;
+// 512 slices 162 / 107 and 310 / 275; 64 slices of head_dim 128 with the ridge (then on the CUDA cores) 74 / 50 and 121 / 86.
 #pragma once
 #include "ns_kernels.cuh"
 #include "small_kernels.cuh"
@@ -353,8 +353,8 @@ __device__ __forceinline__ void wait_done(Ctx& c, int b, int where) {
 
 // The tensor core truncates when it adds to an accumulator; the leading partial product is added to once per K step and
 // loses about an eighth of an ulp each time on the average, which `trunc` (a share of the value) gives back on its way to the
-// small ones.  Without it K2inv and dQ of fp32 calls were up to 1.28 and 1.24 times as far from the oracle as with one add fewer
-// per product, with it 0.83 to 0.98 and 0.90 to 0.99 times.
+// small ones.  Without it K2inv and dQ of fp32 calls were up to 1.28 and 1.24 times as far from the oracle as with an accumulator
+// of its own for x1 y1 (one addition fewer per product), with it 0.83 to 0.98 and 0.90 to 0.99 times.
 // A product that is added to one before adds its small terms onto the large value as well: two products in an accumulator are three
 // times as many truncating additions as one, three five times.  (With one product's share for all, dL/dK2 was 1.6 to 2.2 times as far
 // from 64 bits as FP32 sums are, with theirs 1.2 to 1.3 times; mean over 16 to 64 landmarks, J = 4 to 8.)
@@ -416,7 +416,7 @@ __device__ __forceinline__ void take(Ctx& c, int b, uint32_t col, uint32_t set, 
 //   4J        k2inv = Z K2^T (ridge only)                                     K2 in slot 0
 // Even s: accumulator 0, odd s: accumulator 1.  Y is formed before W: Z is in registers too, so its slot
 // stays free, and W goes over R.  FP32 staging of K2, then A: slot 3.
-// Two slices per SM (97 KB, 256 TMEM columns, 112 registers): the epilogues of one run beside the products of the other.
+// Two slices per SM (97 KB, 256 TMEM columns, 96 registers): the epilogues of one run beside the products of the other.
 constexpr int kFwdStage = 3;
 struct FwdParams {
   ns::NsFwdParams p;
